@@ -3,6 +3,8 @@
 // the reference's calling convention -- host pointers, caller-owned cache, void return -- and
 // runs every stage on the GPU. Device mirrors of the weights and of the latent cache are kept
 // in a process-wide registry, created on first sight.
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdlib>
@@ -15,6 +17,8 @@
 #include <cuda_fp16.h>
 
 #include "cwk_common.cuh"
+#include "host_pool.cuh"
+#include "lin_split_tc.cuh"
 
 int cwk_mla_decode_rows(cwk_ctx *ctx, const void *q, const void *cache, int64_t ld, int rows, int nh, int L, int R,
                         float scale, void *out);
@@ -179,102 +183,6 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const void *Wv, const fl
     }
 }
 
-// A chunk of tokens: four rows x four tokens per warp, so that a lane's 16 bytes of a weight row meet four tokens' activations
-// and a token's activations meet four rows -- the one-token form, run per token, reads every activation from L1 once per row
-// and is bound by that. A warp covers the whole width of its rows (lane l takes pieces l, l + 32, ...), eight warps = 32 rows
-// per block, blockIdx.y = group of four tokens; f32 accumulate, the lanes' sums by shuffles.
-template <int KIND>
-__device__ __forceinline__ void unpack16(const uint4 &v, float *o) {      // 8 bf16, 4 f32 or 16 e4m3 (those 256 times too small)
-    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-    if (KIND == GEMV_BF16) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) { o[2 * q] = __uint_as_float(u[q] << 16); o[2 * q + 1] = __uint_as_float(u[q] & 0xffff0000u); }
-    } else if (KIND == GEMV_F32) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) o[q] = __uint_as_float(u[q]);
-    } else {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t mag = u[q] & 0x7f7f7f7fu, sg = u[q] & 0x80808080u;
-            if (__vcmpeq4(mag, 0x7f7f7f7fu)) {             // a NaN code in the word: code by code
-#pragma unroll
-                for (int e = 0; e < 4; e++) o[4 * q + e] = e4m3_val((u[q] >> (8 * e)) & 0xffu) * 0.00390625f;
-            } else {
-                const uint32_t h01 = ((mag & 0x7fu) << 7) | ((mag & 0x7f00u) << 15) | ((sg & 0x80u) << 8) | ((sg & 0x8000u) << 16);
-                const uint32_t h23 = ((mag >> 9) & 0x3f80u) | ((mag >> 1) & 0x3f800000u) | ((sg >> 8) & 0x8000u) | (sg & 0x80000000u);
-                const float2 f01 = __half22float2(*reinterpret_cast<const __half2 *>(&h01));
-                const float2 f23 = __half22float2(*reinterpret_cast<const __half2 *>(&h23));
-                o[4 * q] = f01.x; o[4 * q + 1] = f01.y; o[4 * q + 2] = f23.x; o[4 * q + 3] = f23.y;
-            }
-        }
-    }
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(256) gemm_rows_kernel(const void *Wv, const float *scales, const float *x, float *y, int rows, int k,
-                                                        int64_t ldx, int64_t ldy, int ntok) {
-    constexpr int E = KIND == GEMV_BF16 ? 8 : KIND == GEMV_F32 ? 4 : 16, EB = 16 / E, R = 4, TOK = 4;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = (blockIdx.x * 8 + warp) * R, t0 = blockIdx.y * TOK;
-    if (r0 >= rows) return;
-    const float *xt[TOK];
-#pragma unroll
-    for (int t = 0; t < TOK; t++) xt[t] = x + (int64_t)min(t0 + t, ntok - 1) * ldx;
-    const uint8_t *w[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) w[r] = reinterpret_cast<const uint8_t *>(Wv) + (int64_t)min(r0 + r, rows - 1) * k * EB;
-    const int nkb = (k + 127) / 128;
-    float acc[R][TOK];
-#pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-        for (int t = 0; t < TOK; t++) acc[r][t] = 0.f;
-    // (loads of the next step issued ahead of this step's arithmetic were measured: the registers they hold cost more
-    // in resident warps than the overlap gives -- 2.37 against 1.67 ms for the widest projection of a 512-token chunk)
-    for (int j = lane * E; j + E <= k; j += 32 * E) {
-        uint4 wv[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) wv[r] = ld_weight16(w[r] + (int64_t)j * EB);
-        float xv[TOK][E];
-#pragma unroll
-        for (int t = 0; t < TOK; t++)
-#pragma unroll
-            for (int q = 0; q < E / 4; q++) {
-                const float4 f = *reinterpret_cast<const float4 *>(xt[t] + j + 4 * q);
-                xv[t][4 * q] = f.x; xv[t][4 * q + 1] = f.y; xv[t][4 * q + 2] = f.z; xv[t][4 * q + 3] = f.w;
-            }
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            float o[E];
-            unpack16<KIND>(wv[r], o);
-            float m = 1.f;
-            if (KIND == GEMV_FP8) m = scales[(int64_t)(min(r0 + r, rows - 1) / 128) * nkb + (j >> 7)] * 256.0f;
-#pragma unroll
-            for (int t = 0; t < TOK; t++) {
-                float d = 0.f;
-#pragma unroll
-                for (int e = 0; e < E; e++) d += o[e] * xv[t][e];
-                acc[r][t] += KIND == GEMV_FP8 ? d * m : d;
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-        for (int t = 0; t < TOK; t++) {
-            float a = acc[r][t];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (lane == 0 && r0 + r < rows && t0 + t < ntok) y[(int64_t)(t0 + t) * ldy + r0 + r] = a;
-        }
-}
-
-// Whether gemm_rows_kernel takes the operands: whole 16-byte pieces, aligned rows.
-bool gemm_rows_ok(const void *W, const float *x, int64_t k, int64_t ldx, int kind) {
-    const int E = kind == GEMV_BF16 ? 8 : kind == GEMV_F32 ? 4 : 16;
-    return k % (32 * E) == 0 && (ldx & 3) == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
-}
-
 // y[t][0..rows) = W . x[t] for n tokens. kind: GEMV_BF16 / GEMV_F32 / GEMV_FP8. W2 != NULL: also y2 = W2 . x[t] (same kind,
 // same k) in the same launch.
 template <int TOK>
@@ -296,14 +204,6 @@ void launch_gemv_tok(cwk_ctx *ctx, int kind, const void *W, const float *scales,
 void launch_gemv(cwk_ctx *ctx, int kind, const void *W, const float *scales, const float *x, float *y, int64_t rows, int64_t k, int n,
                  int64_t ldx, int64_t ldy, const void *W2 = nullptr, const float *scales2 = nullptr, float *y2 = nullptr, int64_t rows2 = 0,
                  int64_t ldy2 = 0) {
-    if (n >= 4 && !W2 && gemm_rows_ok(W, x, k, ldx, kind)) {
-        const dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((n + 3) / 4));
-        if (kind == GEMV_BF16) gemm_rows_kernel<GEMV_BF16><<<grid, 256, 0, ctx->stream>>>(W, scales, x, y, (int)rows, (int)k, ldx, ldy, n);
-        else if (kind == GEMV_F32) gemm_rows_kernel<GEMV_F32><<<grid, 256, 0, ctx->stream>>>(W, scales, x, y, (int)rows, (int)k, ldx, ldy, n);
-        else gemm_rows_kernel<GEMV_FP8><<<grid, 256, 0, ctx->stream>>>(W, scales, x, y, (int)rows, (int)k, ldx, ldy, n);
-        ctx->launches++;
-        return;
-    }
     if (n >= 4) launch_gemv_tok<4>(ctx, kind, W, scales, x, y, rows, k, n, ldx, ldy, W2, scales2, y2, rows2, ldy2);
     else launch_gemv_tok<1>(ctx, kind, W, scales, x, y, rows, k, n, ldx, ldy, W2, scales2, y2, rows2, ldy2);
 }
@@ -372,6 +272,42 @@ __global__ void __launch_bounds__(256) rms_scale_pair_kernel(float *xa, int na, 
                                                              float eps, uint16_t *row_out, void *host_row, int host_bf16) {
     if (blockIdx.x == 0) rms_scale_row(xa, na, wa, eps, nullptr, nullptr, 0);
     else rms_scale_row(xb, nb, wb, eps, row_out, host_row, host_bf16);
+}
+
+// The two norms of a chunk on the tensor path, one block per (token, row): adds up the split partial sums of the joint
+// q_a | kv_a projection (part [splits][n][na + nb]), then the q_a row leaves as three bf16 planes (the next projection's
+// operand), the kv_a row as the narrowed cache row and, where the caller's cache is f32, as f32. The sum of squares runs in
+// the order of rms_scale_row.
+__global__ void __launch_bounds__(256) norm_chunk_kernel(const float *part, int splits, int n, int na, int nb, const uint16_t *wa, const uint16_t *wb,
+                                                         float eps, uint16_t *planes, uint16_t *cache_rows, float *kv_out) {
+    extern __shared__ __align__(16) float s_row[];
+    const int t = blockIdx.x, len = blockIdx.y ? nb : na, ld = na + nb;
+    const float *src = part + (int64_t)t * ld + (blockIdx.y ? na : 0);
+    for (int i = threadIdx.x * 4; i < len; i += 1024) {    // (na and nb are multiples of 8)
+        float4 v = *reinterpret_cast<const float4 *>(src + i);
+#pragma unroll 8
+        for (int s = 1; s < splits; s++) {
+            const float4 w = *reinterpret_cast<const float4 *>(src + (int64_t)s * n * ld + i);
+            v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+        }
+        *reinterpret_cast<float4 *>(s_row + i) = v;
+    }
+    __syncthreads();
+    if (blockIdx.y) {
+        rms_scale_row(s_row, nb, wb, eps, cache_rows + (int64_t)t * nb, kv_out ? kv_out + (int64_t)t * nb : nullptr, 0);
+        return;
+    }
+    rms_scale_row(s_row, na, wa, eps, nullptr, nullptr, 0);
+    for (int i = threadIdx.x; i < na; i += 256) {          // (the values this thread scaled itself)
+        const float v = s_row[i];
+        const __nv_bfloat16 h = __float2bfloat16_rn(v);
+        const float r = v - __bfloat162float(h);
+        const __nv_bfloat16 m = __float2bfloat16_rn(r);
+        uint16_t *o = planes + (int64_t)t * na + i;
+        o[0] = __bfloat16_as_ushort(h);
+        o[(int64_t)n * na] = __bfloat16_as_ushort(m);
+        o[2 * (int64_t)n * na] = __bfloat16_as_ushort(__float2bfloat16_rn(r - __bfloat162float(m)));
+    }
 }
 
 // q_abs[t][h][c] = sum_r q[t][h][r] * W_k[h][r][c] (src/attention.c:741-744), W_k = rows [h*kv_dim, +nope) of
@@ -512,64 +448,6 @@ __global__ void __launch_bounds__(256) unabsorb_kernel(const uint16_t *cacc, con
     if (lane == 0) attn[idx] = acc;
 }
 
-// The same for a chunk of tokens: four value rows x four tokens per warp (a lane's 16 bytes of a W_v row meet four tokens'
-// accumulators and the other way round), eight warps = 32 rows per block; grid (vdim / 32, groups of four tokens, heads).
-// kv_lora a multiple of 256, vdim a multiple of 4, 16-byte aligned operands.
-__global__ void __launch_bounds__(256) unabsorb_rows_kernel(const uint16_t *cacc, const uint16_t *kvb, int nh, int nope, int vdim,
-                                                            int kv_lora, float *attn, int ntok) {
-    constexpr int R = 4, TOK = 4;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.z, r0 = (blockIdx.x * 8 + warp) * R, t0 = blockIdx.y * TOK;
-    if (r0 >= vdim) return;
-    const uint16_t *w[R], *c[TOK];
-#pragma unroll
-    for (int r = 0; r < R; r++) w[r] = kvb + ((int64_t)h * (nope + vdim) + nope + min(r0 + r, vdim - 1)) * kv_lora;
-#pragma unroll
-    for (int t = 0; t < TOK; t++) c[t] = cacc + ((int64_t)min(t0 + t, ntok - 1) * nh + h) * kv_lora;
-    float acc[R][TOK];
-#pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-        for (int t = 0; t < TOK; t++) acc[r][t] = 0.f;
-    for (int j = lane * 8; j + 8 <= kv_lora; j += 256) {
-        uint4 wv[R], cv[TOK];
-#pragma unroll
-        for (int r = 0; r < R; r++) wv[r] = ld_weight16(w[r] + j);
-#pragma unroll
-        for (int t = 0; t < TOK; t++) cv[t] = *reinterpret_cast<const uint4 *>(c[t] + j);
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            const uint32_t wu[4] = {wv[r].x, wv[r].y, wv[r].z, wv[r].w};
-#pragma unroll
-            for (int t = 0; t < TOK; t++) {
-                const uint32_t cu[4] = {cv[t].x, cv[t].y, cv[t].z, cv[t].w};
-                float d = 0.f;
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    d += __uint_as_float(wu[q] << 16) * __uint_as_float(cu[q] << 16) +
-                         __uint_as_float(wu[q] & 0xffff0000u) * __uint_as_float(cu[q] & 0xffff0000u);
-                acc[r][t] += d;
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-        for (int t = 0; t < TOK; t++) {
-            float a = acc[r][t];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (lane == 0 && r0 + r < vdim && t0 + t < ntok) attn[((int64_t)(t0 + t) * nh + h) * vdim + r0 + r] = a;
-        }
-}
-
-void launch_unabsorb(cudaStream_t st, const uint16_t *cacc, const uint16_t *kvb, int nh, int nope, int vdim, int kv_lora, float *attn, int tokens) {
-    if (tokens >= 4 && kv_lora % 256 == 0 && ((reinterpret_cast<uintptr_t>(kvb) | reinterpret_cast<uintptr_t>(cacc)) & 15) == 0)
-        unabsorb_rows_kernel<<<dim3((vdim + 31) / 32, (tokens + 3) / 4, nh), 256, 0, st>>>(cacc, kvb, nh, nope, vdim, kv_lora, attn, tokens);
-    else
-        unabsorb_kernel<<<dim3((nh * vdim + 7) / 8, tokens), 256, 0, st>>>(cacc, kvb, nh, nope, vdim, kv_lora, attn);
-}
-
 // Indexer scores over the f32 pool rows, the reference's order (src/attention.c:573-582 with dot_f32's scalar
 // grouping :249-258): per head four strided accumulators with separate multiply and add, (s0+s1)+(s2+s3), then any
 // remainder in order; ReLU; times the head weight; heads summed in order. One thread per pool row.
@@ -595,6 +473,12 @@ __global__ void __launch_bounds__(128) pool_scores_kernel(const float *pool, int
         total = __fadd_rn(total, __fmul_rn(d, wt[h]));
     }
     sc[c] = total;
+}
+
+// what each token of a chunk sees: rows 0 .. pos0 + t
+__global__ void chunk_lens_kernel(int32_t *len, int n, int pos0) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) len[t] = pos0 + t + 1;
 }
 
 __global__ void scale_vec_kernel(float *x, int n, float s) {
@@ -642,6 +526,9 @@ struct Registry {
     void *pin = nullptr;          // page-locked staging; pin_dev: the same memory as the device addresses it (NULL: not addressable)
     void *pin_dev = nullptr;
     size_t pin_bytes = 0;
+    CwkHostPool *pool = nullptr;  // copies of a chunk's activations (never freed: its threads sleep on it)
+    cudaStream_t up = nullptr, down = nullptr;
+    std::vector<cudaEvent_t> events;
 } g;
 
 void set_err(cwkc_error *err, int status, const char *fmt, ...) {
@@ -977,51 +864,205 @@ int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const flo
     return CWK_OK;
 }
 
-// A chunk of n tokens of a layer without an indexer: every stage batched over the tokens, the attention as n
-// decode-shaped problems over one shared cache (row t sees rows 0..pos0+t), src/attention.c:943-1024.
+// ---- a chunk's activations between the caller's pageable arrays and the device -------------------------------------
+// A chunk runs in pieces of some 256 tokens, so that the link works in both directions under the GPU's work: a piece's
+// activations are copied into page-locked memory by several threads while the piece before is computed, and its results
+// are on their way back while the next is. On 16 host cores, 8.4 MB: 790 us through the driver's own staging (one thread),
+// 230 us this way; 530 and 260 us back.
+constexpr int CHUNK_PIECE = 256;
+// Within a piece the copy and the link overlap too, COPY_GROUP bytes at a time, each shared out in blocks of COPY_BLOCK.
+constexpr size_t COPY_BLOCK = 64 * 1024, COPY_GROUP = 1024 * 1024, COPY_STAGED_MAX = 128u << 20;      // larger chunks: the driver's own staging
+
+bool ensure_copy_streams() {
+    if (g.pool) return true;
+    if (cudaStreamCreateWithFlags(&g.up, cudaStreamNonBlocking) != cudaSuccess || cudaStreamCreateWithFlags(&g.down, cudaStreamNonBlocking) != cudaSuccess) return false;
+    g.pool = new CwkHostPool();
+    return true;
+}
+cudaEvent_t pool_event(size_t i) {
+    while (g.events.size() <= i) {
+        cudaEvent_t e = nullptr;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+        g.events.push_back(e);
+    }
+    return g.events[i];
+}
+
+// The layer's contractions on the tensor cores (lin_split_tc.cu), where the shapes are whole 64-wide blocks.
+bool chunk_tc_ok(const Layer &ly, int64_t n) {
+    CwkSplitGemm a;                                        // every contraction length and weight width of the layer
+    a.A = (const uint16_t *)16; a.W = (const uint16_t *)ly.qa->data; a.Y = (void *)16; a.n = (int)n; a.ldy = 64;
+    for (const WeightMirror *w : {ly.qa, ly.qb, ly.kva, ly.o, ly.kvb}) {
+        if (w->kind != CWKC_WEIGHT_BF16) return false;
+        a.rows = (int)w->rows; a.k = (int)w->cols; a.lda = a.ldw = w->cols;
+        if (!cwk_split_gemm_ok(a)) return false;
+    }
+    return n >= 4 && n <= (1 << 20) && ly.nope % 64 == 0 && ly.vdim % 8 == 0 && ly.kvb->cols == ly.kv_lora && (ly.nh * (int64_t)ly.vdim) % 64 == 0 &&
+           (size_t)std::max(ly.q_lora, ly.kv_lora) * 4 <= 48 * 1024;
+}
+
+// A chunk of n tokens of a layer without an indexer: every stage batched over the tokens of a piece, the attention as
+// decode-shaped problems over one shared cache (row t sees rows 0..pos0+t), src/attention.c:943-1024. The contractions
+// run on the tensor cores with the activations as three bf16 planes (chunk_tc_ok), or row by row on CUDA cores.
 int chunk_steps(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos0, int64_t n, const float *X_host, float *Out_host, cwkc_error *err) {
     cudaStream_t st = ctx->stream;
     const int64_t H = ly.H;
     const int nh = ly.nh, nope = ly.nope, vdim = ly.vdim, q_lora = ly.q_lora, kv_lora = ly.kv_lora, kv_dim = ly.kv_dim;
-    const size_t per_f = (size_t)H * 2 + q_lora + (size_t)nh * nope + kv_lora + (size_t)nh * vdim;
-    const size_t need = (size_t)n * (per_f * 4 + (size_t)nh * kv_lora * 2 * 2 + 4) + 1024;
-    if (!ensure_bufs(need, 64, err)) return CWK_ERR_MEMORY;
-    float *d_x = g.d_buf, *d_qa = d_x + n * H, *d_q = d_qa + n * q_lora, *d_kva = d_q + n * (size_t)nh * nope;
-    float *d_attn = d_kva + n * kv_lora, *d_out = d_attn + n * (size_t)nh * vdim;
-    uint16_t *d_qabs = (uint16_t *)(((uintptr_t)(d_out + n * H) + 63) & ~(uintptr_t)63), *d_cacc = d_qabs + n * (size_t)nh * kv_lora;
-    int32_t *d_len = (int32_t *)(d_cacc + n * (size_t)nh * kv_lora);
+    const int64_t qw = (int64_t)nh * nope, vw = (int64_t)nh * vdim;
+    std::vector<int> pieces;
+    for (int64_t left = n; left > 0; left -= pieces.back()) pieces.push_back(left > CHUNK_PIECE + CHUNK_PIECE / 2 ? CHUNK_PIECE : (int)left);
+    const int64_t m = *std::max_element(pieces.begin(), pieces.end());
+    const bool tc = chunk_tc_ok(ly, *std::min_element(pieces.begin(), pieces.end()));
+    // device scratch, in bytes from g.d_buf: the activations of the whole chunk, the stages between of one piece
+    size_t need = 0;
+    auto take = [&](size_t bytes) { const size_t at = need; need += (bytes + 255) & ~(size_t)255; return at; };
+    const size_t o_x = take((size_t)n * H * 4), o_out = take((size_t)n * H * 4), o_kva = take((size_t)n * kv_lora * 4), o_len = take((size_t)n * 4);
+    const size_t o_qabs = take((size_t)m * nh * kv_lora * 2), o_cacc = take((size_t)m * nh * kv_lora * 2);
+    const size_t o_qa = take((size_t)m * q_lora * (tc ? 6 : 4)), o_q = take((size_t)m * qw * (tc ? 6 : 4)), o_attn = take((size_t)m * vw * (tc ? 6 : 4));
+    const size_t o_xp = tc ? take((size_t)m * H * 6) : 0;
+    size_t part_floats = 0;
+    for (const int np : pieces)
+        if (tc)
+            part_floats = std::max({part_floats, (size_t)np * (q_lora + kv_lora) * cwk_split_gemm_splits(ctx, np, q_lora, kv_lora, (int)H),
+                                    (size_t)np * qw * cwk_split_gemm_splits(ctx, np, (int)qw, 0, q_lora), (size_t)np * H * cwk_split_gemm_splits(ctx, np, (int)H, 0, (int)vw)});
+    const size_t o_part = take(part_floats * 4);
+    const size_t rb = ly.host_row_bytes, xb = (size_t)H * 4;                   // per token
+    const bool staged = (size_t)n * (2 * xb + rb) <= COPY_STAGED_MAX && (xb & 15) == 0 && ((uintptr_t)X_host & 15) == 0 && ensure_copy_streams();
+    if (!ensure_bufs(need, staged ? (size_t)n * (2 * xb + rb) : 64, err)) return CWK_ERR_MEMORY;
+    uint8_t *d = (uint8_t *)g.d_buf, *pin_x = (uint8_t *)g.pin, *pin_out = pin_x + (size_t)n * xb, *pin_rows = pin_out + (size_t)n * xb;
+    float *d_x = (float *)(d + o_x), *d_out = (float *)(d + o_out), *d_kva = (float *)(d + o_kva), *d_part = (float *)(d + o_part);
+    uint16_t *d_qabs = (uint16_t *)(d + o_qabs), *d_cacc = (uint16_t *)(d + o_cacc);
+    int32_t *d_len = (int32_t *)(d + o_len);
     int s = sync_cache(ctx, ly, capacity, pos0);
     if (s != CWK_OK) { set_err(err, s, "latent cache mirror failed"); return s; }
     CacheMirror &cm = *ly.cm;
-    std::vector<int32_t> lens((size_t)n);
-    for (int64_t t = 0; t < n; t++) lens[(size_t)t] = (int32_t)(pos0 + t + 1);
-    if (cudaMemcpyAsync(d_x, X_host, (size_t)n * H * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(d_len, lens.data(), (size_t)n * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess) {
-        set_err(err, CWK_ERR_CUDA, "chunk upload failed");
-        return CWK_ERR_CUDA;
+    const float eps = ly.spec->rms_norm_eps_f;
+    chunk_lens_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_len, (int)n, (int)pos0);
+
+    auto device_piece = [&](int64_t t0, int np) -> int {
+        const float *x = d_x + t0 * H;
+        float *out = d_out + t0 * H, *kva = d_kva + t0 * kv_lora;
+        uint16_t *rows = cm.dev + (size_t)(pos0 + t0) * kv_lora;
+        if (tc) {
+            uint16_t *d_xp = (uint16_t *)(d + o_xp), *d_qa = (uint16_t *)(d + o_qa), *d_q = (uint16_t *)(d + o_q);
+            if ((s = cwk_split_planes(ctx, x, np, (int)H, d_xp)) != CWK_OK) return s;
+            CwkSplitGemm a;                                // q_a and kv_a together
+            a.n = np;
+            a.A = d_xp; a.lda = a.ldw = H; a.k = (int)H;
+            a.W = (const uint16_t *)ly.qa->data; a.w_rows = a.rows = q_lora; a.W2 = (const uint16_t *)ly.kva->data; a.rows2 = kv_lora;
+            a.splits = cwk_split_gemm_splits(ctx, np, q_lora, kv_lora, (int)H);
+            a.Y = d_part; a.ldy = q_lora + kv_lora;
+            if ((s = cwk_split_gemm(ctx, a)) != CWK_OK) return s;
+            norm_chunk_kernel<<<dim3((unsigned)np, 2), 256, (size_t)std::max(q_lora, kv_lora) * 4, st>>>(d_part, a.splits, np, q_lora, kv_lora, ly.qa_n, ly.kva_n,
+                                                                                                     eps, d_qa, rows, ly.lbf ? nullptr : kva);
+            CwkSplitGemm q;
+            q.n = np;
+            q.A = d_qa; q.lda = q.ldw = q_lora; q.k = q_lora; q.W = (const uint16_t *)ly.qb->data; q.w_rows = qw; q.rows = (int)qw; q.ldy = qw;
+            q.splits = cwk_split_gemm_splits(ctx, np, (int)qw, 0, q_lora);
+            q.out = q.splits > 1 ? CwkSplitGemm::F32 : CwkSplitGemm::PLANES;
+            q.Y = q.splits > 1 ? (void *)d_part : (void *)d_q;
+            if ((s = cwk_split_gemm(ctx, q)) != CWK_OK) return s;
+            if (q.splits > 1 && (s = cwk_sum_partials(ctx, d_part, q.splits, np, (int)qw, nullptr, d_q)) != CWK_OK) return s;
+            CwkSplitGemm ab;                               // q_abs[t][h] = q[t][h] . W_k[h]
+            ab.n = np;
+            ab.A = d_q; ab.lda = qw; ab.k = nope; ab.heads = nh; ab.W = (const uint16_t *)ly.kvb->data; ab.w_rows = ly.kvb->rows; ab.ldw = kv_lora;
+            ab.w_head_rows = kv_dim; ab.w_k_rows = true; ab.rows = kv_lora; ab.out = CwkSplitGemm::BF16; ab.Y = d_qabs; ab.ldy = (int64_t)nh * kv_lora;
+            if ((s = cwk_split_gemm(ctx, ab)) != CWK_OK) return s;
+            ctx->launches += 1;
+        } else {
+            float *d_qa = (float *)(d + o_qa), *d_q = (float *)(d + o_q);
+            dev_linear(ctx, ly.qa, x, d_qa, np, H, q_lora);
+            dev_linear(ctx, ly.kva, x, kva, np, H, kv_lora);
+            rms_scale_kernel<<<(unsigned)np, 256, 0, st>>>(d_qa, q_lora, q_lora, ly.qa_n, eps, nullptr, 0);
+            rms_scale_kernel<<<(unsigned)np, 256, 0, st>>>(kva, kv_lora, kv_lora, ly.kva_n, eps, rows, kv_lora);
+            dev_linear(ctx, ly.qb, d_qa, d_q, np, q_lora, qw);
+            launch_absorb_q(st, d_q, (const uint16_t *)ly.kvb->data, nh, nope, kv_dim, kv_lora, d_qabs, np);
+            ctx->launches += 3;
+        }
+        s = cwk_mla_decode(ctx, d_qabs, cm.dev, 0, kv_lora, d_len + t0, (int)(pos0 + t0 + np), nullptr, 0, np, nh, kv_lora, 0, 1.0f / sqrtf((float)nope), d_cacc, 0);
+        if (s != CWK_OK) return s;
+        if (tc) {
+            uint16_t *d_attn = (uint16_t *)(d + o_attn);
+            CwkSplitGemm u;                                // attn[t][h] = W_v[h] . c_acc[t][h]
+            u.n = np;
+            u.planes = 1; u.A = d_cacc; u.lda = (int64_t)nh * kv_lora; u.k = kv_lora; u.heads = nh; u.W = (const uint16_t *)ly.kvb->data; u.w_rows = ly.kvb->rows;
+            u.ldw = kv_lora; u.w_head_rows = kv_dim; u.w_row_off = nope; u.rows = vdim; u.out = CwkSplitGemm::PLANES; u.Y = d_attn; u.ldy = vw;
+            if ((s = cwk_split_gemm(ctx, u)) != CWK_OK) return s;
+            CwkSplitGemm o;
+            o.n = np;
+            o.A = d_attn; o.lda = o.ldw = vw; o.k = (int)vw; o.W = (const uint16_t *)ly.o->data; o.w_rows = H; o.rows = (int)H; o.ldy = H;
+            o.splits = cwk_split_gemm_splits(ctx, np, (int)H, 0, (int)vw);
+            o.Y = o.splits > 1 ? d_part : out;
+            if ((s = cwk_split_gemm(ctx, o)) != CWK_OK) return s;
+            if (o.splits > 1 && (s = cwk_sum_partials(ctx, d_part, o.splits, np, (int)H, out, nullptr)) != CWK_OK) return s;
+        } else {
+            float *d_attn = (float *)(d + o_attn);
+            unabsorb_kernel<<<dim3((nh * vdim + 7) / 8, (unsigned)np), 256, 0, st>>>(d_cacc, (const uint16_t *)ly.kvb->data, nh, nope, vdim, kv_lora, d_attn);
+            ctx->launches += 1;
+            dev_linear(ctx, ly.o, d_attn, out, np, vw, H);
+        }
+        return CWK_OK;
+    };
+    auto rows_src = [&](int64_t t0) { return ly.lbf ? (const void *)(cm.dev + (size_t)(pos0 + t0) * kv_lora) : (const void *)(d_kva + t0 * kv_lora); };
+    uint8_t *host_rows = ly.host_layer + (size_t)pos0 * rb;
+    auto quiet = [&](int st_, const char *what) {          // nothing of this call stays in flight behind an error
+        cudaStreamSynchronize(st);
+        if (staged) { cudaStreamSynchronize(g.up); cudaStreamSynchronize(g.down); }
+        if (what) set_err(err, st_, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
+        else set_err(err, st_, "%s", cwk_last_error(ctx));
+        return st_;
+    };
+    struct Back { uint8_t *dst, *pin; size_t len; };
+    std::vector<Back> back;                                // groups on their way back, an event each (pool_event(2 + index))
+    auto send = [&](uint8_t *pin, const void *src, uint8_t *dst, size_t bytes, bool &ok) {
+        for (size_t o = 0; o < bytes && ok; o += COPY_GROUP) {
+            const size_t len = std::min(COPY_GROUP, bytes - o);
+            cudaEvent_t e = pool_event(2 + back.size());
+            ok = e && cudaMemcpyAsync(pin + o, (const uint8_t *)src + o, len, cudaMemcpyDeviceToHost, g.down) == cudaSuccess && cudaEventRecord(e, g.down) == cudaSuccess;
+            back.push_back({dst + o, pin + o, len});
+        }
+    };
+    int64_t t0 = 0;
+    for (size_t i = 0; i < pieces.size(); t0 += pieces[i++]) {
+        const int np = pieces[i];
+        const size_t at = (size_t)t0 * xb, bytes = (size_t)np * xb;
+        bool ok;
+        if (staged) {
+            ok = true;
+            for (size_t lo = at; lo < at + bytes && ok; lo += COPY_GROUP) {
+                const size_t len = std::min(COPY_GROUP, at + bytes - lo);
+                g.pool->run((int)((len + COPY_BLOCK - 1) / COPY_BLOCK), [&](int b) {
+                    const size_t o = lo + (size_t)b * COPY_BLOCK;
+                    cwk_copy_to_pinned(pin_x + o, (const uint8_t *)X_host + o, std::min(COPY_BLOCK, lo + len - o));
+                });
+                ok = cudaMemcpyAsync((uint8_t *)d_x + lo, pin_x + lo, len, cudaMemcpyHostToDevice, g.up) == cudaSuccess;
+            }
+            cudaEvent_t up = pool_event(0);
+            ok = ok && up && cudaEventRecord(up, g.up) == cudaSuccess && cudaStreamWaitEvent(st, up, 0) == cudaSuccess;
+        } else
+            ok = cudaMemcpyAsync((uint8_t *)d_x + at, (const uint8_t *)X_host + at, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
+        if (!ok) return quiet(CWK_ERR_CUDA, "chunk upload failed");
+        if ((s = device_piece(t0, np)) != CWK_OK) return quiet(s, nullptr);
+        if (staged) {
+            cudaEvent_t computed = pool_event(1);
+            ok = computed && cudaEventRecord(computed, st) == cudaSuccess && cudaStreamWaitEvent(g.down, computed, 0) == cudaSuccess;
+            send(pin_rows + (size_t)t0 * rb, rows_src(t0), host_rows + (size_t)t0 * rb, (size_t)np * rb, ok);
+            send(pin_out + at, (const uint8_t *)d_out + at, (uint8_t *)Out_host + at, bytes, ok);
+        }
+        else
+            ok = cudaMemcpyAsync(host_rows + (size_t)t0 * rb, rows_src(t0), (size_t)np * rb, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+                 cudaMemcpyAsync((uint8_t *)Out_host + at, (const uint8_t *)d_out + at, bytes, cudaMemcpyDeviceToHost, st) == cudaSuccess;
+        if (!ok) return quiet(CWK_ERR_CUDA, "chunk download failed");
     }
-    dev_linear(ctx, ly.qa, d_x, d_qa, (int)n, H, q_lora);
-    dev_linear(ctx, ly.kva, d_x, d_kva, (int)n, H, kv_lora);
-    rms_scale_kernel<<<(unsigned)n, 256, 0, st>>>(d_qa, q_lora, q_lora, ly.qa_n, ly.spec->rms_norm_eps_f, nullptr, 0);
-    rms_scale_kernel<<<(unsigned)n, 256, 0, st>>>(d_kva, kv_lora, kv_lora, ly.kva_n, ly.spec->rms_norm_eps_f, cm.dev + (size_t)pos0 * kv_lora, kv_lora);
-    dev_linear(ctx, ly.qb, d_qa, d_q, (int)n, q_lora, (int64_t)nh * nope);
-    launch_absorb_q(st, d_q, (const uint16_t *)ly.kvb->data, nh, nope, kv_dim, kv_lora, d_qabs, (int)n);
-    ctx->launches += 3;
-    s = cwk_mla_decode(ctx, d_qabs, cm.dev, 0, kv_lora, d_len, (int)(pos0 + n), nullptr, 0, (int)n, nh, kv_lora, 0, 1.0f / sqrtf((float)nope),
-                       d_cacc, 0);
-    if (s != CWK_OK) { set_err(err, s, "%s", cwk_last_error(ctx)); return s; }
-    launch_unabsorb(st, d_cacc, (const uint16_t *)ly.kvb->data, nh, nope, vdim, kv_lora, d_attn, (int)n);
-    ctx->launches += 1;
-    dev_linear(ctx, ly.o, d_attn, d_out, (int)n, (int64_t)nh * vdim, H);
-    // results and the chunk's cache rows back to the caller (pageable memory: synchronous copies)
-    bool ok = cudaMemcpyAsync(Out_host, d_out, (size_t)n * H * 4, cudaMemcpyDeviceToHost, st) == cudaSuccess;
-    if (ly.lbf) ok = ok && cudaMemcpyAsync(ly.host_layer + (size_t)pos0 * ly.host_row_bytes, cm.dev + (size_t)pos0 * kv_lora, (size_t)n * kv_lora * 2, cudaMemcpyDeviceToHost, st) == cudaSuccess;
-    else ok = ok && cudaMemcpyAsync(ly.host_layer + (size_t)pos0 * ly.host_row_bytes, d_kva, (size_t)n * kv_lora * 4, cudaMemcpyDeviceToHost, st) == cudaSuccess;
-    if (!ok || cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
-        set_err(err, CWK_ERR_CUDA, "GPU chunk failed: %s", cudaGetErrorString(cudaGetLastError()));
-        return CWK_ERR_CUDA;
+    for (size_t i = 0; i < back.size(); i++) {             // results out of page-locked memory, group by group as they arrive
+        if (cudaEventSynchronize(g.events[2 + i]) != cudaSuccess) return quiet(CWK_ERR_CUDA, "GPU chunk failed");
+        const Back &r = back[i];
+        g.pool->run((int)((r.len + COPY_BLOCK - 1) / COPY_BLOCK), [&](int b) {
+            const size_t o = (size_t)b * COPY_BLOCK;
+            memcpy(r.dst + o, r.pin + o, std::min(COPY_BLOCK, r.len - o));
+        });
     }
+    if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) return quiet(CWK_ERR_CUDA, "GPU chunk failed");
     if (cwk_check_device_error(ctx) != CWK_OK) { set_err(err, CWK_ERR_STATE, "%s", cwk_last_error(ctx)); return CWK_ERR_STATE; }
     note_row_written(ly, pos0 + n - 1);
     return CWK_OK;
