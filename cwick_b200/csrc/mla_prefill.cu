@@ -203,6 +203,19 @@ bool cwk_mla_prefill_attn_tc_ok(const void *Q, const void *cache, const void *Wu
 int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, const void *Wuk, void *kx, int *flags, int64_t pos0, int n, int nh,
                             float scale, void *out, int exact_only);
 
+// Which attention route is the faster one for a chunk of n queries behind pos0 rows. The expansion covers every cached
+// row once, whatever n, and its attention works in tiles of 128 queries; the absorbed route costs a pass of the decode
+// kernel per query. In microseconds, measured with 64 heads: expansion 0.018 per row; attention 0.74 per 64-key tile and 5
+// per item (128 queries x head x half), the items dealt over the SMs; absorbed 0.032 per query and 128-key tile and 0.42 per
+// query around it. 509 queries after 3001 rows: 230 against 640; 64 queries after 32704: 970 against 550.
+static bool expanded_keys_pay(const cwk_ctx *ctx, int n, int64_t pos0, int nh) {
+    const double T = (double)(pos0 + n), mean = (double)pos0 + 0.5 * n;
+    const double items = (double)((n + 127) / 128) * nh * 2, rounds = items <= ctx->sm_count ? 1.0 : items / ctx->sm_count + 0.5;
+    const double expanded = 0.018 * T * nh / 64 + rounds * (0.74 * (mean / 64 + 1) + 5.0);
+    const double absorbed = n * (0.032 * (mean / 128 + 1) + 0.42) * nh / 64;
+    return expanded < absorbed;
+}
+
 // Absorb: Qfull[t][h][0:L] = q[t][h][0:nope] . W_uk[h] ([nope][L] row-major bf16), and
 // Qfull[t][h][L:L+rope] = RoPE(q[t][h][nope:nope+rope], pos0+t). The identity is
 // q_abs = W_k^T q of src/attention.c:741-744 (gemv_bf16_t), batched over tokens.
@@ -294,10 +307,8 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
     // The attention takes one of two routes. Queries as MMA rows against per-head expanded keys (mla_prefill_attn.cu)
     // needs Kx bf16 [pos0+n][nh][qd] and no Qfull; the absorbed route (the decode kernel once per query row) needs
     // Qfull bf16 [n][nh][row]. The same workspace region serves whichever runs.
-    // The expansion covers every cached row, so it pays when the chunk is a fair share of the context (always for a
-    // prompt from position 0); a short chunk after a long history takes the absorbed route.
     const bool expanded_keys = ctx->force_mla_path != 0 && ctx->force_mla_path != 1 && ctx->force_mla_path != 2 && ctx->force_mla_path != 4 && pos0 + n <= 32768 &&
-                               (int64_t)n * 4 >= pos0 + n;
+                               expanded_keys_pay(ctx, n, pos0, nh);
     const size_t b_kx = up((size_t)(pos0 + n) * nh * qd * 2);
     const size_t b_q = up((size_t)n * nh * qd * 2), b_qf = expanded_keys ? std::max(b_kx, up((size_t)n * nh * row * 2)) : up((size_t)n * nh * row * 2),
                  b_len = up((size_t)n * 4) + up(((size_t)((n + 127) / 128) * nh * 2 + 3) * 4);
