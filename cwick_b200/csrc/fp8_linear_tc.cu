@@ -11,13 +11,18 @@
 // order of src/tensor.c:511-520). Two TMEM accumulators alternate so the MMA of
 // block kb+1 runs while block kb is being promoted.
 //
-// Block tile 128 (rows of X) x 256 (two scale column blocks), K step 128 = one scale block per
-// pipeline stage, two stages. An operand tile arrives as ONE TMA box of two 64-wide column blocks
-// (a TMA operation costs some 400 cycles whatever its size, and a 128 x 128 tile with 64-wide steps
-// is bound by that, not by the MMAs). The MMA is M 128 x N 256: at N = 256 the operand reads leave
-// shared-memory bandwidth for the incoming tiles. Warp 0 = TMA producer, warp 1 = MMA issuer + TMEM
-// owner, warps 4..11 = promotion / epilogue (TMEM lane quarter = warp % 4; warps 4-7 own output
-// columns 0-127 of the tile, warps 8-11 columns 128-255).
+// A pair of CTAs (a cluster of two) takes tiles of 256 rows of X x 256 outputs (two scale column blocks), K step 128 = one
+// scale block per pipeline stage, three stages. The tile's MMA spans the pair (M 256 x N 256): each CTA holds its own 128
+// rows of X and one half of the 256 weight rows, so that 64 KB per SM and step arrive for 1024 cycles of MMAs. With a
+// 128 x 256 tile per SM it was 96 KB, and the ~56 B/clk an SM gets from L2 while all of them load made the step 1.8 k cycles
+// (o_proj, 4096 tokens, 8192 -> 4096: 251 us). An operand tile arrives as ONE TMA box of two 64-wide column blocks (a TMA
+// operation costs some 400 cycles whatever its size).
+// The pairs are persistent: whole waves of tiles first; the tiles left over are cut along K into parts so that the last
+// round is as full as the others (a chunk of a few tiles is all last round), their partial sums added by a second kernel.
+// Warp 0 = TMA producer, warp 1 = TMEM owner and, in the pair's first CTA, MMA issuer for both, warps 4..11 = promotion /
+// epilogue of the CTA's own 128 rows (TMEM lane quarter = warp % 4; warps 4-7 own output columns 0-127 of the tile,
+// warps 8-11 columns 128-255); they write out while the next tile's first blocks are multiplied.
+#include <algorithm>
 #include <map>
 #include <tuple>
 
@@ -25,10 +30,11 @@
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 128;
-constexpr int STAGES = 2;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;      // 32 KB + 64 KB
-constexpr int G_OFF_BAR = STAGES * (A_BYTES + B_BYTES);          // 196608
+constexpr int BM = 256, BN = 256, BK = 128;
+constexpr int STAGES = 3;
+constexpr int A_BYTES = BM / 2 * BK * 2, B_BYTES = BN / 2 * BK * 2;   // 32 KB + 32 KB per CTA
+constexpr int G_OFF_STG = STAGES * (A_BYTES + B_BYTES);          // 196608: eight 4 KB staging tiles of the epilogue
+constexpr int G_OFF_BAR = G_OFF_STG + 8 * 4096;
 constexpr int G_SMEM = G_OFF_BAR + 256 + 1024;
 constexpr uint32_t G_TMEM_COLS = 512;                             // two 256-column partial accumulators
 constexpr int G_THREADS = 384;
@@ -69,8 +75,7 @@ __global__ void __launch_bounds__(256) e4m3_to_bf16_kernel(const uint8_t *src, u
 }
 
 // One launch serves one projection, or two that share the activations X (q_a and kv_a of the MLA
-// prefill: alone they fill 1.3 and 0.65 waves of the SMs): column tiles [0, tiles_a) belong to the
-// first weight matrix, the rest to the second.
+// prefill): column tiles [0, tiles_a) belong to the first weight matrix, the rest to the second.
 struct GemmProblem {
     const float *scale_inv;
     int64_t cols;
@@ -79,12 +84,38 @@ struct GemmProblem {
 };
 struct GemmParams {
     GemmProblem pr[2];
-    int tiles_a;               // column tiles of the first problem
+    int tiles_a, tiles_n, tiles_m;   // column tiles of the first problem and of both, row tiles
+    int full, splits;                // tiles done whole; parts of K each later tile is cut into
+    float *part;                     // partial sums of the cut tiles [tile - full][part][256][256]
     int64_t n, k;
     int *err;
 };
 
-__global__ void __launch_bounds__(G_THREADS, 1)
+struct GemmUnit {
+    int second, col0, row0, kb0, kb1, slot;      // slot: which partial-sum tile (-1: a whole tile)
+};
+// Work unit u: tiles 0 .. full - 1, then the parts of the tiles after them. Row tiles vary fastest: pairs that run at the
+// same time share weight tiles and, between them, all of X.
+__device__ __forceinline__ GemmUnit gemm_unit(int u, const GemmParams &p, int nkb) {
+    GemmUnit g;
+    int tile = u, part = 0, parts = 1;
+    g.slot = -1;
+    if (u >= p.full && p.splits > 1) {
+        tile = p.full + (u - p.full) / p.splits;
+        part = (u - p.full) % p.splits;
+        parts = p.splits;
+        g.slot = u - p.full;
+    }
+    const int tn = tile / p.tiles_m;
+    g.second = tn >= p.tiles_a;
+    g.col0 = (tn - (g.second ? p.tiles_a : 0)) * BN;
+    g.row0 = (tile % p.tiles_m) * BM;
+    g.kb0 = nkb * part / parts;
+    g.kb1 = nkb * (part + 1) / parts;
+    return g;
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1)
 fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                      const __grid_constant__ CUtensorMap tm_w2, const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -96,138 +127,191 @@ fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + G_OFF_BAR + 8 * GB_COUNT + 8);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int second = (int)blockIdx.x >= p.tiles_a;
-    GemmProblem pp;            // field-wise select: indexing the parameter struct with a run-time index would copy it to local memory
-    pp.scale_inv = second ? p.pr[1].scale_inv : p.pr[0].scale_inv;
-    pp.cols = second ? p.pr[1].cols : p.pr[0].cols;
-    pp.Y = second ? p.pr[1].Y : p.pr[0].Y;
-    pp.out_bf16 = second ? p.pr[1].out_bf16 : p.pr[0].out_bf16;
-    const int col0 = ((int)blockIdx.x - (second ? p.tiles_a : 0)) * BN, row0 = blockIdx.y * BM;
+    const int rank = (int)cluster_rank();
     const int nkb = (int)(p.k / 128);              // scale blocks along K = pipeline steps
+    const int units = p.splits > 1 ? p.full + (p.tiles_n * p.tiles_m - p.full) * p.splits : p.tiles_n * p.tiles_m;
+    const int u0 = (int)blockIdx.x >> 1, du = (int)gridDim.x >> 1;
 
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_x) : "memory");
-        if (second) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w2) : "memory");
-        else asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
-        for (int i = 0; i < GB_COUNT; i++) mbar_init(bar(i), (i >= GB_PEMPTY) ? 256u : 1u);
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
+        if (p.tiles_n > p.tiles_a) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w2) : "memory");
+        for (int i = 0; i < GB_COUNT; i++) mbar_init(bar(i), (i >= GB_PEMPTY) ? 16u : 1u);      // PEMPTY: the promotion warps of both CTAs
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(G_TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(G_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
 
     if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
-            int issued = 0;
-            for (int s = 0; s < nkb && ok; s++) {
-                const int slot = s % STAGES, use = s / STAGES;
-                ok = mbar_wait(bar(GB_EMPTY + slot), (uint32_t)((use & 1) ^ 1), p.err, 401);
-                if (!ok) break;
-                mbar_expect_tx(bar(GB_FULL + slot), A_BYTES + B_BYTES);
-                tma_load_3d(base + slot * (A_BYTES + B_BYTES), &tm_x, 0, row0, s * 2, bar(GB_FULL + slot));
-                // (the maps are kernel parameters: their addresses must stay in parameter space, so no pointer select)
-                if (second) tma_load_3d(base + slot * (A_BYTES + B_BYTES) + A_BYTES, &tm_w2, 0, col0, s * 2, bar(GB_FULL + slot));
-                else tma_load_3d(base + slot * (A_BYTES + B_BYTES) + A_BYTES, &tm_w, 0, col0, s * 2, bar(GB_FULL + slot));
-                issued = s + 1;
+            int c = 0;                                       // steps issued so far, over all units
+            for (int u = u0; u < units && ok; u += du) {
+                const GemmUnit g = gemm_unit(u, p, nkb);
+                for (int kb = g.kb0; kb < g.kb1 && ok; kb++, c++) {
+                    const int slot = c % STAGES, use = c / STAGES;
+                    ok = mbar_wait(bar(GB_EMPTY + slot), (uint32_t)((use & 1) ^ 1), p.err, 401);
+                    if (!ok) break;
+                    // both CTAs' tiles are counted at the first CTA's barrier, where the issuer waits
+                    if (rank == 0) mbar_expect_tx(bar(GB_FULL + slot), 2 * (A_BYTES + B_BYTES));
+                    const uint32_t full = cluster_addr(bar(GB_FULL + slot), 0), a0 = base + slot * (A_BYTES + B_BYTES);
+                    tma_load_3d_pair(a0, &tm_x, 0, g.row0 + rank * (BM / 2), kb * 2, full);
+                    // (the maps are kernel parameters: their addresses must stay in parameter space, so no pointer select)
+                    if (g.second) tma_load_3d_pair(a0 + A_BYTES, &tm_w2, 0, g.col0 + rank * (BN / 2), kb * 2, full);
+                    else tma_load_3d_pair(a0 + A_BYTES, &tm_w, 0, g.col0 + rank * (BN / 2), kb * 2, full);
+                }
             }
-            if (!ok)      // drain the copies still in flight before leaving
-                for (int s = (issued > STAGES ? issued - STAGES : 0); s < issued; s++)
+            if (!ok && rank == 0)      // drain the copies still in flight before leaving
+                for (int s = (c > STAGES ? c - STAGES : 0); s < c; s++)
                     mbar_wait(bar(GB_FULL + s % STAGES), (uint32_t)((s / STAGES) & 1), p.err, 402);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (lane == 0 && rank == 0) {
             constexpr uint32_t ID = idesc_bf16(BM, BN, 0, 0);
             bool ok = true;
-            for (int kb = 0; kb < nkb && ok; kb++) {
-                const int pb = kb & 1, puse = kb >> 1, slot = kb % STAGES, use = kb / STAGES;
-                ok = mbar_wait(bar(GB_PEMPTY + pb), (uint32_t)((puse & 1) ^ 1), p.err, 403);
-                if (ok) ok = mbar_wait(bar(GB_FULL + slot), (uint32_t)(use & 1), p.err, 404);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a0 = base + slot * (A_BYTES + B_BYTES), b0 = a0 + A_BYTES;
-                const uint64_t da = smem_desc(a0, 16, 1024), db = smem_desc(b0, 16, 1024);   // one build per stage, constant adds per MMA
+            int c = 0;
+            for (int u = u0; u < units && ok; u += du) {
+                const GemmUnit g = gemm_unit(u, p, nkb);
+                for (int kb = g.kb0; kb < g.kb1 && ok; kb++, c++) {
+                    const int pb = c & 1, puse = c >> 1, slot = c % STAGES, use = c / STAGES;
+                    ok = mbar_wait(bar(GB_PEMPTY + pb), (uint32_t)((puse & 1) ^ 1), p.err, 403);
+                    if (ok) ok = mbar_wait(bar(GB_FULL + slot), (uint32_t)(use & 1), p.err, 404);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a0 = base + slot * (A_BYTES + B_BYTES), b0 = a0 + A_BYTES;
+                    const uint64_t da = smem_desc(a0, 16, 1024), db = smem_desc(b0, 16, 1024);   // one build per stage, constant adds per MMA
 #pragma unroll
-                for (int ks = 0; ks < 8; ks++)          // 64-wide column block ks >> 2 of each operand, 32 bytes per 16-wide step
-                    umma_bf16(tmem + pb * 256, da + (uint64_t)(((ks >> 2) * (BM * 128) + (ks & 3) * 32) >> 4),
-                              db + (uint64_t)(((ks >> 2) * (BN * 128) + (ks & 3) * 32) >> 4), ID, ks != 0);
-                umma_commit(bar(GB_EMPTY + slot));        // stage may be refilled once these MMAs are done
-                umma_commit(bar(GB_PFULL + pb));
+                    for (int ks = 0; ks < 8; ks++)          // 64-wide column block ks >> 2 of each operand, 32 bytes per 16-wide step
+                        umma_bf16_pair(tmem + pb * 256, da + (uint64_t)(((ks >> 2) * (BM / 2 * 128) + (ks & 3) * 32) >> 4),
+                                       db + (uint64_t)(((ks >> 2) * (BN / 2 * 128) + (ks & 3) * 32) >> 4), ID, ks != 0);
+                    umma_commit_pair(bar(GB_EMPTY + slot));        // stage may be refilled once these MMAs are done
+                    umma_commit_pair(bar(GB_PFULL + pb));
+                }
             }
         }
     } else if (warp >= 4) {
         const int q = warp & 3, ch = (warp - 4) >> 2;
-        const int row = q * 32 + lane;
-        const int cbase = col0 + ch * 128;             // first output column of this warp's 128
-        const bool live = cbase < pp.cols;              // a tile past the last column block: only keep the barriers moving
         const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
         const int64_t ncb = (p.k + 127) / 128;
-        const float *srow = pp.scale_inv + (int64_t)(live ? cbase / 128 : 0) * ncb;
-        float acc[128];
-#pragma unroll
-        for (int j = 0; j < 128; j++) acc[j] = 0.f;
+        uint8_t *stg = sm + G_OFF_STG + (warp - 4) * 4096;
         bool ok = true;
-        for (int kb = 0; kb < nkb; kb++) {
-            const int pb = kb & 1, puse = kb >> 1;
-            ok = mbar_wait(bar(GB_PFULL + pb), (uint32_t)(puse & 1), p.err, 405);
-            if (!ok) break;
-            tc_fence_after();
-            if (live) {
-                const float sc = __ldg(srow + kb);
+        int c = 0;
+        for (int u = u0; u < units && ok; u += du) {
+            const GemmUnit g = gemm_unit(u, p, nkb);
+            // (field-wise selects: indexing the parameter struct with a run-time index would copy it to local memory)
+            const int64_t cols = g.second ? p.pr[1].cols : p.pr[0].cols;
+            const int cbase = g.col0 + ch * 128;             // first output column of this warp's 128
+            const bool live = cbase < cols;                  // a tile past the last column block: only keep the barriers moving
+            const float *srow = (g.second ? p.pr[1].scale_inv : p.pr[0].scale_inv) + (int64_t)(live ? cbase / 128 : 0) * ncb;
+            float acc[128];
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    uint32_t v[32];                              // two loads in flight per wait
-                    TMEM_LD16(v, 0, tlane + pb * 256 + ch * 128 + c * 32);
-                    TMEM_LD16(v, 16, tlane + pb * 256 + ch * 128 + c * 32 + 16);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int j = 0; j < 128; j++) acc[j] = 0.f;
+            for (int kb = g.kb0; kb < g.kb1; kb++, c++) {
+                const int pb = c & 1, puse = c >> 1;
+                ok = mbar_wait(bar(GB_PFULL + pb), (uint32_t)(puse & 1), p.err, 405);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                if (live) {
+                    const float sc = __ldg(srow + kb);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) acc[c * 32 + j] = fmaf(__uint_as_float(v[j]), sc, acc[c * 32 + j]);
-                }
-            }
-            tc_fence_before();
-            mbar_arrive(bar(GB_PEMPTY + pb));
-        }
-        if (ok && live && row0 + row < p.n) {
-            const int64_t r = row0 + row;
-            if (pp.out_bf16) {
-                uint16_t *y = (uint16_t *)pp.Y + r * pp.cols + cbase;
+                    for (int cc = 0; cc < 4; cc++) {
+                        uint32_t v[32];                              // two loads in flight per wait
+                        TMEM_LD16(v, 0, tlane + pb * 256 + ch * 128 + cc * 32);
+                        TMEM_LD16(v, 16, tlane + pb * 256 + ch * 128 + cc * 32 + 16);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int j = 0; j < 128; j += 8) {
-                    if (cbase + j + 8 <= pp.cols) {
-                        uint4 w;
-                        w.x = pack_bf16x2(acc[j], acc[j + 1]); w.y = pack_bf16x2(acc[j + 2], acc[j + 3]);
-                        w.z = pack_bf16x2(acc[j + 4], acc[j + 5]); w.w = pack_bf16x2(acc[j + 6], acc[j + 7]);
-                        *reinterpret_cast<uint4 *>(y + j) = w;
-                    } else {
-                        for (int e = 0; e < 8; e++)
-                            if (cbase + j + e < pp.cols) y[j + e] = (uint16_t)(pack_bf16x2(acc[j + e], 0.f) & 0xffffu);
+                        for (int j = 0; j < 32; j++) acc[cc * 32 + j] = fmaf(__uint_as_float(v[j]), sc, acc[cc * 32 + j]);
                     }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(cluster_addr(bar(GB_PEMPTY + pb), 0));
+            }
+            if (!ok || !live) continue;
+            // A thread holds one row; whole 128-byte lines leave through the warp's staging tile, four rows per instruction.
+            const int r0 = g.row0 + rank * (BM / 2) + q * 32;
+            const bool bf16 = g.slot < 0 && (g.second ? p.pr[1].out_bf16 : p.pr[0].out_bf16);
+            uint8_t *y;                                          // row r0, column cbase
+            int64_t row_bytes;
+            int rows_left, cols_left = (int)(cols - cbase);
+            if (g.slot >= 0) {
+                row_bytes = BN * 4;
+                y = (uint8_t *)(p.part + (int64_t)g.slot * BM * BN + (int64_t)(rank * (BM / 2) + q * 32) * BN + ch * 128);
+                rows_left = 32; cols_left = 128;
+            } else {
+                row_bytes = cols * (bf16 ? 2 : 4);
+                y = (uint8_t *)(g.second ? p.pr[1].Y : p.pr[0].Y) + (int64_t)r0 * row_bytes + (int64_t)cbase * (bf16 ? 2 : 4);
+                rows_left = (int)min((int64_t)32, p.n - r0);
+            }
+            auto flush = [&](int col, int el) {                  // the staging tile's 128 bytes per row, at column `col` (8-column pieces are whole)
+                __syncwarp();
+#pragma unroll
+                for (int r8 = 0; r8 < 8; r8++) {
+                    const int rr = r8 * 4 + (lane >> 3), jj = lane & 7;
+                    const uint4 w = *reinterpret_cast<const uint4 *>(stg + rr * 128 + ((jj ^ (rr & 7)) << 4));
+                    if (rr < rows_left && col + (jj + 1) * (16 / el) <= cols_left) *reinterpret_cast<uint4 *>(y + (int64_t)rr * row_bytes + col * el + jj * 16) = w;
+                }
+                __syncwarp();
+            };
+            if (bf16) {
+#pragma unroll
+                for (int cc = 0; cc < 2; cc++) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        *reinterpret_cast<uint4 *>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                            make_uint4(pack_bf16x2(acc[cc * 64 + 8 * j], acc[cc * 64 + 8 * j + 1]), pack_bf16x2(acc[cc * 64 + 8 * j + 2], acc[cc * 64 + 8 * j + 3]),
+                                       pack_bf16x2(acc[cc * 64 + 8 * j + 4], acc[cc * 64 + 8 * j + 5]), pack_bf16x2(acc[cc * 64 + 8 * j + 6], acc[cc * 64 + 8 * j + 7]));
+                    flush(cc * 64, 2);
                 }
             } else {
-                float *y = (float *)pp.Y + r * pp.cols + cbase;
 #pragma unroll
-                for (int j = 0; j < 128; j += 4) {
-                    if (cbase + j + 4 <= pp.cols) {
-                        *reinterpret_cast<float4 *>(y + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-                    } else {
-                        for (int e = 0; e < 4; e++)
-                            if (cbase + j + e < pp.cols) y[j + e] = acc[j + e];
-                    }
+                for (int cc = 0; cc < 4; cc++) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        *reinterpret_cast<float4 *>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                            make_float4(acc[cc * 32 + 4 * j], acc[cc * 32 + 4 * j + 1], acc[cc * 32 + 4 * j + 2], acc[cc * 32 + 4 * j + 3]);
+                    flush(cc * 32, 4);
                 }
             }
         }
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();                                          // the pair's barriers and tensor memory stay until both are done
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G_TMEM_COLS) : "memory");
     }
+}
+
+// Adds up the parts of the tiles that were cut along K, in order. Four columns per thread, 64 threads per row.
+__global__ void __launch_bounds__(256) fp8_sum_parts_kernel(const GemmParams p) {
+    const int tile = p.full + (int)blockIdx.y, tn = tile / p.tiles_m;
+    const bool second = tn >= p.tiles_a;
+    const int row = (int)blockIdx.x * 4 + (int)(threadIdx.x >> 6), c = (int)(threadIdx.x & 63) * 4;
+    const int64_t r = (int64_t)(tile % p.tiles_m) * BM + row, col = (int64_t)(tn - (second ? p.tiles_a : 0)) * BN + c;
+    const int64_t cols = second ? p.pr[1].cols : p.pr[0].cols;
+    if (r >= p.n || col >= cols) return;                     // (cols is a multiple of 8: four columns are in or out together)
+    const float *src = p.part + (int64_t)blockIdx.y * p.splits * BM * BN + row * BN + c;
+    float4 v = *reinterpret_cast<const float4 *>(src);
+#pragma unroll 4
+    for (int s = 1; s < p.splits; s++) {
+        const float4 w = *reinterpret_cast<const float4 *>(src + (int64_t)s * BM * BN);
+        v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+    }
+    void *Y = second ? p.pr[1].Y : p.pr[0].Y;
+    if (second ? p.pr[1].out_bf16 : p.pr[0].out_bf16)
+        *reinterpret_cast<uint2 *>((uint16_t *)Y + r * cols + col) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+    else
+        *reinterpret_cast<float4 *>((float *)Y + r * cols + col) = v;
 }
 
 }  // namespace
@@ -291,7 +375,7 @@ static int encode_weight_map(cwk_ctx *ctx, const void *dst_c, int64_t cols, int6
     cuuint32_t es[3] = {1, 1, 1};
     cuuint64_t wd[3] = {64, (cuuint64_t)cols, (cuuint64_t)(k / 64)};
     cuuint64_t st[2] = {(cuuint64_t)k * 2, 128};
-    cuuint32_t wb[3] = {64, BN, 2};
+    cuuint32_t wb[3] = {64, BN / 2, 2};
     if (enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dst, wd, st, wb, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cwk_fail(ctx, CWK_ERR_CUDA, "cuTensorMapEncodeTiled failed for the projection weights");
@@ -337,7 +421,7 @@ int cwk_fp8_linear_tc_launch2(cwk_ctx *ctx, const void *X, int64_t n, int64_t k,
         cuuint32_t es[3] = {1, 1, 1};
         cuuint64_t xd[3] = {64, (cuuint64_t)n, (cuuint64_t)(k / 64)};
         cuuint64_t st[2] = {(cuuint64_t)k * 2, 128};
-        cuuint32_t xb[3] = {64, BM, 2};
+        cuuint32_t xb[3] = {64, BM / 2, 2};
         if (enc(&tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(X), xd, st, xb, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cwk_fail(ctx, CWK_ERR_CUDA, "cuTensorMapEncodeTiled failed for the projection activations");
@@ -352,12 +436,28 @@ int cwk_fp8_linear_tc_launch2(cwk_ctx *ctx, const void *X, int64_t n, int64_t k,
     p.pr[1] = p.pr[0];
     if (W2) { p.pr[1].scale_inv = scale2; p.pr[1].cols = cols2; p.pr[1].Y = Y2; p.pr[1].out_bf16 = out_bf16_2; }
     p.tiles_a = (int)((cols1 + BN - 1) / BN);
+    p.tiles_n = p.tiles_a + (W2 ? (int)((cols2 + BN - 1) / BN) : 0);
+    p.tiles_m = (int)((n + BM - 1) / BM);
     p.n = n; p.k = k; p.err = ctx->dev_err;
-    const int tiles_b = W2 ? (int)((cols2 + BN - 1) / BN) : 0;
-    dim3 grid((unsigned)(p.tiles_a + tiles_b), (unsigned)((n + BM - 1) / BM));
+    // Whole waves, then the rest cut along K into as many parts as fill one more round, each at least four blocks long.
+    const int pairs = std::max(1, ctx->sm_count / 2), tiles = p.tiles_n * p.tiles_m;
+    p.full = tiles / pairs * pairs;
+    const int rest = tiles - p.full;
+    p.splits = rest > 0 ? std::max(1, std::min(pairs / rest, (int)(k / 128 / 4))) : 1;
+    p.part = nullptr;
+    if (p.splits > 1) {
+        s = cwk_reserve_scratch(ctx, (size_t)rest * p.splits * BM * BN * 4);
+        if (s != CWK_OK) return s;
+        p.part = ctx->scratch;
+    }
+    const int units = p.full + rest * p.splits;
     CwkKernelTimer timer(ctx);
-    fp8_linear_tc_kernel<<<grid, G_THREADS, G_SMEM, ctx->stream>>>(tm_x, tm_w, tm_w2, p);
+    fp8_linear_tc_kernel<<<2 * std::min(units, pairs), G_THREADS, G_SMEM, ctx->stream>>>(tm_x, tm_w, tm_w2, p);
     CWK_LAUNCH_CHECK(ctx, "fp8_linear_tc_kernel");
+    if (p.splits > 1) {
+        fp8_sum_parts_kernel<<<dim3(BM / 4, (unsigned)rest), 256, 0, ctx->stream>>>(p);
+        CWK_LAUNCH_CHECK(ctx, "fp8_sum_parts_kernel");
+    }
     return CWK_OK;
 }
 
