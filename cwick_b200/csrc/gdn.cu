@@ -30,7 +30,6 @@ struct GdnParams {
     float *S;              // [B][nh][head_v][head_k]
     float *out;            // [B][n][val_dim]
     int n, nh, kv_group;
-    int n_stride;          // positions per slot in the arrays (>= n: a call's tail after the chunk-parallel part)
     float rms_eps;
 };
 
@@ -53,7 +52,7 @@ template <int HK> struct GdnPos {
 template <int HK> __device__ __forceinline__ void gdn_fetch(const GdnParams &p, int item, int t, int j, int hv, GdnPos<HK> &r) {
     const int vh = item % p.nh, b = item / p.nh, kh = vh / p.kv_group;
     const int key_dim = (p.nh / p.kv_group) * HK, val_dim = p.nh * hv;
-    const float *row = p.up + ((int64_t)b * p.n_stride + t) * (2 * key_dim + val_dim);
+    const float *row = p.up + ((int64_t)b * p.n + t) * (2 * key_dim + val_dim);
 #pragma unroll
     for (int u = 0; u < GdnPos<HK>::PER; u++)
         if (j + u * hv < HK) {
@@ -61,9 +60,9 @@ template <int HK> __device__ __forceinline__ void gdn_fetch(const GdnParams &p, 
             r.k[u] = __ldg(row + key_dim + (int64_t)kh * HK + j + u * hv);
         }
     r.v = __ldg(row + 2 * key_dim + (int64_t)vh * hv + j);
-    r.z = __ldg(p.gate + ((int64_t)b * p.n_stride + t) * val_dim + (int64_t)vh * hv + j);
-    r.gdec = __ldg(p.gdec + ((int64_t)b * p.n_stride + t) * p.nh + vh);
-    r.beta = __ldg(p.beta + ((int64_t)b * p.n_stride + t) * p.nh + vh);
+    r.z = __ldg(p.gate + ((int64_t)b * p.n + t) * val_dim + (int64_t)vh * hv + j);
+    r.gdec = __ldg(p.gdec + ((int64_t)b * p.n + t) * p.nh + vh);
+    r.beta = __ldg(p.beta + ((int64_t)b * p.n + t) * p.nh + vh);
     r.a_log = __ldg(p.a_log + vh);
     r.dt_bias = __ldg(p.dt_bias + vh);
 }
@@ -175,7 +174,7 @@ __global__ void __launch_bounds__(128) gdn_scan_kernel(const __grid_constant__ C
             float o = __fmul_rn(acc, s_rstd);
             o = __fmul_rn(o, nw);
             o = __fmul_rn(o, silu);
-            p.out[((int64_t)b * p.n_stride + t) * val_dim + (int64_t)vh * hv + j] = o;
+            p.out[((int64_t)b * p.n + t) * val_dim + (int64_t)vh * hv + j] = o;
         }
     }
     if (j == copier) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -183,9 +182,9 @@ __global__ void __launch_bounds__(128) gdn_scan_kernel(const __grid_constant__ C
 
 }  // namespace
 
-int cwk_gdn_scan_chunked(cwk_ctx *ctx, int B, int n_stride, int nchunks, int nh, int kv_group, const float *up, const float *gdec,
-                         const float *beta, const float *gate, const float *a_log, const float *dt_bias, const float *norm,
-                         float rms_eps, float *S, float *out);
+bool cwk_gdn_chunked_ok(int kv_group, const float *up, const float *gate, const float *norm, const float *S, const float *out);
+int cwk_gdn_scan_chunked(cwk_ctx *ctx, int B, int n, int nh, int kv_group, const float *up, const float *gdec, const float *beta, const float *gate,
+                         const float *a_log, const float *dt_bias, const float *norm, float rms_eps, float *S, float *out);
 
 extern "C" int cwk_gdn_scan(cwk_ctx *ctx, int B, int n, int nh, int head_k, int head_v, int kv_group, const float *up,
                             const float *gdec, const float *beta, const float *gate, const float *a_log, const float *dt_bias,
@@ -197,23 +196,14 @@ extern "C" int cwk_gdn_scan(cwk_ctx *ctx, int B, int n, int nh, int head_k, int 
         return cwk_fail(ctx, CWK_ERR_UNSUPPORTED, "gdn_scan is built for key dims 64, 128 and value dims 32..128 (got %d, %d)", head_k, head_v);
     if (reinterpret_cast<uintptr_t>(S) & 15) return cwk_fail(ctx, CWK_ERR_ARGUMENT, "gdn_scan: the state must be 16-byte aligned");
     CWK_CUDA(ctx, cudaSetDevice(ctx->device));
-    // A prompt (at least two chunks of 64 positions, head dims 128 x 128) goes through the chunk-parallel form; its last
-    // n % 64 positions, decode steps and every other shape through the position-serial kernel, which keeps the
-    // reference's summation order. cwk_ctx_force_mla_path(ctx, 0) keeps everything on the serial kernel.
-    int done = 0;
-    if (head_k == 128 && head_v == 128 && n >= 128 && ctx->force_mla_path != 0 && (reinterpret_cast<uintptr_t>(up) & 15) == 0) {
-        const int nchunks = n / 64;
-        int s = cwk_gdn_scan_chunked(ctx, B, n, nchunks, nh, kv_group, up, gdec, beta, gate, a_log, dt_bias, norm, rms_eps, S, out);
-        if (s != CWK_OK) return s;
-        done = nchunks * 64;
-        if (done == n) return CWK_OK;
-    }
-    const int key_dim_h = (nh / kv_group) * head_k, val_dim_h = nh * head_v;
+    // A prompt (at least two chunks of 64 positions, head dims 128 x 128) goes through the chunk-parallel form; decode
+    // steps and every other shape through the position-serial kernel, which keeps the reference's summation order.
+    // cwk_ctx_force_mla_path(ctx, 0) keeps everything on the serial kernel.
+    if (head_k == 128 && head_v == 128 && n >= 128 && ctx->force_mla_path != 0 && cwk_gdn_chunked_ok(kv_group, up, gate, norm, S, out))
+        return cwk_gdn_scan_chunked(ctx, B, n, nh, kv_group, up, gdec, beta, gate, a_log, dt_bias, norm, rms_eps, S, out);
     GdnParams p;
-    p.up = up + (int64_t)done * (2 * key_dim_h + val_dim_h); p.gdec = gdec + (int64_t)done * nh; p.beta = beta + (int64_t)done * nh;
-    p.gate = gate + (int64_t)done * val_dim_h; p.a_log = a_log; p.dt_bias = dt_bias; p.norm = norm; p.S = S;
-    p.out = out + (int64_t)done * val_dim_h;
-    p.n = n - done; p.n_stride = n; p.nh = nh; p.kv_group = kv_group; p.rms_eps = rms_eps;
+    p.up = up; p.gdec = gdec; p.beta = beta; p.gate = gate; p.a_log = a_log; p.dt_bias = dt_bias; p.norm = norm; p.S = S; p.out = out;
+    p.n = n; p.nh = nh; p.kv_group = kv_group; p.rms_eps = rms_eps;
     const int nitems = B * nh;
     if ((int64_t)nitems * head_v > 0x7fffffffLL) return cwk_fail(ctx, CWK_ERR_UNSUPPORTED, "gdn_scan: more than 2^31 state rows");
     const size_t smem = (size_t)head_v * head_k * sizeof(float) + 1024;   // + slack to align the tile to the swizzle period

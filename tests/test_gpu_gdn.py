@@ -122,3 +122,32 @@ def test_prompt_goes_through_the_chunk_parallel_scan(attn, B, n):
         tol = 1e-4 if path == -1 else 2e-5
         assert np.abs(got - want).max() <= tol * np.abs(want).max(), (path, float(np.abs(got - want).max()), float(np.abs(want).max()))
         assert np.abs(Sg - S_h).max() <= tol * np.abs(S_h).max(), (path, float(np.abs(Sg - S_h).max()))
+
+
+@pytest.mark.parametrize("B,n,nh,grp", [(1, 129, 8, 1), (2, 191, 8, 4), (1, 320, 16, 8)])
+def test_partial_last_chunk_and_head_groups(attn, B, n, nh, grp):
+    """The chunk-parallel scan at the edges of its last chunk (1 and 63 positions of 64, none missing) and for the key-head
+    groups it serves, against the position-serial kernel on the same inputs."""
+    hk = hv = 128
+    key_dim, val_dim = (nh // grp) * hk, nh * hv
+    g = torch.Generator(device="cuda").manual_seed(n)
+
+    def f32(*s):
+        return torch.randn(*s, device="cuda", generator=g)
+    up = f32(B, n, 2 * key_dim + val_dim)
+    kq = up[:, :, :2 * key_dim].view(B, n, -1, hk)
+    kq /= kq.norm(dim=-1, keepdim=True)
+    args = [up, f32(B, n, nh), f32(B, n, nh), f32(B, n, val_dim), 0.5 * f32(nh), 0.5 * f32(nh), 1 + 0.1 * f32(hv)]
+    S0 = 0.05 * f32(B, nh, hv, hk)
+    res = []
+    for path in (-1, 0):
+        S = S0.clone()
+        assert attn.lib.cwk_ctx_force_mla_path(attn.ctx.h, path) == 0
+        try:
+            out = attn.gdn_scan(*args, S, grp, 1e-6)
+            attn.ctx.sync()
+        finally:
+            attn.lib.cwk_ctx_force_mla_path(attn.ctx.h, -1)
+        res.append((out, S))
+    for got, want in zip(*res):
+        assert float((got - want).norm() / want.norm()) < 5e-6
