@@ -354,10 +354,16 @@ constexpr int CWK_MAX_SPLITS = 512;
 // else here): 64 for one sequence in many splits, 8 for many sequences in few (registers, hence blocks per SM).
 template <bool FOLD, int CWK_MERGE_AHEAD>
 static __global__ void __launch_bounds__(128) lse_merge_kernel(const float *partial, int nsplit, int nh, int D,
-                                                               uint16_t *out, float *rec_out) {
+                                                               uint16_t *out, float *rec_out, const int2 *meta = nullptr) {
     const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t rec_sz = (int64_t)nh * (D + 2);
-    const float *base = partial + (int64_t)b * nsplit * rec_sz;
+    int64_t rec0 = (int64_t)b * nsplit;
+    if (meta) {                                   // a number of records of its own per sequence: {first, count}
+        const int2 m = meta[b];
+        rec0 = m.x;
+        nsplit = m.y;
+    }
+    const float *base = partial + rec0 * rec_sz;
     __shared__ float sw[CWK_MAX_SPLITS];
     __shared__ float red[8];
     // value pass, part one: blockIdx.z picks a 128-column chunk of the row
@@ -421,6 +427,10 @@ static inline void lse_combine_launch(cudaStream_t st, const float *partial, int
     if (nsplit > 32) lse_merge_kernel<false, 64><<<grid, 128, 0, st>>>(partial, nsplit, nh, D, out, nullptr);
     else if (nsplit > 8) lse_merge_kernel<false, 32><<<grid, 128, 0, st>>>(partial, nsplit, nh, D, out, nullptr);
     else lse_merge_kernel<false, 8><<<grid, 128, 0, st>>>(partial, nsplit, nh, D, out, nullptr);
+}
+// `meta[b]` = {first record, number of records} of sequence b, at most CWK_MAX_SPLITS of them
+static inline void lse_combine_ranges_launch(cudaStream_t st, const float *partial, const int2 *meta, int nh, int D, int B, uint16_t *out) {
+    lse_merge_kernel<false, 8><<<dim3(nh, B, (D + 127) / 128), 128, 0, st>>>(partial, 0, nh, D, out, nullptr, meta);
 }
 static inline void lse_fold_launch(cudaStream_t st, const float *partial, int nsplit, int nh, int D, float *rec_out) {
     const dim3 grid(nh, 1, (D + 127) / 128);

@@ -12,7 +12,7 @@
 // not apply so the caller can take the mma.sync path.
 int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int64_t seq_stride,
                              int64_t ld, const int32_t *kv_len, int max_kv_len, int B, int nh,
-                             int R, float scale, float *partial, int nsplit, void *out_direct, const int32_t *sel, int64_t sel_ld);
+                             int R, float scale, float *partial, int nsplit, void *out_direct, const int32_t *sel, int64_t sel_ld, int2 *seq_meta);
 bool cwk_mla_decode_tc_available();
 // persistent tcgen05/TMA kernel with the cross-block reduction inside (mla_decode_sk.cu): bf16 rows to `out`, or one
 // folded record per sequence to `rec_out`
@@ -152,9 +152,29 @@ static int mla_launch(cwk_ctx *ctx, const void *q, const void *cache, int64_t se
     const int max_tiles = (max_kv_len + tile - 1) / tile;
     const int hblocks = (path == 0) ? nh : (nh + 63) / 64;
     int ns = plan_splits(ctx->sm_count, B * hblocks, max_tiles, n_splits > 0 ? n_splits : 0);
+    const size_t rec = (size_t)nh * (L + 2) * sizeof(float);
+    // A batch whose sequences have lengths of their own (known on the device only) and tiles enough for every SM: equal
+    // shares of all tiles instead of equal numbers of splits per sequence, which make the longest sequence's blocks the
+    // call's time and leave SMs without a block. A block that changes sequences pays about two tiles' time for it, so the
+    // shares have to be several tiles long. 64 sequences of 16384..32768 rows: MLA64OLD -> MLA64NEW us.
+    if (path == 2 && !sel && kv_len && B > 1 && seq_stride != 0 && n_splits <= 0 && out && !partial_out && !ctx->keep_splits && ctx->sm_count <= CWK_MAX_SPLITS &&
+        (int64_t)B * max_tiles >= 6 * (int64_t)ctx->sm_count) {
+        const int G = ctx->sm_count;
+        int s = cwk_reserve_scratch(ctx, rec * (size_t)(B + G) + (size_t)B * sizeof(int2));
+        if (s != CWK_OK) return s;
+        int2 *meta = (int2 *)((uint8_t *)ctx->scratch + rec * (size_t)(B + G));
+        {
+            CwkKernelTimer timer(ctx);
+            s = cwk_mla_decode_tc_launch(ctx, q, cache, seq_stride, ld, kv_len, max_kv_len, B, nh, R, scale, ctx->scratch, G, nullptr, nullptr, 0, meta);
+            if (s != CWK_OK) return s;
+        }
+        lse_combine_ranges_launch(ctx->stream, ctx->scratch, meta, nh, L, B, (uint16_t *)out);
+        CWK_LAUNCH_CHECK(ctx, "lse_merge_kernel");
+        ctx->last_nsplit = 0;
+        return CWK_OK;
+    }
     // One split per sequence needs no records at all: the kernel normalises and writes bf16.
     const bool direct = (ns == 1 && out && !partial_out && path != 0);
-    const size_t rec = (size_t)nh * (L + 2) * sizeof(float);
     if (!direct) {
         int s = cwk_reserve_scratch(ctx, rec * ((size_t)ns * B + (ctx->keep_splits ? 1 : 0)));      // keep_splits: room for one folded record behind them
         if (s != CWK_OK) return s;
@@ -165,7 +185,7 @@ static int mla_launch(cwk_ctx *ctx, const void *q, const void *cache, int64_t se
     CwkKernelTimer timer(ctx);
     if (path == 2) {
         int s = cwk_mla_decode_tc_launch(ctx, q, cache, seq_stride, ld, kv_len, max_kv_len, B, nh, R, scale, partial, ns,
-                                         direct ? out : nullptr, sel, sel_ld);
+                                         direct ? out : nullptr, sel, sel_ld, nullptr);
         if (s != CWK_OK) return s;
     } else if (path == 1) {
         static bool attr_set[16] = {false};

@@ -105,10 +105,61 @@ struct TcParams {
     const uint16_t *cache;
     int64_t seq_stride, ld;
     int rope_cols;         // 64, or 0: the ninth block is zeros
+    // Range mode (B > 0; seq_meta set): the tiles of all B sequences, one after another, are dealt out in equal contiguous
+    // ranges, one per block (blockIdx.x): a block may end one sequence and begin the next, and every block has the same
+    // number of tiles whatever the sequences' lengths. The record of sequence b from block g goes to slot b + g (along the
+    // tiles either b or g grows, so slots are unique); seq_meta[b] = {first slot, number of records}.
+    int B;
+    int2 *seq_meta;
 #ifdef CWK_TRACE
     long long *trace;      // developer build only: per-phase clock64 stamps of block (0,0); NULL = off
 #endif
 };
+
+struct Segment {
+    int b, t0, n, kv;      // sequence, first tile, tiles, rows of the sequence
+};
+
+// Range mode: where block blockIdx.x's share of all tiles begins (out[0] = sequence, out[1] = tile in it) and how many tiles
+// it has (out[2]). One warp. The block with a sequence's first tile notes the sequence's first record slot and their
+// number; sequences without rows are noted by the block with the tile before them (block 0: those at the front).
+__device__ __forceinline__ void find_range(const TcParams &p, int lane, int *out) {
+    auto tiles_of = [&](int b) { return b < p.B ? (max(p.kv_len[b], 0) + TILE - 1) / TILE : 0; };
+    int64_t total = 0;
+    for (int b0 = 0; b0 < p.B; b0 += 32) {
+        int v = tiles_of(b0 + lane);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        total += v;
+    }
+    const int64_t G = max((int64_t)1, min((int64_t)gridDim.x, total)), g = blockIdx.x;      // no block between two others is left without a tile
+    const int64_t lo = g < G ? total * g / G : total, hi = g < G ? total * (g + 1) / G : total;
+    auto block_of = [&](int64_t tile) { return ((tile + 1) * G - 1) / total; };
+    int64_t before = 0;
+    for (int b0 = 0; b0 < p.B; b0 += 32) {
+        const int mine = tiles_of(b0 + lane);
+        int v = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        const int64_t s0 = before + v - mine, s1 = s0 + mine;      // this lane's sequence: tiles [s0, s1)
+        if (mine > 0 && s0 <= lo && lo < s1 && hi > lo) {
+            out[0] = b0 + lane;
+            out[1] = (int)(lo - s0);
+        }
+        if (b0 + lane < p.B) {
+            if (mine > 0 && lo <= s0 && s0 < hi) {
+                const int64_t g1 = block_of(s1 - 1);
+                p.seq_meta[b0 + lane] = make_int2(b0 + lane + (int)g, (int)(g1 - g + 1));
+            }
+            if (mine == 0 && (s0 > 0 ? (lo < s0 && s0 <= hi) : g == 0)) p.seq_meta[b0 + lane] = make_int2(0, 0);
+        }
+        before += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) out[2] = (int)(hi - lo);
+}
 
 __global__ void __launch_bounds__(NTHREADS, 1)
 mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
@@ -125,28 +176,51 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     float *s_w = s_alpha + 64;                                        // [16 warps][16] per-warp max / sum
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int split = blockIdx.x, b = p.reverse_b ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
+    const int split = blockIdx.x;
     // With few blocks in the launch (one short sequence), two blocks take each tile: both compute the tile's scores
     // and probabilities, each accumulates and writes one half of the value columns. Half the value MMAs per block,
     // and the records leave through twice as many SMs.
     const int mb0 = p.halves == 2 ? 2 * (int)blockIdx.z : 0, mb1 = p.halves == 2 ? mb0 + 2 : 4;
-    const int kv = p.kv_len ? p.kv_len[b] : p.kv_len_imm;
-    const int ntiles = (kv + TILE - 1) / TILE;
-    const int t0 = (int)((int64_t)ntiles * split / p.nsplit);
-    const int t1 = (int)((int64_t)ntiles * (split + 1) / p.nsplit);
-    const int n = t1 - t0;
-    float *rec = p.partial + ((int64_t)b * p.nsplit + split) * (int64_t)(NH * (L + 2));
+    // this block's tiles: `n` of them, from tile t0 of sequence b (range mode: going on into the sequences after it)
+    int b = p.reverse_b ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y, t0, n;
+    const int ntiles = p.seq_meta ? 0 : ((p.kv_len ? p.kv_len[b] : p.kv_len_imm) + TILE - 1) / TILE;
+    if (p.seq_meta) {
+        __shared__ int s_range[3];
+        if (warp == 2) find_range(p, lane, s_range);
+        __syncthreads();
+        b = s_range[0]; t0 = s_range[1]; n = s_range[2];
+        if (n <= 0) return;
+    } else {
+        t0 = (int)((int64_t)ntiles * split / p.nsplit);
+        n = (int)((int64_t)ntiles * (split + 1) / p.nsplit) - t0;
+    }
+    auto record = [&](int sb) { return p.partial + (p.seq_meta ? (int64_t)sb + split : (int64_t)sb * p.nsplit + split) * (int64_t)(NH * (L + 2)); };
 
     if (n <= 0) {                       // empty split: a record the merge ignores (direct mode: zeros)
         if (p.out) {
             for (int i = tid; i < NH * L / 2; i += NTHREADS) reinterpret_cast<uint32_t *>(p.out + (int64_t)b * NH * L)[i] = 0u;
         } else {
+            float *rec = record(b);
             for (int i = tid; i < NH * (L + 2); i += NTHREADS) rec[i] = (i < NH) ? -INFINITY : 0.f;
         }
         return;
     }
+    // the block's tiles sequence by sequence; a segment is what it has of one
+    auto first_segment = [&]() {
+        Segment s;
+        s.b = b; s.t0 = t0; s.kv = p.kv_len ? p.kv_len[b] : p.kv_len_imm;
+        s.n = p.seq_meta ? min(n, (s.kv + TILE - 1) / TILE - t0) : n;
+        return s;
+    };
+    auto next_segment = [&](Segment &s, int left) {        // left: tiles of the block behind this segment, at least one
+        do {
+            s.b++;
+            s.kv = p.kv_len[s.b];
+        } while (s.kv <= 0);
+        s.t0 = 0;
+        s.n = min(left, (s.kv + TILE - 1) / TILE);
+    };
 
-    const int bz = p.batch_coord_zero ? 0 : b;
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_q) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_kv) : "memory");
@@ -160,10 +234,10 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // Blocks that have one tile more than the others start first when they are few; when they are most of the
         // launch they are the ones to spread.
         if (p.stagger) {
-            const int nlong = ntiles % p.nsplit;                            // blocks with one tile more (0: all alike)
+            const int nlong = p.seq_meta ? 0 : ntiles % p.nsplit;                            // blocks with one tile more (0: all alike)
             const bool longest = nlong != 0 && n == (ntiles + p.nsplit - 1) / p.nsplit;
             int group;
-            if (nlong == 0) group = (split + 3 * b) & 7;
+            if (nlong == 0) group = (split + (p.seq_meta ? 0 : 3 * b)) & 7;
             else if (nlong * 4 <= p.nsplit) group = longest ? 0 : 1 + (split + 3 * b) % 7;      // a few long blocks: they go first
             else group = longest ? (split + 3 * b) % 7 : 7;                 // mostly long blocks: they spread, the few short ones last
             const long long until = clock64() + (long long)group * p.stagger;
@@ -177,10 +251,10 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (!p.sel) {
             for (int k = 0; k < 6; k += 2) {
                 mbar_expect_tx(bar(B_FULL + k), 2 * KV_BLK);
-                tma_load_4d(base + OFF_KV + k * KV_BLK, &tm_kv, 0, t0 * TILE, k, bz, bar(B_FULL + k));
+                tma_load_4d(base + OFF_KV + k * KV_BLK, &tm_kv, 0, t0 * TILE, k, p.batch_coord_zero ? 0 : b, bar(B_FULL + k));
             }
             mbar_expect_tx(bar(B_FULL + 6), 3 * KV_BLK);
-            tma_load_4d(base + OFF_KV + 6 * KV_BLK, &tm_kr, 0, t0 * TILE, 6, bz, bar(B_FULL + 6));
+            tma_load_4d(base + OFF_KV + 6 * KV_BLK, &tm_kr, 0, t0 * TILE, 6, p.batch_coord_zero ? 0 : b, bar(B_FULL + 6));
         }
     }
     if (warp == 1) {
@@ -206,9 +280,20 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             bool ok = true;
             int issued_it[NBLK];
             for (int k = 0; k < NBLK; k++) issued_it[k] = 0;      // tile 0 went out during set-up
+            Segment sg = first_segment();
+            int begin = 0, nq = 1;                                // the block's tile with which the segment begins; queries asked for
             for (int it = 1; it < n && ok; it++) {
                 const uint32_t par_free = (uint32_t)((it & 1) ^ 1);
-                const int row = (t0 + it) * TILE;
+                if (it == begin + sg.n) {                         // the next sequence: its query replaces this one's after the last scores
+                    begin = it;
+                    next_segment(sg, n - it);
+                    ok = mbar_wait(bar(B_SFULL), (uint32_t)((it - 1) & 1), p.err, 107);
+                    if (!ok) break;
+                    mbar_expect_tx(bar(B_QFULL), NBLK * Q_BLK);
+                    tma_load_3d(base + OFF_Q, &tm_q, 0, sg.b * NH, 0, bar(B_QFULL));
+                    nq++;
+                }
+                const int row = (sg.t0 + it - begin) * TILE, bz = p.batch_coord_zero ? 0 : sg.b;
                 for (int k = 0; k < 8 && ok; k += 2) {
                     ok = mbar_wait(bar(B_EMPTY_L + (k >> 1)), par_free, p.err, 102);
                     // the last latent pair and the rope block (= the P^T slot) come free together, at the end of
@@ -230,7 +315,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 }
             }
             if (!ok) {      // drain: do not leave the block with bulk copies in flight
-                mbar_wait(bar(B_QFULL), 0, p.err, 103);
+                mbar_wait(bar(B_QFULL), (uint32_t)((nq - 1) & 1), p.err, 103);
                 for (int k = 0; k < 8; k += 2)
                     if (issued_it[k] >= 0) mbar_wait(bar(B_FULL + k), (uint32_t)(issued_it[k] & 1), p.err, 104);
             }
@@ -240,7 +325,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // 64 threads, two rows of the tile each: a row's 1152 bytes go out as 72 copies of 16 bytes, each to its place
         // in the 128-byte-swizzled block of its 64 columns. One commit group per pair of blocks (three for the last),
         // so that the score MMAs start on the first pair while the others are still arriving.
-        const int pt = tid - 64;
+        const int pt = tid - 64, kv = p.kv_len ? p.kv_len[b] : p.kv_len_imm;
         const uint16_t *cbase = p.cache + (p.batch_coord_zero ? 0 : (int64_t)b * p.seq_stride);
         const int32_t *selb = p.sel + (int64_t)b * p.sel_ld;
         bool ok = true;
@@ -297,9 +382,13 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             // (the issue loop is one thread, and its instruction count bounds the MMA rate at N = 64).
             const uint64_t dK = smem_desc(base + OFF_KV, 16, 1024), dQ = smem_desc(base + OFF_Q, 16, 1024);
             const uint64_t dV = smem_desc(base + OFF_KV, KV_BLK, 1024), dP = smem_desc(base + OFF_KV + RP * KV_BLK, KV_BLK, 1024);
-            bool ok = mbar_wait(bar(B_QFULL), 0, p.err, 201);
+            bool ok = true;
+            Segment sg = first_segment();
+            int begin = 0, nseg = 0;
             for (int it = 0; it < n && ok; it++) {
                 const uint32_t par = (uint32_t)(it & 1);
+                if (it == begin + sg.n) { begin = it; next_segment(sg, n - it); }
+                if (it == begin) ok = mbar_wait(bar(B_QFULL), (uint32_t)(nseg++ & 1), p.err, 201);
                 // S^T = K Q^T over the nine column blocks (4 k-steps of 16 each)
 #pragma unroll
                 for (int k = 0; k < NBLK; k++) {
@@ -322,7 +411,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 if (!ok) break;
                 TRACE(1, it, 3);
                 tc_fence_after();
-                const uint32_t acc0 = it != 0;
+                const uint32_t acc0 = it != begin;
 #pragma unroll
                 for (int mb = 0; mb < 4; mb++) {
                     if (mb >= mb0 && mb < mb1) {
@@ -348,14 +437,12 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int st = tid - 128;                     // 0..511
         const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
         float lpart[HG];
-#pragma unroll
-        for (int h = 0; h < HG; h++) lpart[h] = 0.f;
         if (p.sel) {
             // gather mode: these 512 threads have nothing to do until the first tile's scores exist, so they fetch the
             // first tile (four threads per row; 16-byte copies into the swizzled blocks, one commit group per block pair)
             const int r = st >> 2, part = st & 3;
             const int j = t0 * TILE + r;
-            const bool val = j < kv;
+            const bool val = j < (p.kv_len ? p.kv_len[b] : p.kv_len_imm);
             const uint16_t *src = p.cache + (p.batch_coord_zero ? 0 : (int64_t)b * p.seq_stride) +
                                   (int64_t)(val ? p.sel[(int64_t)b * p.sel_ld + j] : 0) * p.ld;
             const uint32_t drow = base + OFF_KV + r * 128;
@@ -386,7 +473,13 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             mbar_arrive(bar(B_FULL + 6));
         }
         bool ok = true;
-        for (int it = 0; it < n; it++) {
+        Segment sg = first_segment();
+        for (int begin = 0; ok;) {                        // one segment
+        const int end = begin + sg.n, kv = sg.kv;
+        float *rec = record(sg.b);
+#pragma unroll
+        for (int h = 0; h < HG; h++) lpart[h] = 0.f;
+        for (int it = begin; it < end; it++) {
             ok = mbar_wait(bar(B_SFULL), (uint32_t)(it & 1), p.err, 301);
             if (!ok) break;
             if (st == 0) TRACE(2, it, 0);
@@ -395,12 +488,12 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             TMEM_LD16(sr, 0, tlane + COL_S + hb);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (st == 0) TRACE(2, it, 5);
-            const bool valid = (t0 + it) * TILE + row < kv;
+            const bool valid = (sg.t0 + it - begin) * TILE + row < kv;
             float s[HG];
 #pragma unroll
             for (int h = 0; h < HG; h++) s[h] = valid ? __uint_as_float(sr[h]) * p.scale_log2 : -INFINITY;
 
-            if (it == 0) {
+            if (it == begin) {
                 // Reference exponent per head: the score of the tile's first token. Any value works
                 // as long as no score outruns it by more than 2^LAZY_LOG2 (checked next, every tile).
                 if (row == 0) {
@@ -445,7 +538,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 softmax_bar();
 #pragma unroll
                 for (int h = 0; h < HG; h++) lpart[h] *= s_alpha[hb + h];
-                if (it > 0) {
+                if (it > begin) {
                     // O^T columns are heads: scale column h of every dv block by alpha[h]
                     for (int mb = 0; mb < 4; mb++) {
                         uint32_t o[16];
@@ -511,7 +604,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             if (p.out) softmax_bar();
             if (st == 0) TRACE(2, 15, 4);
             for (int mb = mb0; mb < mb1 && ok; mb++) {
-                ok = mbar_wait(bar(mb == 3 ? B_EMPTY_RP : B_EMPTY_L + mb), (uint32_t)((n - 1) & 1), p.err, 302);
+                ok = mbar_wait(bar(mb == 3 ? B_EMPTY_RP : B_EMPTY_L + mb), (uint32_t)((end - 1) & 1), p.err, 302);
                 ok = __all_sync(0xffffffffu, ok);                  // the TMEM load below is warp-wide
                 if (!ok) break;
                 if (st == 0 && mb == 0) TRACE(2, 15, 2);
@@ -521,7 +614,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 TMEM_LD16(o, 0, tlane + COL_O + mb * 64 + h0);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (p.out) {
-                    uint16_t *dst = p.out + ((int64_t)b * NH + h0) * L + mb * 128 + row;
+                    uint16_t *dst = p.out + ((int64_t)sg.b * NH + h0) * L + mb * 128 + row;
 #pragma unroll
                     for (int j = 0; j < 16; j++)
                         dst[j * L] = (uint16_t)(pack_bf16x2(__uint_as_float(o[j]) * s_alpha[h0 + j], 0.f) & 0xffffu);
@@ -531,6 +624,12 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     for (int j = 0; j < 16; j++) dst[j * L] = __uint_as_float(o[j]);
                 }
             }
+        }
+        if (end >= n || !ok) break;
+        tc_fence_before();                                // the accumulator has been read: these threads' next P lets its MMAs go ahead
+        softmax_bar();                                    // the reference exponents and row sums have been read
+        next_segment(sg, n - end);
+        begin = end;
         }
     }
 #ifdef CWK_TRACE
@@ -550,7 +649,7 @@ bool cwk_mla_decode_tc_available() { return true; }
 
 int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int64_t seq_stride, int64_t ld,
                              const int32_t *kv_len, int max_kv_len, int B, int nh, int R, float scale, float *partial,
-                             int nsplit, void *out_direct, const int32_t *sel, int64_t sel_ld) {
+                             int nsplit, void *out_direct, const int32_t *sel, int64_t sel_ld, int2 *seq_meta) {
     const int width = L + R;          // 576, or 512 for a rope-free latent (the rope block then reads as zeros)
     if (nh != NH) return cwk_fail(ctx, CWK_ERR_UNSUPPORTED, "tcgen05 MLA decode is built for 64 heads");
     if (max_kv_len <= 0) return cwk_fail(ctx, CWK_ERR_UNSUPPORTED, "tcgen05 MLA decode needs a non-empty cache");
@@ -578,6 +677,13 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
     p.out = (uint16_t *)out_direct;
     p.sel = sel; p.sel_ld = sel_ld; p.cache = (const uint16_t *)cache; p.seq_stride = seq_stride; p.ld = ld; p.rope_cols = R;
     p.reverse_b = shared_cache ? 1 : 0;
+    p.B = B; p.seq_meta = seq_meta;
+    if (seq_meta) {                    // range mode: nsplit = number of blocks
+        p.halves = 1; p.stagger = 700;
+        mla_decode_tc_kernel<<<nsplit, NTHREADS, SMEM_TOTAL, ctx->stream>>>(*tm_q, *tm_kv, *tm_kr, p);
+        CWK_LAUNCH_CHECK(ctx, "mla_decode_tc_kernel");
+        return CWK_OK;
+    }
     p.halves = ((int64_t)nsplit * B * 2 <= ctx->sm_count) ? 2 : 1;
     {
         const int tiles_per_block = ((max_kv_len + TILE - 1) / TILE + nsplit - 1) / nsplit;

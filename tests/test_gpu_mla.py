@@ -371,3 +371,39 @@ def test_bad_arguments_are_reported_not_run(attn):
         attn.mla_decode_dims(to_bf16_cuda(q), to_bf16_cuda(cache), torch.ones(1, dtype=torch.int32).cuda(),
                              1024, -448, SCALE)
     assert e.value.status in (lib.ERR_ARGUMENT, lib.ERR_UNSUPPORTED)
+
+
+@pytest.mark.parametrize("lens", [
+    [0, 40000, 0, 1, 129, 0, 70000, 128],            # empty sequences in front, between and inside; one block, many blocks
+    [9000] * 13,                                     # alike, not a multiple of the blocks' share
+    [1] * 300 + [120000],                            # blocks that pass through dozens of sequences
+    [0, 0, 0],                                       # nothing at all
+])
+def test_batch_in_equal_shares_of_tiles(attn, lens):
+    """A batch large enough to be dealt out in equal shares of all tiles (blocks end one sequence and begin the next): every
+    sequence against the same kernel on that sequence alone, whose own results the tests above pin to the oracle."""
+    B, rows = len(lens), max(max(lens), 120000 if 0 in lens else 1)
+    g = torch.Generator(device="cuda").manual_seed(B)
+    pool = torch.randn(max(rows, 8192), 576, device="cuda", generator=g).to(torch.bfloat16)
+    big = B * rows <= 2_000_000
+    cache = torch.empty(B, rows, 576, dtype=torch.bfloat16, device="cuda") if big else None
+    if big:
+        for b in range(B):
+            cache[b] = pool.roll(17 * b, 0)[:rows]
+        stride = rows * 576
+    else:                                            # overlapping views of one pool, 64 rows apart
+        extra = torch.randn(64 * B + rows, 576, device="cuda", generator=g).to(torch.bfloat16)
+        cache, stride = extra, 64 * 576
+    q = torch.randn(B, 64, 576, device="cuda", generator=g).to(torch.bfloat16)
+    kv = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    got = attn.mla_decode(q, cache, kv, max_kv_len=rows, scale=192 ** -0.5, seq_stride=stride)
+    attn.ctx.sync()
+    flat = cache.reshape(-1, 576)
+    for b in list(range(min(B, 12))) + [B - 1]:
+        if lens[b] == 0:
+            assert not got[b].any()
+            continue
+        one = flat[b * stride // 576:b * stride // 576 + lens[b]]
+        want = attn.mla_decode(q[b:b + 1], one, kv[b:b + 1], max_kv_len=lens[b], scale=192 ** -0.5)
+        attn.ctx.sync()
+        assert float((got[b].float() - want[0].float()).norm() / want.float().norm()) < 5e-3, (b, lens[b])
