@@ -1,4 +1,5 @@
-"""Builds libcwk_attn.so (every CUDA source under csrc/) for sm_100a with nvcc.
+"""Builds libcwk_attn.so (every CUDA source under csrc/) for sm_100a with nvcc, and _pycall.so, the CPython entry points
+of the decode calls (csrc/pycall.c), with the host compiler.
 
 The library is built in-tree next to this file so that it travels with the
 source tree; nothing is installed. `python -m cwick_b200.build` rebuilds it.
@@ -7,10 +8,12 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcwk_attn.so")
+PYCALL = os.path.join(HERE, "_pycall.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -28,10 +31,10 @@ def sources():
 
 
 def needs_build():
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(PYCALL):
         return True
-    t = os.path.getmtime(LIB)
-    deps = sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + \
+    t = min(os.path.getmtime(LIB), os.path.getmtime(PYCALL))
+    deps = sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + [os.path.join(CSRC, "pycall.c")] + \
         glob.glob(os.path.join(os.path.dirname(HERE), "include", "*.h"))
     return any(os.path.getmtime(d) > t for d in deps)
 
@@ -60,6 +63,8 @@ def build(force=False, verbose=False):
         raise RuntimeError("nvcc failed")
     cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-lcudart"]
     subprocess.check_call(cmd)
+    subprocess.check_call([os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
+                           os.path.join(CSRC, "pycall.c"), "-o", PYCALL, "-L" + HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"])
     return LIB
 
 

@@ -1,4 +1,5 @@
-"""ctypes binding of libcwk_attn.so -- the only way this package computes.
+"""Binding of libcwk_attn.so -- the only way this package computes: ctypes for every entry point, and a compiled module for
+the few that a decode step calls (`fast`).
 
 There is no CPU or eager fallback: if the shared library is missing or the
 process has no CUDA device, `load()` / `Context()` raise.
@@ -102,6 +103,17 @@ def load():
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def fast(lib, name):
+    """The entry point `name`, called with plain integers (addresses, sizes) and floats: through the compiled module where it
+    belongs to the loaded library and has the function, else through ctypes."""
+    if lib is _lib:
+        from . import _pycall
+        fn = getattr(_pycall, name, None)
+        if fn is not None:
+            return fn
+    return getattr(lib, name)
 
 
 class CwkError(RuntimeError):

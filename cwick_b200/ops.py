@@ -26,6 +26,10 @@ class Attn:
         self.device = device
         self.ctx = _lib.Context(device, stream=torch.cuda.current_stream(device).cuda_stream)
         self.lib = self.ctx.lib
+        self._h = self.ctx.h.value
+        # the calls of a decode step: plain integers and floats in, status out
+        self._mla_decode, self._gqa_decode, self._dsa_select, self._gdn_scan = (
+            _lib.fast(self.lib, "cwk_" + n) for n in ("mla_decode", "gqa_decode", "dsa_select", "gdn_scan"))
 
     # ---- MLA ---------------------------------------------------------------
     def mla_decode(self, q, cache, kv_len, max_kv_len=None, sel=None, scale=None, seq_stride=None,
@@ -45,10 +49,11 @@ class Attn:
             scale = 1.0 / math.sqrt(192.0 if R else L)
         if out is None:
             out = torch.empty(B, nh, L, dtype=torch.bfloat16, device=q.device)
-        sel_ld = sel.shape[-1] if sel is not None else 0
-        self.ctx.check(self.lib.cwk_mla_decode(self.ctx.h, _p(q), _p(cache), seq_stride, ld, _p(kv_len),
-                                               max_kv_len, _p(sel), sel_ld, B, nh, L, R, scale, _p(out),
-                                               n_splits))
+        st = self._mla_decode(self._h, q.data_ptr(), cache.data_ptr(), seq_stride, ld, kv_len.data_ptr(), max_kv_len,
+                              None if sel is None else sel.data_ptr(), 0 if sel is None else sel.shape[-1], B, nh, L, R, scale,
+                              out.data_ptr(), n_splits)
+        if st:
+            self.ctx.check(st)
         return out
 
     def mla_decode_dims(self, q, cache, kv_len, L, R, scale, max_kv_len=None, sel=None, seq_stride=None,
@@ -128,9 +133,11 @@ class Attn:
         sel = torch.full((B, want + 1), -1, dtype=torch.int32, device=keys.device)
         nsel = torch.zeros(B, dtype=torch.int32, device=keys.device)
         sc = torch.zeros(B, T, dtype=torch.float32, device=keys.device) if return_scores else None
-        self.ctx.check(self.lib.cwk_dsa_select(self.ctx.h, _p(keys), _p(kscale), T, _p(q), _p(wt), _p(n), max_n, B, ih, hd,
-                                               want, 1 if keep_self else 0, _p(sel), want + 1, _p(nsel),
-                                               _p(sc) if sc is not None else None))
+        st = self._dsa_select(self._h, keys.data_ptr(), kscale.data_ptr(), T, q.data_ptr(), wt.data_ptr(), n.data_ptr(), max_n, B, ih,
+                              hd, want, 1 if keep_self else 0, sel.data_ptr(), want + 1, nsel.data_ptr(),
+                              None if sc is None else sc.data_ptr())
+        if st:
+            self.ctx.check(st)
         return (sel, nsel, sc) if return_scores else (sel, nsel)
 
     # ---- GQA -----------------------------------------------------------------
@@ -145,8 +152,10 @@ class Attn:
             max_kv_len = int(kv_len.max().item())
         if out is None:
             out = torch.empty(B, nh, hd, dtype=torch.bfloat16, device=q.device)
-        self.ctx.check(self.lib.cwk_gqa_decode(self.ctx.h, _p(q), _p(K), _p(V), T * nkv * hd, _p(kv_len),
-                                               max_kv_len, B, nh, nkv, hd, scale, _p(out), n_splits))
+        st = self._gqa_decode(self._h, q.data_ptr(), K.data_ptr(), V.data_ptr(), T * nkv * hd, kv_len.data_ptr(), max_kv_len, B, nh, nkv,
+                              hd, scale, out.data_ptr(), n_splits)
+        if st:
+            self.ctx.check(st)
         return out
 
     def gqa_prefill(self, Q, K, V, pos, scale=None):
@@ -213,8 +222,10 @@ class Attn:
         B, n, _ = up.shape
         _, nh, hv, hk = S.shape
         out = torch.empty(B, n, nh * hv, dtype=torch.float32, device=up.device)
-        self.ctx.check(self.lib.cwk_gdn_scan(self.ctx.h, B, n, nh, hk, hv, kv_group, _p(up), _p(gdec), _p(beta), _p(gate), _p(a_log),
-                                             _p(dt_bias), _p(norm), rms_eps, _p(S), _p(out)))
+        st = self._gdn_scan(self._h, B, n, nh, hk, hv, kv_group, up.data_ptr(), gdec.data_ptr(), beta.data_ptr(), gate.data_ptr(),
+                            a_log.data_ptr(), dt_bias.data_ptr(), norm.data_ptr(), rms_eps, S.data_ptr(), out.data_ptr())
+        if st:
+            self.ctx.check(st)
         return out
 
     def mm_select(self, index_keys, iq, limit, block_size, topk_blocks, cap=4096):
