@@ -61,6 +61,9 @@ int cwk_check_cuda(cwk_ctx *ctx, cudaError_t e, const char *what);
 int cwk_reserve_scratch(cwk_ctx *ctx, size_t bytes);
 int cwk_reserve_stage(cwk_ctx *ctx, size_t dev_bytes, size_t pin_bytes);
 int cwk_reserve_work(cwk_ctx *ctx, size_t bytes);
+// Device buffers that go from one context to the next (cwk_ctx.cu).
+cudaError_t cwk_buffer_alloc(int device, size_t bytes, void **p, size_t *granted);
+void cwk_buffer_free(int device, void *p, size_t bytes);
 // After a stream synchronise: turn a kernel-side give-up code into CWK_ERR_STATE.
 int cwk_check_device_error(cwk_ctx *ctx);
 // Allocate the error word on first use: pinned, mapped host memory, so the host reads it without a copy.
@@ -110,6 +113,25 @@ struct CwkKernelTimer {
         int _s = cwk_check_cuda((ctx), cudaGetLastError(), name);      \
         if (_s != CWK_OK) return _s;                                   \
     } while (0)
+
+// ---- kernels of a decode step that may start before the one in front of them is done -----------------------------------
+// A decode step at small batch is a chain of kernels of a few microseconds, and half as much again is the time from one
+// kernel's end to the next one's first instruction. Launched this way, a kernel's blocks come up while the kernel before
+// still runs, set themselves up, and wait in cwk_pdl_wait() until that one is complete and its results are visible. Every
+// kernel launched this way calls cwk_pdl_wait() before it touches global memory that a kernel may have written, and
+// cwk_pdl_launch() to let the next one come up. (A kernel that never calls the latter lets it up when it ends: so other
+// kernels in the stream need know nothing of this.)
+template <class... K, class... A>
+static inline cudaError_t cwk_launch_early(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = &at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+__device__ __forceinline__ void cwk_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void cwk_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- device helpers ---------------------------------------------------------
 __device__ __forceinline__ float bf16_bits_to_f32(uint16_t b) {

@@ -358,6 +358,8 @@ static __global__ void __launch_bounds__(128) lse_merge_kernel(const float *part
     const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t rec_sz = (int64_t)nh * (D + 2);
     int64_t rec0 = (int64_t)b * nsplit;
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     if (meta) {                                   // a number of records of its own per sequence: {first, count}
         const int2 m = meta[b];
         rec0 = m.x;
@@ -424,13 +426,12 @@ static __global__ void __launch_bounds__(128) lse_merge_kernel(const float *part
 static inline void lse_combine_launch(cudaStream_t st, const float *partial, int nsplit, int nh, int D, int B,
                                       uint16_t *out) {
     const dim3 grid(nh, B, (D + 127) / 128);
-    if (nsplit > 32) lse_merge_kernel<false, 64><<<grid, 128, 0, st>>>(partial, nsplit, nh, D, out, nullptr);
-    else if (nsplit > 8) lse_merge_kernel<false, 32><<<grid, 128, 0, st>>>(partial, nsplit, nh, D, out, nullptr);
-    else lse_merge_kernel<false, 8><<<grid, 128, 0, st>>>(partial, nsplit, nh, D, out, nullptr);
+    auto kern = nsplit > 32 ? lse_merge_kernel<false, 64> : nsplit > 8 ? lse_merge_kernel<false, 32> : lse_merge_kernel<false, 8>;
+    (void)cwk_launch_early(kern, grid, dim3(128), 0, st, partial, nsplit, nh, D, out, (float *)nullptr, (const int2 *)nullptr);
 }
 // `meta[b]` = {first record, number of records} of sequence b, at most CWK_MAX_SPLITS of them
 static inline void lse_combine_ranges_launch(cudaStream_t st, const float *partial, const int2 *meta, int nh, int D, int B, uint16_t *out) {
-    lse_merge_kernel<false, 8><<<dim3(nh, B, (D + 127) / 128), 128, 0, st>>>(partial, 0, nh, D, out, nullptr, meta);
+    (void)cwk_launch_early(lse_merge_kernel<false, 8>, dim3(nh, B, (D + 127) / 128), dim3(128), 0, st, partial, 0, nh, D, out, (float *)nullptr, meta);
 }
 static inline void lse_fold_launch(cudaStream_t st, const float *partial, int nsplit, int nh, int D, float *rec_out) {
     const dim3 grid(nh, 1, (D + 127) / 128);

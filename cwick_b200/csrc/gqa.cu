@@ -1,6 +1,6 @@
-// gqa.cu -- Qwen3.5-style grouped-query attention: single-query decode
-// (split over the key range, merged by lse_merge_kernel) and causal prefill.
-// Both run flash_rows_kernel with K and V as separate streams.
+// gqa.cu -- Qwen3.5-style grouped-query attention: entry points of the single-query decode (gqa_decode.cu; more than eight
+// query heads per KV head: flash_rows_kernel, split over the key range and merged by lse_merge_kernel) and of causal prefill
+// (mla_prefill_attn.cu, or flash_rows_kernel with K and V as separate streams).
 #include <algorithm>
 #include <cmath>
 
@@ -37,6 +37,8 @@ static int gqa_prefill_launch(cwk_ctx *ctx, const FlashRowsParams &p, int nblock
     return CWK_OK;
 }
 
+int cwk_gqa_decode_streams(cwk_ctx *ctx, const void *q, const void *K, const void *V, int64_t seq_stride, const int32_t *kv_len, int max_kv_len,
+                           const int32_t *sel, int64_t sel_ld, int B, int nh, int nkv, int hd, float scale, void *out, int max_blocks);
 int cwk_gqa_prefill_tc(cwk_ctx *ctx, const void *Q, const void *K, const void *V, int64_t pos, int n, int nh, int nkv, int hd,
                        float scale, void *out, int *flags);
 
@@ -55,6 +57,10 @@ static int gqa_decode_impl(cwk_ctx *ctx, const void *q, const void *K, const voi
     if (((uintptr_t)K | (uintptr_t)V | (uintptr_t)q) % 16 != 0 || (seq_stride % 8) != 0)
         return cwk_fail(ctx, CWK_ERR_ARGUMENT, "gqa_decode: pointers must be 16-byte aligned");
     CWK_CUDA(ctx, cudaSetDevice(ctx->device));
+    // up to eight query heads per KV head: a warp's MMA columns (gqa_decode.cu); more take the row kernel below
+    if (group <= 8)
+        return cwk_gqa_decode_streams(ctx, q, K, V, seq_stride, kv_len, max_kv_len, sel, sel_ld, B, nh, nkv, hd, scale, out,
+                                      n_splits > 0 ? (int)std::min<int64_t>((int64_t)n_splits * B * nkv, 1 << 20) : 0);
     const int max_tiles = std::max(1, (max_kv_len + 63) / 64);
     int ns = n_splits > 0 ? std::min(std::min(n_splits, max_tiles), CWK_MAX_SPLITS) : 1;
     if (n_splits <= 0) {

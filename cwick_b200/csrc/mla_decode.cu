@@ -156,7 +156,7 @@ static int mla_launch(cwk_ctx *ctx, const void *q, const void *cache, int64_t se
     // A batch whose sequences have lengths of their own (known on the device only) and tiles enough for every SM: equal
     // shares of all tiles instead of equal numbers of splits per sequence, which make the longest sequence's blocks the
     // call's time and leave SMs without a block. A block that changes sequences pays about two tiles' time for it, so the
-    // shares have to be several tiles long. 64 sequences of 16384..32768 rows: MLA64OLD -> MLA64NEW us.
+    // shares have to be several tiles long. 64 sequences of 16384..32768 rows: 497 -> 434 us.
     if (path == 2 && !sel && kv_len && B > 1 && seq_stride != 0 && n_splits <= 0 && out && !partial_out && !ctx->keep_splits && ctx->sm_count <= CWK_MAX_SPLITS &&
         (int64_t)B * max_tiles >= 6 * (int64_t)ctx->sm_count) {
         const int G = ctx->sm_count;

@@ -177,6 +177,16 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int split = blockIdx.x;
+    cwk_pdl_launch();
+    if (tid == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_q) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_kv) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_kr) : "memory");
+        for (int i = 0; i < B_COUNT; i++)
+            mbar_init(bar(i), i == B_PFULL ? (uint32_t)NSOFT : (p.sel && i < B_EMPTY_L) ? (uint32_t)NSOFT : 1u);      // gather: 512 arrivals fill a block
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cwk_pdl_wait();
     // With few blocks in the launch (one short sequence), two blocks take each tile: both compute the tile's scores
     // and probabilities, each accumulates and writes one half of the value columns. Half the value MMAs per block,
     // and the records leave through twice as many SMs.
@@ -222,12 +232,6 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     };
 
     if (tid == 0) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_q) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_kv) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_kr) : "memory");
-        for (int i = 0; i < B_COUNT; i++)
-            mbar_init(bar(i), i == B_PFULL ? (uint32_t)NSOFT : (p.sel && i < B_EMPTY_L) ? (uint32_t)NSOFT : 1u);      // gather: 512 arrivals fill a block
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // A full wave of blocks with many tiles each: blocks that start together stay in lockstep for their first tiles
         // (every SM loads, then every SM computes, and HBM idles through the compute phases: 10 k cycles per tile against
         // 7 k once they have drifted apart), so eight groups of blocks start a fraction of a tile period apart.
@@ -680,8 +684,8 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
     p.B = B; p.seq_meta = seq_meta;
     if (seq_meta) {                    // range mode: nsplit = number of blocks
         p.halves = 1; p.stagger = 700;
-        mla_decode_tc_kernel<<<nsplit, NTHREADS, SMEM_TOTAL, ctx->stream>>>(*tm_q, *tm_kv, *tm_kr, p);
-        CWK_LAUNCH_CHECK(ctx, "mla_decode_tc_kernel");
+        CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel, dim3(nsplit), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
+        ctx->launches++;
         return CWK_OK;
     }
     p.halves = ((int64_t)nsplit * B * 2 <= ctx->sm_count) ? 2 : 1;
@@ -689,7 +693,7 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
         const int tiles_per_block = ((max_kv_len + TILE - 1) / TILE + nsplit - 1) / nsplit;
         p.stagger = ((int64_t)nsplit * B * 2 > ctx->sm_count && tiles_per_block >= 6) ? 700 : 0;
     }
-    mla_decode_tc_kernel<<<dim3(nsplit, B, p.halves), NTHREADS, SMEM_TOTAL, ctx->stream>>>(*tm_q, *tm_kv, *tm_kr, p);
-    CWK_LAUNCH_CHECK(ctx, "mla_decode_tc_kernel");
+    CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel, dim3(nsplit, B, p.halves), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
+    ctx->launches++;
     return CWK_OK;
 }

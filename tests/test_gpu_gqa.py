@@ -113,3 +113,26 @@ def test_prefill_last_row_equals_decode(attn):
         dec = attn.gqa_decode(Q[row:row + 1].contiguous(), K[None, :row + 1].contiguous(),
                               V[None, :row + 1].contiguous(), torch.tensor([row + 1], dtype=torch.int32).cuda())
         close(bf16_to_np(pre[row]), bf16_to_np(dec[0]), max_abs=4e-3)
+
+
+@pytest.mark.parametrize("hd", [256, 128])
+@pytest.mark.parametrize("nh,nkv", [(16, 4), (8, 1), (6, 2), (24, 3), (8, 8), (32, 2)])
+@pytest.mark.parametrize("lens", [[0, 17, 0, 1, 2500, 64, 0], [3, 3, 3], [0, 0], [5000]])
+def test_decode_streams_against_f32(attn, hd, nh, nkv, lens):
+    """Equal shares of all steps per block over sequences of any lengths (empty ones in front, between, behind), one, two or
+    four KV heads per block, one to eight query heads per KV head, and sixteen (the row kernel): against float32."""
+    B, T = len(lens), max(max(lens), 1)
+    g = torch.Generator(device="cuda").manual_seed(nh + T)
+    q = torch.randn(B, nh, hd, device="cuda", generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(B, T, nkv, hd, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    k[:, ::7] *= 3                                   # scores that outrun the first ones
+    got = attn.gqa_decode(q, k, v, torch.tensor(lens, dtype=torch.int32, device="cuda"), max_kv_len=T)
+    attn.ctx.sync()
+    for b in range(B):
+        if lens[b] == 0:
+            assert not got[b].any()
+            continue
+        kk, vv = (x[b, :lens[b]].float().repeat_interleave(nh // nkv, 1) for x in (k, v))
+        s = torch.einsum("hd,thd->ht", q[b].float(), kk) / hd ** 0.5
+        want = torch.einsum("ht,thd->hd", torch.softmax(s, -1), vv)
+        assert float((got[b].float() - want).norm() / want.norm()) < 5e-3, b
