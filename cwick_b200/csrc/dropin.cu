@@ -23,6 +23,9 @@
 int cwk_mla_decode_rows(cwk_ctx *ctx, const void *q, const void *cache, int64_t ld, int rows, int nh, int L, int R,
                         float scale, void *out);
 
+// one sequence's attention left as split records in the context's scratch
+int cwk_mla_launch_splits(cwk_ctx *ctx, const void *q, const void *cache, int64_t ld, int rows, int nh, int L, int R, float scale, float **partial_out,
+                          int *nsplit_out);
 int cwk_mla_decode(cwk_ctx *ctx, const void *q, const void *cache, int64_t seq_stride, int64_t ld, const int32_t *kv_len,
                    int max_kv_len, const int32_t *sel, int64_t sel_ld, int B, int nh, int L, int R, float scale, void *out,
                    int n_splits);
@@ -576,6 +579,8 @@ void dev_linear(cwk_ctx *ctx, const WeightMirror *w, const float *x, float *y, i
     launch_gemv(ctx, kind, w->data, w->scales, x, y, w->rows, w->cols, n, ldx, ldy);
 }
 
+#include "token_step.cuh"
+
 // Values of a small vector tensor as f32 on the device (cwick_tensor_value, src/tensor.c:767-774).
 float *mirror_vector_f32(const cwkc_tensor *t, int64_t n) {
     if (!t || !t->data) return nullptr;
@@ -716,6 +721,39 @@ int sync_indexer(cwk_ctx *ctx, Layer &ly) {
     return CWK_OK;
 }
 
+// The chain of token_step.cuh takes a layer of whole 16-byte rows with a latent of 512 and value heads of 128.
+bool token_chain_ok(const Layer &ly, const float *d_x) {
+    return ly.qa->kind == ly.kva->kind && ly.qa->cols == ly.kva->cols && gemv_token_ok(ly.qa, d_x) && gemv_token_ok(ly.kva, d_x) && gemv_token_ok(ly.qb, d_x) &&
+           gemv_token_ok(ly.o, d_x) && (ly.H | ly.q_lora | ly.kv_lora) % 4 == 0 && ly.q_lora <= 12288 && ly.nh * (int64_t)ly.nope % 4 == 0 && ly.kv_lora == 512 &&
+           ly.vdim == 128 && (reinterpret_cast<uintptr_t>(ly.kvb->data) & 15) == 0;
+}
+int token_chain(cwk_ctx *ctx, Layer &ly, int64_t pos, const float *d_x, float *d_qa, float *d_q, float *d_kva, float *d_attn, uint16_t *d_qabs, void *a_row,
+                float *a_out) {
+    const int nh = ly.nh, nope = ly.nope, kv_lora = ly.kv_lora, kv_dim = ly.kv_dim;
+    auto weights = [](const WeightMirror *w) {
+        return Prefetch{w->data, (size_t)w->rows * w->cols * (w->kind == CWKC_WEIGHT_BF16 ? 2 : w->kind == CWKC_WEIGHT_F32 ? 4 : 1)};
+    };
+    const Prefetch none{nullptr, 0};
+    uint16_t *row = ly.cm->dev + (size_t)pos * kv_lora;
+    CWK_CUDA(ctx, gemv_token(ctx, ly.qa, d_x, d_qa, ly.kva, d_kva, nullptr, weights(ly.qb), weights(ly.kvb)));
+    const TokenNorm nm{ly.qa_n, ly.kva_n, ly.spec->rms_norm_eps_f, d_kva, kv_lora, row, a_row, ly.lbf ? 1 : 0};
+    CWK_CUDA(ctx, gemv_token(ctx, ly.qb, d_qa, d_q, nullptr, nullptr, &nm, none, none));
+    CWK_CUDA(ctx, cwk_launch_early(absorb_token_kernel, dim3(nh, kv_lora / 256), dim3(512), 0, ctx->stream, (const float *)d_q, (const uint16_t *)ly.kvb->data, nope, kv_dim,
+                                   kv_lora, d_qabs));
+    float *partial = nullptr;
+    int nsplit = 0;
+    const Prefetch wo = weights(ly.o);
+    ctx->prefetch = wo.p; ctx->prefetch_bytes = wo.bytes;              // (the attention's bytes are few: HBM is free for o_proj's)
+    const int s = cwk_mla_launch_splits(ctx, d_qabs, ly.cm->dev, kv_lora, (int)(pos + 1), nh, kv_lora, 0, 1.0f / sqrtf((float)nope), &partial, &nsplit);
+    ctx->prefetch = nullptr; ctx->prefetch_bytes = 0;
+    if (s != CWK_OK) return s;
+    CWK_CUDA(ctx, cwk_launch_early(merge_unabsorb_kernel, dim3(nh, 2), dim3(512), 0, ctx->stream, (const float *)partial, nsplit, nh, (const uint16_t *)ly.kvb->data, nope,
+                                   d_attn));
+    ctx->launches += 2;
+    CWK_CUDA(ctx, gemv_token(ctx, ly.o, d_attn, a_out, nullptr, nullptr, nullptr, none, none));
+    return CWK_OK;
+}
+
 // One token of one layer, the reference's mla_latent_decode (src/attention.c:642-902) stage by stage on the device.
 // x_host/out_host: H floats each. Returns a cwk status; the message goes to err.
 int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const float *x_host, float *out_host, cwkc_error *err) {
@@ -751,6 +789,12 @@ int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const flo
     float *a_out = pin_dev ? (float *)(pin_dev + ((uint8_t *)p_out - (uint8_t *)g.pin)) : nullptr;
     memcpy(p_x, x_host, (size_t)H * 4);
     cudaMemcpyAsync(d_x, p_x, (size_t)H * 4, cudaMemcpyHostToDevice, st);
+    int64_t nlist = pos + 1;
+    bool use_sel = false;
+    if (!ly.idx && a_row && a_out && token_chain_ok(ly, d_x)) {
+        s = token_chain(ctx, ly, pos, d_x, d_qa, d_q, d_kva, d_attn, d_qabs, a_row, a_out);
+        if (s != CWK_OK) { set_err(err, s, "%s", cwk_last_error(ctx)); return s; }
+    } else {
     if (ly.qa->kind == ly.kva->kind && ly.qa->cols == ly.kva->cols) {      // q_a and kv_a read the same x: one launch
         const int kind = ly.qa->kind == CWKC_WEIGHT_BF16 ? GEMV_BF16 : ly.qa->kind == CWKC_WEIGHT_F32 ? GEMV_F32 : GEMV_FP8;
         launch_gemv(ctx, kind, ly.qa->data, ly.qa->scales, d_x, d_qa, ly.qa->rows, ly.qa->cols, 1, 0, 0, ly.kva->data, ly.kva->scales, d_kva,
@@ -771,8 +815,6 @@ int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const flo
     ctx->launches += 2;
 
     // ---- DSA indexer (src/attention.c:716-735): absorb this position, then pick the rows to attend to ----
-    int64_t nlist = pos + 1;
-    bool use_sel = false;
     if (ly.idx) {
         cwkc_indexer_state *ist = ly.idx;
         IndexMirror &im = *ly.im;
@@ -852,6 +894,7 @@ int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const flo
     else {
         dev_linear(ctx, ly.o, d_attn, d_out, 1, 0, 0);
         cudaMemcpyAsync(p_out, d_out, (size_t)H * 4, cudaMemcpyDeviceToHost, st);
+    }
     }
     if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
         set_err(err, CWK_ERR_CUDA, "GPU decode failed: %s", cudaGetErrorString(cudaGetLastError()));
