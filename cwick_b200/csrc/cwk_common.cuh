@@ -36,9 +36,6 @@ struct cwk_ctx {
     int force_mla_path = -1;
     bool keep_splits = false;   // internal: leave split records in scratch (no merge, no fold)
     int last_nsplit = 0;
-    // internal: a range that the MLA decode kernel tells L2 to fetch while it runs (the weights that come next)
-    const void *prefetch = nullptr;
-    size_t prefetch_bytes = 0;
     // optional event pairs around main kernels (cwk_ctx_profile)
     bool profiling = false;
     std::vector<cudaEvent_t> ev;      // pool, pairs (2i, 2i+1)

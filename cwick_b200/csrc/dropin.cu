@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256) gemv_bf16_kernel(const uint16_t *W, const
 
 // In place: x <- x / sqrt(mean(x^2) + eps) * w (cwick_rms_norm + apply_bf16_vec, src/tensor.c:780-791,
 // src/attention.c:70-73), one block per row (blockIdx.x). Optionally also narrows the result to bf16 the way the
-// reference narrows a latent-cache row (src/util.c:202-210) into row_out + row * row_ld.
+// reference narrows a latent-cache row (src/util.c:202-210) into row_out + row * row_ld. Threads 0 .. 255 of a block.
 __device__ __forceinline__ void rms_scale_row(float *x, int n, const uint16_t *w, float eps, uint16_t *row_out, void *host_row, int host_bf16) {
     __shared__ double red[8];
     double ss = 0.0;
@@ -249,7 +249,7 @@ __device__ __forceinline__ void rms_scale_row(float *x, int n, const uint16_t *w
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    __syncthreads();
+    asm volatile("bar.sync 1, 256;" ::: "memory");         // (the calling block may have other threads)
     const double tot = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
     const float inv = __fdiv_rn(1.0f, (float)sqrt(tot / (double)n + (double)eps));
     for (int i = threadIdx.x; i < n; i += 256) {
@@ -722,35 +722,32 @@ int sync_indexer(cwk_ctx *ctx, Layer &ly) {
 }
 
 // The chain of token_step.cuh takes a layer of whole 16-byte rows with a latent of 512 and value heads of 128.
-bool token_chain_ok(const Layer &ly, const float *d_x) {
-    return ly.qa->kind == ly.kva->kind && ly.qa->cols == ly.kva->cols && gemv_token_ok(ly.qa, d_x) && gemv_token_ok(ly.kva, d_x) && gemv_token_ok(ly.qb, d_x) &&
-           gemv_token_ok(ly.o, d_x) && (ly.H | ly.q_lora | ly.kv_lora) % 4 == 0 && ly.q_lora <= 12288 && ly.nh * (int64_t)ly.nope % 4 == 0 && ly.kv_lora == 512 &&
-           ly.vdim == 128 && (reinterpret_cast<uintptr_t>(ly.kvb->data) & 15) == 0;
+bool token_chain_ok(const cwk_ctx *ctx, const Layer &ly) {
+    return ly.qa->kind == ly.kva->kind && ly.qa->cols == ly.kva->cols && gemv_token_ok(ctx, ly.qa) && gemv_token_ok(ctx, ly.kva) && gemv_token_ok(ctx, ly.qb) &&
+           gemv_token_ok(ctx, ly.o) && (ly.H | ly.q_lora | ly.kv_lora) % 4 == 0 && ly.q_lora <= 8192 && ly.nh * (int64_t)ly.vdim <= 8192 && ly.nh * (int64_t)ly.nope % 4 == 0 &&
+           ly.kv_lora == 512 && ly.vdim == 128 && (reinterpret_cast<uintptr_t>(ly.kvb->data) & 15) == 0;
 }
+// d_attn: two parts of nh * 128 values
 int token_chain(cwk_ctx *ctx, Layer &ly, int64_t pos, const float *d_x, float *d_qa, float *d_q, float *d_kva, float *d_attn, uint16_t *d_qabs, void *a_row,
                 float *a_out) {
     const int nh = ly.nh, nope = ly.nope, kv_lora = ly.kv_lora, kv_dim = ly.kv_dim;
-    auto weights = [](const WeightMirror *w) {
-        return Prefetch{w->data, (size_t)w->rows * w->cols * (w->kind == CWKC_WEIGHT_BF16 ? 2 : w->kind == CWKC_WEIGHT_F32 ? 4 : 1)};
-    };
-    const Prefetch none{nullptr, 0};
-    uint16_t *row = ly.cm->dev + (size_t)pos * kv_lora;
-    CWK_CUDA(ctx, gemv_token(ctx, ly.qa, d_x, d_qa, ly.kva, d_kva, nullptr, weights(ly.qb), weights(ly.kvb)));
-    const TokenNorm nm{ly.qa_n, ly.kva_n, ly.spec->rms_norm_eps_f, d_kva, kv_lora, row, a_row, ly.lbf ? 1 : 0};
-    CWK_CUDA(ctx, gemv_token(ctx, ly.qb, d_qa, d_q, nullptr, nullptr, &nm, none, none));
+    TokenInput in{};
+    in.x = d_x;
+    CWK_CUDA(ctx, gemv_token(ctx, ly.qa, d_qa, ly.kva, d_kva, X_PLAIN, in));
+    in = TokenInput{d_qa, nullptr, ly.qa_n, ly.kva_n, ly.spec->rms_norm_eps_f, d_kva, kv_lora, ly.cm->dev + (size_t)pos * kv_lora, a_row, ly.lbf ? 1 : 0};
+    CWK_CUDA(ctx, gemv_token(ctx, ly.qb, d_q, nullptr, nullptr, X_NORM, in));
     CWK_CUDA(ctx, cwk_launch_early(absorb_token_kernel, dim3(nh, kv_lora / 256), dim3(512), 0, ctx->stream, (const float *)d_q, (const uint16_t *)ly.kvb->data, nope, kv_dim,
                                    kv_lora, d_qabs));
     float *partial = nullptr;
     int nsplit = 0;
-    const Prefetch wo = weights(ly.o);
-    ctx->prefetch = wo.p; ctx->prefetch_bytes = wo.bytes;              // (the attention's bytes are few: HBM is free for o_proj's)
     const int s = cwk_mla_launch_splits(ctx, d_qabs, ly.cm->dev, kv_lora, (int)(pos + 1), nh, kv_lora, 0, 1.0f / sqrtf((float)nope), &partial, &nsplit);
-    ctx->prefetch = nullptr; ctx->prefetch_bytes = 0;
     if (s != CWK_OK) return s;
     CWK_CUDA(ctx, cwk_launch_early(merge_unabsorb_kernel, dim3(nh, 2), dim3(512), 0, ctx->stream, (const float *)partial, nsplit, nh, (const uint16_t *)ly.kvb->data, nope,
                                    d_attn));
     ctx->launches += 2;
-    CWK_CUDA(ctx, gemv_token(ctx, ly.o, d_attn, a_out, nullptr, nullptr, nullptr, none, none));
+    in = TokenInput{};
+    in.x = d_attn; in.x2 = d_attn + nh * 128;
+    CWK_CUDA(ctx, gemv_token(ctx, ly.o, a_out, nullptr, nullptr, X_SUM, in));
     return CWK_OK;
 }
 
@@ -764,13 +761,13 @@ int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const flo
     // floats: x[H] qa[q_lora] q[nh*nope] kva[kv_lora] attn[nh*vdim] out[H] iq[ih*ihd] iwt[ih] isc[pool_cap] | bf16: qabs, cacc | int32: sel
     const int64_t pool_cap = ly.idx ? ly.idx->pool_cap : 0;
     const int64_t topk = ly.idx ? ly.spec->index_topk : 0;
-    const size_t nf = (size_t)H * 2 + q_lora + (size_t)nh * nope + kv_lora + (size_t)nh * vdim + (size_t)ih * ihd + ih + pool_cap + 64;
+    const size_t nf = (size_t)H * 2 + q_lora + (size_t)nh * nope + kv_lora + (size_t)2 * nh * vdim + (size_t)ih * ihd + ih + pool_cap + 64;
     const size_t nsel = (size_t)topk + kp + 4;
     const size_t need = nf * 4 + (size_t)nh * kv_lora * 2 * 2 + nsel * 4 + 512;
     const size_t pin_need = (size_t)H * 4 * 2 + (size_t)kv_lora * 4 + (size_t)(2 * ihd + ih * ihd + ih + pool_cap) * 4 + nsel * 4 + 256;
     if (!ensure_bufs(need, pin_need, err)) return CWK_ERR_MEMORY;
     float *d_x = g.d_buf, *d_qa = d_x + H, *d_q = d_qa + q_lora, *d_kva = d_q + (size_t)nh * nope;
-    float *d_attn = d_kva + kv_lora, *d_out = d_attn + (size_t)nh * vdim, *d_iq = d_out + H, *d_iwt = d_iq + (size_t)ih * ihd;
+    float *d_attn = d_kva + kv_lora, *d_out = d_attn + (size_t)2 * nh * vdim, *d_iq = d_out + H, *d_iwt = d_iq + (size_t)ih * ihd;
     float *d_isc = d_iwt + ih;
     uint16_t *d_qabs = (uint16_t *)(((uintptr_t)(d_isc + pool_cap) + 63) & ~(uintptr_t)63), *d_cacc = d_qabs + (size_t)nh * kv_lora;
     int32_t *d_sel = (int32_t *)(d_cacc + (size_t)nh * kv_lora);
@@ -791,7 +788,7 @@ int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const flo
     cudaMemcpyAsync(d_x, p_x, (size_t)H * 4, cudaMemcpyHostToDevice, st);
     int64_t nlist = pos + 1;
     bool use_sel = false;
-    if (!ly.idx && a_row && a_out && token_chain_ok(ly, d_x)) {
+    if (!ly.idx && a_row && a_out && token_chain_ok(ctx, ly)) {
         s = token_chain(ctx, ly, pos, d_x, d_qa, d_q, d_kva, d_attn, d_qabs, a_row, a_out);
         if (s != CWK_OK) { set_err(err, s, "%s", cwk_last_error(ctx)); return s; }
     } else {

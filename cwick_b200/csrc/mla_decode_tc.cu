@@ -105,8 +105,6 @@ struct TcParams {
     const uint16_t *cache;
     int64_t seq_stride, ld;
     int rope_cols;         // 64, or 0: the ninth block is zeros
-    const uint8_t *prefetch;      // a range for L2, each block a share of it
-    size_t prefetch_share, prefetch_bytes;
     // Range mode (B > 0; seq_meta set): the tiles of all B sequences, one after another, are dealt out in equal contiguous
     // ranges, one per block (blockIdx.x): a block may end one sequence and begin the next, and every block has the same
     // number of tiles whatever the sequences' lengths. The record of sequence b from block g goes to slot b + g (along the
@@ -280,13 +278,6 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #define TRACE(role, it, ev) do { } while (0)
 #endif
 
-    if (warp == 3 && lane == 0 && p.prefetch_share) {      // (this block's own tile has been asked for)
-        const size_t blk = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-        size_t at = blk * p.prefetch_share;
-        const size_t end = min(at + p.prefetch_share, p.prefetch_bytes & ~(size_t)15);
-        for (; at < end; at += 65536)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.prefetch + at), "r"((uint32_t)min(end - at, (size_t)65536)) : "memory");
-    }
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (lane == 0 && !p.sel) {
@@ -691,7 +682,6 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
     p.sel = sel; p.sel_ld = sel_ld; p.cache = (const uint16_t *)cache; p.seq_stride = seq_stride; p.ld = ld; p.rope_cols = R;
     p.reverse_b = shared_cache ? 1 : 0;
     p.B = B; p.seq_meta = seq_meta;
-    p.prefetch = nullptr; p.prefetch_share = p.prefetch_bytes = 0;
     if (seq_meta) {                    // range mode: nsplit = number of blocks
         p.halves = 1; p.stagger = 700;
         CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel, dim3(nsplit), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
@@ -702,11 +692,6 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
     {
         const int tiles_per_block = ((max_kv_len + TILE - 1) / TILE + nsplit - 1) / nsplit;
         p.stagger = ((int64_t)nsplit * B * 2 > ctx->sm_count && tiles_per_block >= 6) ? 700 : 0;
-    }
-    if (ctx->prefetch_bytes) {
-        const size_t blocks = (size_t)nsplit * B * p.halves;
-        p.prefetch = (const uint8_t *)ctx->prefetch; p.prefetch_bytes = ctx->prefetch_bytes;
-        p.prefetch_share = ((ctx->prefetch_bytes + blocks - 1) / blocks + 15) & ~(size_t)15;
     }
     CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel, dim3(nsplit, B, p.halves), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
     ctx->launches++;

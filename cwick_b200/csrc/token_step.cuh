@@ -5,33 +5,23 @@
 // chain of eight kernels adds to that is latency -- a kernel comes up, asks for its first bytes, waits a microsecond, and at
 // its end HBM idles until the next one has done the same (100 us per call). So here every kernel (1) comes up while the one
 // before still runs (cwk_launch_early) and asks for its first weights, which depend on nothing, before it waits for its
-// activations; (2) the first projection and the attention, which leave HBM idle, tell L2 to fetch the weights that are next
-// (`Prefetch`); and (3) small steps ride along: the two norms in the q_b projection's blocks, the merge of the attention's
-// split records in the un-absorb.
+// activations; and (2) small steps ride along: the two norms in the q_b projection's blocks, the merge of the attention's
+// split records in the un-absorb. (Telling L2 from the first projection and from the attention to fetch the weights that
+// come next made a call 1 to 3 us longer.)
 #pragma once
 
-struct Prefetch {               // a range to bring into L2, dealt out to a grid's blocks
-    const void *p;
-    size_t bytes;
-};
-// One thread of every block; 16-byte units, at most 64 KB per instruction.
-__device__ __forceinline__ void prefetch_share(const Prefetch &f, int block, int blocks) {
-    if (!f.bytes) return;
-    const size_t share = ((f.bytes + blocks - 1) / blocks + 15) & ~(size_t)15;
-    size_t at = (size_t)block * share;
-    const size_t end = at + share < f.bytes ? at + share : (f.bytes & ~(size_t)15);
-    while (at < end) {
-        const uint32_t n = (uint32_t)(end - at < 65536 ? end - at : 65536);
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const uint8_t *)f.p + at), "r"(n) : "memory");
-        at += n;
-    }
-}
-
-// y[r] = W[r] . x for one token (as gemv_rows_kernel, rows of whole 16-byte pieces only). NORM: x is first normalised,
-// x / sqrt(mean(x^2) + eps) * w, by every block for itself (its values in shared memory, the sum in rms_scale_row's order);
-// the launch's last block then is not a projection block but does the kv_a row: normalised in place, narrowed into the
-// cache row and written to the caller's staging.
-struct TokenNorm {
+// y[r] = W[r] . x for one token (as gemv_rows_kernel, rows of whole 16-byte pieces only). The grid is what fits on the SMs at
+// once, two blocks of sixteen warps each, and a block goes through a contiguous range of rows: with a block per few rows, a
+// second wave of blocks came up in the middle of every projection, each asking for its first bytes anew (q_b 12 us, now 6).
+// wpr warps share a pair of rows, so that an activation read from shared memory or L1 meets two weights (at one, those
+// reads take as long as HBM needs for the weights), chosen so that the rounds come out even. A block's results leave together: the
+// last projection's go to host memory, and a row of its own is a bus transaction of four bytes.
+// What x is: X_PLAIN as it is; X_NORM x / sqrt(mean(x^2) + eps) * w, worked out by every block for itself; X_SUM x + x2. In the
+// last two the values are kept in shared memory. X_NORM: the launch's last block is not a projection block but does the
+// kv_a row: normalised in place, narrowed into the cache row and written to the caller's staging.
+enum { X_PLAIN = 0, X_NORM = 1, X_SUM = 2 };
+struct TokenInput {
+    const float *x, *x2;
     const uint16_t *w, *wkv;
     float eps;
     float *kva;
@@ -40,90 +30,144 @@ struct TokenNorm {
     void *host_row;
     int host_bf16;
 };
-template <int KIND, bool NORM>
-__global__ void __launch_bounds__(256) gemv_token_kernel(const void *Wv, const float *scales, const float *x, float *y, int rows, int k, int rpb, int nb1,
-                                                         const void *W2, const float *scales2, float *y2, int rows2, const TokenNorm nm, const Prefetch f0,
-                                                         const Prefetch f1) {
-    constexpr int E = KIND == GEMV_BF16 ? 8 : KIND == GEMV_F32 ? 4 : 16, EB = 16 / E, AHEAD = 8;
+constexpr int TG_WARPS = 16, TG_MAX_ROWS = 512;      // rows per block (a block's results wait in shared memory)
+template <int KIND, int XIN>
+__global__ void __launch_bounds__(32 * TG_WARPS, 2) gemv_token_kernel(const void *Wv, const float *scales, float *y, int rows, int k, int wpr, int blocks,
+                                                                     const void *W2, const float *scales2, float *y2, int rows2, const TokenInput in) {
+    constexpr int E = KIND == GEMV_BF16 ? 8 : KIND == GEMV_F32 ? 4 : 16, EB = 16 / E, AHEAD = 4;
     extern __shared__ __align__(16) float s_x[];
-    __shared__ float s_part[8];
+    __shared__ float s_part[2][TG_WARPS][2], s_y[TG_MAX_ROWS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     cwk_pdl_launch();
-    if (NORM && blockIdx.x == gridDim.x - 1) {
+    if (XIN == X_NORM && blockIdx.x == blocks) {
         cwk_pdl_wait();
-        rms_scale_row(nm.kva, nm.nkv, nm.wkv, nm.eps, nm.row_out, nm.host_row, nm.host_bf16);
+        if (threadIdx.x < 256) rms_scale_row(in.kva, in.nkv, in.wkv, in.eps, in.row_out, in.host_row, in.host_bf16);
         return;
     }
-    const int wpr = 8 / rpb;                               // warps per row
-    int bx = blockIdx.x;
-    if (bx >= nb1) { bx -= nb1; Wv = W2; scales = scales2; y = y2; rows = rows2; }
-    const int r = bx * rpb + warp / wpr, part = warp % wpr;
-    const bool live = r < rows;
-    const uint8_t *w = reinterpret_cast<const uint8_t *>(Wv) + (int64_t)(live ? r : 0) * k * EB;
-    const float *sc = KIND == GEMV_FP8 ? scales + (int64_t)((live ? r : 0) / 128) * ((k + 127) / 128) : nullptr;
+    const int slots = TG_WARPS / wpr, slot = warp / wpr, part = warp % wpr;      // pairs at a time; this warp's pair and share of it
     const int step = wpr * 32 * E, j0 = (part * 32 + lane) * E;
-    uint4 v[AHEAD];
+    const int all = rows + rows2, lo = (int)((int64_t)all * blockIdx.x / blocks), hi = (int)((int64_t)all * (blockIdx.x + 1) / blocks);
+    uint4 v[2][AHEAD];
+    const uint8_t *w[2] = {nullptr, nullptr};
+    const float *sc[2] = {nullptr, nullptr};
+    int r = lo + 2 * slot;
+    auto ask = [&]() {                                     // the first pieces of rows r and r + 1 (an odd last one twice)
+        if (r >= hi) return;
 #pragma unroll
-    for (int u = 0; u < AHEAD; u++)
-        if (j0 + u * step < k) v[u] = ld_weight16(w + (int64_t)(j0 + u * step) * EB);
-    if ((lane & 7) == 0)                                   // the row's further lines on their way to L2
-        for (int j = j0 + AHEAD * step; j < k; j += step) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (int64_t)j * EB));
-    if (threadIdx.x == 0) {
-        prefetch_share(f0, blockIdx.x, gridDim.x);
-        prefetch_share(f1, blockIdx.x, gridDim.x);
-    }
+        for (int i = 0; i < 2; i++) {
+            const int q = min(r + i, hi - 1);
+            const bool second = q >= rows;
+            const int rr = second ? q - rows : q;
+            w[i] = reinterpret_cast<const uint8_t *>(second ? W2 : Wv) + (int64_t)rr * k * EB;
+            if (KIND == GEMV_FP8) sc[i] = (second ? scales2 : scales) + (int64_t)(rr / 128) * ((k + 127) / 128);
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++)
+                if (j0 + u * step < k) v[i][u] = ld_weight16(w[i] + (int64_t)(j0 + u * step) * EB);
+        }
+    };
+    ask();
     cwk_pdl_wait();
-    if (NORM) {
-        for (int i = threadIdx.x; i < k; i += 256) s_x[i] = x[i];      // (each thread scales what it read)
-        rms_scale_row(s_x, k, nm.w, nm.eps, nullptr, nullptr, 0);
+    const float *x = in.x;
+    if (XIN == X_NORM) {
+        __shared__ double s_ss[TG_WARPS];
+        double ss = 0.0;
+        for (int i = threadIdx.x; i < k; i += 32 * TG_WARPS) {
+            const float f = x[i];
+            s_x[i] = f;                                    // (each thread scales what it wrote)
+            ss += (double)f * (double)f;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) s_ss[warp] = ss;
+        __syncthreads();
+        double tot = s_ss[lane & (TG_WARPS - 1)];
+#pragma unroll
+        for (int o = TG_WARPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        const float inv = __fdiv_rn(1.0f, (float)sqrt(tot / (double)k + (double)in.eps));
+        for (int i = threadIdx.x; i < k; i += 32 * TG_WARPS) s_x[i] = s_x[i] * inv * bf16_bits_to_f32(in.w[i]);
+        __syncthreads();
+        x = s_x;
+    } else if (XIN == X_SUM) {
+        for (int i = threadIdx.x * 4; i < k; i += 128 * TG_WARPS) {
+            float4 a = *reinterpret_cast<const float4 *>(x + i);
+            const float4 b = *reinterpret_cast<const float4 *>(in.x2 + i);
+            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+            *reinterpret_cast<float4 *>(s_x + i) = a;
+        }
         __syncthreads();
         x = s_x;
     }
-    float acc = 0.f;
-    int j = j0;
+    for (int it = 0; lo + it * 2 * slots < hi; it++) {     // (every warp of a block goes round as often)
+        float acc[2] = {0.f, 0.f};
+        const int row = r;
+        if (r < hi) {
 #pragma unroll
-    for (int u = 0; u < AHEAD; u++)
-        if (j0 + u * step < k) acc += gemv_piece<KIND>(v[u], x, j0 + u * step, sc);
-    for (j = j0 + AHEAD * step; j + (AHEAD - 1) * step < k; j += AHEAD * step) {
+            for (int u = 0; u < AHEAD; u++)
+                if (j0 + u * step < k) {
+                    acc[0] += gemv_piece<KIND>(v[0][u], x, j0 + u * step, sc[0]);
+                    acc[1] += gemv_piece<KIND>(v[1][u], x, j0 + u * step, sc[1]);
+                }
+            for (int j = j0 + AHEAD * step; j < k; j += AHEAD * step) {
 #pragma unroll
-        for (int u = 0; u < AHEAD; u++) v[u] = ld_weight16(w + (int64_t)(j + u * step) * EB);
+                for (int u = 0; u < AHEAD; u++)
+                    if (j + u * step < k) {
+                        v[0][u] = ld_weight16(w[0] + (int64_t)(j + u * step) * EB);
+                        v[1][u] = ld_weight16(w[1] + (int64_t)(j + u * step) * EB);
+                    }
 #pragma unroll
-        for (int u = 0; u < AHEAD; u++) acc += gemv_piece<KIND>(v[u], x, j + u * step, sc);
+                for (int u = 0; u < AHEAD; u++)
+                    if (j + u * step < k) {
+                        acc[0] += gemv_piece<KIND>(v[0][u], x, j + u * step, sc[0]);
+                        acc[1] += gemv_piece<KIND>(v[1][u], x, j + u * step, sc[1]);
+                    }
+            }
+        }
+        r += 2 * slots;
+        ask();                                             // the next pair's pieces, under this one's sums
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+            acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], o);
+        }
+        if (wpr > 1) {
+            if (lane == 0) { s_part[it & 1][warp][0] = acc[0]; s_part[it & 1][warp][1] = acc[1]; }
+            __syncthreads();
+            acc[0] = acc[1] = 0.f;
+            for (int i = 0; i < wpr; i++) { acc[0] += s_part[it & 1][slot * wpr + i][0]; acc[1] += s_part[it & 1][slot * wpr + i][1]; }
+        }
+        if (part == 0 && lane < 2 && row + lane < hi) s_y[row + lane - lo] = acc[lane];
     }
-    for (; j < k; j += step) acc += gemv_piece<KIND>(ld_weight16(w + (int64_t)j * EB), x, j, sc);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (wpr == 1) {
-        if (lane == 0 && live) y[r] = acc;
-        return;
-    }
-    if (lane == 0) s_part[warp] = acc;
     __syncthreads();
-    if (part == 0 && lane == 0 && live) {
-        float sum = 0.f;
-        for (int i = 0; i < wpr; i++) sum += s_part[warp + i];
-        y[r] = sum;
-    }
+    for (int i = threadIdx.x; i < hi - lo; i += 32 * TG_WARPS) (lo + i < rows ? y[lo + i] : y2[lo + i - rows]) = s_y[i];
 }
-bool gemv_token_ok(const WeightMirror *w, const void *x) {
+bool gemv_token_ok(const cwk_ctx *ctx, const WeightMirror *w) {
     const int E = w->kind == CWKC_WEIGHT_BF16 ? 8 : w->kind == CWKC_WEIGHT_F32 ? 4 : 16;
-    return w->cols % E == 0 && ((reinterpret_cast<uintptr_t>(w->data) | reinterpret_cast<uintptr_t>(x)) & 15) == 0 && w->rows < (1 << 30);
+    return w->cols % E == 0 && (reinterpret_cast<uintptr_t>(w->data) & 15) == 0 && w->rows <= (int64_t)TG_MAX_ROWS * ctx->sm_count;
 }
-// w2 != NULL: a second matrix of the same kind and width, in the same launch. norm != NULL: NORM (no second matrix).
-cudaError_t gemv_token(cwk_ctx *ctx, const WeightMirror *w, const float *x, float *y, const WeightMirror *w2, float *y2, const TokenNorm *norm, Prefetch f0, Prefetch f1) {
-    int rpb = 8;                                           // fewer rows per block until the grid is a few blocks per SM
-    const int64_t rows2 = w2 ? w2->rows : 0;
-    while (rpb > 1 && (w->rows + rpb - 1) / rpb + (rows2 + rpb - 1) / rpb < 4 * (int64_t)ctx->sm_count) rpb >>= 1;
-    const int nb1 = (int)((w->rows + rpb - 1) / rpb), nb2 = (int)((rows2 + rpb - 1) / rpb);
-    const TokenNorm nm = norm ? *norm : TokenNorm{};
+// w2 != NULL: a second matrix of the same kind and width, in the same launch (X_PLAIN).
+cudaError_t gemv_token(cwk_ctx *ctx, const WeightMirror *w, float *y, const WeightMirror *w2, float *y2, int xin, const TokenInput &in) {
+    const int64_t rows2 = w2 ? w2->rows : 0, all = w->rows + rows2;
+    const int E = w->kind == CWKC_WEIGHT_BF16 ? 8 : w->kind == CWKC_WEIGHT_F32 ? 4 : 16;
+    const int pieces = (int)(w->cols / E);                 // of a row
+    const int cap = 2 * ctx->sm_count - (xin == X_NORM ? 1 : 0);      // blocks that are resident together
+    const int blocks = (int)std::min<int64_t>((all + 1) / 2, cap);
+    const int64_t pairs = ((all + blocks - 1) / blocks + 1) / 2;
+    int wpr = 1;
+    int64_t best = -1;
+    for (int c = 1; c <= TG_WARPS; c <<= 1) {              // least time of a block: rounds x (pieces per lane + what a round costs besides)
+        const int64_t rounds = (pairs + TG_WARPS / c - 1) / (TG_WARPS / c), cost = rounds * ((pieces + 32 * c - 1) / (32 * c) * 2 + (c > 1 ? 3 : 2));
+        if (best < 0 || cost < best) { best = cost; wpr = c; }
+    }
     auto go = [&](auto kern) {
         ctx->launches++;
-        return cwk_launch_early(kern, dim3((unsigned)(nb1 + nb2 + (norm ? 1 : 0))), dim3(256), norm ? (size_t)w->cols * 4 : 0, ctx->stream, (const void *)w->data, (const float *)w->scales, x, y,
-                                (int)w->rows, (int)w->cols, rpb, nb1, (const void *)(w2 ? w2->data : nullptr), (const float *)(w2 ? w2->scales : nullptr), y2, (int)rows2, nm, f0, f1);
+        return cwk_launch_early(kern, dim3((unsigned)(blocks + (xin == X_NORM ? 1 : 0))), dim3(32 * TG_WARPS), xin == X_PLAIN ? 0 : (size_t)w->cols * 4, ctx->stream,
+                                (const void *)w->data, (const float *)w->scales, y, (int)w->rows, (int)w->cols, wpr, blocks, (const void *)(w2 ? w2->data : nullptr),
+                                (const float *)(w2 ? w2->scales : nullptr), y2, (int)rows2, in);
     };
-    if (w->kind == CWKC_WEIGHT_BF16) return norm ? go(gemv_token_kernel<GEMV_BF16, true>) : go(gemv_token_kernel<GEMV_BF16, false>);
-    if (w->kind == CWKC_WEIGHT_F32) return norm ? go(gemv_token_kernel<GEMV_F32, true>) : go(gemv_token_kernel<GEMV_F32, false>);
-    return norm ? go(gemv_token_kernel<GEMV_FP8, true>) : go(gemv_token_kernel<GEMV_FP8, false>);
+    auto kinds = [&](auto bf16, auto f32, auto fp8) { return w->kind == CWKC_WEIGHT_BF16 ? go(bf16) : w->kind == CWKC_WEIGHT_F32 ? go(f32) : go(fp8); };
+    if (xin == X_NORM) return kinds(gemv_token_kernel<GEMV_BF16, X_NORM>, gemv_token_kernel<GEMV_F32, X_NORM>, gemv_token_kernel<GEMV_FP8, X_NORM>);
+    if (xin == X_SUM) return kinds(gemv_token_kernel<GEMV_BF16, X_SUM>, gemv_token_kernel<GEMV_F32, X_SUM>, gemv_token_kernel<GEMV_FP8, X_SUM>);
+    return kinds(gemv_token_kernel<GEMV_BF16, X_PLAIN>, gemv_token_kernel<GEMV_F32, X_PLAIN>, gemv_token_kernel<GEMV_FP8, X_PLAIN>);
 }
 
 // q_abs[h][c] = sum_r q[h][r] W_k[h][r][c] (src/attention.c:741-744) for one token: grid (heads, kv_lora / 256), 512 threads,
@@ -161,34 +205,32 @@ __global__ void __launch_bounds__(512) absorb_token_kernel(const float *q, const
     }
 }
 
-// The attention's split records of one token (nsplit x [heads][512 + 2], flash_rows.cuh's layout) merged, and the result,
-// rounded to bf16 as the merge on its own would leave it, taken through W_v (src/attention.c:812-815): grid (heads, 2),
-// 512 threads; a block merges its head's 512 columns and does half of the head's 128 value rows, four per warp, whose weights
-// are on their way before the records are there.
-__global__ void __launch_bounds__(512) merge_unabsorb_kernel(const float *partial, int nsplit, int nh, const uint16_t *kvb, int nope, float *attn) {
-    constexpr int L = 512, VD = 128, AHEAD = 32;
-    __shared__ float s_w[512], s_red[32];
-    __shared__ __align__(16) float s_c[L];
-    const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+// The attention's split records of one token (nsplit <= 512 of [heads][512 + 2], flash_rows.cuh's layout) merged, and the
+// result, rounded to bf16 as the merge on its own would leave it, taken through W_v (src/attention.c:812-815): grid (heads,
+// 2), 512 threads. A block merges 256 of its head's 512 columns, two threads a column (each half of the records), and forms
+// those columns' part of the head's 128 values, eight per warp, whose weights are on their way before the records are
+// there; attn [2][heads][128] has the two parts, added up by the next projection.
+__global__ void __launch_bounds__(512, 2) merge_unabsorb_kernel(const float *partial, int nsplit, int nh, const uint16_t *kvb, int nope, float *attn) {
+    constexpr int L = 512, VD = 128, AHEAD = 16;
+    __shared__ float s_w[512], s_red[32], s_half[256];
+    __shared__ __align__(16) float s_c[256];
+    const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c0 = blockIdx.y * 256;
     const int64_t rec = (int64_t)nh * (L + 2);
     cwk_pdl_launch();
-    uint4 v[4][2];
-    const int r0 = blockIdx.y * (VD / 2) + warp * 4;
+    uint4 v[8];
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint16_t *w = kvb + ((int64_t)h * (nope + VD) + nope + r0 + r) * L;
-        v[r][0] = ld_weight16(w + lane * 8);
-        v[r][1] = ld_weight16(w + 256 + lane * 8);
-    }
+    for (int r = 0; r < 8; r++) v[r] = ld_weight16(kvb + ((int64_t)h * (nope + VD) + nope + warp * 8 + r) * L + c0 + lane * 8);
     cwk_pdl_wait();
-    const float *col = partial + 2 * nh + (int64_t)h * L + tid;
+    const int lo = tid < 256 ? 0 : (nsplit + 1) / 2, hi = tid < 256 ? (nsplit + 1) / 2 : nsplit;      // this thread's records
+    const float *col = partial + 2 * nh + (int64_t)h * L + c0 + (tid & 255);
     float o[AHEAD];
 #pragma unroll
-    for (int s = 0; s < AHEAD; s++) o[s] = s < nsplit ? col[s * rec] : 0.f;
-    float m = -INFINITY, l = 0.f;                          // this thread's record (nsplit <= 512)
+    for (int s = 0; s < AHEAD; s++) o[s] = lo + s < hi ? col[(lo + s) * rec] : 0.f;
+    float m = -INFINITY, l = 0.f;                          // record `tid`
     if (tid < nsplit) {
+        const float mm = partial[tid * rec + h];
         l = partial[tid * rec + nh + h];
-        if (l > 0.f) m = partial[tid * rec + h];
+        if (l > 0.f) m = mm;
     }
     float M = m;
 #pragma unroll
@@ -211,22 +253,24 @@ __global__ void __launch_bounds__(512) merge_unabsorb_kernel(const float *partia
     float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int s = 0; s < AHEAD; s++)
-        if (s < nsplit) a[s & 3] += s_w[s] * o[s];
-    for (int s0 = AHEAD; s0 < nsplit; s0 += AHEAD) {
+        if (lo + s < hi) a[s & 3] += s_w[lo + s] * o[s];
+    for (int s0 = lo + AHEAD; s0 < hi; s0 += AHEAD) {
 #pragma unroll
-        for (int s = 0; s < AHEAD; s++) o[s] = s0 + s < nsplit ? col[(s0 + s) * rec] : 0.f;
+        for (int s = 0; s < AHEAD; s++) o[s] = s0 + s < hi ? col[(s0 + s) * rec] : 0.f;
 #pragma unroll
         for (int s = 0; s < AHEAD; s++)
-            if (s0 + s < nsplit) a[s & 3] += s_w[s0 + s] * o[s];
+            if (s0 + s < hi) a[s & 3] += s_w[s0 + s] * o[s];
     }
-    const float inv = den > 0.f ? 1.f / den : 0.f;
-    s_c[tid] = __uint_as_float(pack_bf16x2(0.f, ((a[0] + a[1]) + (a[2] + a[3])) * inv) & 0xffff0000u);
+    const float sum = (a[0] + a[1]) + (a[2] + a[3]), inv = den > 0.f ? 1.f / den : 0.f;
+    if (tid >= 256) s_half[tid - 256] = sum;
+    __syncthreads();
+    if (tid < 256) s_c[tid] = __uint_as_float(pack_bf16x2(0.f, (sum + s_half[tid]) * inv) & 0xffff0000u);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-        float t = gemv_piece<GEMV_BF16>(v[r][0], s_c, lane * 8, nullptr) + gemv_piece<GEMV_BF16>(v[r][1], s_c, 256 + lane * 8, nullptr);
+    for (int r = 0; r < 8; r++) {
+        float t = gemv_piece<GEMV_BF16>(v[r], s_c, lane * 8, nullptr);
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
-        if (lane == 0) attn[h * VD + r0 + r] = t;
+        if (lane == 0) attn[((int64_t)blockIdx.y * nh + h) * VD + warp * 8 + r] = t;
     }
 }

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from cwick_b200 import lib as cl, synth
-from cwick_b200.compat import Err, make_spec, tensor
+from cwick_b200.compat import Err, make_spec, tensor, tensor_fp8
 
 pytestmark = pytest.mark.gpu
 
@@ -59,4 +59,56 @@ def test_chunk_against_the_layer_in_double(monkeypatch, H, nh, nope, vdim, q_lor
     np.testing.assert_allclose(got_rows, rows, atol=2e-5 * np.abs(rows).max(), rtol=8e-3 if bf16_cache else 2e-5)
     assert np.linalg.norm(out - want) < 6e-3 * np.linalg.norm(want)
     assert np.array_equal(cache[:pos0], prefix[:pos0] if bf16_cache else synth.bf16_to_f32(prefix[:pos0]))
+    L.cwk_dropin_reset()
+
+
+@pytest.mark.parametrize("pos", [0, 1, 257, 2000])
+@pytest.mark.parametrize("kind", ["bf16", "f32", "fp8"])
+@pytest.mark.parametrize("H,nh,q_lora", [(1024, 64, 640), (336, 2, 208), (48, 1, 16)])
+def test_token_against_the_layer_in_double(monkeypatch, H, nh, q_lora, kind, pos):
+    """One-token decode at latent 512 and value heads of 128: rows per block even and odd, fewer rows than blocks, activations
+    shorter than a warp's reads, one split record and many."""
+    import torch
+    nope = vdim = 128
+    kv_lora = 512
+    monkeypatch.setenv("CWICK_LATENT_BF16", "1")
+    L = cl.load()
+    fn = L["cwick_attention_mla_decode"]
+    fn.restype = None
+    fn.argtypes = [C.c_void_p] * 11 + [C.c_int64] * 3 + [C.c_void_p] * 5
+    L.cwk_dropin_reset()
+    shapes = [(q_lora, H), (nh * nope, q_lora), (kv_lora, H), (nh * (nope + vdim), kv_lora), (H, nh * vdim)]
+    w = [synth.normal_bf16(6, i, s, s[1] ** -0.5) for i, s in enumerate(shapes)]
+    keep, t, wide = [], [], []
+    for i, (a, s) in enumerate(zip(w, shapes)):
+        if kind == "f32" and i != 3:
+            b = synth.bf16_to_f32(a)
+            t.append(tensor(b, *s))
+            t[-1].kind = 2
+            keep.append(b)
+        elif kind == "fp8" and i != 3:
+            c = (torch.from_numpy(synth.bf16_to_f32(a)) * 16).to(torch.float8_e4m3fn)
+            b, sc = c.view(torch.uint8).numpy(), np.full(((s[0] + 127) // 128, (s[1] + 127) // 128), 1 / 16, np.float32)
+            sc[-1, -1] = 1 / 32
+            t.append(tensor_fp8(b, sc, *s))
+            keep += [b, sc]
+            a = synth.f32_to_bf16((c.float().numpy() * np.repeat(np.repeat(sc, 128, 0), 128, 1)[:s[0], :s[1]]).astype(np.float32))
+        else:
+            t.append(tensor(a, *s))
+        wide.append(a)
+    ones = synth.f32_to_bf16(np.ones(max(q_lora, kv_lora), np.float32))
+    t += [tensor(ones, 1, q_lora), tensor(ones, 1, kv_lora)]
+    spec = make_spec(H, nh, nope, vdim, q_lora, kv_lora, 1e-6)
+    x = synth.normal(6, 11, H).astype(np.float32)
+    cache = synth.normal_bf16(6, 12, (pos + 1, kv_lora))
+    before = cache[:pos].copy()
+    out, err = np.zeros(H, np.float32), Err()
+    ref = C.byref
+    fn(C.addressof(spec), ref(t[0]), ref(t[1]), ref(t[2]), ref(t[3]), None, ref(t[4]), ref(t[5]), ref(t[6]), cache.ctypes.data, None, pos + 1, pos, 0,
+       None, None, x.ctypes.data, out.ctypes.data, ref(err))
+    assert err.status == 0, err.message
+    want, rows = _layer(x[None].astype(np.float64), wide, synth.bf16_to_f32(before).astype(np.float64), 1e-6, nh, nope, vdim)
+    np.testing.assert_allclose(synth.bf16_to_f32(cache[pos:]), rows, atol=2e-5 * np.abs(rows).max(), rtol=8e-3)
+    assert np.linalg.norm(out - want[0]) < 8e-3 * np.linalg.norm(want)
+    assert np.array_equal(cache[:pos], before)
     L.cwk_dropin_reset()
