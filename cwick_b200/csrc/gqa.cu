@@ -115,7 +115,7 @@ int cwk_gqa_prefill(cwk_ctx *ctx, const void *Q, const void *K, const void *V, i
     // head dim 256 on the tcgen05/TMA prefill kernel (queries as MMA rows, K/V tiles by TMA from the caches); forcing a
     // general path on the context (cwk_ctx_force_mla_path 0 or 1) keeps the mma.sync kernel for A/B runs
     if (hd == 256 && ctx->force_mla_path != 0 && ctx->force_mla_path != 1) {
-        const size_t flags_bytes = ((size_t)((n + 127) / 128) * nh + 3) * sizeof(int);
+        const size_t flags_bytes = ((size_t)((n + 127) / 128) * nh + ctx->sm_count + 3) * sizeof(int);
         int s = cwk_reserve_work(ctx, flags_bytes);
         if (s != CWK_OK) return s;
         s = cwk_gqa_prefill_tc(ctx, Q, K, V, pos, n, nh, nkv, hd, scale, out, (int *)ctx->work);

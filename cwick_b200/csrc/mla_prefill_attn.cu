@@ -55,8 +55,8 @@ struct PaCfg {
     static constexpr int OFF_C = PA_OFF_K + PA_KST * K_BYTES;
     static constexpr int OFF_P = OFF_C + CST * PA_C_BYTES;
     static constexpr int OFF_BAR = OFF_P + 2 * PA_P_BYTES;
-    static constexpr int OFF_X = OFF_BAR + 512;        // [4][128] f32 maxima, [4][128] f32 sums exchanged between the softmax groups; 8 item numbers
-    static constexpr int SMEM = OFF_X + 4096 + 64 + 1024;
+    static constexpr int OFF_X = OFF_BAR + 512;        // [4][128] f32 maxima, [4][128] f32 sums exchanged between the softmax groups; 8 items of 16 bytes
+    static constexpr int SMEM = OFF_X + 4096 + 128 + 1024;
     static_assert(SMEM <= 232448, "shared-memory budget");
     static_assert(384 + DQK / 2 <= 512, "tensor-memory budget");
 };
@@ -77,13 +77,21 @@ struct AttnParams {
     int group;          // GQA: query heads per KV head (MLA: unused)
     int64_t pos0;
     float scale_log2;
-    int *flags;         // one word per item: fast form sets it, exact form runs only where it is set
+    int *flags;         // one word per item (share mode: per item + block): fast form sets it, exact form runs only where it is set
     int *counter;       // [3]: item counters of the fast and the exact form, number of flags raised; zero at launch
     int *err;
+    // Share mode (shares > 0): the key tiles of all items, one after another, are dealt out to the blocks in equal contiguous
+    // shares, whatever the items' number and lengths; what a block does of an item that is not all its own is left as a record
+    // (record_of), and attn_merge_kernel joins them.
+    int shares;         // number of blocks
+    int head_tiles;     // key tiles of one (head, half)
+    float *records;     // [2 * shares][PA_RECORD]
 };
+constexpr int PA_RECORD = PA_QT * (PA_DV + 2);         // floats: O as [PA_DV / 4][row][4], m [row], l [row]
 
 struct AttnItem {
-    int q0, h, half, nt;
+    int q0, h, half, lo, nt;   // key tiles lo .. nt - 1
+    int rec, flag;             // where the result goes as a record (-1: into the output); index of the flag
 };
 
 // Work item w of the attention grid: query tiles from the longest to the shortest inside one (head, half), then the next
@@ -95,14 +103,37 @@ __device__ __forceinline__ AttnItem attn_item(int w, const AttnParams &p, int nq
     it.h = hh % p.nh;
     it.half = hh / p.nh;                                                   // GQA: the grid has one "half", always 0
     const int64_t last_q = p.pos0 + min(it.q0 + PA_QT - 1, p.n - 1);     // keys 0 .. pos0 + (last query of the item): tiles of 64
+    it.lo = 0;
     it.nt = (int)(last_q / PA_KT) + 1;
+    it.rec = -1;
+    it.flag = w;
     return it;
 }
 
+// Share mode: where an item is cut. A segment's first tile must show every row of the item a key (the rows' reference
+// exponents come from it): cuts inside the diagonal move down to its first tile.
+__device__ __forceinline__ int attn_cut(int tile, const AttnItem &it, const AttnParams &p) {
+    return tile <= 0 ? 0 : tile >= it.nt ? it.nt : min(tile, (int)((p.pos0 + it.q0) / PA_KT));
+}
+__device__ __forceinline__ int64_t share_begin(int g, int64_t total_tiles, int shares) { return total_tiles * g / shares; }
+// The part of block g (tiles u0 .. u1 - 1 of all) in item `it`, which begins at tile `at` of all; false: none.
+__device__ __forceinline__ bool attn_segment(AttnItem &it, int w, int g, int64_t at, int64_t u0, int64_t u1, const AttnParams &p) {
+    const int nt = it.nt, lo = attn_cut((int)max((int64_t)-1, min((int64_t)nt, u0 - at)), it, p), hi = attn_cut((int)max((int64_t)-1, min((int64_t)nt, u1 - at)), it, p);
+    it.lo = lo;
+    it.nt = hi;
+    it.rec = lo > 0 ? 2 * g : hi < nt ? 2 * g + 1 : -1;      // (only a block's first segment begins inside an item, only its last ends inside one)
+    it.flag = w + g;                                         // (from one segment to the next w or g goes up)
+    return hi > lo;
+}
+
+// Softmax groups and tiles. A tile's scores go from tensor memory through registers into P in a chain (barrier, load, maximum,
+// exponentials, barrier, store, fence) that takes longer than its MMAs. So in the fast form two of the four groups take the even tiles
+// and two the odd ones, a row's 64 keys between them, and the chains of two tiles overlap.
+//
 // Persistent: one block per SM takes items from a global counter until none is left. The first TMA operation of a
 // block waits several thousand cycles for its tensor map, tensor memory is allocated once, and the loads of the next
 // item run under the epilogue of this one.
-template <int NWG, class CFG, bool GQA>      // NWG softmax warp groups: 2 or 4 = fast form (a row's 64 keys shared by 2 or 4 threads), 1 = exact form
+template <int NWG, class CFG, bool GQA>      // NWG softmax warp groups: 4 = fast form, 1 = exact form
 __global__ void __launch_bounds__(128 + 128 * NWG, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_c, const AttnParams p) {
     constexpr int PA_DQK = CFG::DQK, PA_K_BYTES = CFG::K_BYTES, PA_CST = CFG::CST, PA_OFF_C = CFG::OFF_C, PA_OFF_P = CFG::OFF_P,
@@ -114,10 +145,13 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t bar0 = base + PA_OFF_BAR;
     auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + PA_OFF_BAR + 8 * PB_COUNT + 8);
-    volatile int *s_item = reinterpret_cast<volatile int *>(sm + PA_OFF_X + 4096);      // ring of 8 item numbers
+    int4 *s_item = reinterpret_cast<int4 *>(sm + PA_OFF_X + 4096);      // ring of 8 items: {number, first tile, end, record}
+    constexpr int TG = NWG == 4 ? 2 : 1;             // groups that share a tile
     float *s_m = reinterpret_cast<float *>(sm + PA_OFF_X), *s_l = s_m + 512;              // [4][128] each
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     if (NWG == 1 && p.counter[2] == 0) return;                   // the repair pass: the fast form raised no flag
     const int nq = (p.n + PA_QT - 1) / PA_QT;
     const int total = nq * p.nh * (GQA ? 1 : 2);
@@ -126,8 +160,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_k) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_c) : "memory");
         for (int i = 0; i < PB_COUNT; i++) {
-            const bool by_soft = (i >= PB_SEMPTY && i < PB_PEMPTY) || i == PB_QFULL || i == PB_OFREE || i == PB_XM || i == PB_XL;
-            mbar_init(bar(i), by_soft ? (uint32_t)(128 * NWG) : 1u);
+            const bool by_tile = i >= PB_SEMPTY && i < PB_PEMPTY, by_soft = i == PB_QFULL || i == PB_OFREE || i == PB_XM || i == PB_XL;
+            mbar_init(bar(i), by_tile ? (uint32_t)(128 * TG) : by_soft ? (uint32_t)(128 * NWG) : 1u);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -140,10 +174,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
 
-    // item k of this block, as published by the key producer (-1: no more)
-    auto next_item = [&](int k, int &w) -> bool {
+    // item k of this block, as published by the key producer (w < 0: no more)
+    auto next_item = [&](int k, int &w, AttnItem &it) -> bool {
         if (!mbar_wait(bar(PB_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1031)) return false;
-        w = s_item[k & 7];
+        const int4 v = s_item[k & 7];
+        w = v.x;
+        it = attn_item(max(w, 0), p, nq);
+        it.lo = v.y; it.nt = v.z; it.rec = v.w;
+        if (p.shares) it.flag = w + (int)blockIdx.x;
         return true;
     };
 
@@ -152,16 +190,39 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         if (lane == 0) {
             bool ok = true;
             int kc = 0;                              // key tiles issued so far (ring position and phase run across items)
+            const int hh_n = p.nh * (GQA ? 1 : 2);
+            const int64_t all = (int64_t)p.head_tiles * hh_n, u0 = p.shares ? share_begin(blockIdx.x, all, p.shares) : 0,
+                          u1 = p.shares ? share_begin(blockIdx.x + 1, all, p.shares) : 0;
+            int sw = 0;                              // share mode: the next item, and where it begins
+            int64_t at = 0;
+            if (p.shares) {
+                sw = (int)(u0 / p.head_tiles) * nq;
+                at = u0 / p.head_tiles * p.head_tiles;
+                for (int nt; sw < total && at + (nt = attn_item(sw, p, nq).nt) <= u0; sw++) at += nt;
+            }
             for (int k = 0; ok; k++) {
-                int w = atomicAdd(p.counter + (NWG == 1 ? 1 : 0), 1);
-                if (NWG == 1)                         // the repair pass takes flagged items only
-                    while (w < total && p.flags[w] == 0) w = atomicAdd(p.counter + 1, 1);
-                if (w >= total) w = -1;
-                s_item[k & 7] = w;                    // the roles of a block stay within a few tiles of each other: 8 slots cannot wrap
+                int w = -1;
+                AttnItem it{};
+                if (p.shares) {
+                    while (sw < total && at < u1) {
+                        it = attn_item(sw, p, nq);
+                        const int nt = it.nt;
+                        const bool mine = attn_segment(it, sw, blockIdx.x, at, u0, u1, p);
+                        at += nt;
+                        sw++;
+                        if (mine && (NWG > 1 || p.flags[it.flag] != 0)) { w = sw - 1; break; }      // (the repair pass takes flagged ones only)
+                    }
+                } else {
+                    w = atomicAdd(p.counter + (NWG == 1 ? 1 : 0), 1);
+                    if (NWG == 1)                     // the repair pass takes flagged items only
+                        while (w < total && p.flags[w] == 0) w = atomicAdd(p.counter + 1, 1);
+                    if (w >= total) w = -1;
+                    it = attn_item(max(w, 0), p, nq);
+                }
+                s_item[k & 7] = make_int4(w, it.lo, it.nt, it.rec);      // the roles of a block stay within a few tiles of each other: 8 slots cannot wrap
                 mbar_arrive(bar(PB_ITEM + (k & 7)));
                 if (w < 0) break;
-                const AttnItem it = attn_item(w, p, nq);
-                for (int i = 0; i < it.nt && ok; i++, kc++) {
+                for (int i = it.lo; i < it.nt && ok; i++, kc++) {
                     const int ks = kc % PA_KST, ku = kc / PA_KST;
                     ok = mbar_wait(bar(PB_KEMPTY + ks), (uint32_t)((ku & 1) ^ 1), p.err, 1001);
                     if (!ok) break;
@@ -182,10 +243,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             int cc = 0;
             for (int k = 0; ok; k++) {
                 int w;
-                ok = next_item(k, w);
+                AttnItem it;
+                ok = next_item(k, w, it);
                 if (!ok || w < 0) break;
-                const AttnItem it = attn_item(w, p, nq);
-                for (int i = 0; i < it.nt && ok; i++, cc++) {
+                for (int i = it.lo; i < it.nt && ok; i++, cc++) {
                     const int cs = cc % PA_CST, cu = cc / PA_CST;
                     ok = mbar_wait(bar(PB_CEMPTY + cs), (uint32_t)((cu & 1) ^ 1), p.err, 1002);
                     if (!ok) break;
@@ -208,14 +269,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             int kc = 0;                              // score tiles issued so far
             for (int k = 0; ok; k++) {
                 int w;
-                ok = next_item(k, w);
+                AttnItem it;
+                ok = next_item(k, w, it);
                 if (!ok || w < 0) break;
-                const AttnItem it = attn_item(w, p, nq);
                 ok = mbar_wait(bar(PB_QFULL), (uint32_t)(k & 1), p.err, 1011);     // the softmax threads have written the item's query tile into tensor memory
                 if (!ok) break;
                 tc_fence_after();
                 // scores of a tile: S[kc % 2] = Q Kx^T, three 64-wide blocks of the 192 dims, four 16-wide steps each
-                for (int i = 0; i < it.nt && ok; i++, kc++) {
+                for (int i = it.lo; i < it.nt && ok; i++, kc++) {
                     const int ks = kc % PA_KST, ku = kc / PA_KST, sb = kc % PA_SBUF, su = kc / PA_SBUF;
                     ok = mbar_wait(bar(PB_KFULL + ks), (uint32_t)(ku & 1), p.err, 1012);
                     if (ok) ok = mbar_wait(bar(PB_SEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1013);
@@ -240,14 +301,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             int cc = 0;                              // value tiles issued so far
             for (int k = 0; ok; k++) {
                 int w;
-                ok = next_item(k, w);
+                AttnItem it;
+                ok = next_item(k, w, it);
                 if (!ok || w < 0) break;
-                const AttnItem it = attn_item(w, p, nq);
                 if (k > 0) {                         // the accumulator of the previous item has been read out
                     ok = mbar_wait(bar(PB_OFREE), (uint32_t)((k - 1) & 1), p.err, 1016);
                     if (!ok) break;
                 }
-                for (int i = 0; i < it.nt && ok; i++, cc++) {
+                for (int i = it.lo; i < it.nt && ok; i++, cc++) {
                     const int cs = cc % PA_CST, cu = cc / PA_CST, pb = cc & 1, pu = cc >> 1;
                     ok = mbar_wait(bar(PB_CFULL + cs), (uint32_t)(cu & 1), p.err, 1014);
                     if (ok) ok = mbar_wait(bar(PB_PFULL + pb), (uint32_t)(pu & 1), p.err, 1015);
@@ -258,7 +319,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     const uint64_t dC = smem_desc(base + PA_OFF_C + cs * PA_C_BYTES, PA_KT * 128, 1024);
 #pragma unroll
                     for (int s = 0; s < 4; s++)
-                        umma_bf16(tmem + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, (s != 0) ? 1u : (uint32_t)(i != 0));
+                        umma_bf16(tmem + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, (s != 0) ? 1u : (uint32_t)(i != it.lo));
                     umma_commit(bar(PB_CEMPTY + cs));
                     umma_commit(bar(PB_PEMPTY + pb));
                 }
@@ -267,18 +328,18 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         }
     } else if (warp >= 4) {
         // ------------------------------------------------------------ softmax, (correction,) epilogue
-        // A thread owns query row `row` (= its TMEM lane) and NC of a tile's 64 key columns.
-        constexpr int NC = PA_KT / NWG;
-        const int q4 = warp & 3, wg = (warp - 4) >> 2;
+        // A thread owns query row `row` (= its TMEM lane) and NC of the 64 key columns of its tiles.
+        constexpr int NC = PA_KT / TG;
+        const int q4 = warp & 3, wg = (warp - 4) >> 2, cg = wg & (TG - 1), odd = wg / TG;      // columns cg * NC .., tiles of parity `odd`
         const int row = q4 * 32 + lane;
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
         bool ok = true;
         int tc = 0;                                  // tiles done so far (score buffer, P buffer and their phases run across items)
         for (int k = 0; ok; k++) {
             int w;
-            ok = next_item(k, w);
+            AttnItem it;
+            ok = next_item(k, w, it);
             if (!ok || w < 0) break;
-            const AttnItem it = attn_item(w, p, nq);
             const int q0 = it.q0, h = it.h, half = it.half, nt = it.nt;
             const int64_t tq = p.pos0 + q0 + row;                    // this row's position: keys 0..tq are visible
             // The query tile is the A operand of every score MMA of the item; it is kept in tensor memory (row = lane, two
@@ -306,21 +367,31 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             };
             if (k == 0) load_query(q0, h);
             float m = 0.f, l = 0.f;
-            for (int i = 0; i < nt && ok; i++, tc++) {
+            // reference exponent of the row: its largest score of the item's first tile, which one pair of groups has. (All arrive:
+            // no P is written before the epilogue of the item before has left the P buffers.)
+            auto reference = [&]() -> bool {
+                mbar_arrive(bar(PB_XM));
+                if (!mbar_wait(bar(PB_XM), (uint32_t)(k & 1), p.err, 1026)) return false;
+                m = fmaxf(s_m[row], s_m[128 + row]);                 // the tile shows every row a key: finite
+                return true;
+            };
+            if (NWG == 4 && (tc & 1) != odd) ok = reference();
+            for (int i = it.lo; i < nt && ok; i++, tc++) {
                 const int sb = tc & 1, su = tc >> 1;             // P buffer of this tile
+                if (NWG == 4 && sb != odd) continue;
                 const int s3 = tc % PA_SBUF;                      // its score buffer
                 ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_SFULL + s3), (uint32_t)((tc / PA_SBUF) & 1), p.err, 1021));   // warp-uniform: the TMEM loads below are warp-wide
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t v[NC];
 #pragma unroll
-                for (int c = 0; c < NC / 16; c++) TMEM_LD16(v, c * 16, tlane + PA_COL_S + s3 * PA_KT + wg * NC + c * 16);
+                for (int c = 0; c < NC / 16; c++) TMEM_LD16(v, c * 16, tlane + PA_COL_S + s3 * PA_KT + cg * NC + c * 16);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 tc_fence_before();
                 mbar_arrive(bar(PB_SEMPTY + s3));
                 float s[NC];
                 float mt = -INFINITY;
-                const int64_t k0 = (int64_t)i * PA_KT + wg * NC;
+                const int64_t k0 = (int64_t)i * PA_KT + cg * NC;
                 if ((int64_t)i * PA_KT + PA_KT - 1 <= p.pos0 + q0) {   // every key of the tile is visible to every row of the item
 #pragma unroll
                     for (int j = 0; j < NC; j++) { s[j] = __uint_as_float(v[j]) * p.scale_log2; mt = fmaxf(mt, s[j]); }
@@ -331,23 +402,20 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                         mt = fmaxf(mt, s[j]);
                     }
                 }
-                if (NWG >= 2) {
-                    if (i == 0) {                                    // reference exponent of the row: its largest score of the first tile
-                        s_m[wg * 128 + row] = mt;
-                        mbar_arrive(bar(PB_XM));
-                        ok = mbar_wait(bar(PB_XM), (uint32_t)(k & 1), p.err, 1026);
+                if (NWG == 4) {
+                    if (i == it.lo) {
+                        s_m[cg * 128 + row] = mt;
+                        ok = reference();
                         if (!ok) break;
-                        m = fmaxf(s_m[row], s_m[128 + row]);         // key 0 is visible to every row: finite
-                        if (NWG == 4) m = fmaxf(m, fmaxf(s_m[256 + row], s_m[384 + row]));
                     } else if (mt > m + PA_RANGE) {
-                        p.flags[w] = 1;                              // out of the range this form covers: the exact form redoes the item
+                        p.flags[it.flag] = 1;                        // out of the range this form covers: the exact form redoes the item
                         atomicAdd(p.counter + 2, 1);
                     }
                 } else {
                     // tcgen05.ld / st are warp-wide instructions: the warp decides together, and a lane that has no
                     // need of it rescales by 1
-                    const bool mine = (i != 0) && (mt > m + PA_LAZY);
-                    if (i == 0) m = mt;
+                    const bool mine = (i != it.lo) && (mt > m + PA_LAZY);
+                    if (i == it.lo) m = mt;
                     if (__any_sync(0xffffffffu, mine)) {
                         // some row's scores outran its reference exponent: rescale what it has accumulated. A row is its
                         // thread's TMEM lane; the value MMAs of the previous tile must have finished writing it.
@@ -384,7 +452,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 uint8_t *prow = sm + PA_OFF_P + sb * PA_P_BYTES + row * 128;
 #pragma unroll
                 for (int c = 0; c < NC / 8; c++)
-                    *reinterpret_cast<uint4 *>(prow + (((wg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                    *reinterpret_cast<uint4 *>(prow + (((cg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 tc_fence_before();
                 mbar_arrive(bar(PB_PFULL + sb));
@@ -393,14 +461,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             {
                 // the next item's query tile: the score MMAs of this item are done with theirs (they precede its last value MMAs)
                 int wn;
-                ok = next_item(k + 1, wn);
+                AttnItem nx;
+                ok = next_item(k + 1, wn, nx);
                 if (!ok) break;
                 if (wn >= 0) {
                     ok = mbar_wait(bar(PB_QEMPTY), (uint32_t)(k & 1), p.err, 1025);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
-                    const AttnItem nx = attn_item(wn, p, nq);
                     load_query(nx.q0, nx.h);
                 }
             }
@@ -408,13 +476,30 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             ok = mbar_wait(bar(PB_ODONE), (uint32_t)(k & 1), p.err, 1024);
             if (!ok) break;
             tc_fence_after();
-            if (NWG >= 2) {                                          // the row's sum is the groups' sums
+            if (NWG == 4) {                                          // the row's sum is the groups' sums
                 s_l[wg * 128 + row] = l;
                 mbar_arrive(bar(PB_XL));
                 ok = mbar_wait(bar(PB_XL), (uint32_t)(k & 1), p.err, 1027);
                 if (!ok) break;
-                l = s_l[row] + s_l[128 + row];
-                if (NWG == 4) l += s_l[256 + row] + s_l[384 + row];
+                l = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
+            }
+            if (it.rec >= 0) {                                       // part of an item: its record
+                float *rec = p.records + (int64_t)it.rec * PA_RECORD;
+                constexpr int CPG = PA_DV / NWG;                     // columns per group
+#pragma unroll 1
+                for (int c = 0; c < CPG / 16; c++) {
+                    const int col = wg * CPG + c * 16;
+                    uint32_t o[16];
+                    TMEM_LD16(o, 0, tlane + PA_COL_O + col);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        *reinterpret_cast<uint4 *>(rec + ((int64_t)(col / 4 + j) * PA_QT + row) * 4) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+                }
+                if (wg == 0) { rec[PA_QT * PA_DV + row] = m; rec[PA_QT * (PA_DV + 1) + row] = l; }
+                tc_fence_before();
+                mbar_arrive(bar(PB_OFREE));
+                continue;
             }
             const float inv = l > 0.f ? 1.f / l : 0.f;
             uint8_t *stg = sm + PA_OFF_P + (warp - 4) * 4096;         // 4 KB per warp: [32 rows][128 B], in the P buffers (idle: the item's value MMAs are done, and the next item's P comes from these threads)
@@ -459,6 +544,94 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
+}
+
+// Share mode: joins the records of an item that more than one block worked on. Grid (items, PA_DV / 16), a row per thread.
+template <bool GQA>
+__global__ void __launch_bounds__(128) attn_merge_kernel(const AttnParams p) {
+    cwk_pdl_launch();
+    const int nq = (p.n + PA_QT - 1) / PA_QT, w = blockIdx.x, row = threadIdx.x, c16 = blockIdx.y;
+    const int64_t all = (int64_t)p.head_tiles * p.nh * (GQA ? 1 : 2);
+    int64_t at = (int64_t)(w / nq) * p.head_tiles;
+    for (int v = w - w % nq; v < w; v++) at += attn_item(v, p, nq).nt;
+    const AttnItem it = attn_item(w, p, nq);
+    int g = (int)(((at + 1) * p.shares - 1) / all);                  // the block that has the item's first tile
+    const int g1 = (int)(((at + it.nt) * p.shares - 1) / all);       // ... its last
+    cwk_pdl_wait();
+    float m = -INFINITY, l = 0.f, o[16] = {};
+    for (; g <= g1; g++) {
+        AttnItem seg = it;
+        if (!attn_segment(seg, w, g, at, share_begin(g, all, p.shares), share_begin(g + 1, all, p.shares), p)) continue;
+        if (seg.rec < 0) return;                                     // one block had all of it, and wrote the output
+        const float *rec = p.records + (int64_t)seg.rec * PA_RECORD;
+        float4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = *reinterpret_cast<const float4 *>(rec + ((int64_t)(c16 * 4 + j) * PA_QT + row) * 4);
+        const float ms = rec[PA_QT * PA_DV + row], ls = rec[PA_QT * (PA_DV + 1) + row];
+        const float mn = fmaxf(m, ms), a = exp2f(m - mn), b = exp2f(ms - mn);      // (ms is finite; the first time a is 0)
+        m = mn;
+        l = l * a + ls * b;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            o[4 * j] = o[4 * j] * a + v[j].x * b; o[4 * j + 1] = o[4 * j + 1] * a + v[j].y * b;
+            o[4 * j + 2] = o[4 * j + 2] * a + v[j].z * b; o[4 * j + 3] = o[4 * j + 3] * a + v[j].w * b;
+        }
+    }
+    if (it.q0 + row >= p.n) return;
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    uint32_t r[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) r[j] = pack_bf16x2(o[2 * j] * inv, o[2 * j + 1] * inv);
+    uint4 *dst = reinterpret_cast<uint4 *>(p.out + ((int64_t)(it.q0 + row) * p.nh + it.h) * (GQA ? PA_DV : PA_L) + it.half * PA_DV + c16 * 16);
+    dst[0] = make_uint4(r[0], r[1], r[2], r[3]);
+    dst[1] = make_uint4(r[4], r[5], r[6], r[7]);
+}
+
+// The attention grid of both shapes: the fast form, the repair pass, and in share mode the merge. Shares where the longest
+// block of item-by-item dealing would have PA_MERGE_TILES more key tiles than an equal share (what records and merge cost).
+constexpr int PA_MERGE_TILES = 10;
+template <class CFG, bool GQA>
+int attn_launch(cwk_ctx *ctx, AttnParams ap, const CUtensorMap &tm_k, const CUtensorMap &tm_c, int exact_only) {
+    static bool attr_set[16] = {false};
+    if (!attr_set[ctx->device & 15]) {
+        CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<1, CFG, GQA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM));
+        CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<4, CFG, GQA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM));
+        attr_set[ctx->device & 15] = true;
+    }
+    const int nq = (ap.n + PA_QT - 1) / PA_QT, heads = ap.nh * (GQA ? 1 : 2), total = nq * heads, G = ctx->sm_count;
+    auto tiles = [&](int qtile) { return (ap.pos0 + std::min((int64_t)(qtile + 1) * PA_QT, (int64_t)ap.n) - 1) / PA_KT + 1; };
+    int64_t head_tiles = 0;
+    for (int i = 0; i < nq; i++) head_tiles += tiles(i);
+    const int64_t all = head_tiles * heads, share = (all + G - 1) / G, waves = (total + G - 1) / G;
+    // one by one: the idle places of the last round are at least the shortest item each
+    const int64_t one_by_one = std::max(tiles(nq - 1), share + (waves * G - total) * tiles(0) / G);
+    ap.shares = 0; ap.records = nullptr; ap.head_tiles = (int)head_tiles;
+    if (one_by_one > share + PA_MERGE_TILES && share >= 2) {
+        const int s = cwk_reserve_scratch(ctx, (size_t)2 * G * PA_RECORD * sizeof(float));
+        if (s != CWK_OK) return s;
+        ap.shares = G; ap.records = ctx->scratch;
+    }
+    const int nflags = total + (ap.shares ? G : 0);
+    ap.counter = ap.flags + nflags;
+    CWK_CUDA(ctx, cudaMemsetAsync(ap.flags, 0, (size_t)(nflags + 3) * sizeof(int), ctx->stream));
+    if (exact_only) {       // every item flagged (any non-zero word), the flag count non-zero, the two item counters back to zero
+        CWK_CUDA(ctx, cudaMemsetAsync(ap.flags, 1, (size_t)(nflags + 3) * sizeof(int), ctx->stream));
+        CWK_CUDA(ctx, cudaMemsetAsync(ap.counter, 0, 2 * sizeof(int), ctx->stream));
+    }
+    const int grid = ap.shares ? G : std::min(total, G);
+    if (!exact_only) {
+        CwkKernelTimer timer(ctx);
+        CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<4, CFG, GQA>, dim3(grid), dim3(640), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
+        CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<4>");
+    }
+    // the repair pass: items whose flag is clear are skipped
+    CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<1, CFG, GQA>, dim3(grid), dim3(256), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
+    CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<1>");
+    if (ap.shares) {
+        CWK_CUDA(ctx, cwk_launch_early(attn_merge_kernel<GQA>, dim3(total, PA_DV / 16), dim3(128), 0, ctx->stream, ap));
+        CWK_LAUNCH_CHECK(ctx, "attn_merge_kernel");
+    }
+    return CWK_OK;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -630,7 +803,7 @@ bool cwk_mla_prefill_attn_tc_ok(const void *Q, const void *cache, const void *Wu
 
 // Q bf16 [n][nh][192] with the rope part already rotated; cache bf16 [pos0 + n][576] (latent | rope key);
 // Wuk bf16 [nh][128][512]; kx = workspace bf16 [nh][pos0 + n][192]; flags = workspace int32, one per item of the
-// attention (ceil(n / 128) x nh x 2) plus three counters; out bf16 [n][nh][512]. exact_only: skip the fast form and run
+// attention (ceil(n / 128) x nh x 2) and per SM plus three counters; out bf16 [n][nh][512]. exact_only: skip the fast form and run
 // the exact form on every item (for tests).
 // Returns CWK_ERR_UNSUPPORTED (no error text) when the tensor path cannot run.
 int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, const void *Wuk, void *kx, int *flags, int64_t pos0, int n, int nh,
@@ -652,8 +825,6 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, cons
     static bool attr_set[16] = {false};
     if (!attr_set[ctx->device & 15]) {
         CWK_CUDA(ctx, cudaFuncSetAttribute(kexp_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KX_SMEM));
-        CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<1, PaMla, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaMla::SMEM));
-        CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<4, PaMla, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaMla::SMEM));
         attr_set[ctx->device & 15] = true;
     }
     {
@@ -665,34 +836,16 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, cons
         kexp_tc_kernel<<<dim3(G, nh), 256, KX_SMEM, ctx->stream>>>(tm_lat, tm_w, kp);
         CWK_LAUNCH_CHECK(ctx, "kexp_tc_kernel");
     }
-    {
-        AttnParams ap;
-        ap.q = (const uint16_t *)Q; ap.out = (uint16_t *)out; ap.n = n; ap.nh = nh; ap.T = T; ap.pos0 = pos0; ap.group = 1; ap.scale_log2 = scale * 1.4426950408889634f; ap.flags = flags;
-        ap.err = ctx->dev_err;
-        const int total = ((n + PA_QT - 1) / PA_QT) * nh * 2;
-        ap.counter = flags + total;
-        CWK_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)(total + 3) * sizeof(int), ctx->stream));
-        if (exact_only) {       // every item flagged (any non-zero word), the flag count non-zero, the two item counters back to zero
-            CWK_CUDA(ctx, cudaMemsetAsync(flags, 1, (size_t)(total + 3) * sizeof(int), ctx->stream));
-            CWK_CUDA(ctx, cudaMemsetAsync(flags + total, 0, 2 * sizeof(int), ctx->stream));
-        }
-        const int grid = std::min(total, ctx->sm_count);
-        if (!exact_only) {
-            CwkKernelTimer timer(ctx);
-            prefill_attn_kernel<4, PaMla, false><<<grid, 640, PaMla::SMEM, ctx->stream>>>(tm_k, tm_c, ap);
-            CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<4>");
-        }
-        // the repair pass: items whose flag is clear are skipped
-        prefill_attn_kernel<1, PaMla, false><<<grid, 256, PaMla::SMEM, ctx->stream>>>(tm_k, tm_c, ap);
-        CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<1>");
-    }
-    return CWK_OK;
+    AttnParams ap{};
+    ap.q = (const uint16_t *)Q; ap.out = (uint16_t *)out; ap.n = n; ap.nh = nh; ap.T = T; ap.pos0 = pos0; ap.group = 1;
+    ap.scale_log2 = scale * 1.4426950408889634f; ap.flags = flags; ap.err = ctx->dev_err;
+    return attn_launch<PaMla, false>(ctx, ap, tm_k, tm_c, exact_only);
 }
 
 // Causal GQA prefill on the same kernel (Qwen3.5 full-attention layers, src/q35_model.c:1713-1746): per query head,
 // 128 consecutive queries are the MMA's rows; keys and values are the 256-wide rows of the head's KV head, streamed in
 // 64-key tiles by TMA straight from the caches. Q bf16 [n][nh][256]; K, V bf16 [pos + n][nkv][256]; out bf16
-// [n][nh][256]; flags = workspace int32 [ceil(n / 128) * nh + 3]. Returns CWK_ERR_UNSUPPORTED (no error text) when the
+// [n][nh][256]; flags = workspace int32 [ceil(n / 128) * nh + number of SMs + 3]. Returns CWK_ERR_UNSUPPORTED (no error text) when the
 // tensor path cannot take the operands.
 int cwk_gqa_prefill_tc(cwk_ctx *ctx, const void *Q, const void *K, const void *V, int64_t pos, int n, int nh, int nkv, int hd,
                        float scale, void *out, int *flags) {
@@ -707,25 +860,8 @@ int cwk_gqa_prefill_tc(cwk_ctx *ctx, const void *Q, const void *K, const void *V
     if (!encode3(&tm_k, K, (uint64_t)T, (uint64_t)nkv * 4, (uint64_t)nkv * hd * 2, PA_KT, 4) ||
         !encode3(&tm_v, V, (uint64_t)T, (uint64_t)nkv * 4, (uint64_t)nkv * hd * 2, PA_KT, 4))
         return cwk_fail(ctx, CWK_ERR_CUDA, "cuTensorMapEncodeTiled failed for the GQA prefill operands");
-    static bool attr_set[16] = {false};
-    if (!attr_set[ctx->device & 15]) {
-        CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<1, PaGqa, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaGqa::SMEM));
-        CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<2, PaGqa, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaGqa::SMEM));
-        attr_set[ctx->device & 15] = true;
-    }
-    AttnParams ap;
+    AttnParams ap{};
     ap.q = (const uint16_t *)Q; ap.out = (uint16_t *)out; ap.n = n; ap.nh = nh; ap.T = T; ap.pos0 = pos; ap.group = nh / nkv;
     ap.scale_log2 = scale * 1.4426950408889634f; ap.flags = flags; ap.err = ctx->dev_err;
-    const int total = ((n + PA_QT - 1) / PA_QT) * nh;
-    ap.counter = flags + total;
-    CWK_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)(total + 3) * sizeof(int), ctx->stream));
-    const int grid = std::min(total, ctx->sm_count);
-    {
-        CwkKernelTimer timer(ctx);
-        prefill_attn_kernel<2, PaGqa, true><<<grid, 384, PaGqa::SMEM, ctx->stream>>>(tm_k, tm_v, ap);
-        CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<2, gqa>");
-    }
-    prefill_attn_kernel<1, PaGqa, true><<<grid, 256, PaGqa::SMEM, ctx->stream>>>(tm_k, tm_v, ap);      // repairs flagged items only
-    CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<1, gqa>");
-    return CWK_OK;
+    return attn_launch<PaGqa, true>(ctx, ap, tm_k, tm_v, 0);
 }

@@ -136,3 +136,27 @@ def test_decode_streams_against_f32(attn, hd, nh, nkv, lens):
         s = torch.einsum("hd,thd->ht", q[b].float(), kk) / hd ** 0.5
         want = torch.einsum("ht,thd->hd", torch.softmax(s, -1), vv)
         assert float((got[b].float() - want).norm() / want.norm()) < 5e-3, b
+
+
+@pytest.mark.parametrize("climb", [False, True])
+@pytest.mark.parametrize("n,pos,nh,nkv", [(1, 3000, 4, 1), (100, 2900, 4, 4), (129, 2063, 16, 4), (512, 4500, 16, 4), (1024, 0, 4, 2), (257, 6, 12, 3),
+                                          (640, 11000, 16, 2)])
+def test_prefill_in_equal_shares_of_tiles(attn, n, pos, nh, nkv, climb):
+    """Few query tiles, many keys: the blocks share items, cuts fall inside and next to the diagonal; with climbing scores the
+    flagged segments are done again."""
+    hd = 256
+    g = torch.Generator(device="cuda").manual_seed(n + pos)
+    Q = torch.randn(n, nh, hd, device="cuda", generator=g).to(torch.bfloat16)
+    K = torch.randn(pos + n, nkv, hd, device="cuda", generator=g)
+    if climb:
+        K = 0.2 * K + torch.linspace(0, 9, pos + n, device="cuda")[:, None, None] * torch.sign(Q[n - 1, 0].float())
+    K = K.to(torch.bfloat16)
+    V = torch.randn(pos + n, nkv, hd, device="cuda", generator=g).to(torch.bfloat16)
+    got = attn.gqa_prefill(Q, K, V, pos)
+    attn.ctx.sync()
+    hidden = torch.arange(pos + n, device="cuda")[None, :] > pos + torch.arange(n, device="cuda")[:, None]
+    for h in range(nh):
+        s = (Q[:, h].double() @ K[:, h // (nh // nkv)].double().T / hd ** 0.5).masked_fill(hidden, -torch.inf)
+        want = torch.softmax(s, -1) @ V[:, h // (nh // nkv)].double()
+        err = (got[:, h].double() - want).norm() / want.norm()
+        assert err < 6e-3, (h, float(err))
