@@ -126,6 +126,25 @@ __device__ __forceinline__ bool attn_segment(AttnItem &it, int w, int g, int64_t
     return hi > lo;
 }
 
+// Two f32 in one register pair and the arithmetic on both at once (half the instructions of the softmax: its warps, not the
+// tensor pipe, are what a tile waits for).
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // Softmax groups and tiles. A tile's scores go from tensor memory through registers into P in a chain (barrier, load, maximum,
 // exponentials, barrier, store, fence) that takes longer than its MMAs. So in the fast form two of the four groups take the even tiles
 // and two the odd ones, a row's 64 keys between them, and the chains of two tiles overlap.
@@ -133,8 +152,9 @@ __device__ __forceinline__ bool attn_segment(AttnItem &it, int w, int g, int64_t
 // Persistent: one block per SM takes items from a global counter until none is left. The first TMA operation of a
 // block waits several thousand cycles for its tensor map, tensor memory is allocated once, and the loads of the next
 // item run under the epilogue of this one.
+template <int NWG> constexpr int PA_THREADS = 128 + 128 * NWG + (NWG == 4 ? 32 : 0);      // (the last warp: second issuer of the scores)
 template <int NWG, class CFG, bool GQA>      // NWG softmax warp groups: 4 = fast form, 1 = exact form
-__global__ void __launch_bounds__(128 + 128 * NWG, 1)
+__global__ void __launch_bounds__(PA_THREADS<NWG>, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_c, const AttnParams p) {
     constexpr int PA_DQK = CFG::DQK, PA_K_BYTES = CFG::K_BYTES, PA_CST = CFG::CST, PA_OFF_C = CFG::OFF_C, PA_OFF_P = CFG::OFF_P,
                   PA_OFF_BAR = CFG::OFF_BAR, PA_OFF_X = CFG::OFF_X;
@@ -146,7 +166,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + PA_OFF_BAR + 8 * PB_COUNT + 8);
     int4 *s_item = reinterpret_cast<int4 *>(sm + PA_OFF_X + 4096);      // ring of 8 items: {number, first tile, end, record}
-    constexpr int TG = NWG == 4 ? 2 : 1;             // groups that share a tile
+    constexpr int TG = NWG == 4 ? 2 : 1, QK_ISSUERS = NWG == 4 ? 2 : 1;      // groups that share a tile; issuers of the score MMAs
     float *s_m = reinterpret_cast<float *>(sm + PA_OFF_X), *s_l = s_m + 512;              // [4][128] each
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -160,8 +180,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_k) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_c) : "memory");
         for (int i = 0; i < PB_COUNT; i++) {
+            // (by tile: an arrival per softmax warp; 32 a warp on one barrier are served one after another)
             const bool by_tile = i >= PB_SEMPTY && i < PB_PEMPTY, by_soft = i == PB_QFULL || i == PB_OFREE || i == PB_XM || i == PB_XL;
-            mbar_init(bar(i), by_tile ? (uint32_t)(128 * TG) : by_soft ? (uint32_t)(128 * NWG) : 1u);
+            mbar_init(bar(i), by_tile ? (uint32_t)(4 * TG) : by_soft ? (uint32_t)(128 * NWG) : i == PB_QEMPTY ? QK_ISSUERS : 1u);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -258,11 +279,13 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 for (int j = (cc > PA_CST ? cc - PA_CST : 0); j < cc; j++)
                     mbar_wait(bar(PB_CFULL + j % PA_CST), (uint32_t)((j / PA_CST) & 1), p.err, 1005);
         }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer of the scores
+    } else if (warp == 1 || warp == 4 + 4 * NWG) {
+        // ------------------------------------------------------------ MMA issuers of the scores
         // The two products have issuers of their own (this warp and warp 3): a wait on an mbarrier costs a
-        // lone thread some 300 cycles even when the phase is long complete, and one thread doing all four
-        // waits of a tile in turn was the longest chain of the kernel.
+        // lone thread some 200 cycles even when the phase is long complete, and one thread doing all four
+        // waits of a tile in turn was the longest chain of the kernel. So was, after that, the one issuer of the scores: two
+        // waits, 12 or 16 MMAs and the commits took it 1650 cycles a tile, of which the tensor pipe works 400 to 500. In the fast
+        // form a second one (the last warp) takes every other tile.
         if (lane == 0) {
             constexpr uint32_t ID_QK = idesc_bf16(128, PA_KT, 0, 0);
             bool ok = true;
@@ -277,6 +300,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 tc_fence_after();
                 // scores of a tile: S[kc % 2] = Q Kx^T, three 64-wide blocks of the 192 dims, four 16-wide steps each
                 for (int i = it.lo; i < it.nt && ok; i++, kc++) {
+                    if (QK_ISSUERS == 2 && (kc & 1) != (warp == 1 ? 0 : 1)) continue;
                     const int ks = kc % PA_KST, ku = kc / PA_KST, sb = kc % PA_SBUF, su = kc / PA_SBUF;
                     ok = mbar_wait(bar(PB_KFULL + ks), (uint32_t)(ku & 1), p.err, 1012);
                     if (ok) ok = mbar_wait(bar(PB_SEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1013);
@@ -326,7 +350,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 if (ok) umma_commit(bar(PB_ODONE));
             }
         }
-    } else if (warp >= 4) {
+    } else {
         // ------------------------------------------------------------ softmax, (correction,) epilogue
         // A thread owns query row `row` (= its TMEM lane) and NC of the 64 key columns of its tiles.
         constexpr int NC = PA_KT / TG;
@@ -376,38 +400,47 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 return true;
             };
             if (NWG == 4 && (tc & 1) != odd) ok = reference();
-            for (int i = it.lo; i < nt && ok; i++, tc++) {
-                const int sb = tc & 1, su = tc >> 1;             // P buffer of this tile
-                if (NWG == 4 && sb != odd) continue;
-                const int s3 = tc % PA_SBUF;                      // its score buffer
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_SFULL + s3), (uint32_t)((tc / PA_SBUF) & 1), p.err, 1021));   // warp-uniform: the TMEM loads below are warp-wide
+            const int tc0 = tc;
+            tc += nt - it.lo;
+            for (int d = NWG == 4 ? (tc0 ^ odd) & 1 : 0; d < nt - it.lo; d += NWG == 4 ? 2 : 1) {
+                const int i = it.lo + d, sb = (tc0 + d) & 1, su = (tc0 + d) >> 1;      // the tile; its score and P buffers and their use
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_SFULL + sb), (uint32_t)(su & 1), p.err, 1021));   // warp-uniform: the TMEM loads below are warp-wide
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t v[NC];
 #pragma unroll
-                for (int c = 0; c < NC / 16; c++) TMEM_LD16(v, c * 16, tlane + PA_COL_S + s3 * PA_KT + cg * NC + c * 16);
+                for (int c = 0; c < NC / 16; c++) TMEM_LD16(v, c * 16, tlane + PA_COL_S + sb * PA_KT + cg * NC + c * 16);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 tc_fence_before();
-                mbar_arrive(bar(PB_SEMPTY + s3));
-                float s[NC];
-                float mt = -INFINITY;
-                const int64_t k0 = (int64_t)i * PA_KT + cg * NC;
-                if ((int64_t)i * PA_KT + PA_KT - 1 <= p.pos0 + q0) {   // every key of the tile is visible to every row of the item
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(PB_SEMPTY + sb));
+                const bool whole = (int64_t)i * PA_KT + PA_KT - 1 <= p.pos0 + q0;      // every key of the tile is visible to every row of the item
+                const int seen = (int)min(tq - (int64_t)i * PA_KT - cg * NC, (int64_t)PA_KT);      // the thread's keys 0 .. seen are visible
+                if (NWG == 4 && i == it.lo) {
+                    float mt = -INFINITY;
 #pragma unroll
-                    for (int j = 0; j < NC; j++) { s[j] = __uint_as_float(v[j]) * p.scale_log2; mt = fmaxf(mt, s[j]); }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < NC; j++) {
-                        s[j] = (k0 + j <= tq) ? __uint_as_float(v[j]) * p.scale_log2 : -INFINITY;
-                        mt = fmaxf(mt, s[j]);
-                    }
+                    for (int j = 0; j < NC; j++) mt = fmaxf(mt, whole || j <= seen ? __uint_as_float(v[j]) * p.scale_log2 : -INFINITY);
+                    s_m[cg * 128 + row] = mt;
+                    ok = reference();
+                    if (!ok) break;
                 }
+                // exponents relative to the reference: scale, difference and below the sum two at a time
+                float s[NC];
+                const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), minus_m = NWG == 4 ? pack_f32x2(-m, -m) : 0;
+#pragma unroll
+                for (int j = 0; j < NC; j += 2)
+                    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), scale2, minus_m), s[j], s[j + 1]);
+                if (!whole) {
+#pragma unroll
+                    for (int j = 0; j < NC; j++)
+                        if (j > seen) s[j] = -INFINITY;
+                }
+                float mt = s[0];
+#pragma unroll
+                for (int j = 1; j + 1 < NC; j += 2) mt = fmaxf(mt, fmaxf(s[j], s[j + 1]));
+                mt = fmaxf(mt, s[NC - 1]);
                 if (NWG == 4) {
-                    if (i == it.lo) {
-                        s_m[cg * 128 + row] = mt;
-                        ok = reference();
-                        if (!ok) break;
-                    } else if (mt > m + PA_RANGE) {
+                    if (mt > PA_RANGE) {
                         p.flags[it.flag] = 1;                        // out of the range this form covers: the exact form redoes the item
                         atomicAdd(p.counter + 2, 1);
                     }
@@ -419,7 +452,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     if (__any_sync(0xffffffffu, mine)) {
                         // some row's scores outran its reference exponent: rescale what it has accumulated. A row is its
                         // thread's TMEM lane; the value MMAs of the previous tile must have finished writing it.
-                        ok = mbar_wait(bar(PB_PEMPTY + ((tc - 1) & 1)), (uint32_t)(((tc - 1) >> 1) & 1), p.err, 1022);
+                        ok = mbar_wait(bar(PB_PEMPTY + ((tc0 + d - 1) & 1)), (uint32_t)(((tc0 + d - 1) >> 1) & 1), p.err, 1022);
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                         tc_fence_after();
@@ -438,16 +471,18 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     }
                 }
                 uint32_t pk[NC / 2];
-                float lsum = 0.f;
+                uint64_t lsum = 0;                                   // two f32 zeros
 #pragma unroll
                 for (int j = 0; j < NC; j += 2) {
-                    const float p0 = exp2f(s[j] - m), p1 = exp2f(s[j + 1] - m);
-                    lsum += p0 + p1;
+                    const float p0 = exp2f(NWG == 4 ? s[j] : s[j] - m), p1 = exp2f(NWG == 4 ? s[j + 1] : s[j + 1] - m);
+                    lsum = add_f32x2(lsum, pack_f32x2(p0, p1));
                     pk[j >> 1] = pack_bf16x2(p0, p1);
                 }
-                l += lsum;
+                float l0, l1;
+                unpack_f32x2(lsum, l0, l1);
+                l += l0 + l1;
                 // the P buffer of this parity was read by the value MMAs two tiles ago
-                ok = mbar_wait(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023);
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023));
                 if (!ok) break;
                 uint8_t *prow = sm + PA_OFF_P + sb * PA_P_BYTES + row * 128;
 #pragma unroll
@@ -455,7 +490,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     *reinterpret_cast<uint4 *>(prow + (((cg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 tc_fence_before();
-                mbar_arrive(bar(PB_PFULL + sb));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(PB_PFULL + sb));
             }
             if (!ok) break;
             {
@@ -621,11 +657,11 @@ int attn_launch(cwk_ctx *ctx, AttnParams ap, const CUtensorMap &tm_k, const CUte
     const int grid = ap.shares ? G : std::min(total, G);
     if (!exact_only) {
         CwkKernelTimer timer(ctx);
-        CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<4, CFG, GQA>, dim3(grid), dim3(640), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
+        CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<4, CFG, GQA>, dim3(grid), dim3(PA_THREADS<4>), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
         CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<4>");
     }
     // the repair pass: items whose flag is clear are skipped
-    CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<1, CFG, GQA>, dim3(grid), dim3(256), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
+    CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<1, CFG, GQA>, dim3(grid), dim3(PA_THREADS<1>), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
     CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<1>");
     if (ap.shares) {
         CWK_CUDA(ctx, cwk_launch_early(attn_merge_kernel<GQA>, dim3(total, PA_DV / 16), dim3(128), 0, ctx->stream, ap));
