@@ -90,14 +90,6 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
     // this block's tiles: a contiguous range of ONE sequence (so q and the weights are loaded once)
     const int blocks_per_seq = gridDim.x;
     const int b = blockIdx.y;
-    const int nb = p.n[b];
-    const int ntile = (nb + IT_KEYS - 1) / IT_KEYS;
-    const int t_begin = (int)((int64_t)ntile * blockIdx.x / blocks_per_seq);
-    const int t_end = (int)((int64_t)ntile * (blockIdx.x + 1) / blocks_per_seq);
-    const int nt = t_end - t_begin;
-    if (blockIdx.x == 0 && tid < 2) p.band[2 * b + tid] = 0;
-    if (nt <= 0) return;
-
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_keys) : "memory");
         for (int i = 0; i < IB_COUNT; i++) {
@@ -108,6 +100,16 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    cwk_pdl_launch();
+    cwk_pdl_wait();
+    const int nb = p.n[b];
+    const int ntile = (nb + IT_KEYS - 1) / IT_KEYS;
+    const int t_begin = (int)((int64_t)ntile * blockIdx.x / blocks_per_seq);
+    const int t_end = (int)((int64_t)ntile * (blockIdx.x + 1) / blocks_per_seq);
+    const int nt = t_end - t_begin;
+    if (blockIdx.x == 0 && tid < 2) p.band[2 * b + tid] = 0;
+    if (nt <= 0) return;
+
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -326,6 +328,8 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
     cg::cluster_group cl = cg::this_cluster();
     const unsigned rank = cl.block_rank();
     const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     const int nb = n[b];
     const float *s = approx + (int64_t)b * stride;
     float *f = refined + (int64_t)b * stride;
@@ -554,14 +558,13 @@ extern "C" int cwk_dsa_select(cwk_ctx *ctx, const void *keys, const float *kscal
     const int bps = std::max(1, std::min(tiles, ctx->sm_count / B));
     {
         CwkKernelTimer timer(ctx);
-        indexer_scores_tc_kernel<<<dim3(bps, B), IT_THREADS, I_SMEM, ctx->stream>>>(tm_keys, p);
+        CWK_CUDA(ctx, cwk_launch_early(indexer_scores_tc_kernel, dim3(bps, B), dim3(IT_THREADS), I_SMEM, ctx->stream, tm_keys, p));
         CWK_LAUNCH_CHECK(ctx, "indexer_scores_tc_kernel");
     }
     {
         CwkKernelTimer timer(ctx);
-        band_classify_kernel<<<dim3(TK_CL, B), TK_THREADS, BC_SMEM, ctx->stream>>>(approx, key_stride, n, want, refined, band_list, band,
-                                                                                  (const uint8_t *)keys, kscale, q, wt, keep_self, sel, sel_ld, nsel,
-                                                                                  (long long *)ctx->tc_trace);
+        CWK_CUDA(ctx, cwk_launch_early(band_classify_kernel, dim3(TK_CL, B), dim3(TK_THREADS), BC_SMEM, ctx->stream, approx, key_stride, n, want, refined, band_list, band,
+                                       (const uint8_t *)keys, kscale, q, wt, keep_self, sel, sel_ld, nsel, (long long *)ctx->tc_trace));
         CWK_LAUNCH_CHECK(ctx, "band_classify_kernel");
     }
     if (scores_out) CWK_CUDA(ctx, cudaMemcpyAsync(scores_out, refined, (size_t)B * key_stride * 4, cudaMemcpyDeviceToDevice, ctx->stream));

@@ -139,6 +139,8 @@ fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         for (int i = 0; i < GB_COUNT; i++) mbar_init(bar(i), (i >= GB_PEMPTY) ? 16u : 1u);      // PEMPTY: the promotion warps of both CTAs
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(G_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -294,6 +296,8 @@ fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
 
 // Adds up the parts of the tiles that were cut along K, in order. Four columns per thread, 64 threads per row.
 __global__ void __launch_bounds__(256) fp8_sum_parts_kernel(const GemmParams p) {
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     const int tile = p.full + (int)blockIdx.y, tn = tile / p.tiles_m;
     const bool second = tn >= p.tiles_a;
     const int row = (int)blockIdx.x * 4 + (int)(threadIdx.x >> 6), c = (int)(threadIdx.x & 63) * 4;
@@ -452,10 +456,10 @@ int cwk_fp8_linear_tc_launch2(cwk_ctx *ctx, const void *X, int64_t n, int64_t k,
     }
     const int units = p.full + rest * p.splits;
     CwkKernelTimer timer(ctx);
-    fp8_linear_tc_kernel<<<2 * std::min(units, pairs), G_THREADS, G_SMEM, ctx->stream>>>(tm_x, tm_w, tm_w2, p);
+    CWK_CUDA(ctx, cwk_launch_early(fp8_linear_tc_kernel, dim3(2 * std::min(units, pairs)), dim3(G_THREADS), G_SMEM, ctx->stream, tm_x, tm_w, tm_w2, p));
     CWK_LAUNCH_CHECK(ctx, "fp8_linear_tc_kernel");
     if (p.splits > 1) {
-        fp8_sum_parts_kernel<<<dim3(BM / 4, (unsigned)rest), 256, 0, ctx->stream>>>(p);
+        CWK_CUDA(ctx, cwk_launch_early(fp8_sum_parts_kernel, dim3(BM / 4, (unsigned)rest), dim3(256), 0, ctx->stream, p));
         CWK_LAUNCH_CHECK(ctx, "fp8_sum_parts_kernel");
     }
     return CWK_OK;

@@ -98,6 +98,8 @@ __global__ void __launch_bounds__(256) norm_rope_rows_warp_kernel(const float *i
     if (r >= nrows) return;
     const float *x = in + r * in_ld;
     const int np = norm_cols / 128;
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     float4 v[MAXV4];
     float ra = 0.f, rb = 0.f;
     if (lane < rope_cols / 2) {
@@ -173,6 +175,7 @@ __global__ void __launch_bounds__(256) rope_tail_kernel(const uint16_t *q, uint1
 // group of heads (blockIdx.y): the angle is formed once per thread and applied to the group's heads. The pairs'
 // divisors base^(2j / n_rope) -- the same values rope_cos_sin forms -- are computed once per block (n_rope <= 256).
 __global__ void __launch_bounds__(256) rope_q_inplace_kernel(uint16_t *q, int n, int nh, int nope, int n_rope, int64_t pos0, float base) {
+    cwk_pdl_launch();
     __shared__ float s_den[128];
     for (int jj = threadIdx.x; jj < n_rope / 2; jj += 256) s_den[jj] = (float)pow((double)base, (double)(2.0f * (float)jj / (float)n_rope));
     __syncthreads();
@@ -188,6 +191,7 @@ __global__ void __launch_bounds__(256) rope_q_inplace_kernel(uint16_t *q, int n,
         cs = (float)cd;
         sn = (float)sd;
     }
+    cwk_pdl_wait();                                        // (the angles are worked out under the kernel before)
     uint16_t *src = q + (int64_t)t * nh * (nope + n_rope) + nope + 2 * j;
 #pragma unroll 8
     for (int h = h0; h < h1; h++) {
@@ -334,8 +338,8 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
     if (!kva_done) s = cwk_fp8_linear(ctx, X, Wqa, Sqa, n, H, q_lora, QA, 0);
     if (s != CWK_OK) return s;
     if (norm_rope_warp_ok(QA, q_lora, q_lora, 0, qa_norm, QAn, q_lora))
-        norm_rope_rows_warp_kernel<12><<<(n + 7) / 8, 256, 0, ctx->stream>>>(QA, q_lora, q_lora, 0, (const uint16_t *)qa_norm, eps, rope_base,
-                                                                             pos0, QAn, q_lora, nullptr, 0, n);
+        CWK_CUDA(ctx, cwk_launch_early(norm_rope_rows_warp_kernel<12>, dim3((n + 7) / 8), dim3(256), 0, ctx->stream, QA, q_lora, q_lora, 0,
+                                       (const uint16_t *)qa_norm, eps, rope_base, pos0, QAn, q_lora, nullptr, 0, n));
     else
         norm_rope_rows_kernel<<<n, 256, 0, ctx->stream>>>(QA, q_lora, q_lora, 0, (const uint16_t *)qa_norm, eps, rope_base,
                                                           pos0, QAn, q_lora, nullptr, 0);
@@ -347,14 +351,14 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
         if (s != CWK_OK) return s;
     }
     if (norm_rope_warp_ok(KVA, row, kv_lora, rope, kva_norm, (uint16_t *)cache + pos0 * row, row))
-        norm_rope_rows_warp_kernel<12><<<(n + 7) / 8, 256, 0, ctx->stream>>>(KVA, row, kv_lora, rope, (const uint16_t *)kva_norm, eps, rope_base,
-                                                                             pos0, (uint16_t *)cache + pos0 * row, row, len, 1, n);
+        CWK_CUDA(ctx, cwk_launch_early(norm_rope_rows_warp_kernel<12>, dim3((n + 7) / 8), dim3(256), 0, ctx->stream, KVA, row, kv_lora, rope,
+                                       (const uint16_t *)kva_norm, eps, rope_base, pos0, (uint16_t *)cache + pos0 * row, row, len, 1, n));
     else
         norm_rope_rows_kernel<<<n, 256, 0, ctx->stream>>>(KVA, row, kv_lora, rope, (const uint16_t *)kva_norm, eps, rope_base,
                                                           pos0, (uint16_t *)cache + pos0 * row, row, len, 1);
     CWK_LAUNCH_CHECK(ctx, "norm_rope_rows_kernel(kv_a)");
     if (expanded_keys && cwk_mla_prefill_attn_tc_ok(Q, cache, Wuk, Qf, out)) {
-        rope_q_inplace_kernel<<<dim3((n * (rope / 2) + 255) / 256, nh >= 8 ? 4 : 1), 256, 0, ctx->stream>>>(Q, n, nh, nope, rope, pos0, rope_base);
+        CWK_CUDA(ctx, cwk_launch_early(rope_q_inplace_kernel, dim3((n * (rope / 2) + 255) / 256, nh >= 8 ? 4 : 1), dim3(256), 0, ctx->stream, Q, n, nh, nope, rope, pos0, rope_base));
         CWK_LAUNCH_CHECK(ctx, "rope_q_inplace_kernel");
         return cwk_mla_prefill_attn_tc(ctx, Q, cache, Wuk, Qf, (int *)((uint8_t *)len + up((size_t)n * 4)), pos0, n, nh, scale, out, ctx->force_mla_path == 3);
     }

@@ -624,8 +624,8 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnParams p) {
 }
 
 // The attention grid of both shapes: the fast form, the repair pass, and in share mode the merge. Shares where the longest
-// block of item-by-item dealing would have PA_MERGE_TILES more key tiles than an equal share (what records and merge cost).
-constexpr int PA_MERGE_TILES = 10;
+// block of item-by-item dealing would have PA_MERGE_TILES more key tiles than an equal share (what records and merge cost: 13 us, a tile 0.65).
+constexpr int PA_MERGE_TILES = 20;
 template <class CFG, bool GQA>
 int attn_launch(cwk_ctx *ctx, AttnParams ap, const CUtensorMap &tm_k, const CUtensorMap &tm_c, int exact_only) {
     static bool attr_set[16] = {false};
@@ -709,6 +709,8 @@ kexp_tc_kernel(const __grid_constant__ CUtensorMap tm_lat, const __grid_constant
         for (int i = 0; i < KB_COUNT; i++) mbar_init(bar(i), i >= KB_DEMPTY ? 128u : 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(256u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -869,7 +871,7 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, cons
         const int ntiles = (T + KX_TOK - 1) / KX_TOK;
         const int G = std::max(1, std::min(ntiles, ctx->sm_count / std::max(1, nh)));
         CwkKernelTimer timer(ctx);
-        kexp_tc_kernel<<<dim3(G, nh), 256, KX_SMEM, ctx->stream>>>(tm_lat, tm_w, kp);
+        CWK_CUDA(ctx, cwk_launch_early(kexp_tc_kernel, dim3(G, nh), dim3(256), KX_SMEM, ctx->stream, tm_lat, tm_w, kp));
         CWK_LAUNCH_CHECK(ctx, "kexp_tc_kernel");
     }
     AttnParams ap{};

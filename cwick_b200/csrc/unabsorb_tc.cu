@@ -52,6 +52,7 @@ unabsorb_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     const int h = blockIdx.y;
     const int ntiles = (p.n + UT_TOK - 1) / UT_TOK;
     const int nt = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;      // tiles g, g + G, ... of this head
+    cwk_pdl_launch();
     if (nt <= 0) return;
 
     if (tid == 0) {
@@ -59,6 +60,9 @@ unabsorb_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
         for (int i = 0; i < UB_COUNT; i++) mbar_init(bar(i), i >= UB_DEMPTY ? 128u : 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cwk_pdl_wait();
+    if (tid == 0) {
         // W_v[h] and the first two ring fills go out before the block-wide set-up
         mbar_expect_tx(bar(UB_WFULL), UT_W_BYTES);
         tma_load_3d(base + UT_OFF_W, &tm_w, 0, h * p.w_head_rows, 0, bar(UB_WFULL));
@@ -216,7 +220,7 @@ extern "C" int cwk_mla_unabsorb(cwk_ctx *ctx, const void *attn, const void *Wv, 
     const int ntiles = (n + UT_TOK - 1) / UT_TOK;
     const int G = std::max(1, std::min(ntiles, ctx->sm_count / std::max(1, nh)));
     CwkKernelTimer timer(ctx);
-    unabsorb_tc_kernel<<<dim3(G, nh), UT_THREADS, UT_SMEM, ctx->stream>>>(tm_a, tm_w, p);
+    CWK_CUDA(ctx, cwk_launch_early(unabsorb_tc_kernel, dim3(G, nh), dim3(UT_THREADS), UT_SMEM, ctx->stream, tm_a, tm_w, p));
     CWK_LAUNCH_CHECK(ctx, "unabsorb_tc_kernel");
     return CWK_OK;
 }

@@ -131,7 +131,7 @@ class Attn:
         if max_n is None:
             max_n = int(n.max().item())
         sel = torch.full((B, want + 1), -1, dtype=torch.int32, device=keys.device)
-        nsel = torch.zeros(B, dtype=torch.int32, device=keys.device)
+        nsel = torch.empty(B, dtype=torch.int32, device=keys.device)      # (every sequence's is written)
         sc = torch.zeros(B, T, dtype=torch.float32, device=keys.device) if return_scores else None
         st = self._dsa_select(self._h, keys.data_ptr(), kscale.data_ptr(), T, q.data_ptr(), wt.data_ptr(), n.data_ptr(), max_n, B, ih,
                               hd, want, 1 if keep_self else 0, sel.data_ptr(), want + 1, nsel.data_ptr(),
