@@ -25,10 +25,10 @@
 //     Per tile: S = Q Kx^T (12 MMAs, M 128 x N 64) into one of two TMEM score buffers; the softmax
 //     warps own one query row per thread (TMEM lane = row, so row maxima and sums need no shuffles),
 //     write P (bf16) to shared memory; O += P lat (4 MMAs, M 128 x N 256). The two products have
-//     issuer threads of their own and three score buffers, so the scores run up to two tiles ahead of the values and
-//     the tensor pipe works under the softmax.
+//     issuer threads of their own (the scores two), so the scores run ahead of the values and the tensor pipe works under
+//     the softmax.
 //     The kernel has two forms. The fast one splits the 64 keys of a row between two softmax warp groups
-//     (two threads per row) and never rescales: a row's reference exponent is its largest score of the first
+//     (two threads per row, another two groups for every other tile) and never rescales: a row's reference exponent is its largest score of the first
 //     tile, later scores may outrun it by up to 2^64 (bf16 P and the f32 accumulators have the range), and a
 //     block that sees more raises a flag. The exact one (one thread per row, lazy rescale of its own TMEM lane
 //     when a score outruns the reference by 2^8) runs right after it and recomputes the flagged blocks only.
