@@ -286,6 +286,8 @@ __global__ void __launch_bounds__(256) norm_chunk_kernel(const float *part, int 
     extern __shared__ __align__(16) float s_row[];
     const int t = blockIdx.x, len = blockIdx.y ? nb : na, ld = na + nb;
     const float *src = part + (int64_t)t * ld + (blockIdx.y ? na : 0);
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     for (int i = threadIdx.x * 4; i < len; i += 1024) {    // (na and nb are multiples of 8)
         float4 v = *reinterpret_cast<const float4 *>(src + i);
 #pragma unroll 8
@@ -950,7 +952,8 @@ int chunk_steps(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos0, int64_t
     const int nh = ly.nh, nope = ly.nope, vdim = ly.vdim, q_lora = ly.q_lora, kv_lora = ly.kv_lora, kv_dim = ly.kv_dim;
     const int64_t qw = (int64_t)nh * nope, vw = (int64_t)nh * vdim;
     std::vector<int> pieces;
-    for (int64_t left = n; left > 0; left -= pieces.back()) pieces.push_back(left > CHUNK_PIECE + CHUNK_PIECE / 2 ? CHUNK_PIECE : (int)left);
+    for (int64_t left = n; left > 0; left -= pieces.back())
+        pieces.push_back(left > CHUNK_PIECE + CHUNK_PIECE / 4 ? CHUNK_PIECE : left > CHUNK_PIECE * 3 / 4 ? CHUNK_PIECE / 2 : (int)left);
     const int64_t m = *std::max_element(pieces.begin(), pieces.end());
     const bool tc = chunk_tc_ok(ly, *std::min_element(pieces.begin(), pieces.end()));
     // device scratch, in bytes from g.d_buf: the activations of the whole chunk, the stages between of one piece
@@ -993,8 +996,8 @@ int chunk_steps(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos0, int64_t
             a.splits = cwk_split_gemm_splits(ctx, np, q_lora, kv_lora, (int)H);
             a.Y = d_part; a.ldy = q_lora + kv_lora;
             if ((s = cwk_split_gemm(ctx, a)) != CWK_OK) return s;
-            norm_chunk_kernel<<<dim3((unsigned)np, 2), 256, (size_t)std::max(q_lora, kv_lora) * 4, st>>>(d_part, a.splits, np, q_lora, kv_lora, ly.qa_n, ly.kva_n,
-                                                                                                     eps, d_qa, rows, ly.lbf ? nullptr : kva);
+            CWK_CUDA(ctx, cwk_launch_early(norm_chunk_kernel, dim3((unsigned)np, 2), dim3(256), (size_t)std::max(q_lora, kv_lora) * 4, st, (const float *)d_part, a.splits, np, q_lora,
+                                           kv_lora, ly.qa_n, ly.kva_n, eps, d_qa, rows, ly.lbf ? nullptr : kva));
             CwkSplitGemm q;
             q.n = np;
             q.A = d_qa; q.lda = q.ldw = q_lora; q.k = q_lora; q.W = (const uint16_t *)ly.qb->data; q.w_rows = qw; q.rows = (int)qw; q.ldy = qw;

@@ -88,6 +88,8 @@ lin_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         for (int i = 0; i < NBAR; i++) mbar_init(bar(i), 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"((uint32_t)BN) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -221,6 +223,8 @@ lin_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
 __global__ void __launch_bounds__(256) split_planes_kernel(const float4 *x, int64_t quads, uint2 *o) {
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     if (i >= quads) return;
     const float4 v = x[i];
     uint32_t a[3], b[3];
@@ -232,6 +236,8 @@ __global__ void __launch_bounds__(256) split_planes_kernel(const float4 *x, int6
 
 __global__ void __launch_bounds__(256) sum_partials_kernel(const float4 *part, int splits, int64_t quads, float4 *out, uint2 *planes) {
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    cwk_pdl_launch();
+    cwk_pdl_wait();
     if (i >= quads) return;
     float4 v = part[i];
     for (int s = 1; s < splits; s++) {
@@ -284,7 +290,7 @@ int launch(cwk_ctx *ctx, const CwkSplitGemm &g) {
     p.w_head_rows = g.w_head_rows; p.w_row_off = g.w_row_off; p.ldy = g.ldy; p.y = g.Y; p.err = ctx->dev_err;
     const dim3 grid((unsigned)(p.nb1 + (g.W2 ? (g.rows2 + BN - 1) / BN : 0)), (unsigned)((g.n + LS_TOK - 1) / LS_TOK),
                     (unsigned)(g.heads > 1 ? g.heads : g.splits));
-    lin_split_kernel<P, BN, WK, OUT><<<grid, 256, C::SMEM, ctx->stream>>>(ta, tw, tw2, p);
+    CWK_CUDA(ctx, cwk_launch_early(lin_split_kernel<P, BN, WK, OUT>, grid, dim3(256), C::SMEM, ctx->stream, ta, tw, tw2, p));
     CWK_LAUNCH_CHECK(ctx, "lin_split_kernel");
     return CWK_OK;
 }
@@ -315,14 +321,14 @@ int cwk_split_gemm(cwk_ctx *ctx, const CwkSplitGemm &g) {
 
 int cwk_split_planes(cwk_ctx *ctx, const float *x, int n, int k, uint16_t *planes) {
     const int64_t quads = (int64_t)n * k / 4;
-    split_planes_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, ctx->stream>>>((const float4 *)x, quads, (uint2 *)planes);
+    CWK_CUDA(ctx, cwk_launch_early(split_planes_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, ctx->stream, (const float4 *)x, quads, (uint2 *)planes));
     CWK_LAUNCH_CHECK(ctx, "split_planes_kernel");
     return CWK_OK;
 }
 
 int cwk_sum_partials(cwk_ctx *ctx, const float *part, int splits, int n, int cols, float *out, uint16_t *planes) {
     const int64_t quads = (int64_t)n * cols / 4;
-    sum_partials_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, ctx->stream>>>((const float4 *)part, splits, quads, (float4 *)out, (uint2 *)planes);
+    CWK_CUDA(ctx, cwk_launch_early(sum_partials_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, ctx->stream, (const float4 *)part, splits, quads, (float4 *)out, (uint2 *)planes));
     CWK_LAUNCH_CHECK(ctx, "sum_partials_kernel");
     return CWK_OK;
 }
