@@ -680,12 +680,18 @@ int attn_launch(cwk_ctx *ctx, AttnParams ap, const CUtensorMap &tm_k, const CUte
 
 // ---------------------------------------------------------------------------------------------------------------
 // Key expansion: Kx[h][c][0:128] = W_uk[h] lat[c], Kx[h][c][128:192] = k_rope[c].
-constexpr int KX_TOK = 128, KX_NOPE = 128;
-constexpr int KX_W_BYTES = KX_NOPE * PA_L * 2;        // 131072: eight [128 d][64 l] blocks
+//
+// Pairs of CTAs (M 256): each has 128 of a tile's 256 tokens and 64 of the head's 128 rows of W_uk, so that the weights take half the
+// shared memory and the latent ring has four stages; with the whole of W_uk in one CTA there was room for two, 64 KB in
+// flight per SM. What a tile waited for was its epilogue on four warps (3510 keys x 64 heads: 64 us, the stores 13, the MMAs
+// 18): now eight, a half of the columns each.
+constexpr int KX_TOK = 128, KX_NOPE = 128, KX_ST = 4;
+constexpr int KX_W_BYTES = KX_NOPE / 2 * PA_L * 2;    // 65536: eight [64 d][64 l] blocks
 constexpr int KX_A_BYTES = KX_TOK * 128 * 2;          // 32768: two [128 tok][64 l] blocks = one 128-wide chunk of the latent
-constexpr int KX_OFF_W = 0, KX_OFF_A = KX_W_BYTES, KX_OFF_STG = KX_OFF_A + 2 * KX_A_BYTES, KX_OFF_BAR = KX_OFF_STG + 4 * 4096;
-constexpr int KX_SMEM = KX_OFF_BAR + 256 + 1024;
-enum { KB_WFULL = 0, KB_AFULL = 1, KB_AEMPTY = 3, KB_DFULL = 5, KB_DEMPTY = 7, KB_COUNT = 9 };
+constexpr int KX_OFF_W = 0, KX_OFF_A = KX_W_BYTES, KX_OFF_STG = KX_OFF_A + KX_ST * KX_A_BYTES, KX_OFF_BAR = KX_OFF_STG + 8 * 4096;
+constexpr int KX_SMEM = KX_OFF_BAR + 256 + 1024, KX_THREADS = 384;
+static_assert(KX_SMEM <= 232448, "shared-memory budget");
+enum { KB_WFULL = 0, KB_AFULL = 1, KB_AEMPTY = KB_AFULL + KX_ST, KB_DFULL = KB_AEMPTY + KX_ST, KB_DEMPTY = KB_DFULL + 2, KB_COUNT = KB_DEMPTY + 2 };
 
 struct KexpParams {
     const uint16_t *cache;    // bf16 [T][576]
@@ -694,7 +700,7 @@ struct KexpParams {
     int *err;
 };
 
-__global__ void __launch_bounds__(256, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(KX_THREADS, 1)
 kexp_tc_kernel(const __grid_constant__ CUtensorMap tm_lat, const __grid_constant__ CUtensorMap tm_w, const KexpParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -705,56 +711,58 @@ kexp_tc_kernel(const __grid_constant__ CUtensorMap tm_lat, const __grid_constant
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + KX_OFF_BAR + 8 * KB_COUNT + 8);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int h = blockIdx.y;
-    const int ntiles = (p.T + KX_TOK - 1) / KX_TOK;
-    const int nt = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;     // tiles g, g + G, ...
+    const int h = blockIdx.y, rank = (int)cluster_rank();
+    const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const int ntiles = (p.T + 2 * KX_TOK - 1) / (2 * KX_TOK);
+    const int nt = (ntiles - pair + pairs - 1) / pairs;                                  // tiles g, g + G, ...
     if (nt <= 0) return;
     const int nch = nt * 4;                                                              // 128-wide chunks of the 512 latent dims
 
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_lat) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
-        for (int i = 0; i < KB_COUNT; i++) mbar_init(bar(i), i >= KB_DEMPTY ? 128u : 1u);
+        for (int i = 0; i < KB_COUNT; i++) mbar_init(bar(i), i >= KB_DEMPTY ? 16u : 1u);      // DEMPTY: the epilogue warps of both CTAs, at the first one's barrier
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cwk_pdl_launch();
     cwk_pdl_wait();
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(256u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(256u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
 
     if (warp == 0) {
         if (lane == 0) {
-            mbar_expect_tx(bar(KB_WFULL), KX_W_BYTES);
-            tma_load_3d(base + KX_OFF_W, &tm_w, 0, h * KX_NOPE, 0, bar(KB_WFULL));
+            if (rank == 0) mbar_expect_tx(bar(KB_WFULL), 2 * KX_W_BYTES);                // both CTAs' bytes are counted where the issuer waits
+            tma_load_3d_pair(base + KX_OFF_W, &tm_w, 0, h * KX_NOPE + rank * (KX_NOPE / 2), 0, cluster_addr(bar(KB_WFULL), 0));
             bool ok = true;
             int issued = 0;
             for (int c = 0; c < nch && ok; c++) {
-                const int slot = c & 1, use = c >> 1;
+                const int slot = c % KX_ST, use = c / KX_ST;
                 ok = mbar_wait(bar(KB_AEMPTY + slot), (uint32_t)((use & 1) ^ 1), p.err, 1101);
                 if (!ok) break;
-                const int tile = (int)blockIdx.x + (c >> 2) * (int)gridDim.x;
-                mbar_expect_tx(bar(KB_AFULL + slot), KX_A_BYTES);
-                tma_load_3d(base + KX_OFF_A + slot * KX_A_BYTES, &tm_lat, 0, tile * KX_TOK, (c & 3) * 2, bar(KB_AFULL + slot));
+                const int tile = pair + (c >> 2) * pairs;
+                if (rank == 0) mbar_expect_tx(bar(KB_AFULL + slot), 2 * KX_A_BYTES);
+                tma_load_3d_pair(base + KX_OFF_A + slot * KX_A_BYTES, &tm_lat, 0, (tile * 2 + rank) * KX_TOK, (c & 3) * 2, cluster_addr(bar(KB_AFULL + slot), 0));
                 issued = c + 1;
             }
-            if (!ok) {
+            if (!ok && rank == 0) {
                 mbar_wait(bar(KB_WFULL), 0, p.err, 1102);
-                for (int c = (issued > 2 ? issued - 2 : 0); c < issued; c++) mbar_wait(bar(KB_AFULL + (c & 1)), (uint32_t)((c >> 1) & 1), p.err, 1103);
+                for (int c = (issued > KX_ST ? issued - KX_ST : 0); c < issued; c++) mbar_wait(bar(KB_AFULL + c % KX_ST), (uint32_t)((c / KX_ST) & 1), p.err, 1103);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t ID = idesc_bf16(128, KX_NOPE, 0, 0);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t ID = idesc_bf16(2 * KX_TOK, KX_NOPE, 0, 0);
             const uint64_t dW = smem_desc(base + KX_OFF_W, 16, 1024);
             bool ok = mbar_wait(bar(KB_WFULL), 0, p.err, 1104);
             for (int c = 0; c < nch && ok; c++) {
-                const int slot = c & 1, use = c >> 1, ti = c >> 2, kc = c & 3, db = ti & 1;
+                const int slot = c % KX_ST, use = c / KX_ST, ti = c >> 2, kc = c & 3, db = ti & 1;
                 if (kc == 0) ok = mbar_wait(bar(KB_DEMPTY + db), (uint32_t)(((ti >> 1) & 1) ^ 1), p.err, 1105);
                 if (ok) ok = mbar_wait(bar(KB_AFULL + slot), (uint32_t)(use & 1), p.err, 1106);
                 if (!ok) break;
@@ -762,34 +770,34 @@ kexp_tc_kernel(const __grid_constant__ CUtensorMap tm_lat, const __grid_constant
                 const uint64_t dA = smem_desc(base + KX_OFF_A + slot * KX_A_BYTES, 16, 1024);
 #pragma unroll
                 for (int s = 0; s < 8; s++)       // chunk kc covers W blocks 2 kc and 2 kc + 1
-                    umma_bf16(tmem + db * KX_NOPE, dA + (uint64_t)(((s >> 2) * (KX_TOK * 128) + (s & 3) * 32) >> 4),
-                              dW + (uint64_t)((((kc * 2 + (s >> 2)) * (KX_NOPE * 128)) + (s & 3) * 32) >> 4), ID, (kc | s) != 0);
-                umma_commit(bar(KB_AEMPTY + slot));
-                if (kc == 3) umma_commit(bar(KB_DFULL + db));
+                    umma_bf16_pair(tmem + db * KX_NOPE, dA + (uint64_t)(((s >> 2) * (KX_TOK * 128) + (s & 3) * 32) >> 4),
+                                   dW + (uint64_t)((((kc * 2 + (s >> 2)) * (KX_NOPE / 2 * 128)) + (s & 3) * 32) >> 4), ID, (kc | s) != 0);
+                umma_commit_pair(bar(KB_AEMPTY + slot));
+                if (kc == 3) umma_commit_pair(bar(KB_DFULL + db));
             }
         }
     } else if (warp >= 4) {
-        const int q4 = warp & 3;
+        const int q4 = warp & 3, half = (warp - 4) >> 2;      // this warp's rows; its 64 columns, and half of the rows' rope tails
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
-        uint8_t *stg = sm + KX_OFF_STG + q4 * 4096;
+        uint8_t *stg = sm + KX_OFF_STG + (warp - 4) * 4096;
         bool ok = true;
         for (int ti = 0; ti < nt && ok; ti++) {
             const int db = ti & 1;
-            const int t0w = ((int)blockIdx.x + ti * (int)gridDim.x) * KX_TOK + q4 * 32;
+            const int t0w = ((pair + ti * pairs) * 2 + rank) * KX_TOK + q4 * 32;
             // rope tail first (independent of the MMAs): 128 bytes per token, eight lanes per row
 #pragma unroll
-            for (int r8 = 0; r8 < 8; r8++) {
-                const int rr = r8 * 4 + (lane >> 3), jj = lane & 7;
+            for (int r8 = 0; r8 < 4; r8++) {
+                const int rr = (half * 4 + r8) * 4 + (lane >> 3), jj = lane & 7;
                 if (t0w + rr < p.T) {
                     const uint4 w = *reinterpret_cast<const uint4 *>(p.cache + (int64_t)(t0w + rr) * PA_ROW + PA_L + jj * 8);
                     *reinterpret_cast<uint4 *>(p.kx + ((int64_t)h * p.T + t0w + rr) * PaMla::DQK + KX_NOPE + jj * 8) = w;
                 }
             }
-            ok = mbar_wait(bar(KB_DFULL + db), (uint32_t)((ti >> 1) & 1), p.err, 1107);
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(KB_DFULL + db), (uint32_t)((ti >> 1) & 1), p.err, 1107));
             if (!ok) break;
             tc_fence_after();
-#pragma unroll 1
-            for (int c = 0; c < 2; c++) {
+            {
+                const int c = half;
                 uint32_t v[64];
                 TMEM_LD16(v, 0, tlane + db * KX_NOPE + c * 64);
                 TMEM_LD16(v, 16, tlane + db * KX_NOPE + c * 64 + 16);
@@ -816,14 +824,16 @@ kexp_tc_kernel(const __grid_constant__ CUtensorMap tm_lat, const __grid_constant
                 __syncwarp();
             }
             tc_fence_before();
-            mbar_arrive(bar(KB_DEMPTY + db));
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(bar(KB_DEMPTY + db), 0));
         }
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();                                          // the pair's barriers and tensor memory stay until both are done
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
     }
 }
 
@@ -863,7 +873,7 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, cons
     const int T = (int)(pos0 + n);
     CUtensorMap tm_lat, tm_w, tm_k, tm_c;
     if (!encode3(&tm_lat, cache, (uint64_t)T, PA_L / 64, PA_ROW * 2, KX_TOK, 2) ||                 // latent dims only: block index 8 (rope) stays out
-        !encode3(&tm_w, Wuk, (uint64_t)nh * KX_NOPE, PA_L / 64, PA_L * 2, KX_NOPE, PA_L / 64) ||
+        !encode3(&tm_w, Wuk, (uint64_t)nh * KX_NOPE, PA_L / 64, PA_L * 2, KX_NOPE / 2, PA_L / 64) ||
         !encode3(&tm_k, kx, (uint64_t)nh * T, 3, PaMla::DQK * 2, PA_KT, 3) ||            // rows past a head's last key belong to the next head: every such key is masked
 
         !encode3(&tm_c, cache, (uint64_t)T, PA_L / 64, PA_ROW * 2, PA_KT, 4))
@@ -876,10 +886,10 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, cons
     {
         KexpParams kp;
         kp.cache = (const uint16_t *)cache; kp.kx = (uint16_t *)kx; kp.T = T; kp.nh = nh; kp.err = ctx->dev_err;
-        const int ntiles = (T + KX_TOK - 1) / KX_TOK;
-        const int G = std::max(1, std::min(ntiles, ctx->sm_count / std::max(1, nh)));
+        const int ntiles = (T + 2 * KX_TOK - 1) / (2 * KX_TOK);
+        const int G = std::max(1, std::min(ntiles, ctx->sm_count / 2 / std::max(1, nh)));      // pairs per head
         CwkKernelTimer timer(ctx);
-        CWK_CUDA(ctx, cwk_launch_early(kexp_tc_kernel, dim3(G, nh), dim3(256), KX_SMEM, ctx->stream, tm_lat, tm_w, kp));
+        CWK_CUDA(ctx, cwk_launch_early(kexp_tc_kernel, dim3(2 * G, nh), dim3(KX_THREADS), KX_SMEM, ctx->stream, tm_lat, tm_w, kp));
         CWK_LAUNCH_CHECK(ctx, "kexp_tc_kernel");
     }
     AttnParams ap{};
