@@ -132,6 +132,7 @@ class Context:
         if st != OK:
             raise CwkError(st, "cwk_ctx_create failed (no CUDA device, or not an sm_100 part)")
         self.h = h
+        self.address = h.value       # the handle as a plain integer, for the calls of `fast`; None once closed, so read at every call
         if stream is not None:
             self.check(self.lib.cwk_ctx_set_stream(self.h, vp(stream)))
 
@@ -161,8 +162,8 @@ class Context:
 
     def close(self):
         if getattr(self, "h", None):
-            self.lib.cwk_ctx_destroy(self.h)
-            self.h = None
+            h, self.h, self.address = self.h, None, None
+            self.lib.cwk_ctx_destroy(h)
 
     def __del__(self):
         try:

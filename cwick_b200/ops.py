@@ -26,7 +26,6 @@ class Attn:
         self.device = device
         self.ctx = _lib.Context(device, stream=torch.cuda.current_stream(device).cuda_stream)
         self.lib = self.ctx.lib
-        self._h = self.ctx.h.value
         # the calls of a decode step: plain integers and floats in, status out
         self._mla_decode, self._gqa_decode, self._dsa_select, self._gdn_scan = (
             _lib.fast(self.lib, "cwk_" + n) for n in ("mla_decode", "gqa_decode", "dsa_select", "gdn_scan"))
@@ -49,7 +48,7 @@ class Attn:
             scale = 1.0 / math.sqrt(192.0 if R else L)
         if out is None:
             out = torch.empty(B, nh, L, dtype=torch.bfloat16, device=q.device)
-        st = self._mla_decode(self._h, q.data_ptr(), cache.data_ptr(), seq_stride, ld, kv_len.data_ptr(), max_kv_len,
+        st = self._mla_decode(self.ctx.address, q.data_ptr(), cache.data_ptr(), seq_stride, ld, kv_len.data_ptr(), max_kv_len,
                               None if sel is None else sel.data_ptr(), 0 if sel is None else sel.shape[-1], B, nh, L, R, scale,
                               out.data_ptr(), n_splits)
         if st:
@@ -133,7 +132,7 @@ class Attn:
         sel = torch.full((B, want + 1), -1, dtype=torch.int32, device=keys.device)
         nsel = torch.empty(B, dtype=torch.int32, device=keys.device)      # (every sequence's is written)
         sc = torch.zeros(B, T, dtype=torch.float32, device=keys.device) if return_scores else None
-        st = self._dsa_select(self._h, keys.data_ptr(), kscale.data_ptr(), T, q.data_ptr(), wt.data_ptr(), n.data_ptr(), max_n, B, ih,
+        st = self._dsa_select(self.ctx.address, keys.data_ptr(), kscale.data_ptr(), T, q.data_ptr(), wt.data_ptr(), n.data_ptr(), max_n, B, ih,
                               hd, want, 1 if keep_self else 0, sel.data_ptr(), want + 1, nsel.data_ptr(),
                               None if sc is None else sc.data_ptr())
         if st:
@@ -152,7 +151,7 @@ class Attn:
             max_kv_len = int(kv_len.max().item())
         if out is None:
             out = torch.empty(B, nh, hd, dtype=torch.bfloat16, device=q.device)
-        st = self._gqa_decode(self._h, q.data_ptr(), K.data_ptr(), V.data_ptr(), T * nkv * hd, kv_len.data_ptr(), max_kv_len, B, nh, nkv,
+        st = self._gqa_decode(self.ctx.address, q.data_ptr(), K.data_ptr(), V.data_ptr(), T * nkv * hd, kv_len.data_ptr(), max_kv_len, B, nh, nkv,
                               hd, scale, out.data_ptr(), n_splits)
         if st:
             self.ctx.check(st)
@@ -222,7 +221,7 @@ class Attn:
         B, n, _ = up.shape
         _, nh, hv, hk = S.shape
         out = torch.empty(B, n, nh * hv, dtype=torch.float32, device=up.device)
-        st = self._gdn_scan(self._h, B, n, nh, hk, hv, kv_group, up.data_ptr(), gdec.data_ptr(), beta.data_ptr(), gate.data_ptr(),
+        st = self._gdn_scan(self.ctx.address, B, n, nh, hk, hv, kv_group, up.data_ptr(), gdec.data_ptr(), beta.data_ptr(), gate.data_ptr(),
                             a_log.data_ptr(), dt_bias.data_ptr(), norm.data_ptr(), rms_eps, S.data_ptr(), out.data_ptr())
         if st:
             self.ctx.check(st)
