@@ -44,6 +44,11 @@ constexpr int PA_QT = 128, PA_KT = 64, PA_DV = 256, PA_L = 512, PA_ROW = 576;
 constexpr int PA_C_BYTES = PA_KT * PA_DV * 2;         // 32768: four [64][64] blocks
 constexpr int PA_P_BYTES = PA_QT * PA_KT * 2;         // 16384: one [128][64] block
 constexpr int PA_KST = 3;
+// "Key tile here" has more barriers than the ring has slots: tile kc arrives at barrier kc % PA_KBAR. The two score issuers take
+// alternate tiles, so with one barrier per slot an issuer would wait for every SECOND phase of it, and a parity wait cannot tell
+// that phase from the one two before: with the copy of tile kc - 3 late and that of kc - 2 not, the issuer of kc - 2 went
+// on to kc before its slot had been filled. With an even number of barriers each has one issuer, which sees all of its phases.
+constexpr int PA_KBAR = 2 * PA_KST;
 constexpr int PA_OFF_K = 0;                            // (the query tile lives in tensor memory, not here)
 // The kernel serves two shapes. MLA prefill: 192-wide expanded keys, the 512 value columns in two halves, three value
 // stages. GQA prefill (Qwen3.5 layers): 256-wide keys and values of one KV head, two value stages (the key tiles are
@@ -67,8 +72,10 @@ constexpr uint32_t PA_COL_O = 0, PA_COL_S = 256, PA_COL_Q = 384;   // S buffers 
 constexpr float PA_LAZY = 8.f;                         // exact form: rescale when a score outruns the reference by 2^8
 constexpr float PA_RANGE = 64.f;                       // fast form: flag the block when a score outruns it by 2^64
 constexpr int PA_SBUF = 2;                             // score buffers in tensor memory
-enum { PB_QFULL = 0, PB_KFULL = 1, PB_KEMPTY = 4, PB_CFULL = 7, PB_CEMPTY = 10, PB_SFULL = 13, PB_SEMPTY = 15, PB_PFULL = 17, PB_PEMPTY = 19,
-       PB_ODONE = 21, PB_QEMPTY = 22, PB_OFREE = 23, PB_XM = 24, PB_XL = 25, PB_ITEM = 26, PB_COUNT = 34 };
+enum { PB_QFULL = 0, PB_KFULL = 1, PB_KEMPTY = PB_KFULL + PA_KBAR, PB_CFULL = PB_KEMPTY + PA_KST, PB_CEMPTY = PB_CFULL + 3, PB_SFULL = PB_CEMPTY + 3,
+       PB_SEMPTY = PB_SFULL + 2, PB_PFULL = PB_SEMPTY + 2, PB_PEMPTY = PB_PFULL + 2, PB_ODONE = PB_PEMPTY + 2, PB_QEMPTY, PB_OFREE, PB_XM, PB_XL, PB_ITEM,
+       PB_COUNT = PB_ITEM + 8 };
+static_assert(PA_KBAR % 2 == 0 && PA_KBAR % PA_KST == 0 && 8 * PB_COUNT + 16 <= 512, "barriers");
 
 struct AttnParams {
     const uint16_t *q;  // bf16 [n][nh][DQK] (MLA: rope part rotated)
@@ -247,14 +254,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     const int ks = kc % PA_KST, ku = kc / PA_KST;
                     ok = mbar_wait(bar(PB_KEMPTY + ks), (uint32_t)((ku & 1) ^ 1), p.err, 1001);
                     if (!ok) break;
-                    mbar_expect_tx(bar(PB_KFULL + ks), PA_K_BYTES);
-                    if (GQA) tma_load_3d(base + PA_OFF_K + ks * PA_K_BYTES, &tm_k, 0, i * PA_KT, (it.h / p.group) * (PA_DQK / 64), bar(PB_KFULL + ks));
-                    else tma_load_3d(base + PA_OFF_K + ks * PA_K_BYTES, &tm_k, 0, it.h * p.T + i * PA_KT, 0, bar(PB_KFULL + ks));
+                    const uint32_t full = bar(PB_KFULL + kc % PA_KBAR);
+                    mbar_expect_tx(full, PA_K_BYTES);
+                    if (GQA) tma_load_3d(base + PA_OFF_K + ks * PA_K_BYTES, &tm_k, 0, i * PA_KT, (it.h / p.group) * (PA_DQK / 64), full);
+                    else tma_load_3d(base + PA_OFF_K + ks * PA_K_BYTES, &tm_k, 0, it.h * p.T + i * PA_KT, 0, full);
                 }
             }
             if (!ok)        // drain the copies still in flight before leaving
                 for (int j = (kc > PA_KST ? kc - PA_KST : 0); j < kc; j++)
-                    mbar_wait(bar(PB_KFULL + j % PA_KST), (uint32_t)((j / PA_KST) & 1), p.err, 1004);
+                    mbar_wait(bar(PB_KFULL + j % PA_KBAR), (uint32_t)((j / PA_KBAR) & 1), p.err, 1004);
         }
     } else if (warp == 2) {
         // ------------------------------------------------------------ TMA producer of the latent ring (its slots come free much
@@ -301,8 +309,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 // scores of a tile: S[kc % 2] = Q Kx^T, three 64-wide blocks of the 192 dims, four 16-wide steps each
                 for (int i = it.lo; i < it.nt && ok; i++, kc++) {
                     if (QK_ISSUERS == 2 && (kc & 1) != (warp == 1 ? 0 : 1)) continue;
-                    const int ks = kc % PA_KST, ku = kc / PA_KST, sb = kc % PA_SBUF, su = kc / PA_SBUF;
-                    ok = mbar_wait(bar(PB_KFULL + ks), (uint32_t)(ku & 1), p.err, 1012);
+                    const int ks = kc % PA_KST, sb = kc % PA_SBUF, su = kc / PA_SBUF;
+                    ok = mbar_wait(bar(PB_KFULL + kc % PA_KBAR), (uint32_t)((kc / PA_KBAR) & 1), p.err, 1012);
                     if (ok) ok = mbar_wait(bar(PB_SEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1013);
                     if (!ok) break;
                     tc_fence_after();

@@ -182,3 +182,24 @@ def test_absorbed_route_agrees_with_the_expanded_key_route(attn):
     close(bf16_to_np(a)[[0, 1, 63, 64, 200, 332]], want)
     close(bf16_to_np(b)[[0, 1, 63, 64, 200, 332]], want)
     close(bf16_to_np(a), bf16_to_np(b))
+
+
+def test_keys_from_memory_behind_a_long_context(attn):
+    """16256 rows of 64 heads are 400 MB of expanded keys, more than L2 holds: their tiles reach the attention kernel from
+    memory, at uneven times and out of order. The same bytes from every call, and the absorbed route's values."""
+    n, pos0, nh, H, q_lora = 256, 16000, 64, 512, 256
+    m = make_model(57, H, q_lora, nh)
+    X = synth.normal_bf16(57, 9, (n, H))
+    cache0 = np.zeros((pos0 + n, LAT + ROPE), np.uint16)
+    cache0[:pos0] = synth.normal_bf16(57, 10, (pos0, LAT + ROPE))
+    dev = {k: (torch.from_numpy(v).cuda() if v.dtype != np.uint16 else to_bf16_cuda(v)) for k, v in m.items()}
+    x, cache = to_bf16_cuda(X), to_bf16_cuda(cache0)
+    args = (x, dev["Wqa"], dev["Sqa"], dev["Wqb"], dev["Sqb"], dev["Wkva"], dev["Skva"], dev["qa_n"], dev["kva_n"], dev["Wuk"], cache, pos0, nh)
+    first = attn.mla_prefill(*args)
+    for _ in range(40):
+        again = attn.mla_prefill(*args)
+    attn.ctx.sync()
+    assert torch.equal(first, again)
+    absorbed = _forced(attn, 2, lambda: attn.mla_prefill(*args))
+    attn.ctx.sync()
+    close(bf16_to_np(first), bf16_to_np(absorbed))
