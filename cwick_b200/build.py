@@ -1,5 +1,5 @@
-"""Builds libcwk_attn.so (every CUDA source under csrc/) for sm_100a with nvcc, and _pycall.so, the CPython entry points
-of the decode calls (csrc/pycall.c), with the host compiler.
+"""Builds libcwk_attn.so (every CUDA source under csrc/) for sm_100a with nvcc, and _pycall, the CPython entry points
+of the decode calls (csrc/pycall.c), with the host compiler and for the interpreter that runs this.
 
 The library is built in-tree next to this file so that it travels with the
 source tree; nothing is installed. `python -m cwick_b200.build` rebuilds it.
@@ -13,7 +13,8 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcwk_attn.so")
-PYCALL = os.path.join(HERE, "_pycall.so")
+# (the suffix names the interpreter: another one does not find this file, and binds through ctypes)
+PYCALL = os.path.join(HERE, "_pycall" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -30,17 +31,38 @@ def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
 
+def _older(path, deps):
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
+
+
+def _headers():
+    return glob.glob(os.path.join(os.path.dirname(HERE), "include", "*.h"))
+
+
 def needs_build():
-    if not os.path.exists(LIB) or not os.path.exists(PYCALL):
-        return True
-    t = min(os.path.getmtime(LIB), os.path.getmtime(PYCALL))
-    deps = sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + [os.path.join(CSRC, "pycall.c")] + \
-        glob.glob(os.path.join(os.path.dirname(HERE), "include", "*.h"))
-    return any(os.path.getmtime(d) > t for d in deps)
+    return _older(LIB, sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + _headers())
+
+
+def build_pycall(force=False):
+    """The compiled binding. Without it (no CPython headers here, another interpreter) the calls go through ctypes, so a
+    failure is reported and is not an error; a module of an older source does not stay behind it."""
+    src = os.path.join(CSRC, "pycall.c")
+    if not force and not _older(PYCALL, [src] + _headers()):
+        return
+    for old in (PYCALL, os.path.join(HERE, "_pycall.so")):
+        if os.path.exists(old):
+            os.remove(old)
+    cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o", PYCALL, "-L" + HERE,
+           "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+    try:
+        subprocess.run(cmd, check=True, capture_output=True, text=True)
+    except (OSError, subprocess.CalledProcessError) as e:
+        sys.stderr.write("_pycall was not built (calls go through ctypes, 2.4 us more each): %s\n" % (getattr(e, "stderr", None) or e))
 
 
 def build(force=False, verbose=False):
     if not force and not needs_build():
+        build_pycall()
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     objdir = os.path.join(HERE, "build")
@@ -63,8 +85,7 @@ def build(force=False, verbose=False):
         raise RuntimeError("nvcc failed")
     cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-lcudart"]
     subprocess.check_call(cmd)
-    subprocess.check_call([os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
-                           os.path.join(CSRC, "pycall.c"), "-o", PYCALL, "-L" + HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"])
+    build_pycall(force=True)
     return LIB
 
 

@@ -106,13 +106,15 @@ def load():
 
 
 def fast(lib, name):
-    """The entry point `name`, called with plain integers (addresses, sizes) and floats: through the compiled module where it
-    belongs to the loaded library and has the function, else through ctypes."""
+    """The entry point `name`, called with plain integers (addresses, sizes) and floats: through the compiled module where
+    this interpreter has one, else through ctypes."""
     if lib is _lib:
-        from . import _pycall
-        fn = getattr(_pycall, name, None)
-        if fn is not None:
-            return fn
+        try:
+            from . import _pycall
+        except ImportError:                  # not built, or built for another interpreter
+            pass
+        else:
+            return getattr(_pycall, name)
     return getattr(lib, name)
 
 
