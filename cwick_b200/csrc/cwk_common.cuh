@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/cwk_attn.h"
+#include "buffer_pool.cuh"
 
 struct cwk_ctx {
     int device = 0;
@@ -21,6 +22,7 @@ struct cwk_ctx {
     // workspace of the composite entry points (prefill): separate from the split scratch
     void *work = nullptr;
     size_t work_bytes = 0;
+    CwkBufferUse use;                         // where scratch and work are in use
     // FP8 weights widened to bf16 for the tensor-core projection
     void *wbf16 = nullptr;
     size_t wbf16_bytes = 0;
@@ -61,9 +63,6 @@ int cwk_check_cuda(cwk_ctx *ctx, cudaError_t e, const char *what);
 int cwk_reserve_scratch(cwk_ctx *ctx, size_t bytes);
 int cwk_reserve_stage(cwk_ctx *ctx, size_t dev_bytes, size_t pin_bytes);
 int cwk_reserve_work(cwk_ctx *ctx, size_t bytes);
-// Device buffers that go from one context to the next (cwk_ctx.cu).
-cudaError_t cwk_buffer_alloc(int device, size_t bytes, void **p, size_t *granted);
-void cwk_buffer_free(int device, void *p, size_t bytes);
 // After a stream synchronise: turn a kernel-side give-up code into CWK_ERR_STATE.
 int cwk_check_device_error(cwk_ctx *ctx);
 // Allocate the error word on first use: pinned, mapped host memory, so the host reads it without a copy.

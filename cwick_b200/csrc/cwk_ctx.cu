@@ -1,66 +1,27 @@
 // cwk_ctx.cu -- context lifecycle, error text, scratch and staging buffers.
 #include <cstdarg>
 
-#include <mutex>
-
 #include "cwk_common.cuh"
 
-// ---- device buffers between contexts ---------------------------------------------------------------------------------
-// A context that goes leaves its work buffers to the next one on its device: a server makes and drops contexts with its
-// request slots, and a few megabytes from cudaMalloc take half a millisecond of the next slot's first call. At most
-// POOL_BYTES per device wait here, given back when the device's last context goes. Every buffer comes in after a
-// device synchronise (a context may have used several streams), so it has no user left.
 namespace {
-constexpr size_t POOL_BYTES = 256u << 20;
-struct PoolBuffer {
-    void *p;
-    size_t bytes;
-};
-struct Pool {
-    std::vector<PoolBuffer> free_;
-    size_t held = 0;
-    int contexts = 0;
-};
-std::mutex g_pool_mu;
-Pool g_pool[16];
-Pool &pool_of(int device) { return g_pool[device & 15]; }
-}  // namespace
+CwkBufferPool g_pool;
 
-// At least `bytes` on the current device, which is `device`; *granted is what there is.
-cudaError_t cwk_buffer_alloc(int device, size_t bytes, void **p, size_t *granted) {
-    {
-        std::lock_guard<std::mutex> l(g_pool_mu);
-        Pool &pool = pool_of(device);
-        int best = -1;
-        for (int i = 0; i < (int)pool.free_.size(); i++) {
-            const size_t have = pool.free_[i].bytes;
-            if (have >= bytes && have / 4 <= bytes && (best < 0 || have < pool.free_[best].bytes)) best = i;
-        }
-        if (best >= 0) {
-            *p = pool.free_[best].p;
-            *granted = pool.free_[best].bytes;
-            pool.held -= *granted;
-            pool.free_.erase(pool.free_.begin() + best);
-            return cudaSuccess;
-        }
+// At least `bytes` in a buffer of the context; one that is too small makes room for one of `want`.
+int reserve(cwk_ctx *ctx, void **p, size_t *have, size_t bytes, size_t want) {
+    ctx->use.use(ctx->stream);
+    if (bytes <= *have) return CWK_OK;
+    if (*p) {
+        CWK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        void *old = *p;
+        const size_t n = *have;
+        *p = nullptr;
+        *have = 0;
+        CWK_CUDA(ctx, g_pool.free(ctx->device, old, n, ctx->use.known()));
     }
-    *granted = bytes;
-    return cudaMalloc(p, bytes);
+    CWK_CUDA(ctx, g_pool.alloc(ctx->device, want, p, have));
+    return CWK_OK;
 }
-// The caller has synchronised the device.
-void cwk_buffer_free(int device, void *p, size_t bytes) {
-    if (!p) return;
-    {
-        std::lock_guard<std::mutex> l(g_pool_mu);
-        Pool &pool = pool_of(device);
-        if (pool.contexts > 0 && pool.held + bytes <= POOL_BYTES) {
-            pool.free_.push_back({p, bytes});
-            pool.held += bytes;
-            return;
-        }
-    }
-    cudaFree(p);
-}
+}  // namespace
 
 int cwk_fail(cwk_ctx *ctx, int status, const char *fmt, ...) {
     if (ctx) {
@@ -78,29 +39,8 @@ int cwk_check_cuda(cwk_ctx *ctx, cudaError_t e, const char *what) {
                     "%s: %s", what, cudaGetErrorString(e));
 }
 
-int cwk_reserve_scratch(cwk_ctx *ctx, size_t bytes) {
-    if (bytes <= ctx->scratch_bytes) return CWK_OK;
-    if (ctx->scratch) {
-        CWK_CUDA(ctx, cudaDeviceSynchronize());
-        cwk_buffer_free(ctx->device, ctx->scratch, ctx->scratch_bytes);
-        ctx->scratch = nullptr;
-        ctx->scratch_bytes = 0;
-    }
-    CWK_CUDA(ctx, cwk_buffer_alloc(ctx->device, bytes + (bytes >> 2), (void **)&ctx->scratch, &ctx->scratch_bytes));
-    return CWK_OK;
-}
-
-int cwk_reserve_work(cwk_ctx *ctx, size_t bytes) {
-    if (bytes <= ctx->work_bytes) return CWK_OK;
-    if (ctx->work) {
-        CWK_CUDA(ctx, cudaDeviceSynchronize());
-        cwk_buffer_free(ctx->device, ctx->work, ctx->work_bytes);
-        ctx->work = nullptr;
-        ctx->work_bytes = 0;
-    }
-    CWK_CUDA(ctx, cwk_buffer_alloc(ctx->device, bytes, &ctx->work, &ctx->work_bytes));
-    return CWK_OK;
-}
+int cwk_reserve_scratch(cwk_ctx *ctx, size_t bytes) { return reserve(ctx, (void **)&ctx->scratch, &ctx->scratch_bytes, bytes, bytes + (bytes >> 2)); }
+int cwk_reserve_work(cwk_ctx *ctx, size_t bytes) { return reserve(ctx, &ctx->work, &ctx->work_bytes, bytes, bytes); }
 
 int cwk_reserve_stage(cwk_ctx *ctx, size_t dev_bytes, size_t pin_bytes) {
     if (dev_bytes > ctx->stage_dev_bytes) {
@@ -163,10 +103,7 @@ int cwk_ctx_create(int device, cwk_ctx **out) {
         return CWK_ERR_CUDA;
     }
     c->own_stream = true;
-    {
-        std::lock_guard<std::mutex> l(g_pool_mu);
-        pool_of(device).contexts++;
-    }
+    g_pool.add_context(device);
     *out = c;
     return CWK_OK;
 }
@@ -174,10 +111,10 @@ int cwk_ctx_create(int device, cwk_ctx **out) {
 void cwk_ctx_destroy(cwk_ctx *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
-    cudaDeviceSynchronize();
-    cwk_buffer_free(ctx->device, ctx->scratch, ctx->scratch_bytes);
+    const bool idle = ctx->use.idle(ctx->stream);
+    g_pool.free(ctx->device, ctx->scratch, ctx->scratch_bytes, idle);
     if (ctx->stage_dev) cudaFree(ctx->stage_dev);
-    cwk_buffer_free(ctx->device, ctx->work, ctx->work_bytes);
+    g_pool.free(ctx->device, ctx->work, ctx->work_bytes, idle);
     if (ctx->wbf16) cudaFree(ctx->wbf16);
     if (ctx->stage_pin) cudaFreeHost(ctx->stage_pin);
     if (ctx->dev_err) cudaFreeHost(ctx->dev_err);
@@ -186,25 +123,17 @@ void cwk_ctx_destroy(cwk_ctx *ctx) {
     cwk_fp8_weight_cache_free(ctx);
     for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
-    std::vector<PoolBuffer> last;
-    {
-        std::lock_guard<std::mutex> l(g_pool_mu);
-        Pool &pool = pool_of(ctx->device);
-        if (--pool.contexts == 0) {
-            last.swap(pool.free_);
-            pool.held = 0;
-        }
-    }
-    for (const PoolBuffer &b : last) cudaFree(b.p);
+    g_pool.drop_context(ctx->device);
     delete ctx;
 }
 
 int cwk_ctx_set_stream(cwk_ctx *ctx, void *cuda_stream) {
     if (!ctx) return CWK_ERR_ARGUMENT;
     if (ctx->own_stream && ctx->stream) {
-        cudaStreamSynchronize(ctx->stream);
+        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) ctx->use.lose();
         cudaStreamDestroy(ctx->stream);
-    }
+    } else if (ctx->stream != (cudaStream_t)cuda_stream && (ctx->scratch || ctx->work))
+        ctx->use.lose();                                   // (the stream before, which is the caller's, may still have work)
     ctx->stream = (cudaStream_t)cuda_stream;
     ctx->own_stream = false;
     return CWK_OK;
