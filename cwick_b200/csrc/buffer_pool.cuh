@@ -44,7 +44,7 @@ private:
 
 class CwkBufferPool {
 public:
-    static constexpr size_t POOL_BYTES = 256u << 20;
+    static constexpr size_t POOL_BYTES = 384u << 20;      // one of the largest workspaces (gdn_chunk.cu, 320 MB), or many of the others
 
     void add_context(int device) {
         std::lock_guard<std::mutex> l(mu_);

@@ -105,11 +105,16 @@ struct GdnChunkParams {
     float *S, *out;
     float *ws;                    // per (slot, head, chunk): W [64][128] | U~, then U, transposed [128][64] | M [64][64] | S0 [128 value][128 key] | G [64], its remainders [64]
     int n;                        // positions per slot
-    int nchunks, nh, kv_group;
+    int left;                     // positions of a slot from the segment's first on (the arrays begin there)
+    int nchunks, nh, kv_group;    // chunks of the segment
     float rms_eps;
 };
 constexpr int WS_U = GC * GD, WS_M = 2 * GC * GD, WS_S = WS_M + GC * GC, WS_G = WS_S + GD * GD;
 constexpr int64_t WS_PER = WS_G + 2 * GC;
+// Bytes of workspace in use at a time. A cut costs the ends of three kernels, most of it the last, half-empty wave of the
+// prep kernel: 4096 positions x 32 heads (303 MB) 573 us whole, 607 in two segments, 669 in four; 16384 positions 2207 whole
+// (1.2 GB), 2286 in four segments. So a prompt of that common size stays whole, and longer ones stay within its bound.
+constexpr int64_t WS_MAX = 320 << 20;
 
 __device__ __forceinline__ float *ws_of(const GdnChunkParams &p, int b, int vh, int c) {
     return p.ws + (((int64_t)b * p.nh + vh) * p.nchunks + c) * WS_PER;
@@ -170,7 +175,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnChunkPa
     const int c = blockIdx.x, kh = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int key_dim = (p.nh / p.kv_group) * GD, val_dim = p.nh * GD, qkv_dim = 2 * key_dim + val_dim;
     const int64_t pos0 = (int64_t)b * p.n + (int64_t)c * GC;
-    const int valid = min(GC, p.n - c * GC);
+    const int valid = min(GC, p.left - c * GC);
     const float *row0 = p.up + pos0 * qkv_dim;
     for (int x = tid; x < GC * (GD / 4); x += 256) {
         const int t = x >> 5, q = x & 31;
@@ -422,7 +427,7 @@ __global__ void __launch_bounds__(256, 1) gdn_chunk_scan_kernel(const GdnChunkPa
     const float *ksrc = p.up + ((int64_t)b * p.n + warp) * qkv_dim + key_dim + (int64_t)kh * GD + lane * 4;
     auto issue = [&](int c) {                              // chunks in order
         if (c < p.nchunks) {
-            const int valid = p.n - c * GC - warp;
+            const int valid = p.left - c * GC - warp;
             float *dw = sW + (c & 1) * GC * GD, *dk = sK + (c & 1) * GC * GD;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -588,7 +593,7 @@ __global__ void __launch_bounds__(512, 1) gdn_chunk_out_kernel(const GdnChunkPar
         if (li >= items) return;
         const int c = li % p.nchunks, bh = li / p.nchunks, vh = bh % p.nh, b = bh / p.nh;      // (slot, head, chunk) with the chunk fastest
         lw = p.ws + (int64_t)li * WS_PER;
-        lvalid = cr < p.n - c * GC;
+        lvalid = cr < p.left - c * GC;
         lq = p.up + ((int64_t)b * p.n + (int64_t)c * GC + (lvalid ? cr : 0)) * qkv_dim + (int64_t)(vh / p.kv_group) * GD + cq;
     };
     auto issue = [&](int step) {
@@ -663,7 +668,7 @@ __global__ void __launch_bounds__(512, 1) gdn_chunk_out_kernel(const GdnChunkPar
                     for (int i = 0; i < 4; i++) r[m][k][i] += acc[m][k].sum(i);
         }
         const int64_t pos0 = (int64_t)b * p.n + (int64_t)c * GC;
-        const int valid = min(GC, p.n - c * GC);
+        const int valid = min(GC, p.left - c * GC);
 #pragma unroll
         for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -718,8 +723,17 @@ bool cwk_gdn_chunked_ok(int kv_group, const float *up, const float *gate, const 
 
 int cwk_gdn_scan_chunked(cwk_ctx *ctx, int B, int n, int nh, int kv_group, const float *up, const float *gdec, const float *beta, const float *gate,
                          const float *a_log, const float *dt_bias, const float *norm, float rms_eps, float *S, float *out) {
-    const int nchunks = (n + GC - 1) / GC;
-    int s = cwk_reserve_work(ctx, (size_t)B * nh * nchunks * WS_PER * sizeof(float));
+    // Segments of chunks, one after another, and groups of slots where there are many: the workspace is bounded whatever the
+    // prompt's length, and the state goes from segment to segment in S.
+    const int all = (n + GC - 1) / GC;
+    const auto even = [](int total, int64_t most) {        // as few parts of at most `most` as it takes, alike
+        const int parts = (int)((total + most - 1) / most);
+        return (total + parts - 1) / parts;
+    };
+    constexpr int64_t room = WS_MAX / (WS_PER * (int64_t)sizeof(float));
+    const int nb = even(B, std::max<int64_t>(1, std::min<int64_t>(B, room / ((int64_t)nh * std::min(all, 8)))));
+    const int seg = even(all, std::max<int64_t>(1, std::min<int64_t>(all, room / ((int64_t)nh * nb))));
+    int s = cwk_reserve_work(ctx, (size_t)nb * nh * seg * WS_PER * sizeof(float));
     if (s != CWK_OK) return s;
     static bool attr_set[16] = {false};
     if (!attr_set[ctx->device & 15]) {
@@ -728,18 +742,27 @@ int cwk_gdn_scan_chunked(cwk_ctx *ctx, int B, int n, int nh, int kv_group, const
         CWK_CUDA(ctx, cudaFuncSetAttribute(gdn_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_STAGES * OUT_STAGE_FLOATS * 4));
         attr_set[ctx->device & 15] = true;
     }
+    const int64_t val_dim = (int64_t)nh * GD, qkv_dim = 2 * (int64_t)(nh / kv_group) * GD + val_dim;
     GdnChunkParams p;
-    p.up = up; p.gdec = gdec; p.beta = beta; p.gate = gate; p.a_log = a_log; p.dt_bias = dt_bias; p.norm = norm; p.S = S; p.out = out;
-    p.ws = (float *)ctx->work; p.n = n; p.nchunks = nchunks; p.nh = nh; p.kv_group = kv_group; p.rms_eps = rms_eps;
-    gdn_chunk_prep_kernel<<<dim3(nchunks, nh / kv_group, B), 256, PREP_FLOATS * 4, ctx->stream>>>(p);
-    CWK_LAUNCH_CHECK(ctx, "gdn_chunk_prep_kernel");
-    {
-        CwkKernelTimer timer(ctx);
-        gdn_chunk_scan_kernel<<<dim3(GD / GJ, nh, B), 256, SCAN_FLOATS * 4, ctx->stream>>>(p);
-        CWK_LAUNCH_CHECK(ctx, "gdn_chunk_scan_kernel");
+    p.a_log = a_log; p.dt_bias = dt_bias; p.norm = norm; p.ws = (float *)ctx->work; p.n = n; p.nh = nh; p.kv_group = kv_group; p.rms_eps = rms_eps;
+    for (int b0 = 0; b0 < B; b0 += nb) {
+        const int slots = std::min(nb, B - b0);
+        p.S = S + (int64_t)b0 * nh * GD * GD;
+        for (int c0 = 0; c0 < all; c0 += seg) {
+            const int64_t at = (int64_t)b0 * n + (int64_t)c0 * GC;
+            p.up = up + at * qkv_dim; p.gdec = gdec + at * nh; p.beta = beta + at * nh; p.gate = gate + at * val_dim; p.out = out + at * val_dim;
+            p.left = n - c0 * GC; p.nchunks = std::min(seg, all - c0);
+            gdn_chunk_prep_kernel<<<dim3(p.nchunks, nh / kv_group, slots), 256, PREP_FLOATS * 4, ctx->stream>>>(p);
+            CWK_LAUNCH_CHECK(ctx, "gdn_chunk_prep_kernel");
+            {
+                CwkKernelTimer timer(ctx);
+                gdn_chunk_scan_kernel<<<dim3(GD / GJ, nh, slots), 256, SCAN_FLOATS * 4, ctx->stream>>>(p);
+                CWK_LAUNCH_CHECK(ctx, "gdn_chunk_scan_kernel");
+            }
+            const int items = slots * nh * p.nchunks;
+            gdn_chunk_out_kernel<<<std::min(items, ctx->sm_count), 512, OUT_STAGES * OUT_STAGE_FLOATS * 4, ctx->stream>>>(p, items);
+            CWK_LAUNCH_CHECK(ctx, "gdn_chunk_out_kernel");
+        }
     }
-    const int items = B * nh * nchunks;
-    gdn_chunk_out_kernel<<<std::min(items, ctx->sm_count), 512, OUT_STAGES * OUT_STAGE_FLOATS * 4, ctx->stream>>>(p, items);
-    CWK_LAUNCH_CHECK(ctx, "gdn_chunk_out_kernel");
     return CWK_OK;
 }

@@ -409,7 +409,8 @@ CWK_API int cwk_kda_step(cwk_ctx *ctx, int B, int nh, int hd, float lower, float
  * head_k 64 or 128, head_v a multiple of 32 up to 128. A decode step and a short call run position by position, in the
  * reference's summation order. A prompt (n >= 128, head dims 128 x 128, 16-byte aligned arrays) runs chunk-parallel, 64
  * positions at a time: the same recurrence with its f32 sums in another order, so those results agree with the reference
- * to rounding (about 1e-5 relative), not bit for bit; its workspace inside the context is 148 KB per (slot, head, chunk).
+ * to rounding (about 1e-5 relative), not bit for bit; its workspace inside the context is 148 KB per (slot, head, chunk),
+ * 320 MB at most: longer prompts and more slots go in segments.
  * cwk_ctx_force_mla_path(ctx, 0) keeps every call on the position-serial kernel. */
 CWK_API int cwk_gdn_scan(cwk_ctx *ctx, int B, int n, int nh, int head_k, int head_v, int kv_group, const float *up,
                          const float *gdec, const float *beta, const float *gate, const float *a_log, const float *dt_bias,

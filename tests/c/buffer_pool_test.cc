@@ -82,11 +82,12 @@ int main() {
     {   // at most POOL_BYTES wait
         CwkBufferPool pool;
         pool.add_context(0);
-        void *p[6];
-        size_t n[6];
-        for (int i = 0; i < 6; i++) pool.alloc(0, 60 * MB, &p[i], &n[i]);
-        for (int i = 0; i < 6; i++) pool.free(0, p[i], n[i], true);
-        CHECK(live.size() == CwkBufferPool::POOL_BYTES / (60 * MB) && frees == 2);
+        constexpr int fit = CwkBufferPool::POOL_BYTES / (60 * MB), all = fit + 2;
+        void *p[all];
+        size_t n[all];
+        for (int i = 0; i < all; i++) pool.alloc(0, 60 * MB, &p[i], &n[i]);
+        for (int i = 0; i < all; i++) pool.free(0, p[i], n[i], true);
+        CHECK(live.size() == fit && frees == 2);
         pool.drop_context(0);
         CHECK(live.empty());
         frees = 0;

@@ -79,7 +79,7 @@ def test_prompt_goes_through_the_chunk_parallel_scan(attn, B, n):
     """A prompt of at least two 64-position chunks (head dims 128 x 128) is scanned chunk-parallel: the same recurrence
     with its sums in another order, so the bar is a tolerance (1e-4 relative to the largest output / state entry), against
     the oracle AND against the position-serial kernel (forced with path 0), whose order is the reference's. 200 and 1000
-    are not multiples of 64: the tail runs on the serial kernel, from the state the chunks left."""
+    are not multiples of 64: the last chunk is filled up with positions that change nothing."""
     o = orc.oracle()
     nh, hk, hv, grp = 8, 128, 128, 2
     key_dim, val_dim = (nh // grp) * hk, nh * hv
@@ -151,3 +151,51 @@ def test_partial_last_chunk_and_head_groups(attn, B, n, nh, grp):
         res.append((out, S))
     for got, want in zip(*res):
         assert float((got - want).norm() / want.norm()) < 5e-6
+
+
+def _inputs(B, n, nh, grp, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+
+    def f32(*s):
+        return torch.randn(*s, device="cuda", generator=g)
+    key_dim, val_dim = nh // grp * 128, nh * 128
+    up = f32(B, n, 2 * key_dim + val_dim)
+    kq = up[:, :, :2 * key_dim].view(B, n, -1, 128)
+    kq /= kq.norm(dim=-1, keepdim=True)
+    return [up, f32(B, n, nh), f32(B, n, nh), f32(B, n, val_dim), 0.5 * f32(nh), 0.5 * f32(nh), 1 + 0.1 * f32(128)], 0.05 * f32(B, nh, 128, 128)
+
+
+@pytest.mark.parametrize("B,n,nh,grp", [(1, 64 * 72 + 5, 32, 2),      # two segments, the last one shorter and with a partial chunk
+                                        (1, 64 * 140, 32, 2),         # whole segments
+                                        (2, 64 * 40 + 1, 32, 2),      # both slots in each segment
+                                        (80, 130, 32, 2),             # groups of slots
+                                        (1, 129, 2400, 8)])           # more heads than the workspace takes: chunk by chunk
+def test_segments_and_groups_of_slots(attn, B, n, nh, grp):
+    """A prompt that the bounded workspace cuts into segments, and into groups of slots, against the position-serial kernel."""
+    args, S0 = _inputs(B, n, nh, grp, 7 * n + B)
+    res = []
+    for path in (-1, 0):
+        S = S0.clone()
+        assert attn.lib.cwk_ctx_force_mla_path(attn.ctx.h, path) == 0
+        try:
+            out = attn.gdn_scan(*args, S, grp, 1e-6)
+            attn.ctx.sync()
+        finally:
+            attn.lib.cwk_ctx_force_mla_path(attn.ctx.h, -1)
+        res.append((out, S))
+    for got, want in zip(*res):
+        assert float((got - want).norm() / want.norm()) < 5e-6
+
+
+@pytest.mark.parametrize("B,n", [(1, 32768), (64, 256)])
+def test_workspace_is_bounded(B, n):
+    """The device memory that a prompt takes beside its arrays does not grow with its length or its slots."""
+    from cwick_b200.ops import Attn
+    args, S = _inputs(B, n, 32, 2, n)
+    out = torch.empty(B, n, 32 * 128, device="cuda")
+    a = Attn(0)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    a.ctx.check(a.lib.cwk_gdn_scan(a.ctx.h, B, n, 32, 128, 128, 2, *[dp(t) for t in args], 1e-6, dp(S), dp(out)))
+    a.ctx.sync()
+    assert before - torch.cuda.mem_get_info()[0] <= 352 << 20
