@@ -186,6 +186,69 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const void *Wv, const fl
     }
 }
 
+// A chunk of tokens: four rows x four tokens per warp, so that a lane's 16 bytes of a weight row meet four tokens' activations
+// and a token's activations meet four rows -- the one-token form, run per group of tokens, reads every activation from L1 once
+// per row and is bound by that. A warp covers the whole width of its rows (lane l takes pieces l, l + 32, ...), eight warps = 32
+// rows per block, blockIdx.y = group of four tokens; f32 accumulate, the lanes' sums by shuffles. BF16 weights: the chunk entry
+// point takes no others. It serves the layers that the tensor path refuses (chunk_tc_ok).
+__global__ void __launch_bounds__(256) gemm_rows_kernel(const uint16_t *W, const float *x, float *y, int rows, int k, int64_t ldx, int64_t ldy, int ntok) {
+    constexpr int R = 4, TOK = 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r0 = (blockIdx.x * 8 + warp) * R, t0 = blockIdx.y * TOK;
+    if (r0 >= rows) return;
+    const float *xt[TOK];
+#pragma unroll
+    for (int t = 0; t < TOK; t++) xt[t] = x + (int64_t)min(t0 + t, ntok - 1) * ldx;
+    const uint16_t *w[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) w[r] = W + (int64_t)min(r0 + r, rows - 1) * k;
+    float acc[R][TOK];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) acc[r][t] = 0.f;
+    // (loads of the next step issued ahead of this step's arithmetic were measured: the registers they hold cost more
+    // in resident warps than the overlap gives -- 2.37 against 1.67 ms for the widest projection of a 512-token chunk)
+    for (int j = lane * 8; j + 8 <= k; j += 256) {
+        uint4 wv[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) wv[r] = ld_weight16(w[r] + j);
+        float xv[TOK][8];
+#pragma unroll
+        for (int t = 0; t < TOK; t++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const float4 f = *reinterpret_cast<const float4 *>(xt[t] + j + 4 * q);
+                xv[t][4 * q] = f.x; xv[t][4 * q + 1] = f.y; xv[t][4 * q + 2] = f.z; xv[t][4 * q + 3] = f.w;
+            }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const uint32_t u[4] = {wv[r].x, wv[r].y, wv[r].z, wv[r].w};
+#pragma unroll
+            for (int t = 0; t < TOK; t++) {
+                float d = 0.f;
+#pragma unroll
+                for (int q = 0; q < 4; q++) d += __uint_as_float(u[q] << 16) * xv[t][2 * q] + __uint_as_float(u[q] & 0xffff0000u) * xv[t][2 * q + 1];
+                acc[r][t] += d;
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) {
+            float a = acc[r][t];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0 && r0 + r < rows && t0 + t < ntok) y[(int64_t)(t0 + t) * ldy + r0 + r] = a;
+        }
+}
+
+// Whether gemm_rows_kernel takes the operands: whole 16-byte pieces for every lane, aligned rows.
+bool gemm_rows_ok(const void *W, const float *x, int64_t k, int64_t ldx, int kind) {
+    return kind == GEMV_BF16 && k % 256 == 0 && (ldx & 3) == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
+}
+
 // y[t][0..rows) = W . x[t] for n tokens. kind: GEMV_BF16 / GEMV_F32 / GEMV_FP8. W2 != NULL: also y2 = W2 . x[t] (same kind,
 // same k) in the same launch.
 template <int TOK>
@@ -207,6 +270,11 @@ void launch_gemv_tok(cwk_ctx *ctx, int kind, const void *W, const float *scales,
 void launch_gemv(cwk_ctx *ctx, int kind, const void *W, const float *scales, const float *x, float *y, int64_t rows, int64_t k, int n,
                  int64_t ldx, int64_t ldy, const void *W2 = nullptr, const float *scales2 = nullptr, float *y2 = nullptr, int64_t rows2 = 0,
                  int64_t ldy2 = 0) {
+    if (n >= 4 && !W2 && gemm_rows_ok(W, x, k, ldx, kind)) {
+        gemm_rows_kernel<<<dim3((unsigned)((rows + 31) / 32), (unsigned)((n + 3) / 4)), 256, 0, ctx->stream>>>((const uint16_t *)W, x, y, (int)rows, (int)k, ldx, ldy, n);
+        ctx->launches++;
+        return;
+    }
     if (n >= 4) launch_gemv_tok<4>(ctx, kind, W, scales, x, y, rows, k, n, ldx, ldy, W2, scales2, y2, rows2, ldy2);
     else launch_gemv_tok<1>(ctx, kind, W, scales, x, y, rows, k, n, ldx, ldy, W2, scales2, y2, rows2, ldy2);
 }
@@ -451,6 +519,64 @@ __global__ void __launch_bounds__(256) unabsorb_kernel(const uint16_t *cacc, con
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) attn[idx] = acc;
+}
+
+// The same for a chunk of tokens: four value rows x four tokens per warp (a lane's 16 bytes of a W_v row meet four tokens'
+// accumulators and the other way round), eight warps = 32 rows per block; grid (vdim / 32, groups of four tokens, heads).
+// kv_lora a multiple of 256, vdim a multiple of 4, 16-byte aligned operands.
+__global__ void __launch_bounds__(256) unabsorb_rows_kernel(const uint16_t *cacc, const uint16_t *kvb, int nh, int nope, int vdim,
+                                                            int kv_lora, float *attn, int ntok) {
+    constexpr int R = 4, TOK = 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = blockIdx.z, r0 = (blockIdx.x * 8 + warp) * R, t0 = blockIdx.y * TOK;
+    if (r0 >= vdim) return;
+    const uint16_t *w[R], *c[TOK];
+#pragma unroll
+    for (int r = 0; r < R; r++) w[r] = kvb + ((int64_t)h * (nope + vdim) + nope + min(r0 + r, vdim - 1)) * kv_lora;
+#pragma unroll
+    for (int t = 0; t < TOK; t++) c[t] = cacc + ((int64_t)min(t0 + t, ntok - 1) * nh + h) * kv_lora;
+    float acc[R][TOK];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) acc[r][t] = 0.f;
+    for (int j = lane * 8; j + 8 <= kv_lora; j += 256) {
+        uint4 wv[R], cv[TOK];
+#pragma unroll
+        for (int r = 0; r < R; r++) wv[r] = ld_weight16(w[r] + j);
+#pragma unroll
+        for (int t = 0; t < TOK; t++) cv[t] = *reinterpret_cast<const uint4 *>(c[t] + j);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const uint32_t wu[4] = {wv[r].x, wv[r].y, wv[r].z, wv[r].w};
+#pragma unroll
+            for (int t = 0; t < TOK; t++) {
+                const uint32_t cu[4] = {cv[t].x, cv[t].y, cv[t].z, cv[t].w};
+                float d = 0.f;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    d += __uint_as_float(wu[q] << 16) * __uint_as_float(cu[q] << 16) +
+                         __uint_as_float(wu[q] & 0xffff0000u) * __uint_as_float(cu[q] & 0xffff0000u);
+                acc[r][t] += d;
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) {
+            float a = acc[r][t];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0 && r0 + r < vdim && t0 + t < ntok) attn[((int64_t)(t0 + t) * nh + h) * vdim + r0 + r] = a;
+        }
+}
+
+void launch_unabsorb(cudaStream_t st, const uint16_t *cacc, const uint16_t *kvb, int nh, int nope, int vdim, int kv_lora, float *attn, int tokens) {
+    if (tokens >= 4 && kv_lora % 256 == 0 && ((reinterpret_cast<uintptr_t>(kvb) | reinterpret_cast<uintptr_t>(cacc)) & 15) == 0)
+        unabsorb_rows_kernel<<<dim3((vdim + 31) / 32, (tokens + 3) / 4, nh), 256, 0, st>>>(cacc, kvb, nh, nope, vdim, kv_lora, attn, tokens);
+    else
+        unabsorb_kernel<<<dim3((nh * vdim + 7) / 8, tokens), 256, 0, st>>>(cacc, kvb, nh, nope, vdim, kv_lora, attn);
 }
 
 // Indexer scores over the f32 pool rows, the reference's order (src/attention.c:573-582 with dot_f32's scalar
@@ -887,7 +1013,7 @@ int token_step(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos, const flo
     s = cwk_mla_decode(ctx, d_qabs, cm.dev, 0, kv_lora, nullptr, (int)nlist, use_sel ? d_sel : nullptr, use_sel ? (int64_t)nlist : 0, 1, nh,
                        kv_lora, 0, 1.0f / sqrtf((float)nope), d_cacc, 0);
     if (s != CWK_OK) { set_err(err, s, "%s", cwk_last_error(ctx)); return s; }
-    unabsorb_kernel<<<dim3((nh * vdim + 7) / 8, 1), 256, 0, st>>>(d_cacc, (const uint16_t *)ly.kvb->data, nh, nope, vdim, kv_lora, d_attn);
+    launch_unabsorb(st, d_cacc, (const uint16_t *)ly.kvb->data, nh, nope, vdim, kv_lora, d_attn, 1);
     ctx->launches += 1;
     if (a_out) dev_linear(ctx, ly.o, d_attn, a_out, 1, 0, 0);
     else {
@@ -1040,7 +1166,7 @@ int chunk_steps(cwk_ctx *ctx, Layer &ly, int64_t capacity, int64_t pos0, int64_t
             if (o.splits > 1 && (s = cwk_sum_partials(ctx, d_part, o.splits, np, (int)H, out, nullptr)) != CWK_OK) return s;
         } else {
             float *d_attn = (float *)(d + o_attn);
-            unabsorb_kernel<<<dim3((nh * vdim + 7) / 8, (unsigned)np), 256, 0, st>>>(d_cacc, (const uint16_t *)ly.kvb->data, nh, nope, vdim, kv_lora, d_attn);
+            launch_unabsorb(st, d_cacc, (const uint16_t *)ly.kvb->data, nh, nope, vdim, kv_lora, d_attn, np);
             ctx->launches += 1;
             dev_linear(ctx, ly.o, d_attn, out, np, vw, H);
         }

@@ -62,6 +62,14 @@ def test_chunk_against_the_layer_in_double(monkeypatch, H, nh, nope, vdim, q_lor
     L.cwk_dropin_reset()
 
 
+@pytest.mark.parametrize("n,pos0", [(4, 0), (5, 1), (35, 70), (300, 0)])
+@pytest.mark.parametrize("H,nh,nope,vdim,q_lora,kv_lora", [(512, 4, 96, 128, 256, 512),      # a head width that is no multiple of 64
+                                                           (264, 3, 40, 72, 512, 256)])      # and contractions that are no multiples of 256
+def test_chunk_off_the_tensor_path(monkeypatch, H, nh, nope, vdim, q_lora, kv_lora, n, pos0):
+    """Layers that the tensor path refuses: row kernels over groups of four tokens and rows, with remainders of both."""
+    test_chunk_against_the_layer_in_double(monkeypatch, H, nh, nope, vdim, q_lora, kv_lora, n, pos0, True)
+
+
 @pytest.mark.parametrize("pos", [0, 1, 257, 2000])
 @pytest.mark.parametrize("kind", ["bf16", "f32", "fp8"])
 @pytest.mark.parametrize("H,nh,q_lora", [(1024, 64, 640), (336, 2, 208), (48, 1, 16)])
