@@ -639,9 +639,14 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnParams p) {
     dst[1] = make_uint4(r[4], r[5], r[6], r[7]);
 }
 
-// The attention grid of both shapes: the fast form, the repair pass, and in share mode the merge. Shares where the longest
-// block of item-by-item dealing would have PA_MERGE_TILES more key tiles than an equal share (what records and merge cost: 13 us, a tile 0.65).
-constexpr int PA_MERGE_TILES = 20;
+// The attention grid of both shapes: the fast form, the repair pass, and in share mode the merge. Shares where the longest block
+// of item-by-item dealing would have more than PA_MERGE_TILES key tiles above an equal share: what the records, their merge and
+// its launch cost. Dealt and shared, us, keys and values from memory (16 query heads, 4 KV heads of 256):
+//   512 queries after 1500 (19 tiles above the share) 39.5 / 45.5, after 2500 (28) 51.4 / 51.4, after 4000 (41) 68 / 60
+//   128 queries after 1500 (23) 37.0 / 41.3, after 2000 (30) 42.6 / 41.5, after 4000 (57) 66 / 45
+//   700 queries after 3000 (23) 57.1 / 62.9, after 4000 (28) 68.7 / 70.1, after 6000 (39) 91 / 86
+// and the whole MLA prompt of 64 heads: 256 queries after 4000 (17) 247 / 254, after 6000 (25) 321 / 321, after 14000 (59) 606 / 595.
+constexpr int PA_MERGE_TILES = 28;
 template <class CFG, bool GQA>
 int attn_launch(cwk_ctx *ctx, AttnParams ap, const CUtensorMap &tm_k, const CUtensorMap &tm_c, int exact_only) {
     static bool attr_set[16] = {false};

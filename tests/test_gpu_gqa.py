@@ -160,3 +160,9 @@ def test_prefill_in_equal_shares_of_tiles(attn, n, pos, nh, nkv, climb):
         want = torch.softmax(s, -1) @ V[:, h // (nh // nkv)].double()
         err = (got[:, h].double() - want).norm() / want.norm()
         assert err < 6e-3, (h, float(err))
+
+
+@pytest.mark.parametrize("n,pos,nh,nkv", [(129, 2150, 16, 4), (129, 2300, 16, 4), (512, 2400, 16, 4), (512, 2700, 16, 4)])
+def test_prefill_on_both_sides_of_the_line_for_shares(attn, n, pos, nh, nkv):
+    """The last lengths whose items go out one by one and the first that are shared."""
+    test_prefill_in_equal_shares_of_tiles(attn, n, pos, nh, nkv, False)
