@@ -209,14 +209,18 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, cons
 
 // Which attention route is the faster one for a chunk of n queries behind pos0 rows. The expansion covers every cached
 // row once, whatever n, and its attention works in tiles of 128 queries; the absorbed route costs a pass of the decode
-// kernel per query. In microseconds, measured with 64 heads: expansion 0.018 per row; attention 0.74 per 64-key tile and 5
-// per item (128 queries x head x half), the items dealt over the SMs; absorbed 0.032 per query and 128-key tile and 0.42 per
-// query around it. 509 queries after 3001 rows: 230 against 640; 64 queries after 32704: 970 against 550.
+// kernel per query. In microseconds, fitted to whole calls with 64 heads: expansion 0.012 per row; attention 0.64 per 64-key tile
+// and 5 per item (128 queries x head x half), the items dealt over the SMs; absorbed 0.033 per query and 128-key tile, 0.08 per
+// query around it (0.4 where the queries are more than the SMs: there the other route is far ahead anyway) and 18 for launches
+// that do not come up early. Calls measured near the line, absorbed / expanded:
+//   4 queries after 300 rows 90 / 80, after 1000 92 / 99;          16 after 300 95 / 80, after 1000 97 / 96, after 3000 108 / 139
+//   32 after 1000 114 / 100, after 3000 125 / 139;                 64 after 3000 163 / 143, after 8000 245 / 255
+//   96 after 8000 332 / 274, after 32000 826 / 814;                129 after 8000 356 / 345, after 16000 637 / 610, after 32000 1083 / 1191
 static bool expanded_keys_pay(const cwk_ctx *ctx, int n, int64_t pos0, int nh) {
     const double T = (double)(pos0 + n), mean = (double)pos0 + 0.5 * n;
     const double items = (double)((n + 127) / 128) * nh * 2, rounds = items <= ctx->sm_count ? 1.0 : items / ctx->sm_count + 0.5;
-    const double expanded = 0.018 * T * nh / 64 + rounds * (0.74 * (mean / 64 + 1) + 5.0);
-    const double absorbed = n * (0.032 * (mean / 128 + 1) + 0.42) * nh / 64;
+    const double expanded = 0.012 * T * nh / 64 + rounds * (0.64 * (mean / 64 + 1) + 5.0);
+    const double absorbed = 18.0 + n * (0.033 * (mean / 128 + 1) + 0.08) * nh / 64;
     return expanded < absorbed;
 }
 

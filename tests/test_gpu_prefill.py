@@ -203,3 +203,21 @@ def test_keys_from_memory_behind_a_long_context(attn):
     absorbed = _forced(attn, 2, lambda: attn.mla_prefill(*args))
     attn.ctx.sync()
     close(bf16_to_np(first), bf16_to_np(absorbed))
+
+
+@pytest.mark.parametrize("n,pos0", [(1, 0), (1, 63), (2, 300), (5, 0), (16, 127), (31, 640), (64, 1)])
+@pytest.mark.parametrize("nh", [64, 16, 3])
+def test_short_chunks_on_both_routes(attn, n, pos0, nh):
+    """Chunks of a few queries behind short contexts, which the route by estimated time gives to the expanded keys: every row against
+    the oracle, and against the absorbed route."""
+    H, q_lora = 512, 256
+    m = make_model(61 + nh, H, q_lora, nh)
+    X = synth.normal_bf16(61 + n, 9, (n, H))
+    cache0 = np.zeros((pos0 + n, LAT + ROPE), np.uint16)
+    cache0[:pos0] = synth.normal_bf16(61 + n, 10, (pos0, LAT + ROPE))
+    got, gcache = run_gpu(attn, m, X, cache0, pos0, nh)
+    other, ocache = _forced(attn, 2 if nh == 64 else 1, lambda: run_gpu(attn, m, X, cache0, pos0, nh))      # (its tensor form: 64 heads)
+    want, _ = run_oracle(m, X, cache0, pos0, nh, np.arange(n))
+    close(bf16_to_np(got), want)
+    close(bf16_to_np(other), want)
+    close(bf16_to_np(gcache), bf16_to_np(ocache))
