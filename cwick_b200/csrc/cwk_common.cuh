@@ -120,8 +120,10 @@ struct CwkKernelTimer {
 // kernel launched this way calls cwk_pdl_wait() before it touches global memory that a kernel may have written, and
 // cwk_pdl_launch() to let the next one come up. (A kernel that never calls the latter lets it up when it ends: so other
 // kernels in the stream need know nothing of this.)
-// Not while the stream is captured: between the kernels of a replayed graph the ordinary edge is the shorter one (MLA decode of
-// one sequence of 8192, one graph of 512 calls: 14.2 us a call with the attribute, 13.1 without; launched one by one 17.3 -> 14.3).
+// Not while the stream is captured. There the gain is small, and for the chains that are most often replayed it is a loss: in a
+// graph of 20 calls, with the ordinary edge / with the attribute, us a call: MLA decode 1 x 8192 13.2 / 14.0 (launched one by
+// one 17.3 -> 14.3 with it), 64 x 4096 97.0 / 98.5; GQA prompt of 128 16.5 / 18.1; GQA decode 1 x 4096 11.9 / 10.8, 64 x 4096
+// 162 / 161; sparse decode 8 x 65536 93 / 92; MLA prompt of 200 89 / 87, of 509 after 3001 292 / 295; state scan of one slot 5.5 / 5.2.
 template <class... K, class... A>
 static inline cudaError_t cwk_launch_early(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
     cudaLaunchAttribute at;
