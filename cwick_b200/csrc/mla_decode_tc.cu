@@ -161,6 +161,7 @@ __device__ __forceinline__ void find_range(const TcParams &p, int lane, int *out
     if (lane == 0) out[2] = (int)(hi - lo);
 }
 
+template <bool RANGE>
 __global__ void __launch_bounds__(NTHREADS, 1)
 mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
                      const __grid_constant__ CUtensorMap tm_kr, const TcParams p) {
@@ -193,8 +194,8 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const int mb0 = p.halves == 2 ? 2 * (int)blockIdx.z : 0, mb1 = p.halves == 2 ? mb0 + 2 : 4;
     // this block's tiles: `n` of them, from tile t0 of sequence b (range mode: going on into the sequences after it)
     int b = p.reverse_b ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y, t0, n;
-    const int ntiles = p.seq_meta ? 0 : ((p.kv_len ? p.kv_len[b] : p.kv_len_imm) + TILE - 1) / TILE;
-    if (p.seq_meta) {
+    const int ntiles = RANGE ? 0 : ((p.kv_len ? p.kv_len[b] : p.kv_len_imm) + TILE - 1) / TILE;
+    if (RANGE) {
         __shared__ int s_range[3];
         if (warp == 2) find_range(p, lane, s_range);
         __syncthreads();
@@ -204,7 +205,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         t0 = (int)((int64_t)ntiles * split / p.nsplit);
         n = (int)((int64_t)ntiles * (split + 1) / p.nsplit) - t0;
     }
-    auto record = [&](int sb) { return p.partial + (p.seq_meta ? (int64_t)sb + split : (int64_t)sb * p.nsplit + split) * (int64_t)(NH * (L + 2)); };
+    auto record = [&](int sb) { return p.partial + (RANGE ? (int64_t)sb + split : (int64_t)sb * p.nsplit + split) * (int64_t)(NH * (L + 2)); };
 
     if (n <= 0) {                       // empty split: a record the merge ignores (direct mode: zeros)
         if (p.out) {
@@ -219,7 +220,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     auto first_segment = [&]() {
         Segment s;
         s.b = b; s.t0 = t0; s.kv = p.kv_len ? p.kv_len[b] : p.kv_len_imm;
-        s.n = p.seq_meta ? min(n, (s.kv + TILE - 1) / TILE - t0) : n;
+        s.n = RANGE ? min(n, (s.kv + TILE - 1) / TILE - t0) : n;
         return s;
     };
     auto next_segment = [&](Segment &s, int left) {        // left: tiles of the block behind this segment, at least one
@@ -238,10 +239,10 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // Blocks that have one tile more than the others start first when they are few; when they are most of the
         // launch they are the ones to spread.
         if (p.stagger) {
-            const int nlong = p.seq_meta ? 0 : ntiles % p.nsplit;                            // blocks with one tile more (0: all alike)
+            const int nlong = RANGE ? 0 : ntiles % p.nsplit;                                  // blocks with one tile more (0: all alike)
             const bool longest = nlong != 0 && n == (ntiles + p.nsplit - 1) / p.nsplit;
             int group;
-            if (nlong == 0) group = (split + (p.seq_meta ? 0 : 3 * b)) & 7;
+            if (nlong == 0) group = (split + (RANGE ? 0 : 3 * b)) & 7;
             else if (nlong * 4 <= p.nsplit) group = longest ? 0 : 1 + (split + 3 * b) % 7;      // a few long blocks: they go first
             else group = longest ? (split + 3 * b) % 7 : 7;                 // mostly long blocks: they spread, the few short ones last
             const long long until = clock64() + (long long)group * p.stagger;
@@ -288,7 +289,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             int begin = 0, nq = 1;                                // the block's tile with which the segment begins; queries asked for
             for (int it = 1; it < n && ok; it++) {
                 const uint32_t par_free = (uint32_t)((it & 1) ^ 1);
-                if (it == begin + sg.n) {                         // the next sequence: its query replaces this one's after the last scores
+                if (RANGE && it == begin + sg.n) {                // the next sequence: its query replaces this one's after the last scores
                     begin = it;
                     next_segment(sg, n - it);
                     ok = mbar_wait(bar(B_SFULL), (uint32_t)((it - 1) & 1), p.err, 107);
@@ -391,7 +392,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             int begin = 0, nseg = 0;
             for (int it = 0; it < n && ok; it++) {
                 const uint32_t par = (uint32_t)(it & 1);
-                if (it == begin + sg.n) { begin = it; next_segment(sg, n - it); }
+                if (RANGE && it == begin + sg.n) { begin = it; next_segment(sg, n - it); }
                 if (it == begin) ok = mbar_wait(bar(B_QFULL), (uint32_t)(nseg++ & 1), p.err, 201);
                 // S^T = K Q^T over the nine column blocks (4 k-steps of 16 each)
 #pragma unroll
@@ -629,7 +630,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 }
             }
         }
-        if (end >= n || !ok) break;
+        if (!RANGE || end >= n || !ok) break;
         tc_fence_before();                                // the accumulator has been read: these threads' next P lets its MMAs go ahead
         softmax_bar();                                    // the reference exponents and row sums have been read
         next_segment(sg, n - end);
@@ -669,7 +670,8 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
     const bool shared_cache = (seq_stride == 0);
     static bool attr_set[16] = {false};
     if (!attr_set[ctx->device & 15]) {
-        CWK_CUDA(ctx, cudaFuncSetAttribute(mla_decode_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
+        CWK_CUDA(ctx, cudaFuncSetAttribute(mla_decode_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
+        CWK_CUDA(ctx, cudaFuncSetAttribute(mla_decode_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
         attr_set[ctx->device & 15] = true;
     }
     TcParams p;
@@ -684,7 +686,7 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
     p.B = B; p.seq_meta = seq_meta;
     if (seq_meta) {                    // range mode: nsplit = number of blocks
         p.halves = 1; p.stagger = 700;
-        CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel, dim3(nsplit), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
+        CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel<true>, dim3(nsplit), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
         ctx->launches++;
         return CWK_OK;
     }
@@ -693,7 +695,7 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
         const int tiles_per_block = ((max_kv_len + TILE - 1) / TILE + nsplit - 1) / nsplit;
         p.stagger = ((int64_t)nsplit * B * 2 > ctx->sm_count && tiles_per_block >= 6) ? 700 : 0;
     }
-    CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel, dim3(nsplit, B, p.halves), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
+    CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel<false>, dim3(nsplit, B, p.halves), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
     ctx->launches++;
     return CWK_OK;
 }
