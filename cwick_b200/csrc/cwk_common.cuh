@@ -37,6 +37,7 @@ struct cwk_ctx {
     uint64_t launches = 0;
     int force_mla_path = -1;
     bool keep_splits = false;   // internal: leave split records in scratch (no merge, no fold)
+    bool plain_edge = false;    // internal: the decode kernel does not come up under the kernel before
     int last_nsplit = 0;
     // optional event pairs around main kernels (cwk_ctx_profile)
     bool profiling = false;

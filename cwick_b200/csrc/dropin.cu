@@ -25,7 +25,7 @@ int cwk_mla_decode_rows(cwk_ctx *ctx, const void *q, const void *cache, int64_t 
 
 // one sequence's attention left as split records in the context's scratch
 int cwk_mla_launch_splits(cwk_ctx *ctx, const void *q, const void *cache, int64_t ld, int rows, int nh, int L, int R, float scale, float **partial_out,
-                          int *nsplit_out);
+                          int *nsplit_out, bool plain_edge);
 int cwk_mla_decode(cwk_ctx *ctx, const void *q, const void *cache, int64_t seq_stride, int64_t ld, const int32_t *kv_len,
                    int max_kv_len, const int32_t *sel, int64_t sel_ld, int B, int nh, int L, int R, float scale, void *out,
                    int n_splits);
@@ -868,7 +868,7 @@ int token_chain(cwk_ctx *ctx, Layer &ly, int64_t pos, const float *d_x, float *d
                                    kv_lora, d_qabs));
     float *partial = nullptr;
     int nsplit = 0;
-    const int s = cwk_mla_launch_splits(ctx, d_qabs, ly.cm->dev, kv_lora, (int)(pos + 1), nh, kv_lora, 0, 1.0f / sqrtf((float)nope), &partial, &nsplit);
+    const int s = cwk_mla_launch_splits(ctx, d_qabs, ly.cm->dev, kv_lora, (int)(pos + 1), nh, kv_lora, 0, 1.0f / sqrtf((float)nope), &partial, &nsplit, false);
     if (s != CWK_OK) return s;
     CWK_CUDA(ctx, cwk_launch_early(merge_unabsorb_kernel, dim3(nh, 2), dim3(512), 0, ctx->stream, (const float *)partial, nsplit, nh, (const uint16_t *)ly.kvb->data, nope,
                                    d_attn));

@@ -19,7 +19,7 @@
 #include "flash_rows.cuh"
 
 int cwk_mla_launch_splits(cwk_ctx *ctx, const void *q, const void *cache, int64_t ld, int rows, int nh, int L, int R,
-                          float scale, float **partial_out, int *nsplit_out);
+                          float scale, float **partial_out, int *nsplit_out, bool plain_edge);
 
 namespace {
 
@@ -223,7 +223,9 @@ int cwk_mla_decode_kv_split(cwk_ctx *ctx, const void *q, const void *cache, int6
     }
     float *partial = nullptr;
     int ns = 0;
-    int s = cwk_mla_launch_splits(ctx, q, cache, ld, (int)rows, nh, L, R, scale, &partial, &ns);
+    // The kernel before, as a rule the last step's exchange, ends when its peers have published: the decode kernel gains
+    // nothing by coming up for it (one sequence of 131072 rows, a step: 65.4 us with it, 62.2 without).
+    int s = cwk_mla_launch_splits(ctx, q, cache, ld, (int)rows, nh, L, R, scale, &partial, &ns, true);
     if (s != CWK_OK) return s;
     PeerWindows pw;
     for (int g = 0; g < MAX_WORLD; g++) pw.win[g] = (g < world) ? (float *)windows[g] : nullptr;

@@ -228,12 +228,13 @@ int cwk_mla_decode_rows(cwk_ctx *ctx, const void *q, const void *cache, int64_t 
 }
 
 // Split-KV decode of one sequence whose result stays as split records in the context's scratch
-// (the KV-range exchange folds and ships them itself).
+// (the KV-range exchange folds and ships them itself). plain_edge: behind a kernel that lets no other up before it ends.
 int cwk_mla_launch_splits(cwk_ctx *ctx, const void *q, const void *cache, int64_t ld, int rows, int nh, int L, int R,
-                          float scale, float **partial_out, int *nsplit_out) {
+                          float scale, float **partial_out, int *nsplit_out, bool plain_edge) {
     ctx->keep_splits = true;
+    ctx->plain_edge = plain_edge;
     int s = mla_launch(ctx, q, cache, 0, ld, nullptr, rows, nullptr, 0, 1, nh, L, R, scale, nullptr, nullptr, 0);
-    ctx->keep_splits = false;
+    ctx->keep_splits = ctx->plain_edge = false;
     *partial_out = ctx->scratch;
     *nsplit_out = ctx->last_nsplit;
     return s;

@@ -695,6 +695,11 @@ int cwk_mla_decode_tc_launch(cwk_ctx *ctx, const void *q, const void *cache, int
         const int tiles_per_block = ((max_kv_len + TILE - 1) / TILE + nsplit - 1) / nsplit;
         p.stagger = ((int64_t)nsplit * B * 2 > ctx->sm_count && tiles_per_block >= 6) ? 700 : 0;
     }
+    if (ctx->plain_edge) {
+        mla_decode_tc_kernel<false><<<dim3(nsplit, B, p.halves), NTHREADS, SMEM_TOTAL, ctx->stream>>>(*tm_q, *tm_kv, *tm_kr, p);
+        CWK_LAUNCH_CHECK(ctx, "mla_decode_tc_kernel");
+        return CWK_OK;
+    }
     CWK_CUDA(ctx, cwk_launch_early(mla_decode_tc_kernel<false>, dim3(nsplit, B, p.halves), dim3(NTHREADS), SMEM_TOTAL, ctx->stream, *tm_q, *tm_kv, *tm_kr, p));
     ctx->launches++;
     return CWK_OK;
