@@ -72,6 +72,11 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) flash_rows_kernel(const FlashR
     const int wm = warp % WM, wn = warp / WM;
     const int split = blockIdx.x, by = blockIdx.y, b = blockIdx.z;
 
+    if (MODE == MODE_GQA_DEC) {        // launched to come up under the kernel before (cwk_launch_early)
+        cwk_pdl_launch();
+        cwk_pdl_wait();
+    }
+
     // ---- what this block covers -------------------------------------------
     int limit_uniform = 0;          // keys visible to every row (MLA / GQA_DEC)
     int tile_begin = 0, tile_end = 0;

@@ -1,5 +1,5 @@
-// gqa.cu -- Qwen3.5-style grouped-query attention: entry points of the single-query decode (gqa_decode.cu; more than eight
-// query heads per KV head: flash_rows_kernel, split over the key range and merged by lse_merge_kernel) and of causal prefill
+// gqa.cu -- Qwen3.5-style grouped-query attention: entry points of the single-query decode (gqa_decode.cu; little to read, or more
+// than eight query heads per KV head: flash_rows_kernel, split over the key range and merged by lse_merge_kernel) and of causal prefill
 // (mla_prefill_attn.cu, or flash_rows_kernel with K and V as separate streams).
 #include <algorithm>
 #include <cmath>
@@ -18,7 +18,7 @@ static int gqa_decode_launch(cwk_ctx *ctx, const FlashRowsParams &p, int B, int 
         CWK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL));
         attr_set[ctx->device & 15] = true;
     }
-    kern<<<dim3(ns, nkv, B), 256, SM::TOTAL, ctx->stream>>>(p);
+    CWK_CUDA(ctx, cwk_launch_early(kern, dim3(ns, nkv, B), dim3(256), SM::TOTAL, ctx->stream, p));
     CWK_LAUNCH_CHECK(ctx, "flash_rows_kernel<GQA_DEC>");
     return CWK_OK;
 }
@@ -44,6 +44,18 @@ int cwk_gqa_prefill_tc(cwk_ctx *ctx, const void *Q, const void *K, const void *V
 
 extern "C" {
 
+// Which kernel takes a decode step of at most eight query heads per KV head, by the bytes of K and V that there can be to read. The
+// streams of gqa_decode.cu read faster, the row kernel is done sooner where there is little: its tiles of 64 keys and its few records
+// leave less to merge. Streams / rows, keys and values from memory, us a call, replayed as a graph (launched one by one: a
+// microsecond or two more, in the same order):
+//   16 heads, 4 KV heads of 256: 8 MB 10.9 / 7.5, 17 MB (one sequence of 4096) 13.8 / 9.9, 25 MB 15.3 / 12.0, 34 MB 14.0 / 14.4 (four
+//   sequences) and 16.6 / 14.9 (one), 50 MB 16.8 / 18.4 and 19.2 / 18.6
+//   16 heads, 2 KV heads of 128: 8 MB 14.8 / 7.9, 25 MB 15.1 / 12.6, 42 MB 18.0 / 16.6 and 18.7 / 18.6 (sixteen)
+//   8 heads, 8 KV heads of 128 (the row kernel pads one head to sixteen rows): 8 MB 9.7 / 7.5, 17 MB 10.6 / 10.8, 34 MB 14.2 / 15.8
+static bool gqa_rows_sooner(int64_t B, int64_t max_kv_len, int nkv, int group, int hd) {
+    return B * max_kv_len * nkv * hd * 4 <= (int64_t)(group >= 4 ? 24 : 12) << 20;
+}
+
 // sel != NULL: the keys of sequence b are rows sel[b*sel_ld + 0 .. kv_len[b]) of its cache, in that order.
 static int gqa_decode_impl(cwk_ctx *ctx, const void *q, const void *K, const void *V, int64_t seq_stride,
                            const int32_t *kv_len, int max_kv_len, const int32_t *sel, int64_t sel_ld, int B, int nh, int nkv, int hd,
@@ -57,8 +69,8 @@ static int gqa_decode_impl(cwk_ctx *ctx, const void *q, const void *K, const voi
     if (((uintptr_t)K | (uintptr_t)V | (uintptr_t)q) % 16 != 0 || (seq_stride % 8) != 0)
         return cwk_fail(ctx, CWK_ERR_ARGUMENT, "gqa_decode: pointers must be 16-byte aligned");
     CWK_CUDA(ctx, cudaSetDevice(ctx->device));
-    // up to eight query heads per KV head: a warp's MMA columns (gqa_decode.cu); more take the row kernel below
-    if (group <= 8)
+    // up to eight query heads per KV head: a warp's MMA columns (gqa_decode.cu); more, or little to read, take the row kernel below
+    if (group <= 8 && !gqa_rows_sooner(B, max_kv_len, nkv, group, hd))
         return cwk_gqa_decode_streams(ctx, q, K, V, seq_stride, kv_len, max_kv_len, sel, sel_ld, B, nh, nkv, hd, scale, out,
                                       n_splits > 0 ? (int)std::min<int64_t>((int64_t)n_splits * B * nkv, 1 << 20) : 0);
     const int max_tiles = std::max(1, (max_kv_len + 63) / 64);

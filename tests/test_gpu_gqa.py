@@ -166,3 +166,28 @@ def test_prefill_in_equal_shares_of_tiles(attn, n, pos, nh, nkv, climb):
 def test_prefill_on_both_sides_of_the_line_for_shares(attn, n, pos, nh, nkv):
     """The last lengths whose items go out one by one and the first that are shared."""
     test_prefill_in_equal_shares_of_tiles(attn, n, pos, nh, nkv, False)
+
+
+@pytest.mark.parametrize("hd", [128, 256])
+@pytest.mark.parametrize("nh,nkv", [(16, 4), (8, 1), (6, 2), (24, 3), (8, 8)])
+@pytest.mark.parametrize("lens", [[3, 3, 3], [0, 0], [5000], [1, 0, 65, 64, 63], [16] * 20])
+def test_decode_kernels_agree_on_short_sequences(attn, hd, nh, nkv, lens):
+    """What the row kernel takes because there is little to read, and the same through the streams, which a larger bound on the
+    lengths asks for: both against float32."""
+    B, T = len(lens), max(max(lens), 1)
+    g = torch.Generator(device="cuda").manual_seed(nh + T + B)
+    q = torch.randn(B, nh, hd, device="cuda", generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(B, T, nkv, hd, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    k[:, ::7] *= 3
+    kv_len = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    for bound in (T, 1 << 20):
+        got = attn.gqa_decode(q, k, v, kv_len, max_kv_len=bound)
+        attn.ctx.sync()
+        for b in range(B):
+            if lens[b] == 0:
+                assert not got[b].any()
+                continue
+            kk, vv = (x[b, :lens[b]].float().repeat_interleave(nh // nkv, 1) for x in (k, v))
+            s = torch.einsum("hd,thd->ht", q[b].float(), kk) / hd ** 0.5
+            want = torch.einsum("ht,thd->hd", torch.softmax(s, -1), vv)
+            assert float((got[b].float() - want).norm() / want.norm()) < 5e-3, (bound, b)
