@@ -20,11 +20,11 @@
 //     (the accumulator of a half, 128 x 256 f32, is half of tensor memory; both halves recompute
 //     the 192-wide scores, which is cheaper than any exchange). Keys stream in tiles of 64 through a
 //     3-deep ring (24 KB each), latent halves through a 3-deep ring (32 KB each), one TMA box each. The query tile
-//     itself sits in tensor memory (96 columns of bf16 pairs) as the A operand of the score MMAs: shared-memory
-//     bandwidth is what bounds this kernel, and this way the score MMAs read only the keys from it.
+//     itself sits in tensor memory (96 columns of bf16 pairs) as the A operand of the score MMAs, and P beside it (32 columns) as
+//     that of the values': this way the MMAs read only keys and values from shared memory.
 //     Per tile: S = Q Kx^T (12 MMAs, M 128 x N 64) into one of two TMEM score buffers; the softmax
 //     warps own one query row per thread (TMEM lane = row, so row maxima and sums need no shuffles),
-//     write P (bf16) to shared memory; O += P lat (4 MMAs, M 128 x N 256). The two products have
+//     write P (bf16) to tensor memory (GQA: shared memory); O += P lat (4 MMAs, M 128 x N 256). The two products have
 //     issuer threads of their own (the scores two), so the scores run ahead of the values and the tensor pipe works under
 //     the softmax.
 //     The kernel has two forms. The fast one splits the 64 keys of a row between two softmax warp groups
@@ -173,6 +173,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + PA_OFF_BAR + 8 * PB_COUNT + 8);
     int4 *s_item = reinterpret_cast<int4 *>(sm + PA_OFF_X + 4096);      // ring of 8 items: {number, first tile, end, record}
+    // P is the A operand of the value MMAs. Where the query tile leaves room for it (192-wide keys), it lies in tensor memory: 32 KB less
+    // through shared memory per tile and no proxy fence, 183 -> 176 us for 509 queries after 3001 rows. One tile's worth: it is
+    // written when the value MMAs of the tile before are done. (In the place of the scores it comes from, which 256-wide keys would need,
+    // those MMAs are a link of the next scores' chain: 105 -> 117 us for 512 GQA queries after 10488 rows.)
+    constexpr bool OWN_P = PA_COL_Q + PA_DQK / 2 + PA_KT / 2 <= 512;
+    constexpr uint32_t PA_COL_P = PA_COL_Q + PA_DQK / 2;
     constexpr int TG = NWG == 4 ? 2 : 1, QK_ISSUERS = NWG == 4 ? 2 : 1;      // groups that share a tile; issuers of the score MMAs
     float *s_m = reinterpret_cast<float *>(sm + PA_OFF_X), *s_l = s_m + 512;              // [4][128] each
 
@@ -187,9 +193,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_k) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_c) : "memory");
         for (int i = 0; i < PB_COUNT; i++) {
-            // (by tile: an arrival per softmax warp; 32 a warp on one barrier are served one after another)
+            // (an arrival per softmax warp; 32 a warp on one barrier are served one after another)
             const bool by_tile = i >= PB_SEMPTY && i < PB_PEMPTY, by_soft = i == PB_QFULL || i == PB_OFREE || i == PB_XM || i == PB_XL;
-            mbar_init(bar(i), by_tile ? (uint32_t)(4 * TG) : by_soft ? (uint32_t)(128 * NWG) : i == PB_QEMPTY ? QK_ISSUERS : 1u);
+            mbar_init(bar(i), by_tile ? (uint32_t)(4 * TG) : by_soft ? (uint32_t)(4 * NWG) : i == PB_QEMPTY ? QK_ISSUERS : 1u);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -293,42 +299,54 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         // lone thread some 200 cycles even when the phase is long complete, and one thread doing all four
         // waits of a tile in turn was the longest chain of the kernel. So was, after that, the one issuer of the scores: two
         // waits, 12 or 16 MMAs and the commits took it 1650 cycles a tile, of which the tensor pipe works 400 to 500. In the fast
-        // form a second one (the last warp) takes every other tile.
-        if (lane == 0) {
+        // form a second one (the last warp) takes every other tile. All lanes run the issuers' loops and one is elected for the
+        // MMAs (tc_common.cuh): with the values' P in tensor memory 1644 -> 1575 us for a whole prompt of 4096, 372 -> 353 for 509
+        // after 3001.
+        {
             constexpr uint32_t ID_QK = idesc_bf16(128, PA_KT, 0, 0);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint64_t dK0 = smem_desc(base + PA_OFF_K, 16, 1024);
+            const int first = QK_ISSUERS == 2 && warp != 1 ? 1 : 0;
             bool ok = true;
-            int kc = 0;                              // score tiles issued so far
+            int kc = 0;                              // score tiles so far
             for (int k = 0; ok; k++) {
                 int w;
                 AttnItem it;
                 ok = next_item(k, w, it);
                 if (!ok || w < 0) break;
+                const int end = __shfl_sync(0xffffffffu, kc + it.nt - it.lo, 0);
                 ok = mbar_wait(bar(PB_QFULL), (uint32_t)(k & 1), p.err, 1011);     // the softmax threads have written the item's query tile into tensor memory
                 if (!ok) break;
                 tc_fence_after();
-                // scores of a tile: S[kc % 2] = Q Kx^T, three 64-wide blocks of the 192 dims, four 16-wide steps each
-                for (int i = it.lo; i < it.nt && ok; i++, kc++) {
-                    if (QK_ISSUERS == 2 && (kc & 1) != (warp == 1 ? 0 : 1)) continue;
+                // scores of a tile: S[kc % 2] = Q Kx^T, the 64-wide blocks of the key's dims, four 16-wide steps each
+                for (kc += QK_ISSUERS == 2 ? (kc ^ first) & 1 : 0; kc < end && ok; kc += QK_ISSUERS) {
                     const int ks = kc % PA_KST, sb = kc % PA_SBUF, su = kc / PA_SBUF;
                     ok = mbar_wait(bar(PB_KFULL + kc % PA_KBAR), (uint32_t)((kc / PA_KBAR) & 1), p.err, 1012);
                     if (ok) ok = mbar_wait(bar(PB_SEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1013);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint64_t dK = smem_desc(base + PA_OFF_K + ks * PA_K_BYTES, 16, 1024);
+                    const uint64_t dK = dK0 + (uint64_t)((ks * PA_K_BYTES) >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int s = 0; s < PA_DQK / 16; s++)
-                        umma_bf16_ts(tmem + PA_COL_S + sb * PA_KT, tmem + PA_COL_Q + s * 8,       // A: 16 bf16 of every row = 8 TMEM columns per step
-                                     dK + (uint64_t)(((s >> 2) * (PA_KT * 128) + (s & 3) * 32) >> 4), ID_QK, s != 0);
-                    umma_commit(bar(PB_KEMPTY + ks));
-                    umma_commit(bar(PB_SFULL + sb));
+                        for (int s = 0; s < PA_DQK / 16; s++)
+                            umma_bf16_ts(tm + PA_COL_S + sb * PA_KT, tm + PA_COL_Q + s * 8,       // A: 16 bf16 of every row = 8 TMEM columns per step
+                                         dK + (uint64_t)(((s >> 2) * (PA_KT * 128) + (s & 3) * 32) >> 4), ID_QK, s != 0);
+                        umma_commit(bar(PB_KEMPTY + ks));
+                        umma_commit(bar(PB_SFULL + sb));
+                    }
+                    __syncwarp();
                 }
-                if (ok) umma_commit(bar(PB_QEMPTY));       // the query tile may be replaced once these MMAs are done
+                kc = end;
+                if (ok && elect_one()) umma_commit(bar(PB_QEMPTY));       // the query tile may be replaced once these MMAs are done
+                __syncwarp();
             }
         }
     } else if (warp == 3) {
         // ------------------------------------------------------------ MMA issuer of the values
-        if (lane == 0) {
+        {
             constexpr uint32_t ID_PV = idesc_bf16(128, PA_DV, 0, 1);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint64_t dP0 = smem_desc(base + PA_OFF_P, 16, 1024), dC0 = smem_desc(base + PA_OFF_C, PA_KT * 128, 1024);
             bool ok = true;
             int cc = 0;                              // value tiles issued so far
             for (int k = 0; ok; k++) {
@@ -336,26 +354,33 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 AttnItem it;
                 ok = next_item(k, w, it);
                 if (!ok || w < 0) break;
+                const int tiles = __shfl_sync(0xffffffffu, it.nt - it.lo, 0);
                 if (k > 0) {                         // the accumulator of the previous item has been read out
                     ok = mbar_wait(bar(PB_OFREE), (uint32_t)((k - 1) & 1), p.err, 1016);
                     if (!ok) break;
                 }
-                for (int i = it.lo; i < it.nt && ok; i++, cc++) {
+                for (int i = 0; i < tiles && ok; i++, cc++) {
                     const int cs = cc % PA_CST, cu = cc / PA_CST, pb = cc & 1, pu = cc >> 1;
                     ok = mbar_wait(bar(PB_CFULL + cs), (uint32_t)(cu & 1), p.err, 1014);
                     if (ok) ok = mbar_wait(bar(PB_PFULL + pb), (uint32_t)(pu & 1), p.err, 1015);
                     if (!ok) break;
                     tc_fence_after();
                     // values: O += P lat, P [128 q][64 keys] K-major, lat half [64 keys][256] with the 256 contiguous (MN-major, four 64-wide blocks)
-                    const uint64_t dP = smem_desc(base + PA_OFF_P + pb * PA_P_BYTES, 16, 1024);
-                    const uint64_t dC = smem_desc(base + PA_OFF_C + cs * PA_C_BYTES, PA_KT * 128, 1024);
+                    const uint64_t dP = dP0 + (uint64_t)((pb * PA_P_BYTES) >> 4), dC = dC0 + (uint64_t)((cs * PA_C_BYTES) >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int s = 0; s < 4; s++)
-                        umma_bf16(tmem + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, (s != 0) ? 1u : (uint32_t)(i != it.lo));
-                    umma_commit(bar(PB_CEMPTY + cs));
-                    umma_commit(bar(PB_PEMPTY + pb));
+                        for (int s = 0; s < 4; s++) {
+                            const uint32_t acc = s != 0 ? 1u : (uint32_t)(i != 0);
+                            if (OWN_P) umma_bf16_ts(tm + PA_COL_O, tm + PA_COL_P + s * 8, dC + (uint64_t)((s * 2048) >> 4), ID_PV, acc);
+                            else umma_bf16(tm + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, acc);
+                        }
+                        umma_commit(bar(PB_CEMPTY + cs));
+                        umma_commit(bar(PB_PEMPTY + pb));
+                    }
+                    __syncwarp();
                 }
-                if (ok) umma_commit(bar(PB_ODONE));
+                if (ok && elect_one()) umma_commit(bar(PB_ODONE));
+                __syncwarp();
             }
         }
     } else {
@@ -365,6 +390,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         const int q4 = warp & 3, wg = (warp - 4) >> 2, cg = wg & (TG - 1), odd = wg / TG;      // columns cg * NC .., tiles of parity `odd`
         const int row = q4 * 32 + lane;
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
+        auto arrive = [&](int b) {                   // one for the warp, after every lane's accesses
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(b));
+        };
         bool ok = true;
         int tc = 0;                                  // tiles done so far (score buffer, P buffer and their phases run across items)
         for (int k = 0; ok; k++) {
@@ -376,33 +405,32 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             const int64_t tq = p.pos0 + q0 + row;                    // this row's position: keys 0..tq are visible
             // The query tile is the A operand of every score MMA of the item; it is kept in tensor memory (row = lane, two
             // consecutive bf16 per 32-bit column), so that those MMAs read only the keys from shared memory. A thread
-            // copies its row's share: DQK / 2 columns split between the copying groups. The tile of item k + 1 is copied
+            // copies its row's share: DQK / 2 columns split between the groups. The tile of item k + 1 is copied
             // BEFORE the epilogue of item k (below), so that the next item's first scores are computed under that epilogue.
             auto load_query = [&](int q0_, int h_) {
-                constexpr int QG = (NWG == 4 && ((PA_DQK / 2) / 4) % 16 != 0) ? 2 : NWG;      // groups that copy (16-word stores)
-                constexpr int QW = (PA_DQK / 2) / QG;                // 32-bit words per copying thread
+                constexpr int QW = (PA_DQK / 2) / NWG;               // 32-bit words per copying thread
                 const int t = q0_ + row;
                 const uint4 *src = reinterpret_cast<const uint4 *>(p.q + ((int64_t)t * p.nh + h_) * PA_DQK) + wg * (QW / 4);
 #pragma unroll
-                for (int c = 0; c < (wg < QG ? QW / 16 : 0); c++) {
-                    uint32_t wv[16];
+                for (int c = 0; c < QW / 8; c++) {
+                    uint32_t wv[8];
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const uint4 v = (t < p.n) ? src[c * 4 + j] : make_uint4(0, 0, 0, 0);
+                    for (int j = 0; j < 2; j++) {
+                        const uint4 v = (t < p.n) ? src[c * 2 + j] : make_uint4(0, 0, 0, 0);
                         wv[4 * j] = v.x; wv[4 * j + 1] = v.y; wv[4 * j + 2] = v.z; wv[4 * j + 3] = v.w;
                     }
-                    TMEM_ST16(wv, 0, tlane + PA_COL_Q + wg * QW + c * 16);
+                    TMEM_ST8(wv, 0, tlane + PA_COL_Q + wg * QW + c * 8);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
-                mbar_arrive(bar(PB_QFULL));
+                arrive(PB_QFULL);
             };
             if (k == 0) load_query(q0, h);
             float m = 0.f, l = 0.f;
             // reference exponent of the row: its largest score of the item's first tile, which one pair of groups has. (All arrive:
             // no P is written before the epilogue of the item before has left the P buffers.)
             auto reference = [&]() -> bool {
-                mbar_arrive(bar(PB_XM));
+                arrive(PB_XM);
                 if (!mbar_wait(bar(PB_XM), (uint32_t)(k & 1), p.err, 1026)) return false;
                 m = fmaxf(s_m[row], s_m[128 + row]);                 // the tile shows every row a key: finite
                 return true;
@@ -420,8 +448,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 for (int c = 0; c < NC / 16; c++) TMEM_LD16(v, c * 16, tlane + PA_COL_S + sb * PA_KT + cg * NC + c * 16);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(PB_SEMPTY + sb));
+                arrive(PB_SEMPTY + sb);
                 const bool whole = (int64_t)i * PA_KT + PA_KT - 1 <= p.pos0 + q0;      // every key of the tile is visible to every row of the item
                 const int seen = (int)min(tq - (int64_t)i * PA_KT - cg * NC, (int64_t)PA_KT);      // the thread's keys 0 .. seen are visible
                 if (NWG == 4 && i == it.lo) {
@@ -489,17 +516,26 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 float l0, l1;
                 unpack_f32x2(lsum, l0, l1);
                 l += l0 + l1;
-                // the P buffer of this parity was read by the value MMAs two tiles ago
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023));
-                if (!ok) break;
-                uint8_t *prow = sm + PA_OFF_P + sb * PA_P_BYTES + row * 128;
+                if (OWN_P) {
+                    // P has columns of its own once the value MMAs of the tile before are done with them
+                    if (tc0 + d > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + ((tc0 + d - 1) & 1)), (uint32_t)(((tc0 + d - 1) >> 1) & 1), p.err, 1023));
+                    if (!ok) break;
+                    tc_fence_after();
 #pragma unroll
-                for (int c = 0; c < NC / 8; c++)
-                    *reinterpret_cast<uint4 *>(prow + (((cg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    for (int c = 0; c < NC / 32; c++) TMEM_ST16(pk, c * 16, tlane + PA_COL_P + cg * (NC / 2) + c * 16);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                } else {
+                    // the P buffer of this parity was read by the value MMAs two tiles ago
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023));
+                    if (!ok) break;
+                    uint8_t *prow = sm + PA_OFF_P + sb * PA_P_BYTES + row * 128;
+#pragma unroll
+                    for (int c = 0; c < NC / 8; c++)
+                        *reinterpret_cast<uint4 *>(prow + (((cg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
                 tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(PB_PFULL + sb));
+                arrive(PB_PFULL + sb);
             }
             if (!ok) break;
             {
@@ -522,7 +558,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             tc_fence_after();
             if (NWG == 4) {                                          // the row's sum is the groups' sums
                 s_l[wg * 128 + row] = l;
-                mbar_arrive(bar(PB_XL));
+                arrive(PB_XL);
                 ok = mbar_wait(bar(PB_XL), (uint32_t)(k & 1), p.err, 1027);
                 if (!ok) break;
                 l = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
@@ -542,16 +578,16 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 }
                 if (wg == 0) { rec[PA_QT * PA_DV + row] = m; rec[PA_QT * (PA_DV + 1) + row] = l; }
                 tc_fence_before();
-                mbar_arrive(bar(PB_OFREE));
+                arrive(PB_OFREE);
                 continue;
             }
+            // All groups write out (two of four, 64 columns at a time: 12 k cycles an item with the next query's copy; now 8 k)
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            uint8_t *stg = sm + PA_OFF_P + (warp - 4) * 4096;         // 4 KB per warp: [32 rows][128 B], in the P buffers (idle: the item's value MMAs are done, and the next item's P comes from these threads)
+            uint8_t *stg = sm + PA_OFF_P + (warp - 4) * 2048;         // 2 KB per warp: [32 rows][64 B], in the P buffers (idle: the item's value MMAs are done, and the next item's P comes from these threads)
             const int t0w = q0 + q4 * 32;
-            constexpr int EG = NWG > 2 ? 2 : NWG;                     // groups that write out (the staging tiles are the two P buffers: eight warps)
-            constexpr int NCH = PA_DV / 64 / EG;                      // 64-column chunks per writing thread
+            constexpr int NCH = PA_DV / 64 / NWG;                     // 64-column chunks per thread
 #pragma unroll 1
-            for (int c = 0; c < (wg < EG ? NCH : 0); c++) {
+            for (int c = 0; c < NCH; c++) {
                 const int col = (wg * NCH + c) * 64;
                 uint32_t o[64];
                 TMEM_LD16(o, 0, tlane + PA_COL_O + col);
@@ -559,27 +595,33 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 TMEM_LD16(o, 32, tlane + PA_COL_O + col + 32);
                 TMEM_LD16(o, 48, tlane + PA_COL_O + col + 48);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    uint4 wv;
-                    wv.x = pack_bf16x2(__uint_as_float(o[8 * j]) * inv, __uint_as_float(o[8 * j + 1]) * inv);
-                    wv.y = pack_bf16x2(__uint_as_float(o[8 * j + 2]) * inv, __uint_as_float(o[8 * j + 3]) * inv);
-                    wv.z = pack_bf16x2(__uint_as_float(o[8 * j + 4]) * inv, __uint_as_float(o[8 * j + 5]) * inv);
-                    wv.w = pack_bf16x2(__uint_as_float(o[8 * j + 6]) * inv, __uint_as_float(o[8 * j + 7]) * inv);
-                    *reinterpret_cast<uint4 *>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) = wv;
+                if (c == NCH - 1) {
+                    tc_fence_before();
+                    arrive(PB_OFREE);                                // the value MMAs of the next item may overwrite the accumulator
                 }
-                __syncwarp();
 #pragma unroll
-                for (int r8 = 0; r8 < 8; r8++) {
-                    const int rr = r8 * 4 + (lane >> 3), jj = lane & 7;
-                    const uint4 wv = *reinterpret_cast<const uint4 *>(stg + rr * 128 + ((jj ^ (rr & 7)) << 4));
-                    if (t0w + rr < p.n)
-                        *reinterpret_cast<uint4 *>(p.out + ((int64_t)(t0w + rr) * p.nh + h) * (GQA ? PA_DV : PA_L) + half * PA_DV + col + jj * 8) = wv;
+                for (int u = 0; u < 2; u++) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const uint32_t *x = o + u * 32 + 8 * j;
+                        uint4 wv;
+                        wv.x = pack_bf16x2(__uint_as_float(x[0]) * inv, __uint_as_float(x[1]) * inv);
+                        wv.y = pack_bf16x2(__uint_as_float(x[2]) * inv, __uint_as_float(x[3]) * inv);
+                        wv.z = pack_bf16x2(__uint_as_float(x[4]) * inv, __uint_as_float(x[5]) * inv);
+                        wv.w = pack_bf16x2(__uint_as_float(x[6]) * inv, __uint_as_float(x[7]) * inv);
+                        *reinterpret_cast<uint4 *>(stg + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = wv;
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const int rr = r * 8 + (lane >> 2), jj = lane & 3;
+                        const uint4 wv = *reinterpret_cast<const uint4 *>(stg + rr * 64 + ((jj ^ ((rr >> 1) & 3)) << 4));
+                        if (t0w + rr < p.n)
+                            *reinterpret_cast<uint4 *>(p.out + ((int64_t)(t0w + rr) * p.nh + h) * (GQA ? PA_DV : PA_L) + half * PA_DV + col + u * 32 + jj * 8) = wv;
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
-            tc_fence_before();
-            mbar_arrive(bar(PB_OFREE));                              // the value MMAs of the next item may overwrite the accumulator
         }
     }
     tc_fence_before();

@@ -32,6 +32,14 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+// One lane of a converged warp (the same one each time). tcgen05.mma takes its descriptors from uniform registers: a warp whose lanes
+// all run the issue loop and elect one for the instruction itself keeps them there; a loop that one lane runs alone moves them
+// over for every MMA.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e != 0;
+}
 // Bounded wait. Returns false (and records `code`) when it gives up.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err, int code) {
     for (uint32_t i = 0; i < WAIT_LIMIT; i++)
@@ -133,6 +141,12 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
                    "=r"(arr[off + 8]), "=r"(arr[off + 9]), "=r"(arr[off + 10]), "=r"(arr[off + 11]),        \
                    "=r"(arr[off + 12]), "=r"(arr[off + 13]), "=r"(arr[off + 14]), "=r"(arr[off + 15])       \
                  : "r"(taddr))
+#define TMEM_ST8(arr, off, taddr)                                                                           \
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"                   \
+                 ::"r"(arr[off + 0]), "r"(arr[off + 1]), "r"(arr[off + 2]), "r"(arr[off + 3]),              \
+                   "r"(arr[off + 4]), "r"(arr[off + 5]), "r"(arr[off + 6]), "r"(arr[off + 7]),              \
+                   "r"(taddr)                                                                               \
+                 : "memory")
 #define TMEM_ST16(arr, off, taddr)                                                                          \
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" \
                  ::"r"(arr[off + 0]), "r"(arr[off + 1]), "r"(arr[off + 2]), "r"(arr[off + 3]),              \
