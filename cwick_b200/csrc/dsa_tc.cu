@@ -25,7 +25,11 @@
 // Pipeline of step 1 per 128-key tile: TMA (raw E4M3 tile, 16 KB, 8 stages) -> 8 converter warps
 // (cvt.rn.f16x2.e4m3x2; a thread owns a key row and stores its f16 pairs into tensor memory, where
 // they are the MMA's A operand: shared-memory bandwidth bounds this kernel, and so the MMAs read only
-// the query from it) -> MMA issuer (8 MMAs, M 128, N 128) -> 4 epilogue warps (TMEM -> a[c]).
+// the query from it) -> MMA issuer (8 MMAs, M 128, N 128) -> two groups of 4 epilogue warps on alternate
+// tiles (TMEM -> a[c]), three accumulators between them.
+// What bounded it was the chain around the MMAs (520 cycles of a tile's 1.27 k): one group's epilogue of 750 cycles, 640 arrivals a
+// tile at its barriers (now one per warp), an issue loop run by one lane. 8 sequences x 65536 keys: 31.6 -> 25.1 us from
+// cold caches (bytes alone: 10.6).
 // Blocks are persistent over the tiles of one sequence.
 // Every mbarrier wait is bounded and records a code in the context's error word when it gives up.
 #include <algorithm>
@@ -44,13 +48,14 @@ constexpr int IT_QROWS = 2 * IT_IH;                      // q split into f16 hi 
 constexpr int Q_BYTES_I = IT_QROWS * IT_HD * 2;         // 32768: two [128][64] f16 blocks
 constexpr int I_OFF_Q = 0;
 constexpr int I_OFF_RAW = Q_BYTES_I;                    // 8 stages of raw E4M3 tiles (128-byte swizzle)
-constexpr uint32_t I_COL_D = 0, I_COL_A = 256;          // TMEM: two 128-column accumulators, two 64-column A operands (f16 pairs)
+constexpr int IT_ACC = 3;                                // accumulators
+constexpr uint32_t I_COL_D = 0, I_COL_A = IT_ACC * 128; // TMEM: three 128-column accumulators, two 64-column A operands (f16 pairs)
 constexpr int I_OFF_BAR = I_OFF_RAW + RAW_STAGES * RAW_BYTES;
-constexpr int I_OFF_W = I_OFF_BAR + 256;                // 19 words: warp maxima of the query split, 1 / scale, sign masks of the head weights
+constexpr int I_OFF_W = I_OFF_BAR + 256;                // 23 words: warp maxima of the query split, 1 / scale, sign masks of the head weights
 constexpr int I_SMEM = I_OFF_W + 256 + 1024;
-constexpr int IT_THREADS = 512;                          // TMA, MMA, 2 idle | 8 converter warps | 4 epilogue warps
+constexpr int IT_THREADS = 640;                          // TMA, MMA, 2 idle | 8 converter warps | two groups of 4 epilogue warps
 constexpr int IT_CONV = 256;
-enum { IB_RAW_FULL = 0, IB_RAW_EMPTY = 8, IB_A_FULL = 16, IB_A_EMPTY = 18, IB_D_FULL = 20, IB_D_EMPTY = 22, IB_COUNT = 24 };
+enum { IB_RAW_FULL = 0, IB_RAW_EMPTY = 8, IB_A_FULL = 16, IB_A_EMPTY = 18, IB_D_FULL = 20, IB_D_EMPTY = IB_D_FULL + IT_ACC, IB_COUNT = IB_D_EMPTY + IT_ACC };
 
 // M x N f16 x f16 -> f32, both operands K-major
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
@@ -94,8 +99,8 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_keys) : "memory");
         for (int i = 0; i < IB_COUNT; i++) {
             uint32_t cnt = 1u;
-            if (i >= IB_RAW_EMPTY && i < IB_A_EMPTY) cnt = IT_CONV;   // raw_empty, a_full: every converter thread
-            if (i >= IB_D_EMPTY) cnt = 128u;                          // d_empty: every epilogue thread
+            if (i >= IB_RAW_EMPTY && i < IB_A_EMPTY) cnt = IT_CONV / 32;      // raw_empty, a_full: every converter warp
+            if (i >= IB_D_EMPTY) cnt = 4u;                                    // d_empty: every warp of an epilogue group
             mbar_init(bar(i), cnt);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -109,6 +114,13 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
     const int nt = t_end - t_begin;
     if (blockIdx.x == 0 && tid < 2) p.band[2 * b + tid] = 0;
     if (nt <= 0) return;
+    auto load_tile = [&](int i) {
+        const int r = i % RAW_STAGES;
+        mbar_expect_tx(bar(IB_RAW_FULL + r), RAW_BYTES);
+        tma_load_2d(base + I_OFF_RAW + r * RAW_BYTES, &tm_keys, 0, (int)((int64_t)b * p.key_stride + (int64_t)(t_begin + i) * IT_KEYS), bar(IB_RAW_FULL + r));
+    };
+    if (tid == 0)                                             // the first stages are on their way while the query is split
+        for (int i = 0; i < min(nt, RAW_STAGES); i++) load_tile(i);
 
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(512u) : "memory");
@@ -118,9 +130,10 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
     // the magnitude of its head's weight (w ReLU(x) = sign(w) ReLU(|w| x)) and by a power of two that brings the
     // sequence's largest product into [2^13, 2^14); rows 0-63 of the operand hold the f16 roundings, rows 64-127
     // the f16 roundings of the remainders (22 bits of every product survive). Two swizzled [128][64] blocks.
-    float *s_red = reinterpret_cast<float *>(sm + I_OFF_W);           // [16] warp maxima, then [16] = 1 / scale, [17..18] sign masks
+    float *s_red = reinterpret_cast<float *>(sm + I_OFF_W);           // [20] warp maxima, then [20] = 1 / scale, [21..22] sign masks
     {
-        const int h = tid >> 3, d0 = (tid & 7) * 16;
+        const bool splits = tid < IT_IH * 8;                  // eight threads per head
+        const int h = splits ? tid >> 3 : 0, d0 = (tid & 7) * 16;
         const float w = fabsf(p.wt[(int64_t)b * IT_IH + h]);
         float x[16];
         float m = 0.f;
@@ -135,7 +148,7 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
         if (lane == 0) s_red[warp] = m;
         if (tid < IT_IH) {
             const uint32_t neg = __ballot_sync(0xffffffffu, p.wt[(int64_t)b * IT_IH + tid] < 0.f);
-            if (lane == 0) reinterpret_cast<uint32_t *>(s_red)[17 + warp] = neg;
+            if (lane == 0) reinterpret_cast<uint32_t *>(s_red)[21 + warp] = neg;
         }
         __syncthreads();
         m = 0.f;
@@ -148,7 +161,7 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
             scale = __uint_as_float((uint32_t)(127 + sh) << 23);
             inv = __uint_as_float((uint32_t)(127 - sh) << 23);
         }
-        if (tid == 0) s_red[16] = inv;
+        if (tid == 0) s_red[20] = inv;
         uint32_t hi[8], lo[8];
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
@@ -159,7 +172,7 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
             lo[j >> 1] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
         }
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
+        for (int c = 0; c < (splits ? 2 : 0); c++) {
             const int c16 = (tid & 7) * 2 + c;                                 // 16-byte chunk of the 256-byte row
             uint8_t *blk = sm + I_OFF_Q + (c16 >> 3) * (IT_QROWS * 128);
             const int cc = c16 & 7;
@@ -177,32 +190,34 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
     if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
-            for (int i = 0; i < nt && ok; i++) {
-                const int r = i % RAW_STAGES, use = i / RAW_STAGES;
-                ok = mbar_wait(bar(IB_RAW_EMPTY + r), (uint32_t)((use & 1) ^ 1), p.err, 801);
-                if (!ok) break;
-                mbar_expect_tx(bar(IB_RAW_FULL + r), RAW_BYTES);
-                tma_load_2d(base + I_OFF_RAW + r * RAW_BYTES, &tm_keys, 0,
-                            (int)((int64_t)b * p.key_stride + (int64_t)(t_begin + i) * IT_KEYS), bar(IB_RAW_FULL + r));
+            for (int i = RAW_STAGES; i < nt && ok; i++) {
+                ok = mbar_wait(bar(IB_RAW_EMPTY + i % RAW_STAGES), (uint32_t)(((i / RAW_STAGES) & 1) ^ 1), p.err, 801);
+                if (ok) load_tile(i);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t ID = idesc_f16(128, IT_QROWS);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint64_t db = smem_desc(base + I_OFF_Q, 16, 1024);
             bool ok = true;
+            int d = 0, du = 0;                               // accumulator and its use
             for (int i = 0; i < nt && ok; i++) {
                 const int ab = i & 1, use = i >> 1;
-                ok = mbar_wait(bar(IB_A_FULL + ab), (uint32_t)(use & 1), p.err, 803);
-                if (ok) ok = mbar_wait(bar(IB_D_EMPTY + ab), (uint32_t)((use & 1) ^ 1), p.err, 804);
+                ok = mbar_wait(bar(IB_D_EMPTY + d), (uint32_t)((du & 1) ^ 1), p.err, 804);
+                if (ok) ok = mbar_wait(bar(IB_A_FULL + ab), (uint32_t)(use & 1), p.err, 803);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t db = smem_desc(base + I_OFF_Q, 16, 1024);
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 8; ks++)          // A: the converted keys in tensor memory, 16 f16 of every row = 8 columns per step
-                    umma_bf16_ts(tmem + I_COL_D + ab * 128, tmem + I_COL_A + ab * 64 + ks * 8,
-                                 db + (uint64_t)(((ks >> 2) * (IT_QROWS * 128) + (ks & 3) * 32) >> 4), ID, ks != 0);
-                umma_commit(bar(IB_A_EMPTY + ab));
-                umma_commit(bar(IB_D_FULL + ab));
+                    for (int ks = 0; ks < 8; ks++)          // A: the converted keys in tensor memory, 16 f16 of every row = 8 columns per step
+                        umma_bf16_ts(tm + I_COL_D + d * 128, tm + I_COL_A + ab * 64 + ks * 8,
+                                     db + (uint64_t)(((ks >> 2) * (IT_QROWS * 128) + (ks & 3) * 32) >> 4), ID, ks != 0);
+                    umma_commit(bar(IB_A_EMPTY + ab));
+                    umma_commit(bar(IB_D_FULL + d));
+                }
+                __syncwarp();
+                if (++d == IT_ACC) { d = 0; du++; }
             }
         }
     } else if (warp >= 4 && warp < 12) {
@@ -236,52 +251,56 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
-            mbar_arrive(bar(IB_A_FULL + ab));
-            mbar_arrive(bar(IB_RAW_EMPTY + r));
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(bar(IB_A_FULL + ab));
+                mbar_arrive(bar(IB_RAW_EMPTY + r));
+            }
         }
     } else if (warp >= 12) {
         // ---------------- epilogue: hi + lo, ReLU, signed head sum, key scale
+        // (two groups take alternate tiles)
         const int q4 = warp & 3;
         const int row = q4 * 32 + lane;
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
-        const float unscale = s_red[16];
-        const uint32_t neg[2] = {reinterpret_cast<const uint32_t *>(s_red)[17], reinterpret_cast<const uint32_t *>(s_red)[18]};
+        const float unscale = s_red[20];
+        const uint32_t neg[2] = {reinterpret_cast<const uint32_t *>(s_red)[21], reinterpret_cast<const uint32_t *>(s_red)[22]};
         const bool any_neg = (neg[0] | neg[1]) != 0;
         bool ok = true;
-        for (int i = 0; i < nt; i++) {
-            const int ab = i & 1, use = i >> 1;
-            ok = mbar_wait(bar(IB_D_FULL + ab), (uint32_t)(use & 1), p.err, 807);
+        for (int i = (warp - 12) >> 2; i < nt; i += 2) {
+            const int d = i % IT_ACC;
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(IB_D_FULL + d), (uint32_t)((i / IT_ACC) & 1), p.err, 807));
             if (!ok) break;
             tc_fence_after();
             const int64_t key = (int64_t)(t_begin + i) * IT_KEYS + row;
             const float ksc = key < nb ? p.kscale[(int64_t)b * p.key_stride + key] : 0.f;
             float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                uint32_t v[32], u[32];
-                TMEM_LD16(v, 0, tlane + ab * 128 + c * 32);             // codes . q_hi
-                TMEM_LD16(v, 16, tlane + ab * 128 + c * 32 + 16);
-                TMEM_LD16(u, 0, tlane + ab * 128 + 64 + c * 32);        // codes . q_lo
-                TMEM_LD16(u, 16, tlane + ab * 128 + 64 + c * 32 + 16);
+            for (int c = 0; c < 4; c++) {
+                uint32_t v[16], u[16];
+                TMEM_LD16(v, 0, tlane + d * 128 + c * 16);              // codes . q_hi
+                TMEM_LD16(u, 0, tlane + d * 128 + 64 + c * 16);         // codes . q_lo
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (!any_neg) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
+                    for (int j = 0; j < 16; j += 2) {
                         acc0 += fmaxf(__uint_as_float(v[j]) + __uint_as_float(u[j]), 0.f);
                         acc1 += fmaxf(__uint_as_float(v[j + 1]) + __uint_as_float(u[j + 1]), 0.f);
                     }
                 } else {
+                    const uint32_t ng = neg[c >> 1] >> ((c & 1) * 16);
 #pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
+                    for (int j = 0; j < 16; j += 2) {
                         const float r0 = fmaxf(__uint_as_float(v[j]) + __uint_as_float(u[j]), 0.f);
                         const float r1 = fmaxf(__uint_as_float(v[j + 1]) + __uint_as_float(u[j + 1]), 0.f);
-                        acc0 += __uint_as_float(__float_as_uint(r0) ^ (((neg[c] >> j) & 1u) << 31));
-                        acc1 += __uint_as_float(__float_as_uint(r1) ^ (((neg[c] >> (j + 1)) & 1u) << 31));
+                        acc0 += __uint_as_float(__float_as_uint(r0) ^ (((ng >> j) & 1u) << 31));
+                        acc1 += __uint_as_float(__float_as_uint(r1) ^ (((ng >> (j + 1)) & 1u) << 31));
                     }
                 }
             }
             tc_fence_before();
-            mbar_arrive(bar(IB_D_EMPTY + ab));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(IB_D_EMPTY + d));
             if (key < nb) p.sc[(int64_t)b * p.key_stride + key] = (acc0 + acc1) * unscale * ksc;
         }
     }
