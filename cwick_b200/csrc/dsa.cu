@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(128) indexer_scores_fp8_kernel(
 // it in index order, `want` in all (ascending: one list in index order).
 __global__ void __cluster_dims__(TK_CL, 1, 1) __launch_bounds__(TK_THREADS, 1)
 topk_select_kernel(const float *sc, int64_t sc_stride, const int32_t *n, int want, int keep_self, int32_t *sel, int64_t sel_ld,
-                   int32_t *nsel, int ascending, const int32_t *band_list, const int32_t *band_count) {
+                   int32_t *nsel, int ascending) {
     cg::cluster_group cl = cg::this_cluster();
     const unsigned rank = cl.block_rank();
     const int b = blockIdx.y, tid = threadIdx.x;
@@ -89,9 +89,10 @@ topk_select_kernel(const float *sc, int64_t sc_stride, const int32_t *n, int wan
     __shared__ TkShared sh;
     uint32_t kc[TK_PT];
     if (sl.cached) tk_load(s, sl.begin, sl.end, kc);
-    tk_threshold_and_compact(s, sl, kc, nb, want, keep_self, ascending, out, nsel + b,
-                             band_list ? band_list + (int64_t)b * sc_stride : nullptr, band_list ? band_count[2 * b] : 0,
-                             band_list ? band_count[2 * b + 1] : 0, sh);
+    uint32_t thr;
+    int need_eq;
+    tk_radix_select(s, sl, kc, want, sh, thr, need_eq);
+    tk_compact(s, sl, kc, nb, want, keep_self, ascending, out, nsel + b, thr, need_eq, sh);
 }
 
 extern "C" {
@@ -121,7 +122,7 @@ int cwk_topk_select(cwk_ctx *ctx, const float *sc, int64_t sc_stride, const int3
     (void)max_n;
     CWK_CUDA(ctx, cudaSetDevice(ctx->device));
     CwkKernelTimer timer(ctx);
-    topk_select_kernel<<<dim3(TK_CL, B), TK_THREADS, 0, ctx->stream>>>(sc, sc_stride, n, want, keep_self, sel, sel_ld, nsel, 0, nullptr, nullptr);
+    topk_select_kernel<<<dim3(TK_CL, B), TK_THREADS, 0, ctx->stream>>>(sc, sc_stride, n, want, keep_self, sel, sel_ld, nsel, 0);
     CWK_LAUNCH_CHECK(ctx, "topk_select_kernel");
     return CWK_OK;
 }
@@ -136,7 +137,7 @@ int cwk_ds_topk(cwk_ctx *ctx, const float *sc, int64_t sc_stride, const int32_t 
         return cwk_fail(ctx, CWK_ERR_ARGUMENT, "ds_topk: bad argument");
     CWK_CUDA(ctx, cudaSetDevice(ctx->device));
     CwkKernelTimer timer(ctx);
-    topk_select_kernel<<<dim3(TK_CL, B), TK_THREADS, 0, ctx->stream>>>(sc, sc_stride, n, k, 0, out, out_ld, count, 1, nullptr, nullptr);
+    topk_select_kernel<<<dim3(TK_CL, B), TK_THREADS, 0, ctx->stream>>>(sc, sc_stride, n, k, 0, out, out_ld, count, 1);
     CWK_LAUNCH_CHECK(ctx, "topk_select_kernel<ascending>");
     return CWK_OK;
 }

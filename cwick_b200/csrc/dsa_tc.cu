@@ -11,16 +11,17 @@
 //      times |w_h| and a power of two, is split into an f16 high part and an f16 low part (128 MMA
 //      columns), so the MMA D[128 keys][hi|lo] = codes . q^T has exact products and f32
 //      accumulation, and the epilogue adds the two halves, applies ReLU, the signs and the key's scale.
-//   2. band_classify_kernel: a radix select on a[] gives the approximate want-th largest score tau.
+//   2. band_classify_kernel: a histogram of a[] between the row's smallest and largest score (2048 bins; the scoring kernel leaves
+//      the two) gives the bin [tau_lo, tau_hi] of the approximate want-th largest score.
 //      The want-th largest value moves by at most delta when every score moves by at most delta, so
-//      keys with a > tau + 2*delta are certainly selected (refined = +inf), keys with
-//      a < tau - 2*delta certainly are not (-inf), and the band in between is listed. (delta is
+//      keys with a > tau_hi + 2*delta are certainly selected (refined = +inf), keys with
+//      a < tau_lo - 2*delta certainly are not (-inf), and the band in between is listed. (delta is
 //      taken as 2^-9 of the row's largest score, far above the contraction's and the query
-//      split's worst case.)
+//      split's worst case; the bin is at most a quarter of that wide.)
 //   3. the same kernel then re-scores the listed keys in the reference's exact order on CUDA cores (the
 //      cluster's blocks share the list).
-//   4. the selection kernel (csrc/dsa.cu) takes the exact threshold from the re-scored keys and
-//      writes the reference's list in the reference's order.
+//   4. the exact threshold is the (want - certainly selected)-th largest of those; the compaction of csrc/topk_radix.cuh writes
+//      the reference's list in the reference's order.
 //
 // Pipeline of step 1 per 128-key tile: TMA (raw E4M3 tile, 16 KB, 8 stages) -> 8 converter warps
 // (cvt.rn.f16x2.e4m3x2; a thread owns a key row and stores its f16 pairs into tensor memory, where
@@ -77,6 +78,7 @@ struct IdxParams {
     const int32_t *n;         // [B]
     float *sc;                // [B][key_stride]
     int32_t *band;            // [B][2] counters of the classification that follows: zeroed here
+    float2 *range;            // [B][blocks per sequence][8] largest and smallest score of an epilogue warp, for the classification
     int64_t key_stride;
     int *err;
 };
@@ -113,7 +115,11 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
     const int t_end = (int)((int64_t)ntile * (blockIdx.x + 1) / blocks_per_seq);
     const int nt = t_end - t_begin;
     if (blockIdx.x == 0 && tid < 2) p.band[2 * b + tid] = 0;
-    if (nt <= 0) return;
+    float2 *range = p.range + ((int64_t)b * blocks_per_seq + blockIdx.x) * 8;
+    if (nt <= 0) {
+        if (tid < 8) range[tid] = make_float2(-INFINITY, INFINITY);
+        return;
+    }
     auto load_tile = [&](int i) {
         const int r = i % RAW_STAGES;
         mbar_expect_tx(bar(IB_RAW_FULL + r), RAW_BYTES);
@@ -267,6 +273,7 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
         const uint32_t neg[2] = {reinterpret_cast<const uint32_t *>(s_red)[21], reinterpret_cast<const uint32_t *>(s_red)[22]};
         const bool any_neg = (neg[0] | neg[1]) != 0;
         bool ok = true;
+        float mx = -INFINITY, mn = INFINITY;
         for (int i = (warp - 12) >> 2; i < nt; i += 2) {
             const int d = i % IT_ACC;
             ok = __all_sync(0xffffffffu, mbar_wait(bar(IB_D_FULL + d), (uint32_t)((i / IT_ACC) & 1), p.err, 807));
@@ -301,8 +308,19 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(IB_D_EMPTY + d));
-            if (key < nb) p.sc[(int64_t)b * p.key_stride + key] = (acc0 + acc1) * unscale * ksc;
+            const float a = (acc0 + acc1) * unscale * ksc;
+            if (key < nb) {
+                p.sc[(int64_t)b * p.key_stride + key] = a;
+                mx = fmaxf(mx, a);
+                mn = fminf(mn, a);
+            }
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        }
+        if (lane == 0) range[warp - 12] = make_float2(mx, mn);
     }
     tc_fence_before();
     __syncthreads();
@@ -323,17 +341,35 @@ __device__ __forceinline__ float e4m3_to_f32_i(uint32_t b) {
 
 constexpr int BC_KEYS = 64;                                   // band keys re-scored per pass and block
 constexpr int BC_QLD = IT_HD + 4;                             // padded q rows in shared memory
-constexpr int BC_SMEM = (IT_IH * BC_QLD + IT_IH + BC_KEYS * IT_HD + BC_KEYS * (IT_IH + 1)) * 4;
+constexpr int BC_BINS = 2 * TK_THREADS;                       // histogram bins (two per thread), in the place of the re-scored keys
+constexpr int BC_LIST = 1024;                                 // a band of at most so many keys is ranked in shared memory
+constexpr int BC_SMEM = (IT_IH * BC_QLD + IT_IH + BC_KEYS * IT_HD + BC_KEYS * (IT_IH + 1) + BC_LIST + BC_LIST / TK_CL) * 4;
+static_assert(BC_BINS <= BC_KEYS * IT_HD, "the histogram lies in the place of the keys");
 
-// One cluster per sequence: the row's largest approximate score, the exact want-th largest
-// approximate score tau, then the classification of every key: certainly selected (refined =
-// +inf), certainly not (refined = -inf), or in the band |a - tau| <= eps, whose indices are appended
-// to band_list. band_count[2b] counts the band's entries, band_count[2b + 1] the keys above the band
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// One cluster per sequence: the histogram bin of the row's want-th largest approximate score, then the classification of every
+// key: certainly selected (refined = +inf), certainly not (refined = -inf), or in the band around the bin, whose indices are
+// appended to band_list. band_count[2b] counts the band's entries, band_count[2b + 1] the keys above the band
 // (both zeroed by the scoring kernel before it). The same launch then re-scores the band exactly and
 // writes the selection.
+// A chain of cluster-wide steps on 64 of the SMs, so what counts is their number and length. Four radix passes for the approximate
+// threshold (which need not be exact: a bin's width more in the band) became one histogram, four more over the re-scored keys a
+// ranking by comparison; a key's multiplications and additions go two at a time (the same roundings), warps without a key skip the
+// query rows, counters take one atomic per block: 36.7 -> 27.3 us for 8 x 65536 keys (67 k -> 49 k cycles: 13 to 15 k re-scoring, 9 k
+// histogram, 8 k compaction, 5 k classification, 4 k the threshold, the rest barriers and set-up).
 __global__ void __cluster_dims__(TK_CL, 1, 1) __launch_bounds__(TK_THREADS, 1)
 band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int want, float *refined, int32_t *band_list,
-                     int32_t *band_count, const uint8_t *keys, const float *kscale, const float *q, const float *wt,
+                     int32_t *band_count, const float2 *range, int ranges, const uint8_t *keys, const float *kscale, const float *q, const float *wt,
                      int keep_self, int32_t *sel, int64_t sel_ld, int32_t *nsel, long long *trace) {
 #ifdef CWK_TRACE
 #define BTRACE(i) do { if (trace && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) trace[i] = clock64(); } while (0)
@@ -344,9 +380,10 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
     BTRACE(0);
     extern __shared__ __align__(16) float bc_sm[];
     float *sq = bc_sm, *sw = sq + IT_IH * BC_QLD, *skey = sw + IT_IH, *sprod = skey + BC_KEYS * IT_HD;
+    uint32_t *hist = reinterpret_cast<uint32_t *>(skey), *sall = reinterpret_cast<uint32_t *>(sprod + BC_KEYS * (IT_IH + 1)), *sown = sall + BC_LIST;
     cg::cluster_group cl = cg::this_cluster();
     const unsigned rank = cl.block_rank();
-    const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+    const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     cwk_pdl_launch();
     cwk_pdl_wait();
     const int nb = n[b];
@@ -360,9 +397,15 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
         return;
     }
     __shared__ TkShared sh;
-    __shared__ float red[32];
+    __shared__ float red[2][32];
     uint32_t kc[TK_PT];
     if (sl.cached) tk_load(s, sl.begin, sl.end, kc);
+    float mx = -INFINITY, mn = INFINITY;      // the row's largest and smallest score
+    for (int i = tid; i < ranges; i += TK_THREADS) {
+        const float2 v = __ldcg(range + (int64_t)b * ranges + i);
+        mx = fmaxf(mx, v.x);
+        mn = fminf(mn, v.y);
+    }
     // the query and the head weights of this sequence, for the exact re-scoring at the end (padded rows: the heads of a
     // key's 16 threads then read different banks)
     for (int i = tid; i < IT_IH * (IT_HD / 4); i += TK_THREADS) {
@@ -370,41 +413,64 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
         *reinterpret_cast<float4 *>(sq + h * BC_QLD + c * 4) = __ldg(reinterpret_cast<const float4 *>(q + ((int64_t)b * IT_IH + h) * IT_HD) + c);
     }
     if (tid < IT_IH) sw[tid] = wt[(int64_t)b * IT_IH + tid];
-    // largest score of this block's slice (scores are sums of non-negative terms)
-    float m = 0.f;
+    *reinterpret_cast<uint2 *>(hist + 2 * tid) = make_uint2(0u, 0u);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    }
+    if (lane == 0) { red[0][warp] = mx; red[1][warp] = mn; }
+    __syncthreads();
+    mx = red[0][lane];
+    mn = red[1][lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    }
+    BTRACE(1);
+    // Bins of equal width. No width (all scores alike), or scores that are not finite: one bin, and the whole row is re-scored.
+    const float width = (mx - mn) * (1.0f / (BC_BINS - 1)), per_unit = 1.0f / width;
+    const bool wide = width > 0.f && width < INFINITY && per_unit < INFINITY;
+    auto bin_of = [&](float a) { return !wide ? 0 : a == a ? max(0, min(BC_BINS - 1, (int)((a - mn) * per_unit))) : BC_BINS - 1; };      // rises with a
     for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {
         if (!sl.cached) tk_load(s, c0, sl.end, kc);
         const int i0 = c0 + tid * TK_PT;
 #pragma unroll
         for (int j = 0; j < TK_PT; j++)
-            if (i0 + j < sl.end) m = fmaxf(m, fabsf(order_key_inverse(kc[j])));
+            if (i0 + j < sl.end) atomicAdd(hist + bin_of(order_key_inverse(kc[j])), 1u);
     }
+    cl.sync();
+    {
+        uint2 c = make_uint2(0u, 0u);                       // bins 2 tid and 2 tid + 1 of the whole row
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) red[tid >> 5] = m;
-    __syncthreads();
-    if (tid < 32) {
-        m = red[lane];
+        for (unsigned r = 0; r < TK_CL; r++) {
+            const uint2 v = *reinterpret_cast<const uint2 *>(cl.map_shared_rank(hist, r) + 2 * tid);
+            c.x += v.x; c.y += v.y;
+        }
+        uint32_t incl = c.x + c.y;                          // and the bins above them in the warp, then in the block
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) sh.fmax = m;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_down_sync(0xffffffffu, incl, o);
+            if (lane + o < 32) incl += t;
+        }
+        if (lane == 0) sh.tot[warp] = incl;
+        __syncthreads();
+        const uint32_t above = __reduce_add_sync(0xffffffffu, lane > warp ? sh.tot[lane] : 0u) + incl - (c.x + c.y), w = (uint32_t)want;
+        if (above < w && w <= above + c.x + c.y) sh.sel[0] = (uint32_t)(2 * tid) + (w <= above + c.y ? 1u : 0u);
+        __syncthreads();
     }
-    uint32_t prefix;
-    int remaining;
-    BTRACE(1);
-    tk_radix_select(s, sl, kc, want, sh, prefix, remaining);       // its cluster barriers also publish fmax
     BTRACE(2);
-    m = 0.f;
-#pragma unroll
-    for (unsigned r = 0; r < TK_CL; r++) m = fmaxf(m, *cl.map_shared_rank(&sh.fmax, r));
-    const float tau = order_key_inverse(prefix);
+    const float m = fmaxf(fabsf(mx), fabsf(mn));
     const float eps = 2.0f * 0.001953125f * m;              // 2 * delta, delta = 2^-9 of the row's largest score
-    const float hi = tau + eps, lo = tau - eps;
+    // (a hundredth of a bin covers the roundings of bin_of and of these)
+    const float hi = wide ? mn + ((float)sh.sel[0] + 1.01f) * width + eps : INFINITY, lo = wide ? mn + ((float)sh.sel[0] - 0.01f) * width - eps : -INFINITY;
     int32_t *list = band_list + (int64_t)b * stride;
+    uint32_t inb = 0;                                       // this thread's scores of the chunk that are in the band
     for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {
         if (!sl.cached) tk_load(s, c0, sl.end, kc);
         const int i0 = c0 + tid * TK_PT;
-        uint32_t inb = 0;
+        inb = 0;
         float v[TK_PT];
 #pragma unroll
         for (int j = 0; j < TK_PT; j++) {
@@ -420,32 +486,39 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
             for (int j = 0; j < TK_PT; j++)
                 if (i0 + j < sl.end) f[i0 + j] = v[j];
         }
-        {
-            int nab = 0;
+        // band entries and keys above it: counted for the block, one global atomic for both counters (the list's order does not matter)
+        uint32_t mine = __popc(inb);
 #pragma unroll
-            for (int j = 0; j < TK_PT; j++) nab += (i0 + j < sl.end && v[j] > 0.f) ? 1 : 0;
-            nab = __reduce_add_sync(0xffffffffu, nab);
-            if (lane == 0 && nab) atomicAdd(band_count + 2 * b + 1, nab);
-        }
-        // band entries: one global atomic per warp (the list's order does not matter; the rescoring
-        // kernel overwrites refined[] at these indices)
-        const int mine = __popc(inb);
-        int incl = mine;
+        for (int j = 0; j < TK_PT; j++) mine += (i0 + j < sl.end && v[j] > 0.f) ? 0x10000u : 0u;
+        uint32_t incl = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += t;
         }
-        const int wtot = __shfl_sync(0xffffffffu, incl, 31);
-        int at = 0;
-        if (lane == 31 && wtot) at = atomicAdd(band_count + 2 * b, wtot);
-        at = __shfl_sync(0xffffffffu, at, 31) + incl - mine;
+        if (lane == 31) sh.tot[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t tot = sh.tot[lane];
+            uint32_t to = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, to, o);
+                if (lane >= o) to += t;
+            }
+            uint32_t at = 0;
+            if (lane == 31 && to)
+                at = (uint32_t)atomicAdd(reinterpret_cast<unsigned long long *>(band_count + 2 * b), (unsigned long long)(to & 0xffffu) | ((unsigned long long)(to >> 16) << 32));
+            sh.tot[32 + lane] = __shfl_sync(0xffffffffu, at, 31) + ((to - tot) & 0xffffu);
+        }
+        __syncthreads();
+        int at = (int)(sh.tot[32 + warp] + ((incl - mine) & 0xffffu));
 #pragma unroll
         for (int j = 0; j < TK_PT; j++)
             if (inb & (1u << j)) list[at++] = i0 + j;
     }
     BTRACE(3);
-    cl.sync();                              // every block's part of the band list is written (and fmax has been read everywhere)
+    cl.sync();                              // every block's part of the band list is written (and the histograms have been read everywhere)
     BTRACE(4);
     // ---- exact scores of the band (the reference's order: src/attention.c:573-582 with dot_f32's grouping, :249-258).
     // The cluster's blocks share the list evenly; 64 keys per pass: dequantise into shared memory (16 threads per key),
@@ -474,27 +547,30 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
             // reads of one (key, head) pair per thread. Every dot keeps the reference's order: four strided accumulators
             // with separate multiply and add, then (s0 + s1) + (s2 + s3).
             const int ka = (tid >> 5) * 2, ha = lane, hb2 = lane + 32;
-            const float4 *kp0 = reinterpret_cast<const float4 *>(skey + ka * IT_HD), *kp1 = kp0 + IT_HD / 4;
-            const float4 *qp0 = reinterpret_cast<const float4 *>(sq + ha * BC_QLD), *qp1 = reinterpret_cast<const float4 *>(sq + hb2 * BC_QLD);
-            float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f}, b0[4] = {0.f, 0.f, 0.f, 0.f}, b1[4] = {0.f, 0.f, 0.f, 0.f};
+            if (k0 + ka < k_end) {           // (the query rows are most of what this reads from shared memory: not for keys that are not there)
+            const ulonglong2 *kp0 = reinterpret_cast<const ulonglong2 *>(skey + ka * IT_HD), *kp1 = kp0 + IT_HD / 4;
+            const ulonglong2 *qp0 = reinterpret_cast<const ulonglong2 *>(sq + ha * BC_QLD), *qp1 = reinterpret_cast<const ulonglong2 *>(sq + hb2 * BC_QLD);
+            // (products and sums are rounded apart: the sum is acc * 1 + product, with a 1 that the compiler does not see -- it fuses the
+            // pairwise multiplication with a pairwise addition)
+            const uint32_t one_bits = 0x3f800000u + (uint32_t)(nb >> 31);
+            const uint64_t one = ((uint64_t)one_bits << 32) | one_bits;
+            uint64_t a0[2] = {0, 0}, a1[2] = {0, 0}, b0[2] = {0, 0}, b1[2] = {0, 0};      // f32 pairs
 #pragma unroll 4
             for (int i = 0; i < IT_HD / 4; i++) {
-                const float4 k0v = kp0[i], k1v = kp1[i], q0v = qp0[i], q1v = qp1[i];
-                a0[0] = __fadd_rn(a0[0], __fmul_rn(k0v.x, q0v.x)); a0[1] = __fadd_rn(a0[1], __fmul_rn(k0v.y, q0v.y));
-                a0[2] = __fadd_rn(a0[2], __fmul_rn(k0v.z, q0v.z)); a0[3] = __fadd_rn(a0[3], __fmul_rn(k0v.w, q0v.w));
-                a1[0] = __fadd_rn(a1[0], __fmul_rn(k0v.x, q1v.x)); a1[1] = __fadd_rn(a1[1], __fmul_rn(k0v.y, q1v.y));
-                a1[2] = __fadd_rn(a1[2], __fmul_rn(k0v.z, q1v.z)); a1[3] = __fadd_rn(a1[3], __fmul_rn(k0v.w, q1v.w));
-                b0[0] = __fadd_rn(b0[0], __fmul_rn(k1v.x, q0v.x)); b0[1] = __fadd_rn(b0[1], __fmul_rn(k1v.y, q0v.y));
-                b0[2] = __fadd_rn(b0[2], __fmul_rn(k1v.z, q0v.z)); b0[3] = __fadd_rn(b0[3], __fmul_rn(k1v.w, q0v.w));
-                b1[0] = __fadd_rn(b1[0], __fmul_rn(k1v.x, q1v.x)); b1[1] = __fadd_rn(b1[1], __fmul_rn(k1v.y, q1v.y));
-                b1[2] = __fadd_rn(b1[2], __fmul_rn(k1v.z, q1v.z)); b1[3] = __fadd_rn(b1[3], __fmul_rn(k1v.w, q1v.w));
+                const ulonglong2 k0v = kp0[i], k1v = kp1[i], q0v = qp0[i], q1v = qp1[i];
+                a0[0] = fma_f32x2(a0[0], one, mul_f32x2(k0v.x, q0v.x)); a0[1] = fma_f32x2(a0[1], one, mul_f32x2(k0v.y, q0v.y));
+                a1[0] = fma_f32x2(a1[0], one, mul_f32x2(k0v.x, q1v.x)); a1[1] = fma_f32x2(a1[1], one, mul_f32x2(k0v.y, q1v.y));
+                b0[0] = fma_f32x2(b0[0], one, mul_f32x2(k1v.x, q0v.x)); b0[1] = fma_f32x2(b0[1], one, mul_f32x2(k1v.y, q0v.y));
+                b1[0] = fma_f32x2(b1[0], one, mul_f32x2(k1v.x, q1v.x)); b1[1] = fma_f32x2(b1[1], one, mul_f32x2(k1v.y, q1v.y));
             }
-            auto fin = [&](const float (&s4)[4], int kk, int h) {
+            auto fin = [&](const uint64_t (&s2)[2], int kk, int h) {
+                const float s4[4] = {__uint_as_float((uint32_t)s2[0]), __uint_as_float((uint32_t)(s2[0] >> 32)), __uint_as_float((uint32_t)s2[1]), __uint_as_float((uint32_t)(s2[1] >> 32))};
                 float d = __fadd_rn(__fadd_rn(s4[0], s4[1]), __fadd_rn(s4[2], s4[3]));
                 if (d < 0.f) d = 0.f;
                 sprod[kk * (IT_IH + 1) + h] = __fmul_rn(d, sw[h]);
             };
             fin(a0, ka, ha); fin(a1, ka, hb2); fin(b0, ka + 1, ha); fin(b1, ka + 1, hb2);
+            }
         }
         __syncthreads();
         if (tid < BC_KEYS && k0 + tid < k_end) {
@@ -502,17 +578,49 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
 #pragma unroll 8
             for (int h = 0; h < IT_IH; h++) tot = __fadd_rn(tot, sprod[tid * (IT_IH + 1) + h]);
             f[list[k0 + tid]] = tot;
+            if (total <= BC_LIST) sown[k0 - k_begin + tid] = order_key(tot);
         }
         __syncthreads();
     }
-    // ---- the selection itself, on the refined row: the exact threshold is the (want - certainly selected)-th largest of the
-    // re-scored keys; then the reference's list in the reference's order
+    // ---- the selection itself: the exact threshold is the (want - certainly selected)-th largest of the re-scored keys; then the
+    // reference's list in the reference's order
     BTRACE(5);
     cl.sync();                              // every block's re-scored keys are in refined[]
     BTRACE(6);
-    if (sl.cached) tk_load(f, sl.begin, sl.end, kc);
-    tk_threshold_and_compact(f, sl, kc, nb, want, keep_self, 0, out, nsel + b, list, total,
-                             *reinterpret_cast<volatile int32_t *>(band_count + 2 * b + 1), sh);
+    const int kth = max(1, min(want - *reinterpret_cast<volatile int32_t *>(band_count + 2 * b + 1), total));   // holds by construction; clamped against a violated error bound
+    uint32_t thr;
+    int need_eq;
+    if (total <= BC_LIST) {
+        // every block ranks its own keys among all of them; the block that has the kth tells the others
+        if (tid < total) sall[tid] = cl.map_shared_rank(sown, tid / per)[tid % per];
+        __syncthreads();
+        for (int k = warp; k < k_end - k_begin; k += TK_THREADS / 32) {
+            const uint32_t x = sown[k];
+            int gt = 0, ge = 0;
+            for (int i = lane; i < total; i += 32) {
+                gt += sall[i] > x ? 1 : 0;
+                ge += sall[i] >= x ? 1 : 0;
+            }
+            gt = __reduce_add_sync(0xffffffffu, gt);
+            ge = __reduce_add_sync(0xffffffffu, ge);
+            if (gt < kth && kth <= ge && lane < TK_CL)
+                *reinterpret_cast<uint2 *>(cl.map_shared_rank(sh.sel, (unsigned)lane)) = make_uint2(x, (uint32_t)(kth - gt));
+        }
+        cl.sync();
+        thr = sh.sel[0];
+        need_eq = (int)sh.sel[1];
+    } else {
+        tk_list_select(f, list, total, kth, sh, thr, need_eq);
+    }
+    if (sl.cached) {                        // the refined slice, of which only the band has to be read back
+        const int i0 = sl.begin + tid * TK_PT;
+#pragma unroll
+        for (int j = 0; j < TK_PT; j++) {
+            if (inb >> j & 1) kc[j] = order_key(__ldcg(f + i0 + j));
+            else kc[j] = order_key(order_key_inverse(kc[j]) > hi ? INFINITY : -INFINITY);
+        }
+    }
+    tk_compact(f, sl, kc, nb, want, keep_self, 0, out, nsel + b, thr, need_eq, sh);
     BTRACE(7);
 }
 
@@ -536,15 +644,18 @@ extern "C" int cwk_dsa_select(cwk_ctx *ctx, const void *keys, const float *kscal
     }
     const bool tc_ok = ih == IT_IH && hd == IT_HD && ((uintptr_t)keys % 16) == 0 && cwk_encode_tiled_fn() != nullptr &&
                        ctx->force_mla_path != 0 && ctx->force_mla_path != 1;
-    // workspace: approx f32 [B][stride], refined f32 [B][stride], band list int32 [B][stride], band counts [B][2]
+    // workspace: approx f32 [B][stride], refined f32 [B][stride], band list int32 [B][stride], band counts [B][2], ranges [B][blocks][8][2]
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t b_sc = up((size_t)B * key_stride * 4);
-    int s = cwk_reserve_work(ctx, 3 * b_sc + up((size_t)B * 8));
+    const int tiles = (max_n + IT_KEYS - 1) / IT_KEYS;
+    const int bps = std::max(1, std::min(tiles, ctx->sm_count / B));      // scoring blocks per sequence
+    int s = cwk_reserve_work(ctx, 3 * b_sc + up((size_t)B * 8) + (size_t)B * bps * 8 * sizeof(float2));
     if (s != CWK_OK) return s;
     uint8_t *w = (uint8_t *)ctx->work;
     float *approx = (float *)w, *refined = (float *)(w + b_sc);
     int32_t *band_list = (int32_t *)(w + 2 * b_sc);
     int32_t *band = (int32_t *)(w + 3 * b_sc);
+    float2 *range = (float2 *)(w + 3 * b_sc + up((size_t)B * 8));
     if (!tc_ok) {
         // shapes the tensor-core path is not built for: exact scores for every key
         s = cwk_indexer_scores_fp8(ctx, keys, kscale, key_stride, q, wt, n, max_n, B, ih, hd, scores_out ? scores_out : approx);
@@ -572,9 +683,7 @@ extern "C" int cwk_dsa_select(cwk_ctx *ctx, const void *keys, const float *kscal
         attr_set[ctx->device & 15] = true;
     }
     IdxParams p;
-    p.kscale = kscale; p.q = q; p.wt = wt; p.n = n; p.sc = approx; p.band = band; p.key_stride = key_stride; p.err = ctx->dev_err;
-    const int tiles = (max_n + IT_KEYS - 1) / IT_KEYS;
-    const int bps = std::max(1, std::min(tiles, ctx->sm_count / B));
+    p.kscale = kscale; p.q = q; p.wt = wt; p.n = n; p.sc = approx; p.band = band; p.range = range; p.key_stride = key_stride; p.err = ctx->dev_err;
     {
         CwkKernelTimer timer(ctx);
         CWK_CUDA(ctx, cwk_launch_early(indexer_scores_tc_kernel, dim3(bps, B), dim3(IT_THREADS), I_SMEM, ctx->stream, tm_keys, p));
@@ -582,7 +691,7 @@ extern "C" int cwk_dsa_select(cwk_ctx *ctx, const void *keys, const float *kscal
     }
     {
         CwkKernelTimer timer(ctx);
-        CWK_CUDA(ctx, cwk_launch_early(band_classify_kernel, dim3(TK_CL, B), dim3(TK_THREADS), BC_SMEM, ctx->stream, approx, key_stride, n, want, refined, band_list, band,
+        CWK_CUDA(ctx, cwk_launch_early(band_classify_kernel, dim3(TK_CL, B), dim3(TK_THREADS), BC_SMEM, ctx->stream, approx, key_stride, n, want, refined, band_list, band, range, bps * 8,
                                        (const uint8_t *)keys, kscale, q, wt, keep_self, sel, sel_ld, nsel, (long long *)ctx->tc_trace));
         CWK_LAUNCH_CHECK(ctx, "band_classify_kernel");
     }

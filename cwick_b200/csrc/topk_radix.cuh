@@ -32,11 +32,9 @@ struct TkShared {
     uint32_t hist[2][256];               // this block's digit counts, double-buffered across passes
     uint32_t tot[256];                   // the cluster's digit counts
     uint32_t sel[2];                     // chosen prefix, remaining rank
-    unsigned long long cnt[32], off[32], total;   // block scan of (above | equal << 32)
     unsigned long long pub;              // this block's totals, read by the blocks of higher rank
     unsigned long long base;             // totals of the blocks of lower rank
     int tbase;
-    float fmax;
 };
 
 struct TkSlice {
@@ -172,41 +170,57 @@ __device__ __forceinline__ void tk_radix_select(const float *s, const TkSlice sl
     }
 }
 
-// The second half of a selection, for every thread of every block of the row's cluster: the exact threshold (radix select
-// over the row, or, when the row holds +inf / -inf outside a short list of re-scored positions, over that list only), then
-// the ordered compaction into out[]: rows above the threshold in index order, then rows equal to it in index order, `want`
-// in all (ascending: one list in index order). kc holds the slice's keys when sl.cached.
-__device__ __forceinline__ void tk_threshold_and_compact(const float *s, const TkSlice sl, uint32_t (&kc)[TK_PT], int nb, int want,
-                                                         int keep_self, int ascending, int32_t *out, int32_t *nsel_b,
-                                                         const int32_t *band_list, int band_cnt, int band_above, TkShared &sh) {
+// The second half of a selection, for every thread of every block of the row's cluster: the ordered compaction into out[]: rows
+// above the threshold in index order, then rows equal to it in index order, `want` in all (ascending: one list in index order).
+// thr is the integer image of the threshold; need_eq rows equal to it are wanted (the first ones in index order); want - need_eq
+// rows lie above it. kc holds the slice's keys when sl.cached.
+__device__ __forceinline__ void tk_compact(const float *s, const TkSlice sl, uint32_t (&kc)[TK_PT], int nb, int want, int keep_self, int ascending,
+                                           int32_t *out, int32_t *nsel_b, uint32_t thr, int need_eq, TkShared &sh) {
     cg::cluster_group cl = cg::this_cluster();
     const unsigned rank = cl.block_rank();
-    const int tid = threadIdx.x;
-    if (tid == 0) sh.pub = 0;
-    uint32_t thr;
-    int need_eq;
-    if (band_list) {
-        // The row holds +inf / -inf outside a short list of re-scored positions (cwk_dsa_select): the exact
-        // threshold is the (want - certainly selected)-th largest score of that list. Every block of the
-        // cluster finds it for itself; the list is a few hundred entries.
-        const int kth = max(1, min(want - band_above, band_cnt));   // holds by construction; clamped against a violated error bound
-        tk_list_select(s, band_list, band_cnt, kth, sh, thr, need_eq);
-    } else {
-        tk_radix_select(s, sl, kc, want, sh, thr, need_eq);
-    }
-    // thr is the integer image of the threshold; need_eq rows equal to it are wanted (the first
-    // ones in index order); want - need_eq rows lie above it.
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n_gt = want - need_eq;
-    const int lane = tid & 31, warp = tid >> 5;
+    // this thread's rows above and (upper half) equal in the chunk at c0
+    auto count = [&](int c0) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int j = 0; j < TK_PT; j++)
+            if (c0 + tid * TK_PT + j < sl.end) c += (kc[j] > thr ? 1u : 0u) + (kc[j] == thr ? 0x10000u : 0u);
+        return c;
+    };
+    // the same of the block's threads before this one, and of all of them (a chunk is short enough for sixteen bits each)
+    uint32_t before, all;
+    auto scan = [&](uint32_t mine) {
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) sh.tot[warp] = incl;
+        __syncthreads();
+        uint32_t wi = sh.tot[lane];                          // (every warp for itself: no second barrier)
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
+            if (lane >= o) wi += t;
+        }
+        const uint32_t w0 = __shfl_sync(0xffffffffu, wi, (warp + 31) & 31);
+        all = __shfl_sync(0xffffffffu, wi, 31);
+        before = (warp ? w0 : 0u) + incl - mine;
+    };
+    auto wide = [](uint32_t c) { return (unsigned long long)(c & 0xffffu) | ((unsigned long long)(c >> 16) << 32); };
     // this block's totals, for the offsets of the blocks after it
-    {
+    if (sl.cached) {
+        scan(count(sl.begin));
+        if (tid == 0) sh.pub = wide(all);
+    } else {
+        if (tid == 0) sh.pub = 0;
+        __syncthreads();
         unsigned long long mine = 0;
         for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {
-            if (!sl.cached) tk_load(s, c0, sl.end, kc);
-            const int i0 = c0 + tid * TK_PT;
-#pragma unroll
-            for (int j = 0; j < TK_PT; j++)
-                if (i0 + j < sl.end) mine += (kc[j] > thr ? 1ull : 0ull) + (kc[j] == thr ? (1ull << 32) : 0ull);
+            tk_load(s, c0, sl.end, kc);
+            mine += wide(count(c0));
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
@@ -233,42 +247,14 @@ __device__ __forceinline__ void tk_threshold_and_compact(const float *s, const T
             sh.tbase = tbase;
         }
     }
+    // nobody reads a neighbour's shared memory after this: what is left waits for the others only at the end
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     __syncthreads();
-    unsigned long long running = sh.base;
-    const int eq_before_block = (int)(sh.base >> 32);
+    const int og0 = (int)(sh.base & 0xffffffffull), oe0 = (int)(sh.base >> 32);
     const int tbase = sh.tbase;
-    const int eq_quota = max(0, need_eq - eq_before_block);     // ties this block may still take
-    unsigned long long local = 0;                                // (above | equal) in this block's earlier chunks
-    for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {
-        if (!sl.cached) tk_load(s, c0, sl.end, kc);
+    const int eq_quota = max(0, need_eq - oe0);                  // ties this block may still take
+    auto write = [&](int c0, int lg, int le) {                   // lg, le: rows above and equal in this block before this thread's
         const int i0 = c0 + tid * TK_PT;
-        unsigned long long mine = 0;
-#pragma unroll
-        for (int j = 0; j < TK_PT; j++)
-            if (i0 + j < sl.end) mine += (kc[j] > thr ? 1ull : 0ull) + (kc[j] == thr ? (1ull << 32) : 0ull);
-        unsigned long long incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) sh.cnt[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const unsigned long long v = sh.cnt[lane];
-            unsigned long long wi = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long t = __shfl_up_sync(0xffffffffu, wi, o);
-                if (lane >= o) wi += t;
-            }
-            sh.off[lane] = wi - v;
-            if (lane == 31) sh.total = wi;
-        }
-        __syncthreads();
-        const unsigned long long before = local + sh.off[warp] + incl - mine;   // within this block
-        int lg = (int)(before & 0xffffffffull), le = (int)(before >> 32);
-        const int og0 = (int)(running & 0xffffffffull), oe0 = (int)(running >> 32);
 #pragma unroll
         for (int j = 0; j < TK_PT; j++) {
             if (i0 + j < sl.end) {
@@ -283,12 +269,25 @@ __device__ __forceinline__ void tk_threshold_and_compact(const float *s, const T
                 le += eq ? 1 : 0;
             }
         }
-        local += sh.total;
+    };
+    if (sl.cached) {
+        write(sl.begin, (int)(before & 0xffffu), (int)(before >> 16));
+    } else {
+        int lg = 0, le = 0;                                      // in this block's earlier chunks
+        for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {
+            tk_load(s, c0, sl.end, kc);
+            scan(count(c0));
+            write(c0, lg + (int)(before & 0xffffu), le + (int)(before >> 16));
+            lg += (int)(all & 0xffffu);
+            le += (int)(all >> 16);
+            __syncthreads();                                     // the warps' totals have been read
+        }
     }
-    cl.sync();                              // every block's part of the list is written; nobody reads a neighbour's shared memory after this
-    if (rank == 0 && tid == 0) {
-        int cnt = want;
-        if (keep_self && out[cnt - 1] != nb - 1) out[cnt++] = nb - 1;
-        *nsel_b = cnt;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    int cnt = want;
+    if (keep_self) {
+        cl.sync();                          // every block's part of the list is written
+        if (rank == 0 && tid == 0 && out[cnt - 1] != nb - 1) out[cnt++] = nb - 1;
     }
+    if (rank == 0 && tid == 0) *nsel_b = cnt;
 }

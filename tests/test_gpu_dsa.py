@@ -188,6 +188,28 @@ def test_fused_selection_threshold_tie_run(attn):
     assert nsel[0] == ref.size and np.array_equal(sel[0, :nsel[0]].astype(np.int64), ref)
 
 
+@pytest.mark.parametrize("T,want,keep_self,keys", [(3000, 700, False, "alike"), (9000, 1500, True, "few values"), (9000, 512, False, "one far above"),
+                                                   (20000, 2048, True, "narrow"), (66001, 2048, True, "plain"), (2049, 2048, True, "plain")])
+def test_fused_selection_histogram_edges(attn, T, want, keep_self, keys):
+    """The approximate threshold is a bin of a histogram over the row's range: rows without a range (every key is re-scored),
+    bands longer than the list that is ranked in shared memory (1024), ranges set by one key, all scores within the guard band,
+    rows longer than the register slices, one row too many. Lists are exact, order included."""
+    codes, ks, q, wt = make_index_inputs(900 + T + want, 1, T)
+    if keys == "alike":
+        codes[0, :], ks[0, :] = codes[0, 0], ks[0, 0]
+    elif keys == "few values":
+        pick = np.arange(T) % 7
+        codes[0], ks[0] = codes[0, pick], ks[0, pick]
+    elif keys == "one far above":
+        ks[0, T // 3] *= np.float32(200.0)
+    elif keys == "narrow":
+        codes[0], ks[0] = codes[0, 11], ks[0, 11] * (1 + np.float32(1e-4) * synth.uniform(7, 7, T)).astype(np.float32)
+    lens = np.array([T], np.int32)
+    sel, nsel, _ = _select_both_ways(attn, codes, ks, q, wt, lens, want, keep_self)
+    ref = oracle_select(oracle_scores(codes, ks, q, wt)[0], T, want, keep_self)
+    assert nsel[0] == ref.size and np.array_equal(sel[0, :nsel[0]].astype(np.int64), ref)
+
+
 def test_fused_selection_config4_size(attn):
     """BASELINE config 4 dimensions on two sequences: 65536 keys, top 2048."""
     B, T, want = 2, 65536, 2048
