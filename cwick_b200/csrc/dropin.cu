@@ -347,39 +347,72 @@ __global__ void __launch_bounds__(256) rms_scale_pair_kernel(float *xa, int na, 
 
 // The two norms of a chunk on the tensor path, one block per (token, row): adds up the split partial sums of the joint
 // q_a | kv_a projection (part [splits][n][na + nb]), then the q_a row leaves as three bf16 planes (the next projection's
-// operand), the kv_a row as the narrowed cache row and, where the caller's cache is f32, as f32. The sum of squares runs in
-// the order of rms_scale_row.
+// operand), the kv_a row as the narrowed cache row and, where the caller's cache is f32, as f32. The sum of squares is a
+// sum of doubles, as in rms_scale_row, four columns at a time here.
+// A row is a few KB: what it takes is trips to L2, so a thread asks for two pieces of every partial sum and for its weights at
+// once and everything is read and written in pieces of four columns (one value at a time, 2-byte stores: 11 us for 128 tokens of
+// 1536 + 512 in sixteen parts, now 8).
 __global__ void __launch_bounds__(256) norm_chunk_kernel(const float *part, int splits, int n, int na, int nb, const uint16_t *wa, const uint16_t *wb,
                                                          float eps, uint16_t *planes, uint16_t *cache_rows, float *kv_out) {
     extern __shared__ __align__(16) float s_row[];
-    const int t = blockIdx.x, len = blockIdx.y ? nb : na, ld = na + nb;
+    __shared__ double red[8];
+    const int t = blockIdx.x, tid = threadIdx.x, len = blockIdx.y ? nb : na, ld = na + nb;
+    const int64_t step = (int64_t)n * ld;
     const float *src = part + (int64_t)t * ld + (blockIdx.y ? na : 0);
+    const uint16_t *w = blockIdx.y ? wb : wa;
     cwk_pdl_launch();
     cwk_pdl_wait();
-    for (int i = threadIdx.x * 4; i < len; i += 1024) {    // (na and nb are multiples of 8)
-        float4 v = *reinterpret_cast<const float4 *>(src + i);
+    double ss = 0.0;
+    for (int i = tid * 4; i < len; i += 2048) {            // (na and nb are multiples of 8)
+        const bool two = i + 1024 < len;
+        float4 v[2];
+        v[0] = *reinterpret_cast<const float4 *>(src + i);
+        v[1] = two ? *reinterpret_cast<const float4 *>(src + i + 1024) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
         for (int s = 1; s < splits; s++) {
-            const float4 w = *reinterpret_cast<const float4 *>(src + (int64_t)s * n * ld + i);
-            v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+            const float4 x = *reinterpret_cast<const float4 *>(src + s * step + i);
+            v[0].x += x.x; v[0].y += x.y; v[0].z += x.z; v[0].w += x.w;
+            if (two) {
+                const float4 y = *reinterpret_cast<const float4 *>(src + s * step + i + 1024);
+                v[1].x += y.x; v[1].y += y.y; v[1].z += y.z; v[1].w += y.w;
+            }
         }
-        *reinterpret_cast<float4 *>(s_row + i) = v;
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            if (j == 0 || two) {
+                *reinterpret_cast<float4 *>(s_row + i + 1024 * j) = v[j];      // (read back by this thread only)
+                ss += ((double)v[j].x * (double)v[j].x + (double)v[j].y * (double)v[j].y) + ((double)v[j].z * (double)v[j].z + (double)v[j].w * (double)v[j].w);
+            }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((tid & 31) == 0) red[tid >> 5] = ss;
     __syncthreads();
-    if (blockIdx.y) {
-        rms_scale_row(s_row, nb, wb, eps, cache_rows + (int64_t)t * nb, kv_out ? kv_out + (int64_t)t * nb : nullptr, 0);
-        return;
-    }
-    rms_scale_row(s_row, na, wa, eps, nullptr, nullptr, 0);
-    for (int i = threadIdx.x; i < na; i += 256) {          // (the values this thread scaled itself)
-        const float v = s_row[i];
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        const float r = v - __bfloat162float(h);
-        const __nv_bfloat16 m = __float2bfloat16_rn(r);
-        uint16_t *o = planes + (int64_t)t * na + i;
-        o[0] = __bfloat16_as_ushort(h);
-        o[(int64_t)n * na] = __bfloat16_as_ushort(m);
-        o[2 * (int64_t)n * na] = __bfloat16_as_ushort(__float2bfloat16_rn(r - __bfloat162float(m)));
+    const double tot = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+    const float inv = __fdiv_rn(1.0f, (float)sqrt(tot / (double)len + (double)eps));
+    for (int i = tid * 4; i < len; i += 1024) {
+        const float4 v = *reinterpret_cast<const float4 *>(s_row + i);
+        const uint2 g = *reinterpret_cast<const uint2 *>(w + i);
+        float y[4] = {v.x * inv * __uint_as_float(g.x << 16), v.y * inv * __uint_as_float(g.x & 0xffff0000u),
+                      v.z * inv * __uint_as_float(g.y << 16), v.w * inv * __uint_as_float(g.y & 0xffff0000u)};
+        if (blockIdx.y) {
+            uint32_t nbits[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {                  // narrowed the way the reference narrows a cache row (src/util.c:202-210)
+                const uint32_t u = __float_as_uint(y[e]);
+                nbits[e] = ((u + ((u >> 15) & 1u) + ((u >> 16) & 1u)) >> 16) & 0xffffu;
+            }
+            *reinterpret_cast<uint2 *>(cache_rows + (int64_t)t * nb + i) = make_uint2(nbits[0] | (nbits[1] << 16), nbits[2] | (nbits[3] << 16));
+            if (kv_out) *reinterpret_cast<float4 *>(kv_out + (int64_t)t * nb + i) = make_float4(y[0], y[1], y[2], y[3]);
+        } else {
+#pragma unroll
+            for (int pl = 0; pl < 3; pl++) {               // each plane is the bf16 rounding of what the planes before it leave over
+                const uint32_t lo = pack_bf16x2(y[0], y[1]), hi = pack_bf16x2(y[2], y[3]);
+                *reinterpret_cast<uint2 *>(planes + ((int64_t)pl * n + t) * na + i) = make_uint2(lo, hi);
+                y[0] -= __uint_as_float(lo << 16); y[1] -= __uint_as_float(lo & 0xffff0000u);
+                y[2] -= __uint_as_float(hi << 16); y[3] -= __uint_as_float(hi & 0xffff0000u);
+            }
+        }
     }
 }
 
