@@ -87,12 +87,13 @@ __global__ void __launch_bounds__(256) norm_rope_rows_kernel(const float *in, in
 // The same, one WARP per row, for rows whose normalised part is a multiple of 128 columns (at most 128 * MAXV4) and whose
 // rope part is at most 64 columns: a lane keeps its 16-byte pieces of the row in registers, so the row is read once;
 // the sum of squares goes through lane-wise doubles and five shuffles, with no shared memory and no block barrier.
-// 4096 rows are 4096 warps, all resident at once: the call takes about one row's latency.
+// 4096 rows are 4096 warps, all resident at once: the call takes about one row's latency. rot: where each row's (cos, sin) of
+// its rope pairs go as well, for the queries of the same positions (NULL: nowhere).
 template <int MAXV4>
 __global__ void __launch_bounds__(256) norm_rope_rows_warp_kernel(const float *in, int64_t in_ld, int norm_cols, int rope_cols,
                                                                   const uint16_t *weight, float eps, float rope_base, int64_t pos0,
                                                                   uint16_t *out, int64_t out_ld, int *kv_len_out, int ref_narrow,
-                                                                  int64_t nrows) {
+                                                                  int64_t nrows, float2 *rot) {
     const int lane = threadIdx.x & 31;
     const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= nrows) return;
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(256) norm_rope_rows_warp_kernel(const float *i
         float sn, cs;
         rope_cos_sin(pos0 + r, lane, rope_cols, rope_base, cs, sn);
         const float r0 = ra * cs - rb * sn, r1 = rb * cs + ra * sn;
+        if (rot) rot[r * (rope_cols / 2) + lane] = make_float2(cs, sn);
         *reinterpret_cast<uint32_t *>(y + norm_cols + 2 * lane) =
             ref_narrow ? ((uint32_t)narrow_bf16_like_reference(r0) | ((uint32_t)narrow_bf16_like_reference(r1) << 16)) : pack_bf16x2(r0, r1);
     }
@@ -171,7 +173,8 @@ __global__ void __launch_bounds__(256) rope_tail_kernel(const uint16_t *q, uint1
     }
 }
 
-// RoPE of the rope part of q, in place: q[t][h][nope : nope+rope] at position pos0 + t. One thread per (t, pair) and
+// RoPE of the rope part of q, in place, where the kv_a rows did not take the warp kernel above (which leaves the angles to the
+// attention, and that rotates its query tiles itself): q[t][h][nope : nope+rope] at position pos0 + t. One thread per (t, pair) and
 // group of heads (blockIdx.y): the angle is formed once per thread and applied to the group's heads. The pairs'
 // divisors base^(2j / n_rope) -- the same values rope_cos_sin forms -- are computed once per block (n_rope <= 256).
 __global__ void __launch_bounds__(256) rope_q_inplace_kernel(uint16_t *q, int n, int nh, int nope, int n_rope, int64_t pos0, float base) {
@@ -204,7 +207,7 @@ __global__ void __launch_bounds__(256) rope_q_inplace_kernel(uint16_t *q, int n,
 
 int cwk_absorb_tc_launch(cwk_ctx *ctx, const void *Q, int n, int nh, const void *Wuk, void *Qfull);
 bool cwk_mla_prefill_attn_tc_ok(const void *Q, const void *cache, const void *Wuk, const void *kx, const void *out);
-int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, const void *Wuk, void *kx, int *flags, int64_t pos0, int n, int nh,
+int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const float *rot, const void *cache, const void *Wuk, void *kx, int *flags, int64_t pos0, int n, int nh,
                             float scale, void *out, int exact_only);
 
 // Which attention route is the faster one for a chunk of n queries behind pos0 rows. The expansion covers every cached
@@ -309,7 +312,7 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
     CWK_CUDA(ctx, cudaSetDevice(ctx->device));
     const int qd = nope + rope, row = kv_lora + rope;
     // workspace: QA f32 [n][q_lora], QAn bf16 [n][q_lora], KVA f32 [n][row], Q bf16 [n][nh*qd],
-    // Qfull bf16 [n][nh][row], kv_len int32 [n]
+    // Qfull bf16 [n][nh][row], kv_len int32 [n], (cos, sin) of the rope pairs f32 [n][rope]
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t b_qa = up((size_t)n * q_lora * 4), b_qan = up((size_t)n * q_lora * 2), b_kva = up((size_t)n * row * 4);
     // The attention takes one of two routes. Queries as MMA rows against per-head expanded keys (mla_prefill_attn.cu)
@@ -320,7 +323,7 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
     const size_t b_kx = up((size_t)(pos0 + n) * nh * qd * 2);
     const size_t b_q = up((size_t)n * nh * qd * 2), b_qf = expanded_keys ? std::max(b_kx, up((size_t)n * nh * row * 2)) : up((size_t)n * nh * row * 2),
                  b_len = up((size_t)n * 4) + up(((size_t)((n + 127) / 128) * nh * 2 + ctx->sm_count + 3) * 4);
-    int s = cwk_reserve_work(ctx, b_qa + b_qan + b_kva + b_q + b_qf + b_len);
+    int s = cwk_reserve_work(ctx, b_qa + b_qan + b_kva + b_q + b_qf + up(b_len) + (size_t)n * rope * 4);
     if (s != CWK_OK) return s;
     uint8_t *w = (uint8_t *)ctx->work;
     float *QA = (float *)w;
@@ -329,6 +332,7 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
     uint16_t *Q = (uint16_t *)(w + b_qa + b_qan + b_kva);
     uint16_t *Qf = (uint16_t *)(w + b_qa + b_qan + b_kva + b_q);
     int32_t *len = (int32_t *)(w + b_qa + b_qan + b_kva + b_q + b_qf);
+    float *rot = (float *)(w + b_qa + b_qan + b_kva + b_q + b_qf + up(b_len));
 
     // q_a and kv_a share the activations: one launch of the tensor-core GEMM when it takes the shapes
     bool kva_done = false;
@@ -343,7 +347,7 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
     if (s != CWK_OK) return s;
     if (norm_rope_warp_ok(QA, q_lora, q_lora, 0, qa_norm, QAn, q_lora))
         CWK_CUDA(ctx, cwk_launch_early(norm_rope_rows_warp_kernel<12>, dim3((n + 7) / 8), dim3(256), 0, ctx->stream, QA, q_lora, q_lora, 0,
-                                       (const uint16_t *)qa_norm, eps, rope_base, pos0, QAn, q_lora, nullptr, 0, n));
+                                       (const uint16_t *)qa_norm, eps, rope_base, pos0, QAn, q_lora, nullptr, 0, n, nullptr));
     else
         norm_rope_rows_kernel<<<n, 256, 0, ctx->stream>>>(QA, q_lora, q_lora, 0, (const uint16_t *)qa_norm, eps, rope_base,
                                                           pos0, QAn, q_lora, nullptr, 0);
@@ -354,17 +358,20 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
         s = cwk_fp8_linear(ctx, X, Wkva, Skva, n, H, row, KVA, 0);
         if (s != CWK_OK) return s;
     }
+    const bool rotated_later = expanded_keys && cwk_mla_prefill_attn_tc_ok(Q, cache, Wuk, Qf, out) && norm_rope_warp_ok(KVA, row, kv_lora, rope, kva_norm, (uint16_t *)cache + pos0 * row, row);
     if (norm_rope_warp_ok(KVA, row, kv_lora, rope, kva_norm, (uint16_t *)cache + pos0 * row, row))
         CWK_CUDA(ctx, cwk_launch_early(norm_rope_rows_warp_kernel<12>, dim3((n + 7) / 8), dim3(256), 0, ctx->stream, KVA, row, kv_lora, rope,
-                                       (const uint16_t *)kva_norm, eps, rope_base, pos0, (uint16_t *)cache + pos0 * row, row, len, 1, n));
+                                       (const uint16_t *)kva_norm, eps, rope_base, pos0, (uint16_t *)cache + pos0 * row, row, len, 1, n, rotated_later ? (float2 *)rot : nullptr));
     else
         norm_rope_rows_kernel<<<n, 256, 0, ctx->stream>>>(KVA, row, kv_lora, rope, (const uint16_t *)kva_norm, eps, rope_base,
                                                           pos0, (uint16_t *)cache + pos0 * row, row, len, 1);
     CWK_LAUNCH_CHECK(ctx, "norm_rope_rows_kernel(kv_a)");
     if (expanded_keys && cwk_mla_prefill_attn_tc_ok(Q, cache, Wuk, Qf, out)) {
-        CWK_CUDA(ctx, cwk_launch_early(rope_q_inplace_kernel, dim3((n * (rope / 2) + 255) / 256, nh >= 8 ? 4 : 1), dim3(256), 0, ctx->stream, Q, n, nh, nope, rope, pos0, rope_base));
-        CWK_LAUNCH_CHECK(ctx, "rope_q_inplace_kernel");
-        return cwk_mla_prefill_attn_tc(ctx, Q, cache, Wuk, Qf, (int *)((uint8_t *)len + up((size_t)n * 4)), pos0, n, nh, scale, out, ctx->force_mla_path == 3);
+        if (!rotated_later) {
+            CWK_CUDA(ctx, cwk_launch_early(rope_q_inplace_kernel, dim3((n * (rope / 2) + 255) / 256, nh >= 8 ? 4 : 1), dim3(256), 0, ctx->stream, Q, n, nh, nope, rope, pos0, rope_base));
+            CWK_LAUNCH_CHECK(ctx, "rope_q_inplace_kernel");
+        }
+        return cwk_mla_prefill_attn_tc(ctx, Q, rotated_later ? rot : nullptr, cache, Wuk, Qf, (int *)((uint8_t *)len + up((size_t)n * 4)), pos0, n, nh, scale, out, ctx->force_mla_path == 3);
     }
     // absorb on the tensor path (tcgen05); the mma.sync kernel covers a context without the
     // tensor-map encoder or a caller that forced the general kernels

@@ -78,7 +78,8 @@ enum { PB_QFULL = 0, PB_KFULL = 1, PB_KEMPTY = PB_KFULL + PA_KBAR, PB_CFULL = PB
 static_assert(PA_KBAR % 2 == 0 && PA_KBAR % PA_KST == 0 && 8 * PB_COUNT + 16 <= 512, "barriers");
 
 struct AttnParams {
-    const uint16_t *q;  // bf16 [n][nh][DQK] (MLA: rope part rotated)
+    const uint16_t *q;  // bf16 [n][nh][DQK]
+    const float4 *rot;  // MLA: [n][32] (cos, sin) of the rope pairs, two pairs a piece; NULL: q is rotated already
     uint16_t *out;      // bf16 [n][nh][512] (MLA) / [n][nh][256] (GQA)
     int n, nh, T;       // T = pos0 + n cached rows
     int group;          // GQA: query heads per KV head (MLA: unused)
@@ -408,18 +409,30 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             // copies its row's share: DQK / 2 columns split between the groups. The tile of item k + 1 is copied
             // BEFORE the epilogue of item k (below), so that the next item's first scores are computed under that epilogue.
             auto load_query = [&](int q0_, int h_) {
-                constexpr int QW = (PA_DQK / 2) / NWG;               // 32-bit words per copying thread
                 const int t = q0_ + row;
-                const uint4 *src = reinterpret_cast<const uint4 *>(p.q + ((int64_t)t * p.nh + h_) * PA_DQK) + wg * (QW / 4);
+                const uint4 *src = reinterpret_cast<const uint4 *>(p.q + ((int64_t)t * p.nh + h_) * PA_DQK);
 #pragma unroll
-                for (int c = 0; c < QW / 8; c++) {
+                for (int c = 0; c < PA_DQK / 16 / NWG; c++) {        // eight words at a time, the groups in turn
+                    const int w8 = c * NWG + wg;
                     uint32_t wv[8];
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
-                        const uint4 v = (t < p.n) ? src[c * 2 + j] : make_uint4(0, 0, 0, 0);
+                        const uint4 v = (t < p.n) ? src[w8 * 2 + j] : make_uint4(0, 0, 0, 0);
                         wv[4 * j] = v.x; wv[4 * j + 1] = v.y; wv[4 * j + 2] = v.z; wv[4 * j + 3] = v.w;
                     }
-                    TMEM_ST8(wv, 0, tlane + PA_COL_Q + wg * QW + c * 8);
+                    // the rope pairs (the last 64 of 192 columns) are rotated on their way, at the row's position: a kernel of its own, in
+                    // place, was 32 us for 4096 tokens of 64 heads, 13 for 509
+                    if (!GQA && c * NWG * 16 >= PA_DQK - 64 && p.rot && t < p.n) {
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) {
+                            const float4 r = p.rot[(int64_t)t * 16 + w8 * 4 - (PA_DQK - 64) / 4 + j / 2];
+                            const float a0 = __uint_as_float(wv[j] << 16), b0 = __uint_as_float(wv[j] & 0xffff0000u);
+                            const float a1 = __uint_as_float(wv[j + 1] << 16), b1 = __uint_as_float(wv[j + 1] & 0xffff0000u);
+                            wv[j] = pack_bf16x2(a0 * r.x - b0 * r.y, b0 * r.x + a0 * r.y);
+                            wv[j + 1] = pack_bf16x2(a1 * r.z - b1 * r.w, b1 * r.z + a1 * r.w);
+                        }
+                    }
+                    TMEM_ST8(wv, 0, tlane + PA_COL_Q + w8 * 8);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
@@ -912,12 +925,13 @@ bool cwk_mla_prefill_attn_tc_ok(const void *Q, const void *cache, const void *Wu
              reinterpret_cast<uintptr_t>(out)) & 15) == 0;
 }
 
-// Q bf16 [n][nh][192] with the rope part already rotated; cache bf16 [pos0 + n][576] (latent | rope key);
+// Q bf16 [n][nh][192]; rot = (cos, sin) of the rope pairs at the queries' positions, f32 [n][32][2], 16-byte aligned (NULL: Q has been
+// rotated); cache bf16 [pos0 + n][576] (latent | rope key);
 // Wuk bf16 [nh][128][512]; kx = workspace bf16 [nh][pos0 + n][192]; flags = workspace int32, one per item of the
 // attention (ceil(n / 128) x nh x 2) and per SM plus three counters; out bf16 [n][nh][512]. exact_only: skip the fast form and run
 // the exact form on every item (for tests).
 // Returns CWK_ERR_UNSUPPORTED (no error text) when the tensor path cannot run.
-int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, const void *Wuk, void *kx, int *flags, int64_t pos0, int n, int nh,
+int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const float *rot, const void *cache, const void *Wuk, void *kx, int *flags, int64_t pos0, int n, int nh,
                             float scale, void *out, int exact_only) {
     if (!cwk_encode_tiled_fn()) return CWK_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(Wuk) | reinterpret_cast<uintptr_t>(kx) |
@@ -948,7 +962,7 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const void *cache, cons
         CWK_LAUNCH_CHECK(ctx, "kexp_tc_kernel");
     }
     AttnParams ap{};
-    ap.q = (const uint16_t *)Q; ap.out = (uint16_t *)out; ap.n = n; ap.nh = nh; ap.T = T; ap.pos0 = pos0; ap.group = 1;
+    ap.q = (const uint16_t *)Q; ap.rot = (const float4 *)rot; ap.out = (uint16_t *)out; ap.n = n; ap.nh = nh; ap.T = T; ap.pos0 = pos0; ap.group = 1;
     ap.scale_log2 = scale * 1.4426950408889634f; ap.flags = flags; ap.err = ctx->dev_err;
     return attn_launch<PaMla, false>(ctx, ap, tm_k, tm_c, exact_only);
 }
