@@ -428,14 +428,108 @@ static __global__ void __launch_bounds__(128) lse_merge_kernel(const float *part
     }
 }
 
+// The merge of many sequences with few records each, a warp per (sequence, head, 128 C columns) and no block barrier: a lane asks for
+// C pieces of sixteen bytes of the first AHEAD records at once. The kernel above is 128 threads, two barriers and some three
+// microseconds per 128 columns of a head, so that 64 sequences of 3 records (28 MB) took 25 us.
+template <int C, int AHEAD>
+static __global__ void __launch_bounds__(256) lse_merge_warp_kernel(const float *partial, int nsplit, int nh, int D, int items, uint16_t *out, const int2 *meta) {
+    const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int chunks = D / (128 * C), chunk = item % chunks, bh = item / chunks, h = bh % nh, b = bh / nh;
+    const int64_t rec_sz = (int64_t)nh * (D + 2);
+    cwk_pdl_launch();
+    cwk_pdl_wait();
+    if (item >= items) return;
+    int64_t rec0 = (int64_t)b * nsplit;
+    if (meta) {
+        const int2 m = meta[b];
+        rec0 = m.x;
+        nsplit = m.y;
+    }
+    const float *base = partial + rec0 * rec_sz, *ml = base + h;
+    const float *col = base + 2 * nh + (int64_t)h * D + chunk * 128 * C + lane * 4;
+    float4 v[AHEAD][C];
+#pragma unroll
+    for (int s = 0; s < AHEAD; s++)
+#pragma unroll
+        for (int c = 0; c < C; c++) v[s][c] = s < nsplit ? *reinterpret_cast<const float4 *>(col + s * rec_sz + c * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+    // lane s: the record's reference exponent (-inf: nothing in it) and sum
+    auto mine = [&](int s, float &m, float &l) {
+        l = s < nsplit ? ml[s * rec_sz + nh] : 0.f;
+        m = l > 0.f ? ml[s * rec_sz] : -INFINITY;
+    };
+    float m0, l0, M;
+    mine(lane, m0, l0);
+    M = m0;
+    for (int s = lane + 32; s < nsplit; s += 32) {
+        float m, l;
+        mine(s, m, l);
+        M = fmaxf(M, m);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    auto weight = [&](float m) { return m == -INFINITY ? 0.f : __expf(m - M); };
+    float w = weight(m0), den = w * l0;                    // weights of records 0 .. 31
+    for (int s = lane + 32; s < nsplit; s += 32) {
+        float m, l;
+        mine(s, m, l);
+        den += weight(m) * l;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+    float4 a[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) a[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < nsplit; s0 += AHEAD) {           // (AHEAD divides 32)
+        if (s0 > 0) {
+#pragma unroll
+            for (int s = 0; s < AHEAD; s++)
+#pragma unroll
+                for (int c = 0; c < C; c++) v[s][c] = s0 + s < nsplit ? *reinterpret_cast<const float4 *>(col + (s0 + s) * rec_sz + c * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if ((s0 & 31) == 0) {
+                float m, l;
+                mine(s0 + lane, m, l);
+                w = weight(m);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < AHEAD; s++) {
+            const float ws = __shfl_sync(0xffffffffu, w, (s0 + s) & 31);
+            if (s0 + s < nsplit) {                         // (a record without rows has weight 0 and defined values)
+#pragma unroll
+                for (int c = 0; c < C; c++) { a[c].x += ws * v[s][c].x; a[c].y += ws * v[s][c].y; a[c].z += ws * v[s][c].z; a[c].w += ws * v[s][c].w; }
+            }
+        }
+    }
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+    uint16_t *dst = out + ((int64_t)b * nh + h) * D + chunk * 128 * C + lane * 4;
+#pragma unroll
+    for (int c = 0; c < C; c++)
+        *reinterpret_cast<uint2 *>(dst + c * 128) = make_uint2(pack_bf16x2(a[c].x * inv, a[c].y * inv), pack_bf16x2(a[c].z * inv, a[c].w * inv));
+}
+// Whether it takes the merge: whole pieces of 128 columns, sixteen bytes aligned; at most 32 records a sequence (on average); and
+// work enough for its warps, where the kernel above would be 1024 blocks or more, 2048 where a warp goes round twice. Records of 64
+// heads x 512, us, above / this: 64 sequences x 3.3 records 24.0 / 8.8, 32 x 4 12.5 / 4.6, 24 x 7 10.8 / 7.0, 16 x 10 15.8 / 8.4, 8 x 16
+// 8.2 / 4.9, 8 x 17 8.4 / 6.1; below the line 3 x 6 3.7 / 4.0, 2 x 24 4.1 / 5.1, 1 x 12 3.7 / 4.3, and whole calls of 4 x 32 23.1 / 25.3.
+static inline bool lse_merge_by_warps(const float *partial, int few, int nh, int D, int B, const uint16_t *out) {
+    return few <= 32 && nh % 2 == 0 && D % 128 == 0 && (int64_t)B * nh * (D / 128) >= (few <= 16 ? 1024 : 2048) && (reinterpret_cast<uintptr_t>(partial) & 15) == 0 &&
+           (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+}
+static inline void lse_merge_warps_launch(cudaStream_t st, const float *partial, int nsplit, int few, int nh, int D, int B, uint16_t *out, const int2 *meta) {
+    const int most = few <= 4 ? 4 : few <= 8 ? 2 : 1, c = D % (128 * most) == 0 ? most : 1, items = B * nh * (D / (128 * c));
+    auto kern = c == 4 ? lse_merge_warp_kernel<4, 4> : c == 2 ? lse_merge_warp_kernel<2, 8> : lse_merge_warp_kernel<1, 16>;
+    (void)cwk_launch_early(kern, dim3((items + 7) / 8), dim3(256), 0, st, partial, nsplit, nh, D, items, out, meta);
+}
+
 static inline void lse_combine_launch(cudaStream_t st, const float *partial, int nsplit, int nh, int D, int B,
                                       uint16_t *out) {
+    if (lse_merge_by_warps(partial, nsplit, nh, D, B, out)) return lse_merge_warps_launch(st, partial, nsplit, nsplit, nh, D, B, out, nullptr);
     const dim3 grid(nh, B, (D + 127) / 128);
     auto kern = nsplit > 32 ? lse_merge_kernel<false, 64> : nsplit > 8 ? lse_merge_kernel<false, 32> : lse_merge_kernel<false, 8>;
     (void)cwk_launch_early(kern, grid, dim3(128), 0, st, partial, nsplit, nh, D, out, (float *)nullptr, (const int2 *)nullptr);
 }
-// `meta[b]` = {first record, number of records} of sequence b, at most CWK_MAX_SPLITS of them
-static inline void lse_combine_ranges_launch(cudaStream_t st, const float *partial, const int2 *meta, int nh, int D, int B, uint16_t *out) {
+// `meta[b]` = {first record, number of records} of sequence b, at most CWK_MAX_SPLITS of them, `records` in all at most
+static inline void lse_combine_ranges_launch(cudaStream_t st, const float *partial, const int2 *meta, int records, int nh, int D, int B, uint16_t *out) {
+    if (lse_merge_by_warps(partial, records / B, nh, D, B, out)) return lse_merge_warps_launch(st, partial, 0, records / B, nh, D, B, out, meta);
     (void)cwk_launch_early(lse_merge_kernel<false, 8>, dim3(nh, B, (D + 127) / 128), dim3(128), 0, st, partial, 0, nh, D, out, (float *)nullptr, meta);
 }
 static inline void lse_fold_launch(cudaStream_t st, const float *partial, int nsplit, int nh, int D, float *rec_out) {

@@ -168,7 +168,7 @@ static int mla_launch(cwk_ctx *ctx, const void *q, const void *cache, int64_t se
             s = cwk_mla_decode_tc_launch(ctx, q, cache, seq_stride, ld, kv_len, max_kv_len, B, nh, R, scale, ctx->scratch, G, nullptr, nullptr, 0, meta);
             if (s != CWK_OK) return s;
         }
-        lse_combine_ranges_launch(ctx->stream, ctx->scratch, meta, nh, L, B, (uint16_t *)out);
+        lse_combine_ranges_launch(ctx->stream, ctx->scratch, meta, B + G, nh, L, B, (uint16_t *)out);
         CWK_LAUNCH_CHECK(ctx, "lse_merge_kernel");
         ctx->last_nsplit = 0;
         return CWK_OK;

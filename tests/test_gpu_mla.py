@@ -67,6 +67,23 @@ def test_ragged_batch_with_empty_sequence(attn, nsplit):
     close(g, oracle_out(q, cache, lens))
 
 
+@pytest.fixture(scope="module")
+def five_long():
+    q, cache = make_case(78, 5, 64, 4300)
+    lens = np.array([4300, 0, 1, 2100, 4225], np.int32)
+    return to_bf16_cuda(q), to_bf16_cuda(cache), torch.from_numpy(lens).cuda(), oracle_out(q, cache, lens)
+
+
+@pytest.mark.parametrize("nsplit", [2, 4, 5, 8, 9, 16, 17, 32, 33])
+def test_merge_of_split_records(attn, five_long, nsplit):
+    """Both merges (a warp per row and chunk up to 32 records, blocks above) at the ends of their numbers of records ahead,
+    with empty and one-row sequences among the records."""
+    q, cache, lens, want = five_long
+    g = bf16_to_np(attn.mla_decode(q, cache, lens, scale=SCALE, n_splits=nsplit))
+    assert np.all(g[1] == 0)
+    close(g, want)
+
+
 @pytest.mark.parametrize("nh", [16, 40, 128])
 def test_head_counts_other_than_64(attn, nh):
     q, cache = make_case(5 + nh, 2, nh, 300)
