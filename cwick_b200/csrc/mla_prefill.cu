@@ -216,9 +216,9 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const float *rot, const
 // and 5 per item (128 queries x head x half), the items dealt over the SMs; absorbed 0.033 per query and 128-key tile, 0.08 per
 // query around it (0.4 where the queries are more than the SMs: there the other route is far ahead anyway) and 18 for launches
 // that do not come up early. Calls measured near the line, absorbed / expanded:
-//   4 queries after 300 rows 90 / 80, after 1000 92 / 99;          16 after 300 95 / 80, after 1000 97 / 96, after 3000 108 / 139
-//   32 after 1000 114 / 100, after 3000 125 / 139;                 64 after 3000 163 / 143, after 8000 245 / 255
-//   96 after 8000 332 / 274, after 32000 826 / 814;                129 after 8000 356 / 345, after 16000 637 / 610, after 32000 1083 / 1191
+//   4 queries after 300 rows 81 / 73, after 1000 81 / 89;          16 after 300 84 / 73, after 1000 86 / 87, after 3000 95 / 127
+//   32 after 1000 97 / 90, after 3000 110 / 127;                   64 after 3000 136 / 129, after 8000 215 / 232
+//   96 after 8000 270 / 234, after 32000 759 / 736;                129 after 8000 341 / 319, after 16000 595 / 538, after 32000 1025 / 1023
 static bool expanded_keys_pay(const cwk_ctx *ctx, int n, int64_t pos0, int nh) {
     const double T = (double)(pos0 + n), mean = (double)pos0 + 0.5 * n;
     const double items = (double)((n + 127) / 128) * nh * 2, rounds = items <= ctx->sm_count ? 1.0 : items / ctx->sm_count + 0.5;

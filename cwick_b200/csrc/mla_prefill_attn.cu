@@ -16,22 +16,20 @@
 //   kexp_tc_kernel: Kx[h][c][0:128] = W_uk[h] lat[c] (tcgen05, W_uk[h] resident per block as the
 //     K-major B operand, latent tiles streamed), Kx[h][c][128:192] = k_rope[c]. Head-major: a head's 64-key tile is
 //     24 KB of consecutive memory (token-major rows would lie 24 KB apart and crowd a few L2 slices).
-//   prefill_attn_kernel: one block = 128 queries x one head x one half of the 512 value columns
-//     (the accumulator of a half, 128 x 256 f32, is half of tensor memory; both halves recompute
-//     the 192-wide scores, which is cheaper than any exchange). Keys stream in tiles of 64 through a
-//     3-deep ring (24 KB each), latent halves through a 3-deep ring (32 KB each), one TMA box each. The query tile
-//     itself sits in tensor memory (96 columns of bf16 pairs) as the A operand of the score MMAs, and P beside it (32 columns) as
-//     that of the values': this way the MMAs read only keys and values from shared memory.
+//   The attention: one item = 128 queries x one head. The accumulator of one half of the 512 value columns, 128 x 256 f32, is half of
+//     tensor memory, so an item is two blocks' work. Keys stream in tiles of 64 (24 KB), latent halves beside them (32 KB), one TMA box
+//     each. The query tile sits in tensor memory (96 columns of bf16 pairs) as the A operand of the score MMAs, which
+//     so read only the keys from shared memory.
 //     Per tile: S = Q Kx^T (12 MMAs, M 128 x N 64) into one of two TMEM score buffers; the softmax
 //     warps own one query row per thread (TMEM lane = row, so row maxima and sums need no shuffles),
-//     write P (bf16) to tensor memory (GQA: shared memory); O += P lat (4 MMAs, M 128 x N 256). The two products have
-//     issuer threads of their own (the scores two), so the scores run ahead of the values and the tensor pipe works under
-//     the softmax.
-//     The kernel has two forms. The fast one splits the 64 keys of a row between two softmax warp groups
-//     (two threads per row, another two groups for every other tile) and never rescales: a row's reference exponent is its largest score of the first
-//     tile, later scores may outrun it by up to 2^64 (bf16 P and the f32 accumulators have the range), and a
-//     block that sees more raises a flag. The exact one (one thread per row, lazy rescale of its own TMEM lane
-//     when a score outruns the reference by 2^8) runs right after it and recomputes the flagged blocks only.
+//     write P (bf16); O += P lat (4 MMAs, M 128 x N 256). The two products have
+//     issuers of their own, so the scores run ahead of the values and the tensor pipe works under the softmax.
+//     There are two forms. The fast one (prefill_pair_kernel; GQA: prefill_attn_kernel<4>) splits the 64 keys of a row between two
+//     softmax warp groups (two threads per row, another two groups for every other tile) and never rescales: a row's reference
+//     exponent is its largest score of the first tile, later scores may outrun it by up to 2^64 (bf16 P and the f32 accumulators have
+//     the range), and a block that sees more raises a flag. The exact one (prefill_attn_kernel<1>: one thread per row, each half
+//     for itself, lazy rescale of its own TMEM lane when a score outruns the reference by 2^8) runs right after it and recomputes the
+//     flagged items only.
 //
 // Every mbarrier wait is bounded and records a code in the context's error word when it gives up.
 #include <algorithm>
@@ -50,8 +48,8 @@ constexpr int PA_KST = 3;
 // on to kc before its slot had been filled. With an even number of barriers each has one issuer, which sees all of its phases.
 constexpr int PA_KBAR = 2 * PA_KST;
 constexpr int PA_OFF_K = 0;                            // (the query tile lives in tensor memory, not here)
-// The kernel serves two shapes. MLA prefill: 192-wide expanded keys, the 512 value columns in two halves, three value
-// stages. GQA prefill (Qwen3.5 layers): 256-wide keys and values of one KV head, two value stages (the key tiles are
+// prefill_attn_kernel serves two shapes. MLA prefill (its exact form): 192-wide expanded keys, the 512 value columns in two halves, three
+// value stages. GQA prefill (Qwen3.5 layers): 256-wide keys and values of one KV head, two value stages (the key tiles are
 // 32 KB instead of 24 KB). Shared-memory layout and the query tile's width in tensor memory follow from DQK and CST.
 template <int DQK_, int CST_>
 struct PaCfg {
@@ -85,15 +83,15 @@ struct AttnParams {
     int group;          // GQA: query heads per KV head (MLA: unused)
     int64_t pos0;
     float scale_log2;
-    int *flags;         // one word per item (share mode: per item + block): fast form sets it, exact form runs only where it is set
+    int *flags;         // one word per item (share mode: per item + share): fast form sets it, exact form runs only where it is set
     int *counter;       // [3]: item counters of the fast and the exact form, number of flags raised; zero at launch
     int *err;
-    // Share mode (shares > 0): the key tiles of all items, one after another, are dealt out to the blocks in equal contiguous
-    // shares, whatever the items' number and lengths; what a block does of an item that is not all its own is left as a record
-    // (record_of), and attn_merge_kernel joins them.
-    int shares;         // number of blocks
-    int head_tiles;     // key tiles of one (head, half)
-    float *records;     // [2 * shares][PA_RECORD]
+    // Share mode (shares > 0): the key tiles of all items, one after another, are dealt out to the blocks (MLA: pairs of blocks) in
+    // equal contiguous shares, whatever the items' number and lengths; what a share has of an item that is not all its own is left
+    // as a record (record_of), and attn_merge_kernel joins them.
+    int shares;         // number of blocks or pairs
+    int head_tiles;     // key tiles of one head
+    float *records;     // [2 * shares] (MLA: times two halves) [PA_RECORD]
 };
 constexpr int PA_RECORD = PA_QT * (PA_DV + 2);         // floats: O as [PA_DV / 4][row][4], m [row], l [row]
 
@@ -102,14 +100,14 @@ struct AttnItem {
     int rec, flag;             // where the result goes as a record (-1: into the output); index of the flag
 };
 
-// Work item w of the attention grid: query tiles from the longest to the shortest inside one (head, half), then the next
-// (head, half): blocks that run at the same time work on the same few heads, whose keys stay in L2.
+// Work item w of the attention grid: query tiles from the longest to the shortest inside one head, then the next head: blocks that
+// run at the same time work on the same few heads, whose keys stay in L2. (MLA: each of the two halves of the value columns does it.)
 __device__ __forceinline__ AttnItem attn_item(int w, const AttnParams &p, int nq) {
     AttnItem it;
-    const int qtile = nq - 1 - (w % nq), hh = w / nq;
+    const int qtile = nq - 1 - (w % nq);
     it.q0 = qtile * PA_QT;
-    it.h = hh % p.nh;
-    it.half = hh / p.nh;                                                   // GQA: the grid has one "half", always 0
+    it.h = w / nq;
+    it.half = 0;
     const int64_t last_q = p.pos0 + min(it.q0 + PA_QT - 1, p.n - 1);     // keys 0 .. pos0 + (last query of the item): tiles of 64
     it.lo = 0;
     it.nt = (int)(last_q / PA_KT) + 1;
@@ -128,12 +126,13 @@ __device__ __forceinline__ int64_t share_begin(int g, int64_t total_tiles, int s
     const uint32_t t = (uint32_t)total_tiles, q = t / (uint32_t)shares, r = t - q * (uint32_t)shares;
     return (int64_t)(q * (uint32_t)g + r * (uint32_t)g / (uint32_t)shares);
 }
-// The part of block g (tiles u0 .. u1 - 1 of all) in item `it`, which begins at tile `at` of all; false: none.
+template <bool GQA> __device__ __forceinline__ int64_t record_of(int rec, int half) { return GQA ? rec : 2 * rec + half; }
+// The part of share g (tiles u0 .. u1 - 1 of all) in item `it`, which begins at tile `at` of all; false: none.
 __device__ __forceinline__ bool attn_segment(AttnItem &it, int w, int g, int64_t at, int64_t u0, int64_t u1, const AttnParams &p) {
     const int nt = it.nt, lo = attn_cut((int)max((int64_t)-1, min((int64_t)nt, u0 - at)), it, p), hi = attn_cut((int)max((int64_t)-1, min((int64_t)nt, u1 - at)), it, p);
     it.lo = lo;
     it.nt = hi;
-    it.rec = lo > 0 ? 2 * g : hi < nt ? 2 * g + 1 : -1;      // (only a block's first segment begins inside an item, only its last ends inside one)
+    it.rec = lo > 0 ? 2 * g : hi < nt ? 2 * g + 1 : -1;      // (only a share's first segment begins inside an item, only its last ends inside one)
     it.flag = w + g;                                         // (from one segment to the next w or g goes up)
     return hi > lo;
 }
@@ -157,6 +156,42 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
     return r;
 }
 
+// The query tile is the A operand of every score MMA of the item; it is kept in tensor memory (row = lane, two
+// consecutive bf16 per 32-bit column), so that those MMAs read only the keys from shared memory. A thread
+// copies its row's share: DQK / 2 columns split between the groups. The tile of item k + 1 is copied
+// BEFORE the epilogue of item k, so that the next item's first scores are computed under that epilogue.
+template <class CFG, int NWG, bool GQA, class F>      // NWG copying groups; done: says so for the warp
+__device__ __forceinline__ void load_query_tile(const AttnParams &p, int q0_, int h_, int row, int wg, uint32_t tlane, F done) {
+    const int t = q0_ + row;
+    const uint4 *src = reinterpret_cast<const uint4 *>(p.q + ((int64_t)t * p.nh + h_) * CFG::DQK);
+#pragma unroll
+    for (int c = 0; c < CFG::DQK / 16 / NWG; c++) {        // eight words at a time, the groups in turn
+        const int w8 = c * NWG + wg;
+        uint32_t wv[8];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint4 v = (t < p.n) ? src[w8 * 2 + j] : make_uint4(0, 0, 0, 0);
+            wv[4 * j] = v.x; wv[4 * j + 1] = v.y; wv[4 * j + 2] = v.z; wv[4 * j + 3] = v.w;
+        }
+        // the rope pairs (the last 64 of 192 columns) are rotated on their way, at the row's position: a kernel of its own, in
+        // place, was 32 us for 4096 tokens of 64 heads, 13 for 509
+        if (!GQA && c * NWG * 16 >= CFG::DQK - 64 && p.rot && t < p.n) {
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                const float4 r = p.rot[(int64_t)t * 16 + w8 * 4 - (CFG::DQK - 64) / 4 + j / 2];
+                const float a0 = __uint_as_float(wv[j] << 16), b0 = __uint_as_float(wv[j] & 0xffff0000u);
+                const float a1 = __uint_as_float(wv[j + 1] << 16), b1 = __uint_as_float(wv[j + 1] & 0xffff0000u);
+                wv[j] = pack_bf16x2(a0 * r.x - b0 * r.y, b0 * r.x + a0 * r.y);
+                wv[j + 1] = pack_bf16x2(a1 * r.z - b1 * r.w, b1 * r.z + a1 * r.w);
+            }
+        }
+        TMEM_ST8(wv, 0, tlane + PA_COL_Q + w8 * 8);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tc_fence_before();
+    done();
+}
+
 // Softmax groups and tiles. A tile's scores go from tensor memory through registers into P in a chain (barrier, load, maximum,
 // exponentials, barrier, store, fence) that takes longer than its MMAs. So in the fast form two of the four groups take the even tiles
 // and two the odd ones, a row's 64 keys between them, and the chains of two tiles overlap.
@@ -178,12 +213,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + PA_OFF_BAR + 8 * PB_COUNT + 8);
     int4 *s_item = reinterpret_cast<int4 *>(sm + PA_OFF_X + 4096);      // ring of 8 items: {number, first tile, end, record}
-    // P is the A operand of the value MMAs. Where the query tile leaves room for it (192-wide keys), it lies in tensor memory: 32 KB less
-    // through shared memory per tile and no proxy fence, 183 -> 176 us for 509 queries after 3001 rows. One tile's worth: it is
-    // written when the value MMAs of the tile before are done. (In the place of the scores it comes from, which 256-wide keys would need,
-    // those MMAs are a link of the next scores' chain: 105 -> 117 us for 512 GQA queries after 10488 rows.)
-    constexpr bool OWN_P = PA_COL_Q + PA_DQK / 2 + PA_KT / 2 <= 512;
-    constexpr uint32_t PA_COL_P = PA_COL_Q + PA_DQK / 2;
+    // (P stays in shared memory. In the place of the scores it comes from, in tensor memory, the value MMAs are a link of the next
+    // scores' chain: 105 -> 117 us for 512 GQA queries after 10488 rows.)
     constexpr int TG = NWG == 4 ? 2 : 1, QK_ISSUERS = NWG == 4 ? 2 : 1;      // groups that share a tile; issuers of the score MMAs
     float *s_m = reinterpret_cast<float *>(sm + PA_OFF_X), *s_l = s_m + 512;              // [4][128] each
 
@@ -192,7 +223,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     cwk_pdl_wait();
     if (NWG == 1 && p.counter[2] == 0) return;                   // the repair pass: the fast form raised no flag
     const int nq = (p.n + PA_QT - 1) / PA_QT;
-    const int total = nq * p.nh * (GQA ? 1 : 2);
+    const int total = nq * p.nh;
+    const int unit = GQA ? (int)blockIdx.x : (int)blockIdx.x >> 1;      // share mode: whose share this block works on (MLA: one half of it)
 
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_k) : "memory");
@@ -217,10 +249,11 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     auto next_item = [&](int k, int &w, AttnItem &it) -> bool {
         if (!mbar_wait(bar(PB_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1031)) return false;
         const int4 v = s_item[k & 7];
-        w = v.x;
+        w = GQA || v.x < 0 ? v.x : v.x >> 1;
         it = attn_item(max(w, 0), p, nq);
+        it.half = GQA ? 0 : v.x & 1;
         it.lo = v.y; it.nt = v.z; it.rec = v.w;
-        if (p.shares) it.flag = w + (int)blockIdx.x;
+        if (p.shares) it.flag = w + unit;
         return true;
     };
 
@@ -229,9 +262,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         if (lane == 0) {
             bool ok = true;
             int kc = 0;                              // key tiles issued so far (ring position and phase run across items)
-            const int hh_n = p.nh * (GQA ? 1 : 2);
-            const int64_t all = (int64_t)p.head_tiles * hh_n, u0 = p.shares ? share_begin(blockIdx.x, all, p.shares) : 0,
-                          u1 = p.shares ? share_begin(blockIdx.x + 1, all, p.shares) : 0;
+            const int64_t all = (int64_t)p.head_tiles * p.nh, u0 = p.shares ? share_begin(unit, all, p.shares) : 0,
+                          u1 = p.shares ? share_begin(unit + 1, all, p.shares) : 0;
             int sw = 0;                              // share mode: the next item, and where it begins
             int64_t at = 0;
             if (p.shares) {
@@ -240,25 +272,28 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 for (int nt; sw < total && at + (nt = attn_item(sw, p, nq).nt) <= u0; sw++) at += nt;
             }
             for (int k = 0; ok; k++) {
-                int w = -1;
+                int w = -1, half = GQA ? 0 : (int)blockIdx.x & 1;
                 AttnItem it{};
                 if (p.shares) {
                     while (sw < total && at < u1) {
                         it = attn_item(sw, p, nq);
                         const int nt = it.nt;
-                        const bool mine = attn_segment(it, sw, blockIdx.x, at, u0, u1, p);
+                        const bool mine = attn_segment(it, sw, unit, at, u0, u1, p);
                         at += nt;
                         sw++;
                         if (mine && (NWG > 1 || p.flags[it.flag] != 0)) { w = sw - 1; break; }      // (the repair pass takes flagged ones only)
                     }
                 } else {
-                    w = atomicAdd(p.counter + (NWG == 1 ? 1 : 0), 1);
+                    constexpr int H = GQA ? 1 : 2;    // an item is one of its halves here
+                    int hw = atomicAdd(p.counter + (NWG == 1 ? 1 : 0), 1);
                     if (NWG == 1)                     // the repair pass takes flagged items only
-                        while (w < total && p.flags[w] == 0) w = atomicAdd(p.counter + 1, 1);
-                    if (w >= total) w = -1;
+                        while (hw < total * H && p.flags[hw / H] == 0) hw = atomicAdd(p.counter + 1, 1);
+                    w = hw < total * H ? hw / H : -1;
+                    half = hw % H;
                     it = attn_item(max(w, 0), p, nq);
                 }
-                s_item[k & 7] = make_int4(w, it.lo, it.nt, it.rec);      // the roles of a block stay within a few tiles of each other: 8 slots cannot wrap
+                it.half = half;
+                s_item[k & 7] = make_int4(GQA || w < 0 ? w : 2 * w + half, it.lo, it.nt, it.rec);      // the roles of a block stay within a few tiles of each other: 8 slots cannot wrap
                 mbar_arrive(bar(PB_ITEM + (k & 7)));
                 if (w < 0) break;
                 for (int i = it.lo; i < it.nt && ok; i++, kc++) {
@@ -305,8 +340,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         // waits of a tile in turn was the longest chain of the kernel. So was, after that, the one issuer of the scores: two
         // waits, 12 or 16 MMAs and the commits took it 1650 cycles a tile, of which the tensor pipe works 400 to 500. In the fast
         // form a second one (the last warp) takes every other tile. All lanes run the issuers' loops and one is elected for the
-        // MMAs (tc_common.cuh): with the values' P in tensor memory 1644 -> 1575 us for a whole prompt of 4096, 372 -> 353 for 509
-        // after 3001.
+        // MMAs (tc_common.cuh).
         {
             constexpr uint32_t ID_QK = idesc_bf16(128, PA_KT, 0, 0);
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
@@ -376,8 +410,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
 #pragma unroll
                         for (int s = 0; s < 4; s++) {
                             const uint32_t acc = s != 0 ? 1u : (uint32_t)(i != 0);
-                            if (OWN_P) umma_bf16_ts(tm + PA_COL_O, tm + PA_COL_P + s * 8, dC + (uint64_t)((s * 2048) >> 4), ID_PV, acc);
-                            else umma_bf16(tm + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, acc);
+                            umma_bf16(tm + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, acc);
                         }
                         umma_commit(bar(PB_CEMPTY + cs));
                         umma_commit(bar(PB_PEMPTY + pb));
@@ -408,40 +441,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             if (!ok || w < 0) break;
             const int q0 = it.q0, h = it.h, half = it.half, nt = it.nt;
             const int64_t tq = p.pos0 + q0 + row;                    // this row's position: keys 0..tq are visible
-            // The query tile is the A operand of every score MMA of the item; it is kept in tensor memory (row = lane, two
-            // consecutive bf16 per 32-bit column), so that those MMAs read only the keys from shared memory. A thread
-            // copies its row's share: DQK / 2 columns split between the groups. The tile of item k + 1 is copied
-            // BEFORE the epilogue of item k (below), so that the next item's first scores are computed under that epilogue.
-            auto load_query = [&](int q0_, int h_) {
-                const int t = q0_ + row;
-                const uint4 *src = reinterpret_cast<const uint4 *>(p.q + ((int64_t)t * p.nh + h_) * PA_DQK);
-#pragma unroll
-                for (int c = 0; c < PA_DQK / 16 / NWG; c++) {        // eight words at a time, the groups in turn
-                    const int w8 = c * NWG + wg;
-                    uint32_t wv[8];
-#pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        const uint4 v = (t < p.n) ? src[w8 * 2 + j] : make_uint4(0, 0, 0, 0);
-                        wv[4 * j] = v.x; wv[4 * j + 1] = v.y; wv[4 * j + 2] = v.z; wv[4 * j + 3] = v.w;
-                    }
-                    // the rope pairs (the last 64 of 192 columns) are rotated on their way, at the row's position: a kernel of its own, in
-                    // place, was 32 us for 4096 tokens of 64 heads, 13 for 509
-                    if (!GQA && c * NWG * 16 >= PA_DQK - 64 && p.rot && t < p.n) {
-#pragma unroll
-                        for (int j = 0; j < 8; j += 2) {
-                            const float4 r = p.rot[(int64_t)t * 16 + w8 * 4 - (PA_DQK - 64) / 4 + j / 2];
-                            const float a0 = __uint_as_float(wv[j] << 16), b0 = __uint_as_float(wv[j] & 0xffff0000u);
-                            const float a1 = __uint_as_float(wv[j + 1] << 16), b1 = __uint_as_float(wv[j + 1] & 0xffff0000u);
-                            wv[j] = pack_bf16x2(a0 * r.x - b0 * r.y, b0 * r.x + a0 * r.y);
-                            wv[j + 1] = pack_bf16x2(a1 * r.z - b1 * r.w, b1 * r.z + a1 * r.w);
-                        }
-                    }
-                    TMEM_ST8(wv, 0, tlane + PA_COL_Q + w8 * 8);
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();
-                arrive(PB_QFULL);
-            };
+            auto load_query = [&](int q0_, int h_) { load_query_tile<CFG, NWG, GQA>(p, q0_, h_, row, wg, tlane, [&]() { arrive(PB_QFULL); }); };
             if (k == 0) load_query(q0, h);
             float m = 0.f, l = 0.f;
             // reference exponent of the row: its largest score of the item's first tile, which one pair of groups has. (All arrive:
@@ -533,24 +533,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 float l0, l1;
                 unpack_f32x2(lsum, l0, l1);
                 l += l0 + l1;
-                if (OWN_P) {
-                    // P has columns of its own once the value MMAs of the tile before are done with them
-                    if (tc0 + d > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + ((tc0 + d - 1) & 1)), (uint32_t)(((tc0 + d - 1) >> 1) & 1), p.err, 1023));
-                    if (!ok) break;
-                    tc_fence_after();
+                // the P buffer of this parity was read by the value MMAs two tiles ago
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023));
+                if (!ok) break;
+                uint8_t *prow = sm + PA_OFF_P + sb * PA_P_BYTES + row * 128;
 #pragma unroll
-                    for (int c = 0; c < NC / 32; c++) TMEM_ST16(pk, c * 16, tlane + PA_COL_P + cg * (NC / 2) + c * 16);
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                } else {
-                    // the P buffer of this parity was read by the value MMAs two tiles ago
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023));
-                    if (!ok) break;
-                    uint8_t *prow = sm + PA_OFF_P + sb * PA_P_BYTES + row * 128;
-#pragma unroll
-                    for (int c = 0; c < NC / 8; c++)
-                        *reinterpret_cast<uint4 *>(prow + (((cg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                }
+                for (int c = 0; c < NC / 8; c++)
+                    *reinterpret_cast<uint4 *>(prow + (((cg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 tc_fence_before();
                 arrive(PB_PFULL + sb);
             }
@@ -581,7 +571,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 l = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
             }
             if (it.rec >= 0) {                                       // part of an item: its record
-                float *rec = p.records + (int64_t)it.rec * PA_RECORD;
+                float *rec = p.records + record_of<GQA>(it.rec, half) * PA_RECORD;
                 constexpr int CPG = PA_DV / NWG;                     // columns per group
 #pragma unroll 1
                 for (int c = 0; c < CPG / 16; c++) {
@@ -649,7 +639,465 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     }
 }
 
-// Share mode: joins the records of an item that more than one block worked on. Grid (shares, PA_DV / 32), a row per thread:
+// ---- the fast form of the MLA prompt: a pair of CTAs shares its scores ---------------------------------------------------
+// Both halves of the value columns want the same scores, 192 wide, and their exponentials: done by each half for itself they are
+// 384 of 896 multiply-adds per (query, key, head), and a whole prompt is at the power cap. Here the halves are the two CTAs of a
+// cluster. The tiles of all items have running numbers T; the CTA with rank T & 1 forms tile T's scores and P, and P goes to the other by a bulk copy
+// between their shared memories, so that each does half the scores and all of its values. (The first tile of an item gives the
+// rows' reference exponents: both form its scores, one uses them. The row sums are exchanged at the item's end.)
+//
+// 4096 tokens (whole prompt) 1555 -> 1471 us, 509 after 3001 349 -> 330. With the copies issued by the values' issuer, in the order of
+// the tiles, each waited for the peer's copy of the tile before: 2.7 k cycles a tile, 1792 us.
+//
+// P lies in four buffers, tile T in buffer T % 4 of both CTAs: those of its own tiles a CTA's softmax writes, the others the
+// peer fills (an even number: a role that looks at own tiles only sees every phase of their barriers; six of them beside two latent
+// stages instead of three: 1490 and 338 us). A buffer is free for tile T + 4 when the value MMAs of tile T are done in BOTH CTAs, which each tells the
+// other by committing to the same barrier in both. There are eight of these barriers, T % 8: the two softmax sets of a CTA may be
+// an own tile apart, and with four a set could wait for a phase whose predecessor is still open, which a parity wait cannot tell
+// from the one after. tests/test_prefill_pair_protocol.py walks the protocol.
+template <class CFG>
+struct PrCfg {
+    static constexpr int KST = 2, CST = 3;
+    static constexpr int OFF_C = KST * CFG::K_BYTES, OFF_P = OFF_C + CST * PA_C_BYTES, OFF_BAR = OFF_P + 4 * PA_P_BYTES, OFF_X = OFF_BAR + 512;
+    static constexpr int SMEM = OFF_X + 2 * 2048 + 4 * 512 + 128 + 1024;      // maxima [4][128], sums [4][128], row sums here and there [2][128] each, 8 items
+    static_assert(SMEM <= 232448, "shared-memory budget");
+};
+constexpr int PR_THREADS = 672;      // keys, scores, latents, values | 16 softmax warps | sender of P
+enum { PR_QFULL = 0, PR_KFULL, PR_KEMPTY = PR_KFULL + 2, PR_CFULL = PR_KEMPTY + 2, PR_CEMPTY = PR_CFULL + 3, PR_SFULL = PR_CEMPTY + 3, PR_SEMPTY = PR_SFULL + 2,
+       PR_PFULL = PR_SEMPTY + 2, PR_PEMPTY = PR_PFULL + 4, PR_ODONE = PR_PEMPTY + 8, PR_QEMPTY, PR_OFREE, PR_XM, PR_XL, PR_PEER, PR_ITEM = PR_PEER + 2,
+       PR_COUNT = PR_ITEM + 8 };
+static_assert(8 * PR_COUNT + 16 <= 512, "barriers");
+
+// shared memory of this CTA to the same offset in CTA `peer` of the cluster, its bytes counted at that CTA's barrier (multiples of 16 bytes)
+__device__ __forceinline__ void copy_to_peer(uint32_t addr, uint32_t bytes, uint32_t peer_addr, uint32_t peer_bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(peer_addr), "r"(addr), "r"(bytes), "r"(peer_bar)
+                 : "memory");
+}
+// completion of this CTA's MMAs so far, at the same barrier in both CTAs of the pair
+__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
+prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_c, const AttnParams p) {
+    using CFG = PaMla;
+    using L = PrCfg<CFG>;
+    constexpr int NC = PA_KT / 2;                            // key columns per softmax thread
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t *sm = smem_raw + (base - raw);
+    const uint32_t bar0 = base + L::OFF_BAR;
+    auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + L::OFF_BAR + 8 * PR_COUNT + 8);
+    float *s_m = reinterpret_cast<float *>(sm + L::OFF_X), *s_l = s_m + 512, *s_sum = s_l + 512, *s_peer = s_sum + 256;
+    int4 *s_item = reinterpret_cast<int4 *>(s_peer + 256);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = (int)cluster_rank(), unit = (int)blockIdx.x >> 1, units = (int)gridDim.x >> 1;
+    cwk_pdl_launch();
+    cwk_pdl_wait();
+    const int nq = (p.n + PA_QT - 1) / PA_QT, total = nq * p.nh;
+
+    if (tid == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_k) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_c) : "memory");
+        for (int i = 0; i < PR_COUNT; i++) {
+            uint32_t count = 1;
+            if (i == PR_QFULL || i == PR_OFREE || i == PR_XM || i == PR_XL) count = 16;                  // every softmax warp
+            if (i == PR_SEMPTY || i == PR_SEMPTY + 1) count = 8;                                         // the warps of a set
+            if (i >= PR_PFULL && i < PR_PEMPTY) count = ((i - PR_PFULL) & 1) == rank ? 8 : 1;            // ... or the announcement of the peer's copy
+            if (i >= PR_PEMPTY && i < PR_ODONE) count = 2;                                               // the value MMAs of both CTAs
+            mbar_init(bar(i), count);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                          // the peer's barriers are there
+    tc_fence_after();
+    const uint32_t tmem = *s_tmem;
+
+    // item k of this pair, as published by the key producer (w < 0: no more); both CTAs come to the same items by themselves
+    auto next_item = [&](int k, int &w, AttnItem &it) -> bool {
+        if (!mbar_wait(bar(PR_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1431)) return false;
+        const int4 v = s_item[k & 7];
+        w = v.x;
+        it = attn_item(max(w, 0), p, nq);
+        it.half = rank;
+        it.lo = v.y; it.nt = v.z; it.rec = v.w;
+        if (p.shares) it.flag = w + unit;
+        return true;
+    };
+    // the tiles of an item whose first has number T: how many this CTA forms the scores of (the first, and its own), and the i-th of them
+    auto scored = [&](int T, int tiles) { const int f = ((T + 1) & 1) == rank ? 1 : 2; return tiles > f ? 1 + (tiles - f + 1) / 2 : 1; };
+    auto nth = [&](int T, int e) { return e == 0 ? 0 : (((T + 1) & 1) == rank ? 1 : 2) + 2 * (e - 1); };
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ item fetcher and TMA producer of the key ring
+        if (lane == 0) {
+            bool ok = true;
+            int kc = 0, T = 0;                       // key tiles issued so far; number of the item's first tile
+            const int64_t all = (int64_t)p.head_tiles * p.nh, u0 = p.shares ? share_begin(unit, all, p.shares) : 0, u1 = p.shares ? share_begin(unit + 1, all, p.shares) : 0;
+            int sw = 0;                              // share mode: the next item, and where it begins
+            int64_t at = 0;
+            if (p.shares) {
+                sw = (int)u0 / p.head_tiles * nq;
+                at = (int)u0 / p.head_tiles * p.head_tiles;
+                for (int nt; sw < total && at + (nt = attn_item(sw, p, nq).nt) <= u0; sw++) at += nt;
+            }
+            for (int k = 0; ok; k++) {
+                int w = -1;
+                AttnItem it{};
+                if (p.shares) {
+                    while (sw < total && at < u1) {
+                        it = attn_item(sw, p, nq);
+                        const int nt = it.nt;
+                        const bool mine = attn_segment(it, sw, unit, at, u0, u1, p);
+                        at += nt;
+                        sw++;
+                        if (mine) { w = sw - 1; break; }
+                    }
+                } else {
+                    // in rounds, there and back: a pair that had the longer items of one round has the shorter ones of the next
+                    w = k * units + ((k & 1) ? units - 1 - unit : unit);
+                    if (w >= total) w = -1;
+                    it = attn_item(max(w, 0), p, nq);
+                }
+                s_item[k & 7] = make_int4(w, it.lo, it.nt, it.rec);      // the roles of a block stay within a few tiles of each other: 8 slots cannot wrap
+                mbar_arrive(bar(PR_ITEM + (k & 7)));
+                if (w < 0) break;
+                const int tiles = it.nt - it.lo, mine = scored(T, tiles);
+                for (int e = 0; e < mine && ok; e++, kc++) {
+                    const int ks = kc % L::KST;
+                    ok = mbar_wait(bar(PR_KEMPTY + ks), (uint32_t)(((kc / L::KST) & 1) ^ 1), p.err, 1401);
+                    if (!ok) break;
+                    mbar_expect_tx(bar(PR_KFULL + ks), CFG::K_BYTES);
+                    tma_load_3d(base + ks * CFG::K_BYTES, &tm_k, 0, it.h * p.T + (it.lo + nth(T, e)) * PA_KT, 0, bar(PR_KFULL + ks));
+                }
+                T += tiles;
+            }
+            if (!ok)        // drain the copies still in flight before leaving
+                for (int j = max(0, kc - L::KST); j < kc; j++) mbar_wait(bar(PR_KFULL + j % L::KST), (uint32_t)((j / L::KST) & 1), p.err, 1404);
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------------------ TMA producer of the latent ring: every tile, this CTA's half
+        if (lane == 0) {
+            bool ok = true;
+            int cc = 0;
+            for (int k = 0; ok; k++) {
+                int w;
+                AttnItem it;
+                ok = next_item(k, w, it);
+                if (!ok || w < 0) break;
+                for (int i = it.lo; i < it.nt && ok; i++, cc++) {
+                    const int cs = cc % L::CST;
+                    ok = mbar_wait(bar(PR_CEMPTY + cs), (uint32_t)(((cc / L::CST) & 1) ^ 1), p.err, 1402);
+                    if (!ok) break;
+                    mbar_expect_tx(bar(PR_CFULL + cs), PA_C_BYTES);
+                    tma_load_3d(base + L::OFF_C + cs * PA_C_BYTES, &tm_c, 0, i * PA_KT, rank * 4, bar(PR_CFULL + cs));
+                }
+            }
+            if (!ok)
+                for (int j = max(0, cc - L::CST); j < cc; j++) mbar_wait(bar(PR_CFULL + j % L::CST), (uint32_t)((j / L::CST) & 1), p.err, 1405);
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer of the scores
+        constexpr uint32_t ID_QK = idesc_bf16(128, PA_KT, 0, 0);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint64_t dK0 = smem_desc(base, 16, 1024);
+        bool ok = true;
+        int kc = 0, T = 0;
+        for (int k = 0; ok; k++) {
+            int w;
+            AttnItem it;
+            ok = next_item(k, w, it);
+            if (!ok || w < 0) break;
+            const int tiles = __shfl_sync(0xffffffffu, it.nt - it.lo, 0), mine = scored(T, tiles);
+            ok = mbar_wait(bar(PR_QFULL), (uint32_t)(k & 1), p.err, 1411);     // the softmax threads have written the item's query tile into tensor memory
+            if (!ok) break;
+            tc_fence_after();
+            for (int e = 0; e < mine && ok; e++, kc++) {
+                const int ks = kc % L::KST, sb = kc & 1;
+                ok = mbar_wait(bar(PR_KFULL + ks), (uint32_t)((kc / L::KST) & 1), p.err, 1412);
+                if (ok) ok = mbar_wait(bar(PR_SEMPTY + sb), (uint32_t)(((kc >> 1) & 1) ^ 1), p.err, 1413);
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t dK = dK0 + (uint64_t)((ks * CFG::K_BYTES) >> 4);
+                if (elect_one()) {
+#pragma unroll
+                    for (int s = 0; s < CFG::DQK / 16; s++)
+                        umma_bf16_ts(tm + PA_COL_S + sb * PA_KT, tm + PA_COL_Q + s * 8,       // A: 16 bf16 of every row = 8 TMEM columns per step
+                                     dK + (uint64_t)(((s >> 2) * (PA_KT * 128) + (s & 3) * 32) >> 4), ID_QK, s != 0);
+                    umma_commit(bar(PR_KEMPTY + ks));
+                    umma_commit(bar(PR_SFULL + sb));
+                }
+                __syncwarp();
+            }
+            if (ok && elect_one()) umma_commit(bar(PR_QEMPTY));       // the query tile may be replaced once these MMAs are done
+            __syncwarp();
+            T += tiles;
+        }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------ MMA issuer of the values
+        constexpr uint32_t ID_PV = idesc_bf16(128, PA_DV, 0, 1);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint64_t dP0 = smem_desc(base + L::OFF_P, 16, 1024), dC0 = smem_desc(base + L::OFF_C, PA_KT * 128, 1024);
+        bool ok = true;
+        int T = 0, cs = 0, cu = 0;                   // tile, value stage and its use
+        for (int k = 0; ok; k++) {
+            int w;
+            AttnItem it;
+            ok = next_item(k, w, it);
+            if (!ok || w < 0) break;
+            const int tiles = __shfl_sync(0xffffffffu, it.nt - it.lo, 0);
+            if (k > 0) {                         // the accumulator of the previous item has been read out
+                ok = mbar_wait(bar(PR_OFREE), (uint32_t)((k - 1) & 1), p.err, 1416);
+                if (!ok) break;
+            }
+            for (int i = 0; i < tiles && ok; i++, T++) {
+                const int pb = T & 3;
+                const bool own = (T & 1) == rank;
+                if (!own) {                          // (the peer's copy may be here before it is announced)
+                    if (elect_one()) mbar_expect_tx(bar(PR_PFULL + pb), PA_P_BYTES);
+                    __syncwarp();
+                }
+                ok = mbar_wait(bar(PR_CFULL + cs), (uint32_t)(cu & 1), p.err, 1414);
+                if (ok) ok = mbar_wait(bar(PR_PFULL + pb), (uint32_t)((T >> 2) & 1), p.err, 1415);
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t dP = dP0 + (uint64_t)((pb * PA_P_BYTES) >> 4), dC = dC0 + (uint64_t)((cs * PA_C_BYTES) >> 4);
+                if (elect_one()) {
+                    // O += P lat, P [128 q][64 keys] K-major, lat half [64 keys][256] with the 256 contiguous (MN-major, four 64-wide blocks)
+#pragma unroll
+                    for (int s = 0; s < 4; s++)
+                        umma_bf16(tm + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, s != 0 ? 1u : (uint32_t)(i != 0));
+                    umma_commit(bar(PR_CEMPTY + cs));
+                    umma_commit_both(bar(PR_PEMPTY + (T & 7)));
+                }
+                __syncwarp();
+                if (++cs == L::CST) { cs = 0; cu++; }
+            }
+            if (ok && elect_one()) umma_commit(bar(PR_ODONE));
+            __syncwarp();
+        }
+    } else if (warp == 20) {
+        // ------------------------------------------------------------ sender of this CTA's P: as soon as it is there, whatever the values
+        // wait for (in the values' issuer a tile's copy waited for the peer's copy of the tile before: 2.7 k cycles a tile)
+        const uint32_t peer_p = cluster_addr(base + L::OFF_P, (uint32_t)(rank ^ 1)), peer_bar0 = cluster_addr(bar(PR_PFULL), (uint32_t)(rank ^ 1));
+        bool ok = true;
+        int T = 0;
+        for (int k = 0; ok; k++) {
+            int w;
+            AttnItem it;
+            ok = next_item(k, w, it);
+            if (!ok || w < 0) break;
+            const int end = __shfl_sync(0xffffffffu, T + it.nt - it.lo, 0);
+            for (T += (T ^ rank) & 1; T < end && ok; T += 2) {
+                const int pb = T & 3;
+                ok = mbar_wait(bar(PR_PFULL + pb), (uint32_t)((T >> 2) & 1), p.err, 1417);
+                if (!ok) break;
+                if (elect_one()) copy_to_peer(base + L::OFF_P + pb * PA_P_BYTES, PA_P_BYTES, peer_p + pb * PA_P_BYTES, peer_bar0 + 8u * (uint32_t)pb);
+                __syncwarp();
+            }
+            T = end;
+        }
+    } else {
+        // ------------------------------------------------------------ softmax, epilogue
+        // A thread owns query row `row` (= its TMEM lane) and NC of the 64 key columns of its tiles; two groups have a tile between
+        // them, two sets of groups the scored tiles in turn.
+        const int q4 = warp & 3, wg = (warp - 4) >> 2, cg = wg & 1, set = wg >> 1;
+        const int row = q4 * 32 + lane;
+        const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
+        const uint32_t peer_sum = cluster_addr(smem_u32(s_peer), (uint32_t)(rank ^ 1)), peer_bar0 = cluster_addr(bar(PR_PEER), (uint32_t)(rank ^ 1));
+        auto arrive = [&](int b) {                   // one for the warp, after every lane's accesses
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(b));
+        };
+        auto buffer_free = [&](int T) {              // P buffer T % 4 is free for tile T: both CTAs are done with tile T - 4
+            return T < 4 || mbar_wait(bar(PR_PEMPTY + ((T - 4) & 7)), (uint32_t)(((T - 4) >> 3) & 1), p.err, 1423);
+        };
+        bool ok = true;
+        int kc = 0, T = 0;                           // scored tiles so far (score buffer and its phase); number of the item's first tile
+        for (int k = 0; ok; k++) {
+            int w;
+            AttnItem it;
+            ok = next_item(k, w, it);
+            if (!ok || w < 0) break;
+            const int q0 = it.q0, h = it.h, tiles = it.nt - it.lo, mine = scored(T, tiles);
+            const int64_t tq = p.pos0 + q0 + row;                    // this row's position: keys 0..tq are visible
+            if (k == 0) load_query_tile<CFG, 4, false>(p, q0, h, row, wg, tlane, [&]() { arrive(PR_QFULL); });
+            float m = 0.f, l = 0.f;
+            // reference exponent of the row: its largest score of the item's first tile, which one set has. (All arrive: no P is written
+            // before the epilogue of the item before has left the P buffers.)
+            auto reference = [&]() -> bool {
+                arrive(PR_XM);
+                if (!mbar_wait(bar(PR_XM), (uint32_t)(k & 1), p.err, 1426)) return false;
+                m = fmaxf(s_m[row], s_m[128 + row]);                 // the tile shows every row a key: finite
+                return true;
+            };
+            if ((kc & 1) != set) ok = reference();
+            for (int e = (kc ^ set) & 1; e < mine && ok; e += 2) {
+                const int d = nth(T, e), i = it.lo + d, sb = (kc + e) & 1, su = (kc + e) >> 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(PR_SFULL + sb), (uint32_t)(su & 1), p.err, 1421));   // warp-uniform: the TMEM loads below are warp-wide
+                if (!ok) break;
+                tc_fence_after();
+                uint32_t v[NC];
+                TMEM_LD16(v, 0, tlane + PA_COL_S + sb * PA_KT + cg * NC);
+                TMEM_LD16(v, 16, tlane + PA_COL_S + sb * PA_KT + cg * NC + 16);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                arrive(PR_SEMPTY + sb);
+                const bool whole = (int64_t)i * PA_KT + PA_KT - 1 <= p.pos0 + q0;      // every key of the tile is visible to every row of the item
+                const int seen = (int)min(tq - (int64_t)i * PA_KT - cg * NC, (int64_t)PA_KT);      // the thread's keys 0 .. seen are visible
+                if (e == 0) {
+                    float mt = -INFINITY;
+#pragma unroll
+                    for (int j = 0; j < NC; j++) mt = fmaxf(mt, whole || j <= seen ? __uint_as_float(v[j]) * p.scale_log2 : -INFINITY);
+                    s_m[cg * 128 + row] = mt;
+                    ok = reference();
+                    if (!ok) break;
+                    if ((T & 1) != rank) continue;                   // the peer's tile
+                }
+                // exponents relative to the reference: scale, difference and below the sum two at a time
+                float s[NC];
+                const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), minus_m = pack_f32x2(-m, -m);
+#pragma unroll
+                for (int j = 0; j < NC; j += 2)
+                    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), scale2, minus_m), s[j], s[j + 1]);
+                if (!whole) {
+#pragma unroll
+                    for (int j = 0; j < NC; j++)
+                        if (j > seen) s[j] = -INFINITY;
+                }
+                float mt = s[0];
+#pragma unroll
+                for (int j = 1; j + 1 < NC; j += 2) mt = fmaxf(mt, fmaxf(s[j], s[j + 1]));
+                mt = fmaxf(mt, s[NC - 1]);
+                if (mt > PA_RANGE) {
+                    p.flags[it.flag] = 1;                            // out of the range this form covers: the exact form redoes the item
+                    atomicAdd(p.counter + 2, 1);
+                }
+                uint32_t pk[NC / 2];
+                uint64_t lsum = 0;                                   // two f32 zeros
+#pragma unroll
+                for (int j = 0; j < NC; j += 2) {
+                    const float p0 = exp2f(s[j]), p1 = exp2f(s[j + 1]);
+                    lsum = add_f32x2(lsum, pack_f32x2(p0, p1));
+                    pk[j >> 1] = pack_bf16x2(p0, p1);
+                }
+                float l0, l1;
+                unpack_f32x2(lsum, l0, l1);
+                l += l0 + l1;
+                ok = __all_sync(0xffffffffu, buffer_free(T + d));
+                if (!ok) break;
+                uint8_t *prow = sm + L::OFF_P + ((T + d) & 3) * PA_P_BYTES + row * 128;
+#pragma unroll
+                for (int c = 0; c < NC / 8; c++)
+                    *reinterpret_cast<uint4 *>(prow + (((cg * (NC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                arrive(PR_PFULL + ((T + d) & 3));
+            }
+            if (!ok) break;
+            kc += mine;
+            T += tiles;
+            {
+                // the next item's query tile: the score MMAs of this item are done with theirs (they precede its last value MMAs)
+                int wn;
+                AttnItem nx;
+                ok = next_item(k + 1, wn, nx);
+                if (!ok) break;
+                if (wn >= 0) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar(PR_QEMPTY), (uint32_t)(k & 1), p.err, 1425));
+                    if (!ok) break;
+                    tc_fence_after();
+                    load_query_tile<CFG, 4, false>(p, nx.q0, nx.h, row, wg, tlane, [&]() { arrive(PR_QFULL); });
+                }
+            }
+            // ---- the row's sum: this CTA's four groups', then the peer's
+            s_l[wg * 128 + row] = l;
+            arrive(PR_XL);
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(PR_XL), (uint32_t)(k & 1), p.err, 1427));
+            if (!ok) break;
+            if (wg == 0) {
+                s_sum[(k & 1) * 128 + row] = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (tid == 128) {
+                    mbar_expect_tx(bar(PR_PEER + (k & 1)), 512);
+                    copy_to_peer(smem_u32(s_sum + (k & 1) * 128), 512, peer_sum + (k & 1) * 512, peer_bar0 + 8u * (uint32_t)(k & 1));
+                }
+            }
+            l = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
+            // ---- epilogue of the item: O / l -> bf16 -> out[t][h][rank * 256 ..], through staging tiles in the buffers of this CTA's
+            // own P (the peer may be filling the others): free when both CTAs are done with the last two own tiles
+            ok = mbar_wait(bar(PR_PEER + (k & 1)), (uint32_t)((k >> 1) & 1), p.err, 1428);
+            if (ok) ok = mbar_wait(bar(PR_ODONE), (uint32_t)(k & 1), p.err, 1424);
+            const int next_own = T + ((T & 1) == rank ? 0 : 1);      // the own tile after this item, and the one behind it: in these buffers
+            if (ok) ok = buffer_free(next_own);
+            if (ok) ok = buffer_free(next_own + 2);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            l += s_peer[(k & 1) * 128 + row];
+            constexpr int CPG = PA_DV / 4;                           // columns per group
+            uint32_t o[CPG];
+            TMEM_LD16(o, 0, tlane + PA_COL_O + wg * CPG);
+            TMEM_LD16(o, 16, tlane + PA_COL_O + wg * CPG + 16);
+            TMEM_LD16(o, 32, tlane + PA_COL_O + wg * CPG + 32);
+            TMEM_LD16(o, 48, tlane + PA_COL_O + wg * CPG + 48);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            arrive(PR_OFREE);                                        // the value MMAs of the next item may overwrite the accumulator
+            if (it.rec >= 0) {                                       // part of an item: its record
+                float *rec = p.records + record_of<false>(it.rec, rank) * PA_RECORD;
+#pragma unroll
+                for (int j = 0; j < CPG / 4; j++)
+                    *reinterpret_cast<uint4 *>(rec + ((int64_t)(wg * (CPG / 4) + j) * PA_QT + row) * 4) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+                if (wg == 0) { rec[PA_QT * PA_DV + row] = m; rec[PA_QT * (PA_DV + 1) + row] = l; }
+                continue;
+            }
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            uint8_t *stg = sm + L::OFF_P + ((warp - 4) < 8 ? rank : rank + 2) * PA_P_BYTES + ((warp - 4) & 7) * 2048;      // 2 KB per warp: [32 rows][64 B]
+            const int t0w = q0 + q4 * 32;
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const uint32_t *x = o + u * 32 + 8 * j;
+                    uint4 wv;
+                    wv.x = pack_bf16x2(__uint_as_float(x[0]) * inv, __uint_as_float(x[1]) * inv);
+                    wv.y = pack_bf16x2(__uint_as_float(x[2]) * inv, __uint_as_float(x[3]) * inv);
+                    wv.z = pack_bf16x2(__uint_as_float(x[4]) * inv, __uint_as_float(x[5]) * inv);
+                    wv.w = pack_bf16x2(__uint_as_float(x[6]) * inv, __uint_as_float(x[7]) * inv);
+                    *reinterpret_cast<uint4 *>(stg + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = wv;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int rr = r * 8 + (lane >> 2), jj = lane & 3;
+                    const uint4 wv = *reinterpret_cast<const uint4 *>(stg + rr * 64 + ((jj ^ ((rr >> 1) & 3)) << 4));
+                    if (t0w + rr < p.n)
+                        *reinterpret_cast<uint4 *>(p.out + ((int64_t)(t0w + rr) * p.nh + h) * PA_L + rank * PA_DV + wg * CPG + u * 32 + jj * 8) = wv;
+                }
+                __syncwarp();
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                          // nothing of either CTA's is on its way to the other any more
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+// Share mode: joins the records of an item that more than one share has a part of. Grid (shares, PA_DV / 32, halves), a row per thread:
 // the blocks of share g do the item that its end is the first to cut, if there is one (a grid over all items, most of
 // which are whole, took 20 us for 512 of them). 32 columns a thread and 32-bit arithmetic on the shares: 64 items of 512 GQA
 // queries after 10488 rows, 39 MB of records, 12.8 -> 8.9 us (sixteen columns and 64-bit divisions before; asking for the next
@@ -658,8 +1106,8 @@ constexpr int PA_MC = 32;                                            // columns 
 template <bool GQA>
 __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnParams p) {
     cwk_pdl_launch();
-    const int nq = (p.n + PA_QT - 1) / PA_QT, row = threadIdx.x, c0 = (int)blockIdx.y * PA_MC;
-    const int all = p.head_tiles * p.nh * (GQA ? 1 : 2);
+    const int nq = (p.n + PA_QT - 1) / PA_QT, row = threadIdx.x, c0 = (int)blockIdx.y * PA_MC, half = blockIdx.z;
+    const int all = p.head_tiles * p.nh;
     int g = blockIdx.x;
     const int u0 = (int)share_begin(g, all, p.shares), u1 = (int)share_begin(g + 1, all, p.shares);
     int w = u1 / p.head_tiles * nq;                                  // the item with tile u1
@@ -680,7 +1128,7 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnParams p) {
         for (; g <= g1; g++) {
             AttnItem seg = it;
             if (!attn_segment(seg, w, g, at, share_begin(g, all, p.shares), share_begin(g + 1, all, p.shares), p)) continue;
-            const float *rec = p.records + (int64_t)seg.rec * PA_RECORD;
+            const float *rec = p.records + record_of<GQA>(seg.rec, half) * PA_RECORD;
 #pragma unroll
             for (int j = 0; j < PA_MC / 4; j++) v[j] = *reinterpret_cast<const float4 *>(rec + ((int64_t)(c0 / 4 + j) * PA_QT + row) * 4);
             ms = rec[PA_QT * PA_DV + row];
@@ -707,37 +1155,43 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnParams p) {
     uint32_t r[PA_MC / 2];
 #pragma unroll
     for (int j = 0; j < PA_MC / 2; j++) r[j] = pack_bf16x2(o[2 * j] * inv, o[2 * j + 1] * inv);
-    uint4 *dst = reinterpret_cast<uint4 *>(p.out + ((int64_t)(it.q0 + row) * p.nh + it.h) * (GQA ? PA_DV : PA_L) + it.half * PA_DV + c0);
+    uint4 *dst = reinterpret_cast<uint4 *>(p.out + ((int64_t)(it.q0 + row) * p.nh + it.h) * (GQA ? PA_DV : PA_L) + half * PA_DV + c0);
 #pragma unroll
     for (int j = 0; j < PA_MC / 8; j++) dst[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
 }
 
-// The attention grid of both shapes: the fast form, the repair pass, and in share mode the merge. Shares where the longest block
-// of item-by-item dealing would have more than PA_MERGE_TILES key tiles above an equal share: what the records, their merge and
-// its launch cost. Dealt and shared, us, keys and values from memory (16 query heads, 4 KV heads of 256):
+// The attention grid of both shapes: the fast form, the repair pass, and in share mode the merge. Shares where the longest block (or
+// pair) of item-by-item dealing would have more than PA_MERGE_TILES key tiles above an equal share: what the records, their merge and
+// its launch cost. GQA, dealt and shared, us, keys and values from memory (16 query heads, 4 KV heads of 256):
 //   512 queries after 1500 (19 tiles above the share) 39.5 / 45.5, after 2500 (28) 51.4 / 51.4, after 4000 (41) 68 / 60
 //   128 queries after 1500 (23) 37.0 / 41.3, after 2000 (30) 42.6 / 41.5, after 4000 (57) 66 / 45
 //   700 queries after 3000 (23) 57.1 / 62.9, after 4000 (28) 68.7 / 70.1, after 6000 (39) 91 / 86
-// and the whole MLA prompt of 64 heads: 256 queries after 4000 (17) 247 / 254, after 6000 (25) 321 / 321, after 14000 (59) 606 / 595.
-constexpr int PA_MERGE_TILES = 28;
+// MLA: more, and a quarter of the share at least: dealt out item by item, the query tiles of a head run at the same time and read its
+// keys from memory once, in shares one after the other. Up to the attention, dealt and shared (tiles above the share, of the share):
+//   64 heads: 200 queries after 6000 (26 of 164) 258 / 272, 256 after 14000 (60 of 384) 482 / 496, 300 after 20000 (127 of 815) 841 / 867
+//   48 heads: 128 after 3000 (17 of 32) 131 / 138, 128 after 8000 (45 of 82) 228 / 221, 256 after 8000 (90 of 166) 303 / 280
+//   32 heads: 128 after 3000 (28 of 21) 112 / 115, 128 after 8000 (72 of 55) 184 / 162;  16: 128 after 3000 (38 of 11) 97 / 99, 256 after 8000 (73 of 56) 156 / 137
+constexpr int PA_MERGE_TILES = 28, PR_MERGE_TILES = 40;
 template <class CFG, bool GQA>
 int attn_launch(cwk_ctx *ctx, AttnParams ap, const CUtensorMap &tm_k, const CUtensorMap &tm_c, int exact_only) {
     static bool attr_set[16] = {false};
     if (!attr_set[ctx->device & 15]) {
         CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<1, CFG, GQA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM));
-        CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<4, CFG, GQA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM));
+        if constexpr (GQA) CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_kernel<4, CFG, GQA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM));
+        else CWK_CUDA(ctx, cudaFuncSetAttribute(prefill_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PrCfg<CFG>::SMEM));
         attr_set[ctx->device & 15] = true;
     }
-    const int nq = (ap.n + PA_QT - 1) / PA_QT, heads = ap.nh * (GQA ? 1 : 2), total = nq * heads, G = ctx->sm_count;
+    constexpr int H = GQA ? 1 : 2;                                   // blocks that work on an item together
+    const int nq = (ap.n + PA_QT - 1) / PA_QT, total = nq * ap.nh, G = ctx->sm_count / H;
     auto tiles = [&](int qtile) { return (ap.pos0 + std::min((int64_t)(qtile + 1) * PA_QT, (int64_t)ap.n) - 1) / PA_KT + 1; };
     int64_t head_tiles = 0;
     for (int i = 0; i < nq; i++) head_tiles += tiles(i);
-    const int64_t all = head_tiles * heads, share = (all + G - 1) / G, waves = (total + G - 1) / G;
+    const int64_t all = head_tiles * ap.nh, share = (all + G - 1) / G, waves = (total + G - 1) / G;
     // one by one: the idle places of the last round are at least the shortest item each
     const int64_t one_by_one = std::max(tiles(nq - 1), share + (waves * G - total) * tiles(0) / G);
     ap.shares = 0; ap.records = nullptr; ap.head_tiles = (int)head_tiles;
-    if (one_by_one > share + PA_MERGE_TILES && share >= 2 && all < (1LL << 31)) {
-        const int s = cwk_reserve_scratch(ctx, (size_t)2 * G * PA_RECORD * sizeof(float));
+    if (one_by_one > share + (GQA ? (int64_t)PA_MERGE_TILES : std::max<int64_t>(PR_MERGE_TILES, share / 4)) && share >= 2 && all < (1LL << 31)) {
+        const int s = cwk_reserve_scratch(ctx, (size_t)2 * H * G * PA_RECORD * sizeof(float));
         if (s != CWK_OK) return s;
         ap.shares = G; ap.records = ctx->scratch;
     }
@@ -748,17 +1202,18 @@ int attn_launch(cwk_ctx *ctx, AttnParams ap, const CUtensorMap &tm_k, const CUte
         CWK_CUDA(ctx, cudaMemsetAsync(ap.flags, 1, (size_t)(nflags + 3) * sizeof(int), ctx->stream));
         CWK_CUDA(ctx, cudaMemsetAsync(ap.counter, 0, 2 * sizeof(int), ctx->stream));
     }
-    const int grid = ap.shares ? G : std::min(total, G);
     if (!exact_only) {
         CwkKernelTimer timer(ctx);
-        CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<4, CFG, GQA>, dim3(grid), dim3(PA_THREADS<4>), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
-        CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<4>");
+        const int grid = H * (ap.shares ? G : std::min(total, G));
+        if constexpr (GQA) CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<4, CFG, GQA>, dim3(grid), dim3(PA_THREADS<4>), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
+        else CWK_CUDA(ctx, cwk_launch_early(prefill_pair_kernel, dim3(grid), dim3(PR_THREADS), PrCfg<CFG>::SMEM, ctx->stream, tm_k, tm_c, ap));
+        CWK_LAUNCH_CHECK(ctx, "prefill attention");
     }
     // the repair pass: items whose flag is clear are skipped
-    CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<1, CFG, GQA>, dim3(grid), dim3(PA_THREADS<1>), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
+    CWK_CUDA(ctx, cwk_launch_early(prefill_attn_kernel<1, CFG, GQA>, dim3(ap.shares ? H * G : std::min(H * total, ctx->sm_count)), dim3(PA_THREADS<1>), CFG::SMEM, ctx->stream, tm_k, tm_c, ap));
     CWK_LAUNCH_CHECK(ctx, "prefill_attn_kernel<1>");
     if (ap.shares) {
-        CWK_CUDA(ctx, cwk_launch_early(attn_merge_kernel<GQA>, dim3(ap.shares, PA_DV / PA_MC), dim3(128), 0, ctx->stream, ap));
+        CWK_CUDA(ctx, cwk_launch_early(attn_merge_kernel<GQA>, dim3(ap.shares, PA_DV / PA_MC, H), dim3(128), 0, ctx->stream, ap));
         CWK_LAUNCH_CHECK(ctx, "attn_merge_kernel");
     }
     return CWK_OK;

@@ -221,3 +221,23 @@ def test_short_chunks_on_both_routes(attn, n, pos0, nh):
     close(bf16_to_np(got), want)
     close(bf16_to_np(other), want)
     close(bf16_to_np(gcache), bf16_to_np(ocache))
+
+
+@pytest.mark.parametrize("n,pos0", [(200, 6000), (256, 8000)])
+def test_few_heads_in_shares(attn, n, pos0):
+    """16 heads leave most of the pairs of blocks without an item: the key tiles are dealt out in shares and the parts joined.
+    Against the oracle, and with scores beyond the fast form's range (the flagged parts are redone) against the exact form."""
+    nh, H, q_lora = 16, 512, 256
+    m = make_model(71, H, q_lora, nh)
+    X = synth.normal_bf16(71, 9, (n, H))
+    cache0 = np.zeros((pos0 + n, LAT + ROPE), np.uint16)
+    cache0[:pos0] = synth.normal_bf16(71, 10, (pos0, LAT + ROPE))
+    rows = np.array([0, 127, 128, n - 1])
+    got, _ = run_gpu(attn, m, X, cache0, pos0, nh)
+    want, _ = run_oracle(m, X, cache0, pos0, nh, rows)
+    close(bf16_to_np(got)[rows], want)
+    m["Sqb"] = (m["Sqb"] * np.float32(400.0)).astype(np.float32)
+    got, _ = run_gpu(attn, m, X, cache0, pos0, nh)
+    exact, _ = _forced(attn, 3, lambda: run_gpu(attn, m, X, cache0, pos0, nh))
+    assert np.isfinite(bf16_to_np(got)).all()
+    close(bf16_to_np(got), bf16_to_np(exact))
