@@ -903,7 +903,7 @@ int token_chain(cwk_ctx *ctx, Layer &ly, int64_t pos, const float *d_x, float *d
     int nsplit = 0;
     const int s = cwk_mla_launch_splits(ctx, d_qabs, ly.cm->dev, kv_lora, (int)(pos + 1), nh, kv_lora, 0, 1.0f / sqrtf((float)nope), &partial, &nsplit, false);
     if (s != CWK_OK) return s;
-    CWK_CUDA(ctx, cwk_launch_early(merge_unabsorb_kernel, dim3(nh, 2), dim3(512), 0, ctx->stream, (const float *)partial, nsplit, nh, (const uint16_t *)ly.kvb->data, nope,
+    CWK_CUDA(ctx, cwk_launch_early(nsplit > 32 ? merge_unabsorb_kernel<36> : merge_unabsorb_kernel<16>, dim3(nh, 2), dim3(512), 0, ctx->stream, (const float *)partial, nsplit, nh, (const uint16_t *)ly.kvb->data, nope,
                                    d_attn));
     ctx->launches += 2;
     in = TokenInput{};

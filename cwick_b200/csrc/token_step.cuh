@@ -66,15 +66,27 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 2) gemv_token_kernel(const void
         }
     };
     ask();
+    constexpr int NW = 4;                                  // activations at a time, and norm weights asked for ahead
+    uint16_t nw[NW];
+    if (XIN == X_NORM) {
+#pragma unroll
+        for (int u = 0; u < NW; u++) nw[u] = threadIdx.x + u * 32 * TG_WARPS < k ? in.w[threadIdx.x + u * 32 * TG_WARPS] : (uint16_t)0;
+    }
     cwk_pdl_wait();
     const float *x = in.x;
     if (XIN == X_NORM) {
         __shared__ double s_ss[TG_WARPS];
         double ss = 0.0;
-        for (int i = threadIdx.x; i < k; i += 32 * TG_WARPS) {
-            const float f = x[i];
-            s_x[i] = f;                                    // (each thread scales what it wrote)
-            ss += (double)f * (double)f;
+        for (int i = threadIdx.x; i < k; i += NW * 32 * TG_WARPS) {
+            float f[NW];
+#pragma unroll
+            for (int u = 0; u < NW; u++) f[u] = i + u * 32 * TG_WARPS < k ? x[i + u * 32 * TG_WARPS] : 0.f;
+#pragma unroll
+            for (int u = 0; u < NW; u++)
+                if (i + u * 32 * TG_WARPS < k) {
+                    s_x[i + u * 32 * TG_WARPS] = f[u];     // (each thread scales what it wrote)
+                    ss += (double)f[u] * (double)f[u];
+                }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -84,15 +96,28 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 2) gemv_token_kernel(const void
 #pragma unroll
         for (int o = TG_WARPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
         const float inv = __fdiv_rn(1.0f, (float)sqrt(tot / (double)k + (double)in.eps));
-        for (int i = threadIdx.x; i < k; i += 32 * TG_WARPS) s_x[i] = s_x[i] * inv * bf16_bits_to_f32(in.w[i]);
+#pragma unroll
+        for (int u = 0; u < NW; u++) {
+            const int i = threadIdx.x + u * 32 * TG_WARPS;
+            if (i < k) s_x[i] = s_x[i] * inv * bf16_bits_to_f32(nw[u]);
+        }
+        for (int i = threadIdx.x + NW * 32 * TG_WARPS; i < k; i += 32 * TG_WARPS) s_x[i] = s_x[i] * inv * bf16_bits_to_f32(in.w[i]);
         __syncthreads();
         x = s_x;
     } else if (XIN == X_SUM) {
-        for (int i = threadIdx.x * 4; i < k; i += 128 * TG_WARPS) {
-            float4 a = *reinterpret_cast<const float4 *>(x + i);
-            const float4 b = *reinterpret_cast<const float4 *>(in.x2 + i);
-            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-            *reinterpret_cast<float4 *>(s_x + i) = a;
+        for (int i = threadIdx.x * 4; i < k; i += 2 * 128 * TG_WARPS) {      // two pieces of both at a time
+            const bool two = i + 128 * TG_WARPS < k;
+            float4 a[2], b[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                if (u == 0 || two) {
+                    a[u] = *reinterpret_cast<const float4 *>(x + i + u * 128 * TG_WARPS);
+                    b[u] = *reinterpret_cast<const float4 *>(in.x2 + i + u * 128 * TG_WARPS);
+                }
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                if (u == 0 || two)
+                    *reinterpret_cast<float4 *>(s_x + i + u * 128 * TG_WARPS) = make_float4(a[u].x + b[u].x, a[u].y + b[u].y, a[u].z + b[u].z, a[u].w + b[u].w);
         }
         __syncthreads();
         x = s_x;
@@ -209,9 +234,12 @@ __global__ void __launch_bounds__(512) absorb_token_kernel(const float *q, const
 // result, rounded to bf16 as the merge on its own would leave it, taken through W_v (src/attention.c:812-815): grid (heads,
 // 2), 512 threads. A block merges 256 of its head's 512 columns, two threads a column (each half of the records), and forms
 // those columns' part of the head's 128 values, eight per warp, whose weights are on their way before the records are
-// there; attn [2][heads][128] has the two parts, added up by the next projection.
-__global__ void __launch_bounds__(512, 2) merge_unabsorb_kernel(const float *partial, int nsplit, int nh, const uint16_t *kvb, int nope, float *attn) {
-    constexpr int L = 512, VD = 128, AHEAD = 16;
+// there; attn [2][heads][128] has the two parts, added up by the next projection. The kernel is one block per SM and trips to L2, so
+// where the records are more than 32 a thread asks for 36 at once, all of its half for 9216 rows: a call over 8191 rows 84 -> 75 us
+// (16 at a time for every number, in registers for two blocks that there never are; at 1000 rows, 8 records, 16 are 1 us ahead).
+template <int AHEAD>
+__global__ void __launch_bounds__(512, AHEAD > 16 ? 1 : 2) merge_unabsorb_kernel(const float *partial, int nsplit, int nh, const uint16_t *kvb, int nope, float *attn) {
+    constexpr int L = 512, VD = 128;
     __shared__ float s_w[512], s_red[32], s_half[256];
     __shared__ __align__(16) float s_c[256];
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c0 = blockIdx.y * 256;
