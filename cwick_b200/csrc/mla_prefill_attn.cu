@@ -590,7 +590,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             }
             // All groups write out (two of four, 64 columns at a time: 12 k cycles an item with the next query's copy; now 8 k)
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            uint8_t *stg = sm + PA_OFF_P + (warp - 4) * 2048;         // 2 KB per warp: [32 rows][64 B], in the P buffers (idle: the item's value MMAs are done, and the next item's P comes from these threads)
+            // 2 KB per warp, [32 rows][64 B], in the P buffers: the item's value MMAs are done, and the next item's P is written behind
+            // reference(), where all meet. The exact form's warps meet nowhere: each stages in the place of its own rows' P, which
+            // no other warp writes.
+            uint8_t *stg = sm + PA_OFF_P + (warp - 4) * (NWG == 4 ? 2048 : 32 * 128);
             const int t0w = q0 + q4 * 32;
             constexpr int NCH = PA_DV / 64 / NWG;                     // 64-column chunks per thread
 #pragma unroll 1

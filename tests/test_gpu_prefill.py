@@ -167,6 +167,22 @@ def test_scores_out_of_the_fast_forms_range_are_repaired(attn):
     close(g, e)
 
 
+def test_repaired_items_are_the_same_every_time(attn):
+    """The exact form's warps go from one item to the next on their own, and stage their output in shared memory that holds the next item's
+    probabilities: a hundred runs of the case above (most items repaired, several per block), bit for bit. (With a warp's staging in another
+    warp's rows one run in thirty differed.)"""
+    n, nh, H, q_lora = 300, 64, 512, 256
+    m = make_model(43, H, q_lora, nh)
+    m["Sqb"] = (m["Sqb"] * np.float32(400.0)).astype(np.float32)
+    X = synth.normal_bf16(43, 9, (n, H))
+    dev = {k: (torch.from_numpy(v).cuda() if v.dtype != np.uint16 else to_bf16_cuda(v)) for k, v in m.items()}
+    Xd, cache = to_bf16_cuda(X), torch.zeros(n, LAT + ROPE, dtype=torch.bfloat16, device="cuda")
+    outs = [attn.mla_prefill(Xd, dev["Wqa"], dev["Sqa"], dev["Wqb"], dev["Sqb"], dev["Wkva"], dev["Skva"], dev["qa_n"], dev["kva_n"], dev["Wuk"],
+                             cache, 0, nh) for _ in range(100)]
+    attn.ctx.sync()
+    assert all(torch.equal(o, outs[0]) for o in outs)
+
+
 def test_absorbed_route_agrees_with_the_expanded_key_route(attn):
     """The two attention routes of the prefill (queries as MMA rows against expanded keys; the decode
     kernel once per query row against the latent) give the same output within the tolerance, on a chunk
