@@ -114,6 +114,14 @@ struct CwkKernelTimer {
         if (_s != CWK_OK) return _s;                                   \
     } while (0)
 
+// What the FP8 GEMM leaves of output tiles (CWK_FP8_TILE square, numbered column tile * tiles_m + row tile) that it cut along K: from tile
+// `full` on, `splits` f32 tiles each to be added up in order. part == NULL: nothing is left, all sums are in Y.
+constexpr int CWK_FP8_TILE = 256;
+struct CwkFp8Parts {
+    const float *part;
+    int full, splits, tiles_m, tiles_a;                      // tiles_a: column tiles of the first of two projections
+};
+
 // ---- kernels of a decode step that may start before the one in front of them is done -----------------------------------
 // A decode step at small batch is a chain of kernels of a few microseconds, and half as much again is the time from one
 // kernel's end to the next one's first instruction. Launched this way, a kernel's blocks come up while the kernel before

@@ -32,7 +32,7 @@
 
 namespace {
 
-constexpr int BM = 256, BN = 256, BK = 128;
+constexpr int BM = CWK_FP8_TILE, BN = CWK_FP8_TILE, BK = 128;
 constexpr int STAGES = 3;
 constexpr int A_BYTES = BM / 2 * BK * 2, B_BYTES = BN / 2 * BK * 2;   // 32 KB + 32 KB per CTA
 constexpr int G_OFF_STG = STAGES * (A_BYTES + B_BYTES);          // 196608: eight 4 KB staging tiles of the epilogue
@@ -403,9 +403,10 @@ static int encode_weight_map(cwk_ctx *ctx, const void *dst_c, int64_t cols, int6
     return CWK_OK;
 }
 
-// Y1 = X . W1^T (block-scaled), and, when W2 is given, Y2 = X . W2^T in the same launch.
+// Y1 = X . W1^T (block-scaled), and, when W2 is given, Y2 = X . W2^T in the same launch. left: where the parts of the tiles that were
+// cut along K are, for a caller whose next kernel adds them up itself (NULL: added up here). They stay until the stream's next launch after that kernel.
 int cwk_fp8_linear_tc_launch2(cwk_ctx *ctx, const void *X, int64_t n, int64_t k, const void *W1, const float *scale1, int64_t cols1,
-                              void *Y1, int out_bf16_1, const void *W2, const float *scale2, int64_t cols2, void *Y2, int out_bf16_2) {
+                              void *Y1, int out_bf16_1, const void *W2, const float *scale2, int64_t cols2, void *Y2, int out_bf16_2, CwkFp8Parts *left) {
     // vector stores in the epilogue want 16-byte aligned rows
     if ((cols1 % 8) != 0 || (k % 128) != 0 || ((uintptr_t)Y1 % 16) != 0 || ((uintptr_t)X % 16) != 0 ||
         (W2 && ((cols2 % 8) != 0 || ((uintptr_t)Y2 % 16) != 0)))
@@ -475,7 +476,8 @@ int cwk_fp8_linear_tc_launch2(cwk_ctx *ctx, const void *X, int64_t n, int64_t k,
     CwkKernelTimer timer(ctx);
     CWK_CUDA(ctx, cwk_launch_early(fp8_linear_tc_kernel, dim3(2 * std::min(units, pairs)), dim3(G_THREADS), G_SMEM, ctx->stream, tm_x, tm_w, tm_w2, p));
     CWK_LAUNCH_CHECK(ctx, "fp8_linear_tc_kernel");
-    if (p.splits > 1) {
+    if (left) *left = CwkFp8Parts{p.part, p.full, p.splits, p.tiles_m, p.tiles_a};
+    else if (p.splits > 1) {
         CWK_CUDA(ctx, cwk_launch_early(fp8_sum_parts_kernel, dim3(BM / 4, (unsigned)rest), dim3(256), 0, ctx->stream, p));
         CWK_LAUNCH_CHECK(ctx, "fp8_sum_parts_kernel");
     }
@@ -484,5 +486,5 @@ int cwk_fp8_linear_tc_launch2(cwk_ctx *ctx, const void *X, int64_t n, int64_t k,
 
 int cwk_fp8_linear_tc_launch(cwk_ctx *ctx, const void *X, const void *W, const float *scale_inv, int64_t n, int64_t k,
                              int64_t cols, void *Y, int out_bf16) {
-    return cwk_fp8_linear_tc_launch2(ctx, X, n, k, W, scale_inv, cols, Y, out_bf16, nullptr, nullptr, 0, nullptr, 0);
+    return cwk_fp8_linear_tc_launch2(ctx, X, n, k, W, scale_inv, cols, Y, out_bf16, nullptr, nullptr, 0, nullptr, 0, nullptr);
 }

@@ -37,7 +37,7 @@ extern "C" int cwk_fp8_linear(cwk_ctx *ctx, const void *X, const void *W, const 
                               int64_t k, int64_t cols, void *Y, int out_bf16);
 bool cwk_fp8_linear_tc_available();
 int cwk_fp8_linear_tc_launch2(cwk_ctx *ctx, const void *X, int64_t n, int64_t k, const void *W1, const float *scale1, int64_t cols1,
-                              void *Y1, int out_bf16_1, const void *W2, const float *scale2, int64_t cols2, void *Y2, int out_bf16_2);
+                              void *Y1, int out_bf16_1, const void *W2, const float *scale2, int64_t cols2, void *Y2, int out_bf16_2, CwkFp8Parts *left);
 extern "C" int cwk_mla_decode(cwk_ctx *ctx, const void *q, const void *cache, int64_t seq_stride, int64_t ld,
                               const int32_t *kv_len, int max_kv_len, const int32_t *sel, int64_t sel_ld, int B,
                               int nh, int L, int R, float scale, void *out, int n_splits);
@@ -87,31 +87,83 @@ __global__ void __launch_bounds__(256) norm_rope_rows_kernel(const float *in, in
 // The same, one WARP per row, for rows whose normalised part is a multiple of 128 columns (at most 128 * MAXV4) and whose
 // rope part is at most 64 columns: a lane keeps its 16-byte pieces of the row in registers, so the row is read once;
 // the sum of squares goes through lane-wise doubles and five shuffles, with no shared memory and no block barrier.
-// 4096 rows are 4096 warps, all resident at once: the call takes about one row's latency. rot: where each row's (cos, sin) of
-// its rope pairs go as well, for the queries of the same positions (NULL: nowhere).
-template <int MAXV4>
-__global__ void __launch_bounds__(256) norm_rope_rows_warp_kernel(const float *in, int64_t in_ld, int norm_cols, int rope_cols,
-                                                                  const uint16_t *weight, float eps, float rope_base, int64_t pos0,
-                                                                  uint16_t *out, int64_t out_ld, int *kv_len_out, int ref_narrow,
-                                                                  int64_t nrows, float2 *rot) {
+// One launch does the q_a rows and the kv_a rows (b; half of the grid each), and adds up the parts that their GEMM left of tiles that
+// it cut along K, in the order of fp8_sum_parts_kernel, a part of the whole row in flight at a time: latency bounds it, and three kernels one
+// after another (sum, q norm, kv norm, the last behind q_b) waited for their loads three times.
+// Alone with cold caches, 509 tokens: 8.8 + 10.5 + 8.4 -> 13.3 us, 4096 tokens (no parts): 15.4 + 11.6 -> 17.1; the whole prompt of 509 after 3001
+// 331.3 -> 327.2 us, and 324.5 with the angles formed before the wait; 4096 at the power cap, no difference. Four rows a block: 509 rows are 256 blocks.
+// rot: where each row's (cos, sin) of its rope pairs go as well, for the queries of the same positions (NULL: nowhere).
+struct NormRows {
+    const float *in;
+    int64_t in_ld;
+    int norm_cols, rope_cols;
+    const uint16_t *weight;
+    uint16_t *out;
+    int64_t out_ld;
+    int *kv_len_out;
+    int ref_narrow, tile0;                                   // tile0: the rows' first column tile in the GEMM that made them
+    float2 *rot;
+};
+
+template <int MAXV4, bool PARTS>
+__global__ void __launch_bounds__(128) norm_rope_rows_warp_kernel(const NormRows a, const NormRows b, const CwkFp8Parts parts, float eps,
+                                                                  float rope_base, int64_t pos0, int64_t nrows, int blocks) {
     const int lane = threadIdx.x & 31;
-    const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const bool second = (int)blockIdx.x >= blocks;
+    const NormRows &w = second ? b : a;
+    const int64_t r = (int64_t)((int)blockIdx.x - (second ? blocks : 0)) * 4 + (threadIdx.x >> 5);
     if (r >= nrows) return;
-    const float *x = in + r * in_ld;
-    const int np = norm_cols / 128;
+    const int np = w.norm_cols / 128, nrope = w.rope_cols;
+    // a column tile's place for this row: the first of its parts, or NULL where the GEMM wrote the sums
+    const int tm = (int)(r / CWK_FP8_TILE);
+    auto cut = [&](int col) -> const float * {
+        const int tile = PARTS ? (w.tile0 + col / CWK_FP8_TILE) * parts.tiles_m + tm - parts.full : -1;
+        if (tile < 0) return nullptr;
+        return parts.part + (int64_t)tile * parts.splits * (CWK_FP8_TILE * CWK_FP8_TILE) + (int)(r % CWK_FP8_TILE) * CWK_FP8_TILE + col % CWK_FP8_TILE;
+    };
+    const float *x = w.in + r * w.in_ld;
     cwk_pdl_launch();
+    float sn = 0.f, cs = 0.f;                                // the angle needs no input: formed under the GEMM's last tiles
+    if (lane < nrope / 2) rope_cos_sin(pos0 + r, lane, nrope, rope_base, cs, sn);
     cwk_pdl_wait();
     float4 v[MAXV4];
-    float ra = 0.f, rb = 0.f;
-    if (lane < rope_cols / 2) {
-        const float2 ab = *reinterpret_cast<const float2 *>(x + norm_cols + 2 * lane);
-        ra = ab.x; rb = ab.y;
+    float2 ab = make_float2(0.f, 0.f);
+    if (lane < nrope / 2) {
+        const float *p = cut(w.norm_cols + 2 * lane);
+        ab = *reinterpret_cast<const float2 *>(p ? p : x + w.norm_cols + 2 * lane);
+    }
+#pragma unroll
+    for (int c = 0; c < MAXV4; c++)
+        if (c < np) {
+            const float *p = cut(c * 128 + lane * 4);
+            v[c] = *reinterpret_cast<const float4 *>(p ? p : x + c * 128 + lane * 4);
+        }
+    if (PARTS) {
+        for (int s = 1; s < parts.splits; s++) {
+            const int64_t off = (int64_t)s * (CWK_FP8_TILE * CWK_FP8_TILE);
+            float4 t[MAXV4];
+            float2 tr = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < MAXV4; c++) {
+                t[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c < np) {
+                    const float *p = cut(c * 128 + lane * 4);
+                    if (p) t[c] = *reinterpret_cast<const float4 *>(p + off);
+                }
+            }
+            if (lane < nrope / 2) {
+                const float *p = cut(w.norm_cols + 2 * lane);
+                if (p) tr = *reinterpret_cast<const float2 *>(p + off);
+            }
+#pragma unroll
+            for (int c = 0; c < MAXV4; c++) { v[c].x += t[c].x; v[c].y += t[c].y; v[c].z += t[c].z; v[c].w += t[c].w; }
+            ab.x += tr.x; ab.y += tr.y;
+        }
     }
     double ss = 0.0;
 #pragma unroll
     for (int c = 0; c < MAXV4; c++)
         if (c < np) {
-            v[c] = *reinterpret_cast<const float4 *>(x + c * 128 + lane * 4);
             ss += (double)v[c].x * (double)v[c].x;
             ss += (double)v[c].y * (double)v[c].y;
             ss += (double)v[c].z * (double)v[c].z;
@@ -119,16 +171,16 @@ __global__ void __launch_bounds__(256) norm_rope_rows_warp_kernel(const float *i
         }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float inv = __fdiv_rn(1.0f, (float)sqrt(ss / (double)norm_cols + (double)eps));
-    uint16_t *y = out + r * out_ld;
+    const float inv = __fdiv_rn(1.0f, (float)sqrt(ss / (double)w.norm_cols + (double)eps));
+    uint16_t *y = w.out + r * w.out_ld;
 #pragma unroll
     for (int c = 0; c < MAXV4; c++)
         if (c < np) {
-            const uint2 wb = *reinterpret_cast<const uint2 *>(weight + c * 128 + lane * 4);
+            const uint2 wb = *reinterpret_cast<const uint2 *>(w.weight + c * 128 + lane * 4);
             const float o0 = v[c].x * inv * __uint_as_float(wb.x << 16), o1 = v[c].y * inv * __uint_as_float(wb.x & 0xffff0000u);
             const float o2 = v[c].z * inv * __uint_as_float(wb.y << 16), o3 = v[c].w * inv * __uint_as_float(wb.y & 0xffff0000u);
             uint2 pk;
-            if (ref_narrow) {
+            if (w.ref_narrow) {
                 pk.x = (uint32_t)narrow_bf16_like_reference(o0) | ((uint32_t)narrow_bf16_like_reference(o1) << 16);
                 pk.y = (uint32_t)narrow_bf16_like_reference(o2) | ((uint32_t)narrow_bf16_like_reference(o3) << 16);
             } else {
@@ -137,15 +189,13 @@ __global__ void __launch_bounds__(256) norm_rope_rows_warp_kernel(const float *i
             }
             *reinterpret_cast<uint2 *>(y + c * 128 + lane * 4) = pk;
         }
-    if (lane < rope_cols / 2) {
-        float sn, cs;
-        rope_cos_sin(pos0 + r, lane, rope_cols, rope_base, cs, sn);
-        const float r0 = ra * cs - rb * sn, r1 = rb * cs + ra * sn;
-        if (rot) rot[r * (rope_cols / 2) + lane] = make_float2(cs, sn);
-        *reinterpret_cast<uint32_t *>(y + norm_cols + 2 * lane) =
-            ref_narrow ? ((uint32_t)narrow_bf16_like_reference(r0) | ((uint32_t)narrow_bf16_like_reference(r1) << 16)) : pack_bf16x2(r0, r1);
+    if (lane < nrope / 2) {
+        const float r0 = fmaf(ab.x, cs, -(ab.y * sn)), r1 = fmaf(ab.x, sn, ab.y * cs);
+        if (w.rot) w.rot[r * (nrope / 2) + lane] = make_float2(cs, sn);
+        *reinterpret_cast<uint32_t *>(y + w.norm_cols + 2 * lane) =
+            w.ref_narrow ? ((uint32_t)narrow_bf16_like_reference(r0) | ((uint32_t)narrow_bf16_like_reference(r1) << 16)) : pack_bf16x2(r0, r1);
     }
-    if (kv_len_out && lane == 0) kv_len_out[r] = (int)(pos0 + r + 1);
+    if (w.kv_len_out && lane == 0) w.kv_len_out[r] = (int)(pos0 + r + 1);
 }
 
 static bool norm_rope_warp_ok(const float *in, int64_t in_ld, int norm_cols, int rope_cols, const void *weight, const void *out, int64_t out_ld) {
@@ -334,20 +384,28 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
     int32_t *len = (int32_t *)(w + b_qa + b_qan + b_kva + b_q + b_qf);
     float *rot = (float *)(w + b_qa + b_qan + b_kva + b_q + b_qf + up(b_len));
 
-    // q_a and kv_a share the activations: one launch of the tensor-core GEMM when it takes the shapes
+    // q_a and kv_a share the activations: one launch of the tensor-core GEMM when it takes the shapes, and one of both norms behind it
+    uint16_t *rows = (uint16_t *)cache + pos0 * row;
+    const bool q_warp = norm_rope_warp_ok(QA, q_lora, q_lora, 0, qa_norm, QAn, q_lora), kv_warp = norm_rope_warp_ok(KVA, row, kv_lora, rope, kva_norm, rows, row);
+    const bool rotated_later = expanded_keys && cwk_mla_prefill_attn_tc_ok(Q, cache, Wuk, Qf, out) && kv_warp;
+    const NormRows nq{QA, q_lora, q_lora, 0, (const uint16_t *)qa_norm, QAn, q_lora, nullptr, 0, 0, nullptr};
+    NormRows nkv{KVA, row, kv_lora, rope, (const uint16_t *)kva_norm, rows, row, len, 1, 0, rotated_later ? (float2 *)rot : nullptr};
+    const int nb = (n + 3) / 4;
+    CwkFp8Parts parts{};
     bool kva_done = false;
     s = CWK_ERR_UNSUPPORTED;
     if (cwk_fp8_linear_tc_available() && ctx->force_mla_path != 0 && ctx->force_mla_path != 1 && H % 128 == 0 && q_lora % 8 == 0 &&
         row % 8 == 0 && ((uintptr_t)X % 16) == 0) {
-        s = cwk_fp8_linear_tc_launch2(ctx, X, n, H, Wqa, Sqa, q_lora, QA, 0, Wkva, Skva, row, KVA, 0);
+        s = cwk_fp8_linear_tc_launch2(ctx, X, n, H, Wqa, Sqa, q_lora, QA, 0, Wkva, Skva, row, KVA, 0, q_warp && kv_warp ? &parts : nullptr);
         if (s == CWK_OK) kva_done = true;
         else if (s != CWK_ERR_UNSUPPORTED) return s;
     }
+    const bool both = kva_done && q_warp && kv_warp;
     if (!kva_done) s = cwk_fp8_linear(ctx, X, Wqa, Sqa, n, H, q_lora, QA, 0);
     if (s != CWK_OK) return s;
-    if (norm_rope_warp_ok(QA, q_lora, q_lora, 0, qa_norm, QAn, q_lora))
-        CWK_CUDA(ctx, cwk_launch_early(norm_rope_rows_warp_kernel<12>, dim3((n + 7) / 8), dim3(256), 0, ctx->stream, QA, q_lora, q_lora, 0,
-                                       (const uint16_t *)qa_norm, eps, rope_base, pos0, QAn, q_lora, nullptr, 0, n, nullptr));
+    if (both) nkv.tile0 = parts.tiles_a;
+    if (q_warp)
+        CWK_CUDA(ctx, cwk_launch_early(parts.part ? norm_rope_rows_warp_kernel<12, true> : norm_rope_rows_warp_kernel<12, false>, dim3(both ? 2 * nb : nb), dim3(128), 0, ctx->stream, nq, nkv, parts, eps, rope_base, pos0, (int64_t)n, nb));
     else
         norm_rope_rows_kernel<<<n, 256, 0, ctx->stream>>>(QA, q_lora, q_lora, 0, (const uint16_t *)qa_norm, eps, rope_base,
                                                           pos0, QAn, q_lora, nullptr, 0);
@@ -358,14 +416,13 @@ extern "C" int cwk_mla_prefill(cwk_ctx *ctx, const void *X, const void *Wqa, con
         s = cwk_fp8_linear(ctx, X, Wkva, Skva, n, H, row, KVA, 0);
         if (s != CWK_OK) return s;
     }
-    const bool rotated_later = expanded_keys && cwk_mla_prefill_attn_tc_ok(Q, cache, Wuk, Qf, out) && norm_rope_warp_ok(KVA, row, kv_lora, rope, kva_norm, (uint16_t *)cache + pos0 * row, row);
-    if (norm_rope_warp_ok(KVA, row, kv_lora, rope, kva_norm, (uint16_t *)cache + pos0 * row, row))
-        CWK_CUDA(ctx, cwk_launch_early(norm_rope_rows_warp_kernel<12>, dim3((n + 7) / 8), dim3(256), 0, ctx->stream, KVA, row, kv_lora, rope,
-                                       (const uint16_t *)kva_norm, eps, rope_base, pos0, (uint16_t *)cache + pos0 * row, row, len, 1, n, rotated_later ? (float2 *)rot : nullptr));
-    else
-        norm_rope_rows_kernel<<<n, 256, 0, ctx->stream>>>(KVA, row, kv_lora, rope, (const uint16_t *)kva_norm, eps, rope_base,
-                                                          pos0, (uint16_t *)cache + pos0 * row, row, len, 1);
-    CWK_LAUNCH_CHECK(ctx, "norm_rope_rows_kernel(kv_a)");
+    if (!both) {
+        if (kv_warp)
+            CWK_CUDA(ctx, cwk_launch_early(norm_rope_rows_warp_kernel<12, false>, dim3(nb), dim3(128), 0, ctx->stream, nkv, nkv, parts, eps, rope_base, pos0, (int64_t)n, nb));
+        else
+            norm_rope_rows_kernel<<<n, 256, 0, ctx->stream>>>(KVA, row, kv_lora, rope, (const uint16_t *)kva_norm, eps, rope_base, pos0, rows, row, len, 1);
+        CWK_LAUNCH_CHECK(ctx, "norm_rope_rows_kernel(kv_a)");
+    }
     if (expanded_keys && cwk_mla_prefill_attn_tc_ok(Q, cache, Wuk, Qf, out)) {
         if (!rotated_later) {
             CWK_CUDA(ctx, cwk_launch_early(rope_q_inplace_kernel, dim3((n * (rope / 2) + 255) / 256, nh >= 8 ? 4 : 1), dim3(256), 0, ctx->stream, Q, n, nh, nope, rope, pos0, rope_base));

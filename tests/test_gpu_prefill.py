@@ -257,3 +257,27 @@ def test_few_heads_in_shares(attn, n, pos0):
     exact, _ = _forced(attn, 3, lambda: run_gpu(attn, m, X, cache0, pos0, nh))
     assert np.isfinite(bf16_to_np(got)).all()
     close(bf16_to_np(got), bf16_to_np(exact))
+
+
+@pytest.mark.parametrize("n,pos0", [(1, 3), (255, 0), (257, 64), (1030, 5), (2305, 0)])
+def test_norm_adds_up_the_parts_of_cut_tiles(attn, n, pos0):
+    """The norms behind q_a and kv_a add up the tiles that their GEMM cut along K: all of them (up to two row tiles and five), or some (2305
+    tokens are 90 tiles: a wave of 74 whole, then the columns of kv_a from a row tile in their middle on). Cache rows against float64:
+    the reference's narrowing takes less than a bf16 step (2^-7 relative) off; the f32 sums of 2048 products are within 2^-24 * 16 blocks of
+    their magnitude (2^-20 * 4), and an angle of up to 2305 in f32 is off by 2^-24 * 2305 * 2, times values below 4: 1e-3 covers both."""
+    H, nh = 2048, 2
+    m = make_model(77, H, 1536, nh)
+    X = synth.normal_bf16(n, 9, (n, H))
+    cache0 = np.zeros((pos0 + n, LAT + ROPE), np.uint16)
+    out, cache = run_gpu(attn, m, X, cache0, pos0, nh)
+    assert torch.isfinite(out.float()).all()
+    W = torch.from_numpy(m["Wkva"]).cuda().view(torch.float8_e4m3fn).double()
+    W *= torch.from_numpy(m["Skva"]).cuda().double().repeat_interleave(128, 0)[:LAT + ROPE].repeat_interleave(128, 1)
+    kv = to_bf16_cuda(X).double() @ W.T
+    ang = torch.arange(pos0, pos0 + n, device="cuda").double()[:, None] / 10000.0 ** (torch.arange(0, ROPE, 2, device="cuda").double() / ROPE)
+    a, b = kv[:, LAT::2], kv[:, LAT + 1::2]
+    want = torch.empty_like(kv)
+    want[:, :LAT] = kv[:, :LAT] / torch.sqrt((kv[:, :LAT] ** 2).mean(1, keepdim=True) + 1e-6)
+    want[:, LAT::2], want[:, LAT + 1::2] = a * ang.cos() - b * ang.sin(), b * ang.cos() + a * ang.sin()
+    err = (cache[pos0:].double() - want).abs() - 2.0 ** -7 * want.abs()
+    assert err.max() < 1e-3, err.max()
