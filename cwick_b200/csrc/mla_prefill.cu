@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(256) norm_rope_rows_kernel(const float *in, in
 // One launch does the q_a rows and the kv_a rows (b; half of the grid each), and adds up the parts that their GEMM left of tiles that
 // it cut along K, in the order of fp8_sum_parts_kernel, a part of the whole row in flight at a time: latency bounds it, and three kernels one
 // after another (sum, q norm, kv norm, the last behind q_b) waited for their loads three times.
-// Alone with cold caches, 509 tokens: 8.8 + 10.5 + 8.4 -> 13.3 us, 4096 tokens (no parts): 15.4 + 11.6 -> 17.1; the whole prompt of 509 after 3001
-// 331.3 -> 327.2 us, and 324.5 with the angles formed before the wait; 4096 at the power cap, no difference. Four rows a block: 509 rows are 256 blocks.
+// Alone with cold caches, 509 tokens: 8.8 + 10.5 + 8.4 -> 15.9 us, 4096 tokens (no parts): 15.4 + 11.6 -> 19.8; the whole prompt of 509 after 3001
+// 331.3 -> 327.2 us, and 3 less with the angles formed before the wait; 4096 at the power cap, no difference. Four rows a block: 509 rows are 256 blocks.
 // rot: where each row's (cos, sin) of its rope pairs go as well, for the queries of the same positions (NULL: nowhere).
 struct NormRows {
     const float *in;
