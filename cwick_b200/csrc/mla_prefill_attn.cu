@@ -654,8 +654,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
 //
 // P lies in four buffers, tile T in buffer T % 4 of both CTAs: those of its own tiles a CTA's softmax writes, the others the
 // peer fills (an even number: a role that looks at own tiles only sees every phase of their barriers; six of them beside two latent
-// stages instead of three: 1490 and 338 us). A buffer is free for tile T + 4 when the value MMAs of tile T are done in BOTH CTAs, which each tells the
-// other by committing to the same barrier in both. There are eight of these barriers, T % 8: the two softmax sets of a CTA may be
+// stages instead of three: 1490 and 338 us). A buffer is free for tile T + 4 when the value MMAs of tile T are done in BOTH CTAs, and
+// both tell the CTA whose tile it is, which alone writes tile T + 4, and it alone: every arrival from the other CTA is then one that
+// somebody waits for, the last two tiles' before the epilogue, and none is under way when a CTA leaves. There are eight of these
+// barriers, T % 8: the two softmax sets of a CTA may be
 // an own tile apart, and with four a set could wait for a phase whose predecessor is still open, which a parity wait cannot tell
 // from the one after. tests/test_prefill_pair_protocol.py walks the protocol.
 template <class CFG>
@@ -676,9 +678,9 @@ __device__ __forceinline__ void copy_to_peer(uint32_t addr, uint32_t bytes, uint
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(peer_addr), "r"(addr), "r"(bytes), "r"(peer_bar)
                  : "memory");
 }
-// completion of this CTA's MMAs so far, at the same barrier in both CTAs of the pair
-__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+// completion of this CTA's MMAs so far, at the same barrier in the CTAs of the cluster that `ctas` has bits for
+__device__ __forceinline__ void umma_commit_to(uint32_t bar, int ctas) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)ctas) : "memory");
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
@@ -710,7 +712,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             if (i == PR_QFULL || i == PR_OFREE || i == PR_XM || i == PR_XL) count = 16;                  // every softmax warp
             if (i == PR_SEMPTY || i == PR_SEMPTY + 1) count = 8;                                         // the warps of a set
             if (i >= PR_PFULL && i < PR_PEMPTY) count = ((i - PR_PFULL) & 1) == rank ? 8 : 1;            // ... or the announcement of the peer's copy
-            if (i >= PR_PEMPTY && i < PR_ODONE) count = 2;                                               // the value MMAs of both CTAs
+            if (i >= PR_PEMPTY && i < PR_ODONE) count = 2;                                               // the value MMAs of both CTAs (own tiles' barriers)
             mbar_init(bar(i), count);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -880,7 +882,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     for (int s = 0; s < 4; s++)
                         umma_bf16(tm + PA_COL_O, dP + (uint64_t)((s * 32) >> 4), dC + (uint64_t)((s * 2048) >> 4), ID_PV, s != 0 ? 1u : (uint32_t)(i != 0));
                     umma_commit(bar(PR_CEMPTY + cs));
-                    umma_commit_both(bar(PR_PEMPTY + (T & 7)));
+                    umma_commit_to(bar(PR_PEMPTY + (T & 7)), 1 << (T & 1));
                 }
                 __syncwarp();
                 if (++cs == L::CST) { cs = 0; cu++; }
@@ -1093,7 +1095,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync();                                          // nothing of either CTA's is on its way to the other any more
+    cluster_sync();                                          // a CTA's copies and commits to the other have arrived: each was waited for there
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");

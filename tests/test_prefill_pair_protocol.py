@@ -1,7 +1,8 @@
 """The barriers of the MLA prompt attention's pair of CTAs (prefill_pair_kernel), as a model on the CPU: the roles of both CTAs as
-coroutines in random order, MMAs and copies that complete late, waits that see a barrier's parity only. Every P and row sum
+coroutines in random order, MMAs and copies that complete late, waits that see a barrier's parity only. What one CTA sends to the other
+(copies, arrivals of committed MMAs) arrives in any order. Every P and row sum
 must be the tile's or item's own when it is read, no buffer may be written while something still reads it, no barrier may complete twice in a
-phase's stead, and everybody must come to the end."""
+phase's stead, everybody must come to the end, and by then nothing may be on its way to the other CTA, which leaves."""
 import os
 import random
 import re
@@ -42,23 +43,24 @@ class Bar:
 
 
 class Cta:
-    def __init__(self, rank, kst, pbars, both):
+    def __init__(self, rank, kst, pbars, arrivals):
         b = Bar
         self.rank = rank
         self.kfull, self.kempty = [b(1) for _ in range(kst)], [b(1) for _ in range(kst)]
         self.sfull, self.sempty = [b(1), b(1)], [b(1), b(1)]
-        self.pfull, self.pempty = [b(1) for _ in range(4)], [b(2 if both else 1) for _ in range(pbars)]
+        self.pfull, self.pempty = [b(1) for _ in range(4)], [b(arrivals) for _ in range(pbars)]
         self.odone, self.qempty, self.qfull, self.ofree, self.xm, self.xl = b(1), b(1), b(2), b(2), b(2), b(2)
         self.peer = [b(1), b(1)]
         self.k, self.s, self.p, self.readers = [None] * kst, [None, None], [None] * 4, [0] * 4
         self.sum, self.item_m, self.q = [None, None], None, None
 
 
-def model(items, seed, kst, pbars, both=True):
-    """both: a P buffer is free when both CTAs' value products are done with it (False: this CTA's)."""
+def model(items, seed, kst, pbars, told, arrivals=2):
+    """told(T, rank): the CTAs, as bits, that CTA `rank` tells of the end of its value products with tile T."""
     rnd = random.Random(seed)
-    ctas = [Cta(0, kst, pbars, both), Cta(1, kst, pbars, both)]
-    late = []                                                # completions under way: a list per source, in order within it
+    ctas = [Cta(0, kst, pbars, arrivals), Cta(1, kst, pbars, arrivals)]
+    late = []                                                # completions under way in a CTA: a list per source, in order within it
+    sent = []                                                # under way from one CTA to the other, in no order
 
     def wait(bar, parity):
         while not bar.passes(parity):
@@ -127,15 +129,19 @@ def model(items, seed, kst, pbars, both=True):
 
                 def end(pb=pb, T=T):
                     c.readers[pb] -= 1
-                    for x in ctas if both else [c]:
-                        x.pempty[T % pbars].arrive()
+                    for x in ctas:
+                        if told(T, c.rank) >> x.rank & 1:
+                            if x is c:
+                                x.pempty[T % pbars].arrive()
+                            else:
+                                sent.append(x.pempty[T % pbars].arrive)
                 mma.append(end)
                 T += 1
             mma.append(c.odone.arrive)
             yield
 
     def sender(c):
-        copies, other = chain(), ctas[1 - c.rank]
+        other = ctas[1 - c.rank]
         for T in range(c.rank, sum(items), 2):
             pb = T & 3
             yield from wait(c.pfull[pb], T >> 2 & 1)
@@ -149,7 +155,7 @@ def model(items, seed, kst, pbars, both=True):
                     raise Fault("P of tile %d sent into a buffer in use" % T)
                 other.p[pb] = T
                 other.pfull[pb].bytes(1)
-            copies.append(arrive_there)
+            sent.append(arrive_there)
             yield
 
     def free(c, T):
@@ -157,7 +163,7 @@ def model(items, seed, kst, pbars, both=True):
             yield from wait(c.pempty[(T - 4) % pbars], (T - 4) // pbars & 1)
 
     def softmax(c, which):                                   # one of the two sets
-        kc, T, copies, other = 0, 0, chain(), ctas[1 - c.rank]
+        kc, T, other = 0, 0, ctas[1 - c.rank]
         state = c.__dict__.setdefault("soft", {"q": 0})
 
         def query(k):                                        # both sets copy a part; the tile is whole with the second arrival
@@ -202,7 +208,7 @@ def model(items, seed, kst, pbars, both=True):
                 def arrive_there(k=k):
                     other.sum[k & 1] = k
                     other.peer[k & 1].bytes(1)
-                copies.append(arrive_there)
+                sent.append(arrive_there)
             yield from wait(c.peer[k & 1], k >> 1 & 1)
             yield from wait(c.odone, k & 1)
             own = T if T & 1 == c.rank else T + 1
@@ -217,9 +223,14 @@ def model(items, seed, kst, pbars, both=True):
 
     roles = [r for c in ctas for r in (keys(c), scores(c), values(c), sender(c), softmax(c, 0), softmax(c, 1))]
     weight = [rnd.choice((1, 1, 4, 20)) for _ in roles]      # some roles are slow
+    slow = rnd.random() < 0.5                                # the way between the CTAs: nothing arrives until all wait for it
     idle = 0
     while roles:
         ready = [q for q in late if q]
+        if sent and (idle > 100 if slow else rnd.random() < 0.15):
+            sent.pop(rnd.randrange(len(sent)))()
+            idle = 0
+            continue
         if ready and rnd.random() < 0.3:
             rnd.choice(ready).pop(0)()
             idle = 0
@@ -237,26 +248,36 @@ def model(items, seed, kst, pbars, both=True):
         idle = 0 if after != before or ready else idle + 1
         if idle > 5000:
             raise Fault("stuck")
+    if sent:
+        raise Fault("%d arrivals at a CTA that has left" % len(sent))
 
 
 ITEMS = [[1], [2], [3], [1, 1, 1, 1, 1, 1, 1, 1, 1], [2, 1, 2, 1, 3, 1], [5, 4, 3, 2, 1], [7, 1, 6, 2, 9], [12, 11], [1, 8, 1, 1, 8, 3, 3]]
 
 
-def counts():
+def source():
+    """Key slots, barriers of the P buffers and who is told of the end of a tile's value products, as the kernel has them."""
     text = open(SRC).read()
     kst = int(re.search(r"struct PrCfg \{\s*static constexpr int KST = (\d+)", text)[1])
     pbars = int(re.search(r"PR_ODONE = PR_PEMPTY \+ (\d+)", text)[1])
-    return kst, pbars
+    told = eval("lambda T, rank: " + re.search(r"umma_commit_to\(bar\(PR_PEMPTY \+ \(T & 7\)\), ([^;]+)\);", text)[1])
+    return kst, pbars, told
 
 
 @pytest.mark.parametrize("items", ITEMS, ids=str)
 def test_the_pairs_protocol(items):
-    kst, pbars = counts()
+    kst, pbars, told = source()
     for seed in range(12):
-        model(items, seed, kst, pbars)
+        model(items, seed, kst, pbars, told)
 
 
 def test_the_model_finds_buffers_freed_too_early():
     with pytest.raises(Fault):
         for seed in range(100):
-            model([7, 1, 6, 2, 9], seed, 2, 8, both=False)
+            model([7, 1, 6, 2, 9], seed, 2, 8, lambda T, rank: 1 << rank, arrivals=1)
+
+
+def test_the_model_finds_arrivals_that_nobody_waits_for():
+    with pytest.raises(Fault, match="has left"):
+        for seed in range(100):
+            model([7, 1, 6, 2, 9], seed, 2, 8, lambda T, rank: 3)
