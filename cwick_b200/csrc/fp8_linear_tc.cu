@@ -172,6 +172,9 @@ fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                     else tma_load_3d_pair(a0 + A_BYTES, &tm_w, 0, g.col0 + rank * (BN / 2), kb * 2, full);
                 }
             }
+            // the issuer commits to both CTAs: none of these arrivals may still be on its way here when this CTA leaves
+            for (int s = max(0, c - STAGES); s < c && ok; s++)
+                ok = mbar_wait(bar(GB_EMPTY + s % STAGES), (uint32_t)((s / STAGES) & 1), p.err, 406);
             if (!ok && rank == 0)      // drain the copies still in flight before leaving
                 for (int s = (c > STAGES ? c - STAGES : 0); s < c; s++)
                     mbar_wait(bar(GB_FULL + s % STAGES), (uint32_t)((s / STAGES) & 1), p.err, 402);

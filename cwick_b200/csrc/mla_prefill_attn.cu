@@ -1297,6 +1297,9 @@ kexp_tc_kernel(const __grid_constant__ CUtensorMap tm_lat, const __grid_constant
                 tma_load_3d_pair(base + KX_OFF_A + slot * KX_A_BYTES, &tm_lat, 0, (tile * 2 + rank) * KX_TOK, (c & 3) * 2, cluster_addr(bar(KB_AFULL + slot), 0));
                 issued = c + 1;
             }
+            // the issuer commits to both CTAs: none of these arrivals may still be on its way here when this CTA leaves
+            for (int c = max(0, nch - KX_ST); c < nch && ok; c++)
+                ok = mbar_wait(bar(KB_AEMPTY + c % KX_ST), (uint32_t)((c / KX_ST) & 1), p.err, 1108);
             if (!ok && rank == 0) {
                 mbar_wait(bar(KB_WFULL), 0, p.err, 1102);
                 for (int c = (issued > KX_ST ? issued - KX_ST : 0); c < issued; c++) mbar_wait(bar(KB_AFULL + c % KX_ST), (uint32_t)((c / KX_ST) & 1), p.err, 1103);
