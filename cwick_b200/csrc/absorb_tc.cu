@@ -127,7 +127,7 @@ absorb_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const int t = ((int)blockIdx.x + i * (int)gridDim.x) * AT_TOK + q4 * 32 + lane;
 #pragma unroll
             for (int half = 0; half < 2; half++) {
-                if (ok) ok = mbar_wait(bar(AB_DFULL + half), (uint32_t)(i & 1), p.err, 907);
+                if (ok) ok = mbar_wait_warp(bar(AB_DFULL + half), (uint32_t)(i & 1), p.err, 907);
                 if (!ok) break;
                 tc_fence_after();
                 // A thread holds one token row of the accumulator, and rows of Qfull lie 73 KB apart: storing from

@@ -203,16 +203,16 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
         }
     } else if (warp == 1) {
         {
+            uint32_t patience = WAIT_LIMIT;
             constexpr uint32_t ID = idesc_f16(128, IT_QROWS);
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             const uint64_t db = smem_desc(base + I_OFF_Q, 16, 1024);
-            bool ok = true;
             int d = 0, du = 0;                               // accumulator and its use
-            for (int i = 0; i < nt && ok; i++) {
+#pragma unroll 1
+            for (int i = 0; i < nt; i++) {
                 const int ab = i & 1, use = i >> 1;
-                ok = mbar_wait(bar(IB_D_EMPTY + d), (uint32_t)((du & 1) ^ 1), p.err, 804);
-                if (ok) ok = mbar_wait(bar(IB_A_FULL + ab), (uint32_t)(use & 1), p.err, 803);
-                if (!ok) break;
+                mbar_wait_on(bar(IB_D_EMPTY + d), (uint32_t)((du & 1) ^ 1), p.err, 804, patience);
+                mbar_wait_on(bar(IB_A_FULL + ab), (uint32_t)(use & 1), p.err, 803, patience);
                 tc_fence_after();
                 if (elect_one()) {
 #pragma unroll
@@ -225,6 +225,7 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
                 __syncwarp();
                 if (++d == IT_ACC) { d = 0; du++; }
             }
+            settle(patience != WAIT_LIMIT);
         }
     } else if (warp >= 4 && warp < 12) {
         // ---------------- converters: raw E4M3 tile -> f16 pairs in tensor memory, the MMA's A operand
@@ -236,9 +237,8 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
         bool ok = true;
         for (int i = 0; i < nt; i++) {
             const int r = i % RAW_STAGES, ruse = i / RAW_STAGES, ab = i & 1, ause = i >> 1;
-            ok = mbar_wait(bar(IB_RAW_FULL + r), (uint32_t)(ruse & 1), p.err, 805);
-            if (ok) ok = mbar_wait(bar(IB_A_EMPTY + ab), (uint32_t)((ause & 1) ^ 1), p.err, 806);
-            ok = __all_sync(0xffffffffu, ok);            // the TMEM stores below are warp-wide
+            const bool here = mbar_wait(bar(IB_RAW_FULL + r), (uint32_t)(ruse & 1), p.err, 805) && mbar_wait(bar(IB_A_EMPTY + ab), (uint32_t)((ause & 1) ^ 1), p.err, 806);
+            ok = __all_sync(0xffffffffu, here);          // the TMEM stores below are warp-wide
             if (!ok) break;
             tc_fence_after();
             const uint8_t *src = sm + I_OFF_RAW + r * RAW_BYTES + row * 128;
@@ -276,7 +276,7 @@ indexer_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_keys, const IdxP
         float mx = -INFINITY, mn = INFINITY;
         for (int i = (warp - 12) >> 2; i < nt; i += 2) {
             const int d = i % IT_ACC;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(IB_D_FULL + d), (uint32_t)((i / IT_ACC) & 1), p.err, 807));
+            ok = mbar_wait_warp(bar(IB_D_FULL + d), (uint32_t)((i / IT_ACC) & 1), p.err, 807);
             if (!ok) break;
             tc_fence_after();
             const int64_t key = (int64_t)(t_begin + i) * IT_KEYS + row;

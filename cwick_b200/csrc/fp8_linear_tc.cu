@@ -181,18 +181,18 @@ fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         }
     } else if (warp == 1) {
         if (rank == 0) {
+            uint32_t patience = WAIT_LIMIT;
             constexpr uint32_t ID = idesc_bf16(BM, BN, 0, 0);
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             const uint64_t da0 = smem_desc(base, 16, 1024), db0 = smem_desc(base + A_BYTES, 16, 1024);
-            bool ok = true;
             int c = 0, slot = 0, use = 0;
-            for (int u = u0; u < units && ok; u += du) {
+            for (int u = u0; u < units; u += du) {
                 const GemmUnit g = gemm_unit(u, p, nkb);
-                for (int kb = g.kb0; kb < g.kb1 && ok; kb++, c++) {
+#pragma unroll 1
+                for (int kb = g.kb0; kb < g.kb1; kb++, c++) {
                     const int pb = c & 1, puse = c >> 1;
-                    ok = mbar_wait(bar(GB_FULL + slot), (uint32_t)(use & 1), p.err, 404);
-                    if (ok) ok = mbar_wait(bar(GB_PEMPTY + pb), (uint32_t)((puse & 1) ^ 1), p.err, 403);
-                    if (!ok) break;
+                    mbar_wait_on(bar(GB_FULL + slot), (uint32_t)(use & 1), p.err, 404, patience);
+                    mbar_wait_on(bar(GB_PEMPTY + pb), (uint32_t)((puse & 1) ^ 1), p.err, 403, patience);
                     tc_fence_after();
                     const uint64_t off = (uint64_t)((slot * (A_BYTES + B_BYTES)) >> 4);
                     if (elect_one()) {
@@ -207,6 +207,7 @@ fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                     if (++slot == STAGES) { slot = 0; use++; }
                 }
             }
+            settle(patience != WAIT_LIMIT);
         }
     } else if (warp >= 4) {
         const int q = warp & 3, ch = (warp - 4) >> 2;
@@ -227,8 +228,7 @@ fp8_linear_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             for (int j = 0; j < 64; j++) acc2[j] = 0;
             for (int kb = g.kb0; kb < g.kb1; kb++, c++) {
                 const int pb = c & 1, puse = c >> 1;
-                ok = mbar_wait(bar(GB_PFULL + pb), (uint32_t)(puse & 1), p.err, 405);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(bar(GB_PFULL + pb), (uint32_t)(puse & 1), p.err, 405);
                 if (!ok) break;
                 tc_fence_after();
                 if (live) {

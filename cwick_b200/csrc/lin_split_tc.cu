@@ -147,8 +147,7 @@ lin_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     __syncwarp();
     // ---- epilogue: a thread holds one token row of 32 lanes' worth; 128-byte lines leave through a per-warp staging tile,
     // which lies in the weight ring (every copy into it has been consumed once DONE is complete)
-    const bool fine = mbar_wait(bar(DONE), 0, p.err, 1207);
-    if (__all_sync(0xffffffffu, fine)) {
+    if (mbar_wait_warp(bar(DONE), 0, p.err, 1207)) {
         tc_fence_after();
         const int q4 = warp & 3, g2 = warp >> 2;
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);

@@ -279,8 +279,7 @@ __device__ __noinline__ bool segment_epilogue(const SkParams &p, const Seg &s, u
     // Each 128-row block of O^T leaves as soon as its own MMAs have completed (their commit is the
     // barrier that frees the block's latent slot).
     for (int mb = 0; mb < 4 && ok; mb++) {
-        ok = mbar_wait(bar(mb == 3 ? B_EMPTY_RP : B_EMPTY_L + mb), (uint32_t)(itl & 1), p.err, 302);
-        ok = __all_sync(0xffffffffu, ok);                  // the TMEM load below is warp-wide
+        ok = mbar_wait_warp(bar(mb == 3 ? B_EMPTY_RP : B_EMPTY_L + mb), (uint32_t)(itl & 1), p.err, 302);      // the TMEM load below is warp-wide
         if (!ok) break;
         tc_fence_after();
         uint32_t o[16];

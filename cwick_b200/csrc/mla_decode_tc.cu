@@ -485,7 +485,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
         for (int h = 0; h < HG; h++) lpart[h] = 0.f;
         for (int it = begin; it < end; it++) {
-            ok = mbar_wait(bar(B_SFULL), (uint32_t)(it & 1), p.err, 301);
+            ok = mbar_wait_warp(bar(B_SFULL), (uint32_t)(it & 1), p.err, 301);
             if (!ok) break;
             if (st == 0) TRACE(2, it, 0);
             tc_fence_after();
@@ -609,8 +609,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             if (p.out) softmax_bar();
             if (st == 0) TRACE(2, 15, 4);
             for (int mb = mb0; mb < mb1 && ok; mb++) {
-                ok = mbar_wait(bar(mb == 3 ? B_EMPTY_RP : B_EMPTY_L + mb), (uint32_t)((end - 1) & 1), p.err, 302);
-                ok = __all_sync(0xffffffffu, ok);                  // the TMEM load below is warp-wide
+                ok = mbar_wait_warp(bar(mb == 3 ? B_EMPTY_RP : B_EMPTY_L + mb), (uint32_t)((end - 1) & 1), p.err, 302);      // the TMEM load below is warp-wide
                 if (!ok) break;
                 if (st == 0 && mb == 0) TRACE(2, 15, 2);
                 tc_fence_after();

@@ -246,14 +246,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t tmem = *s_tmem;
 
     // item k of this block, as published by the key producer (w < 0: no more)
-    auto next_item = [&](int k, int &w, AttnItem &it) -> bool {
-        if (!mbar_wait(bar(PB_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1031)) return false;
+    auto read_item = [&](int k, int &w, AttnItem &it) {
         const int4 v = s_item[k & 7];
         w = GQA || v.x < 0 ? v.x : v.x >> 1;
         it = attn_item(max(w, 0), p, nq);
         it.half = GQA ? 0 : v.x & 1;
         it.lo = v.y; it.nt = v.z; it.rec = v.w;
         if (p.shares) it.flag = w + unit;
+    };
+    auto next_item = [&](int k, int &w, AttnItem &it) -> bool {      // a warp's
+        if (!mbar_wait_warp(bar(PB_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1031)) return false;
+        read_item(k, w, it);
         return true;
     };
 
@@ -319,8 +322,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             for (int k = 0; ok; k++) {
                 int w;
                 AttnItem it;
-                ok = next_item(k, w, it);
-                if (!ok || w < 0) break;
+                ok = mbar_wait(bar(PB_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1032);
+                if (!ok) break;
+                read_item(k, w, it);
+                if (w < 0) break;
                 for (int i = it.lo; i < it.nt && ok; i++, cc++) {
                     const int cs = cc % PA_CST, cu = cc / PA_CST;
                     ok = mbar_wait(bar(PB_CEMPTY + cs), (uint32_t)((cu & 1) ^ 1), p.err, 1002);
@@ -342,6 +347,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         // form a second one (the last warp) takes every other tile. All lanes run the issuers' loops and one is elected for the
         // MMAs (tc_common.cuh).
         {
+            uint32_t patience = WAIT_LIMIT;
             constexpr uint32_t ID_QK = idesc_bf16(128, PA_KT, 0, 0);
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             const uint64_t dK0 = smem_desc(base + PA_OFF_K, 16, 1024);
@@ -354,15 +360,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 ok = next_item(k, w, it);
                 if (!ok || w < 0) break;
                 const int end = __shfl_sync(0xffffffffu, kc + it.nt - it.lo, 0);
-                ok = mbar_wait(bar(PB_QFULL), (uint32_t)(k & 1), p.err, 1011);     // the softmax threads have written the item's query tile into tensor memory
+                ok = mbar_wait_warp(bar(PB_QFULL), (uint32_t)(k & 1), p.err, 1011);     // the softmax threads have written the item's query tile into tensor memory
                 if (!ok) break;
                 tc_fence_after();
                 // scores of a tile: S[kc % 2] = Q Kx^T, the 64-wide blocks of the key's dims, four 16-wide steps each
-                for (kc += QK_ISSUERS == 2 ? (kc ^ first) & 1 : 0; kc < end && ok; kc += QK_ISSUERS) {
+#pragma unroll 1
+                for (kc += QK_ISSUERS == 2 ? (kc ^ first) & 1 : 0; kc < end; kc += QK_ISSUERS) {
                     const int ks = kc % PA_KST, sb = kc % PA_SBUF, su = kc / PA_SBUF;
-                    ok = mbar_wait(bar(PB_KFULL + kc % PA_KBAR), (uint32_t)((kc / PA_KBAR) & 1), p.err, 1012);
-                    if (ok) ok = mbar_wait(bar(PB_SEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1013);
-                    if (!ok) break;
+                    mbar_wait_on(bar(PB_KFULL + kc % PA_KBAR), (uint32_t)((kc / PA_KBAR) & 1), p.err, 1012, patience);
+                    mbar_wait_on(bar(PB_SEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1013, patience);
                     tc_fence_after();
                     const uint64_t dK = dK0 + (uint64_t)((ks * PA_K_BYTES) >> 4);
                     if (elect_one()) {
@@ -376,13 +382,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     __syncwarp();
                 }
                 kc = end;
-                if (ok && elect_one()) umma_commit(bar(PB_QEMPTY));       // the query tile may be replaced once these MMAs are done
+                if (elect_one()) umma_commit(bar(PB_QEMPTY));       // the query tile may be replaced once these MMAs are done
                 __syncwarp();
             }
+            settle(patience != WAIT_LIMIT);
         }
     } else if (warp == 3) {
         // ------------------------------------------------------------ MMA issuer of the values
         {
+            uint32_t patience = WAIT_LIMIT;
             constexpr uint32_t ID_PV = idesc_bf16(128, PA_DV, 0, 1);
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             const uint64_t dP0 = smem_desc(base + PA_OFF_P, 16, 1024), dC0 = smem_desc(base + PA_OFF_C, PA_KT * 128, 1024);
@@ -395,14 +403,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 if (!ok || w < 0) break;
                 const int tiles = __shfl_sync(0xffffffffu, it.nt - it.lo, 0);
                 if (k > 0) {                         // the accumulator of the previous item has been read out
-                    ok = mbar_wait(bar(PB_OFREE), (uint32_t)((k - 1) & 1), p.err, 1016);
+                    ok = mbar_wait_warp(bar(PB_OFREE), (uint32_t)((k - 1) & 1), p.err, 1016);
                     if (!ok) break;
                 }
-                for (int i = 0; i < tiles && ok; i++, cc++) {
+#pragma unroll 1
+                for (int i = 0; i < tiles; i++, cc++) {
                     const int cs = cc % PA_CST, cu = cc / PA_CST, pb = cc & 1, pu = cc >> 1;
-                    ok = mbar_wait(bar(PB_CFULL + cs), (uint32_t)(cu & 1), p.err, 1014);
-                    if (ok) ok = mbar_wait(bar(PB_PFULL + pb), (uint32_t)(pu & 1), p.err, 1015);
-                    if (!ok) break;
+                    mbar_wait_on(bar(PB_CFULL + cs), (uint32_t)(cu & 1), p.err, 1014, patience);
+                    mbar_wait_on(bar(PB_PFULL + pb), (uint32_t)(pu & 1), p.err, 1015, patience);
                     tc_fence_after();
                     // values: O += P lat, P [128 q][64 keys] K-major, lat half [64 keys][256] with the 256 contiguous (MN-major, four 64-wide blocks)
                     const uint64_t dP = dP0 + (uint64_t)((pb * PA_P_BYTES) >> 4), dC = dC0 + (uint64_t)((cs * PA_C_BYTES) >> 4);
@@ -417,9 +425,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     }
                     __syncwarp();
                 }
-                if (ok && elect_one()) umma_commit(bar(PB_ODONE));
+                if (elect_one()) umma_commit(bar(PB_ODONE));
                 __syncwarp();
             }
+            settle(patience != WAIT_LIMIT);
         }
     } else {
         // ------------------------------------------------------------ softmax, (correction,) epilogue
@@ -448,16 +457,16 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             // no P is written before the epilogue of the item before has left the P buffers.)
             auto reference = [&]() -> bool {
                 arrive(PB_XM);
-                if (!mbar_wait(bar(PB_XM), (uint32_t)(k & 1), p.err, 1026)) return false;
+                if (!mbar_wait_warp(bar(PB_XM), (uint32_t)(k & 1), p.err, 1026)) return false;
                 m = fmaxf(s_m[row], s_m[128 + row]);                 // the tile shows every row a key: finite
                 return true;
             };
-            if (NWG == 4 && (tc & 1) != odd) ok = reference();
+            if (NWG == 4 && (tc & 1) != odd && !reference()) break;
             const int tc0 = tc;
             tc += nt - it.lo;
             for (int d = NWG == 4 ? (tc0 ^ odd) & 1 : 0; d < nt - it.lo; d += NWG == 4 ? 2 : 1) {
                 const int i = it.lo + d, sb = (tc0 + d) & 1, su = (tc0 + d) >> 1;      // the tile; its score and P buffers and their use
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_SFULL + sb), (uint32_t)(su & 1), p.err, 1021));   // warp-uniform: the TMEM loads below are warp-wide
+                ok = mbar_wait_warp(bar(PB_SFULL + sb), (uint32_t)(su & 1), p.err, 1021);   // the TMEM loads below are warp-wide
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t v[NC];
@@ -504,8 +513,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     if (__any_sync(0xffffffffu, mine)) {
                         // some row's scores outran its reference exponent: rescale what it has accumulated. A row is its
                         // thread's TMEM lane; the value MMAs of the previous tile must have finished writing it.
-                        ok = mbar_wait(bar(PB_PEMPTY + ((tc0 + d - 1) & 1)), (uint32_t)(((tc0 + d - 1) >> 1) & 1), p.err, 1022);
-                        ok = __all_sync(0xffffffffu, ok);
+                        ok = mbar_wait_warp(bar(PB_PEMPTY + ((tc0 + d - 1) & 1)), (uint32_t)(((tc0 + d - 1) >> 1) & 1), p.err, 1022);
                         if (!ok) break;
                         tc_fence_after();
                         const float alpha = mine ? exp2f(m - mt) : 1.f;
@@ -534,7 +542,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 unpack_f32x2(lsum, l0, l1);
                 l += l0 + l1;
                 // the P buffer of this parity was read by the value MMAs two tiles ago
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023));
+                ok = mbar_wait_warp(bar(PB_PEMPTY + sb), (uint32_t)((su & 1) ^ 1), p.err, 1023);
                 if (!ok) break;
                 uint8_t *prow = sm + PA_OFF_P + sb * PA_P_BYTES + row * 128;
 #pragma unroll
@@ -552,21 +560,20 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 ok = next_item(k + 1, wn, nx);
                 if (!ok) break;
                 if (wn >= 0) {
-                    ok = mbar_wait(bar(PB_QEMPTY), (uint32_t)(k & 1), p.err, 1025);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(bar(PB_QEMPTY), (uint32_t)(k & 1), p.err, 1025);
                     if (!ok) break;
                     tc_fence_after();
                     load_query(nx.q0, nx.h);
                 }
             }
             // ---- epilogue of the item: O / l -> bf16 -> out[t][h][half * 256 ..], full lines through a staging tile
-            ok = mbar_wait(bar(PB_ODONE), (uint32_t)(k & 1), p.err, 1024);
+            ok = mbar_wait_warp(bar(PB_ODONE), (uint32_t)(k & 1), p.err, 1024);
             if (!ok) break;
             tc_fence_after();
             if (NWG == 4) {                                          // the row's sum is the groups' sums
                 s_l[wg * 128 + row] = l;
                 arrive(PB_XL);
-                ok = mbar_wait(bar(PB_XL), (uint32_t)(k & 1), p.err, 1027);
+                ok = mbar_wait_warp(bar(PB_XL), (uint32_t)(k & 1), p.err, 1027);
                 if (!ok) break;
                 l = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
             }
@@ -728,14 +735,17 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t tmem = *s_tmem;
 
     // item k of this pair, as published by the key producer (w < 0: no more); both CTAs come to the same items by themselves
-    auto next_item = [&](int k, int &w, AttnItem &it) -> bool {
-        if (!mbar_wait(bar(PR_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1431)) return false;
+    auto read_item = [&](int k, int &w, AttnItem &it) {
         const int4 v = s_item[k & 7];
         w = v.x;
         it = attn_item(max(w, 0), p, nq);
         it.half = rank;
         it.lo = v.y; it.nt = v.z; it.rec = v.w;
         if (p.shares) it.flag = w + unit;
+    };
+    auto next_item = [&](int k, int &w, AttnItem &it) -> bool {      // a warp's
+        if (!mbar_wait_warp(bar(PR_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1431)) return false;
+        read_item(k, w, it);
         return true;
     };
     // the tiles of an item whose first has number T: how many this CTA forms the scores of (the first, and its own), and the i-th of them
@@ -790,19 +800,24 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 for (int j = max(0, kc - L::KST); j < kc; j++) mbar_wait(bar(PR_KFULL + j % L::KST), (uint32_t)((j / L::KST) & 1), p.err, 1404);
         }
     } else if (warp == 2) {
-        // ------------------------------------------------------------ TMA producer of the latent ring: every tile, this CTA's half
+        // ------------------------------------------------------------ TMA producer of the latent ring: every tile, this CTA's half; announces the peer's P
         if (lane == 0) {
             bool ok = true;
             int cc = 0;
             for (int k = 0; ok; k++) {
                 int w;
                 AttnItem it;
-                ok = next_item(k, w, it);
-                if (!ok || w < 0) break;
+                ok = mbar_wait(bar(PR_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1432);
+                if (!ok) break;
+                read_item(k, w, it);
+                if (w < 0) break;
                 for (int i = it.lo; i < it.nt && ok; i++, cc++) {
                     const int cs = cc % L::CST;
                     ok = mbar_wait(bar(PR_CEMPTY + cs), (uint32_t)(((cc / L::CST) & 1) ^ 1), p.err, 1402);
                     if (!ok) break;
+                    // the P of the peer's tiles (whose copy may be here before it is announced): what was in its buffer before has been
+                    // multiplied, since the values of tile cc - CST have been
+                    if ((cc & 1) != rank) mbar_expect_tx(bar(PR_PFULL + (cc & 3)), PA_P_BYTES);
                     mbar_expect_tx(bar(PR_CFULL + cs), PA_C_BYTES);
                     tma_load_3d(base + L::OFF_C + cs * PA_C_BYTES, &tm_c, 0, i * PA_KT, rank * 4, bar(PR_CFULL + cs));
                 }
@@ -812,6 +827,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer of the scores
+        uint32_t patience = WAIT_LIMIT;
         constexpr uint32_t ID_QK = idesc_bf16(128, PA_KT, 0, 0);
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         const uint64_t dK0 = smem_desc(base, 16, 1024);
@@ -823,14 +839,14 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             ok = next_item(k, w, it);
             if (!ok || w < 0) break;
             const int tiles = __shfl_sync(0xffffffffu, it.nt - it.lo, 0), mine = scored(T, tiles);
-            ok = mbar_wait(bar(PR_QFULL), (uint32_t)(k & 1), p.err, 1411);     // the softmax threads have written the item's query tile into tensor memory
+            ok = mbar_wait_warp(bar(PR_QFULL), (uint32_t)(k & 1), p.err, 1411);     // the softmax threads have written the item's query tile into tensor memory
             if (!ok) break;
             tc_fence_after();
-            for (int e = 0; e < mine && ok; e++, kc++) {
+#pragma unroll 1
+            for (int e = 0; e < mine; e++, kc++) {
                 const int ks = kc % L::KST, sb = kc & 1;
-                ok = mbar_wait(bar(PR_KFULL + ks), (uint32_t)((kc / L::KST) & 1), p.err, 1412);
-                if (ok) ok = mbar_wait(bar(PR_SEMPTY + sb), (uint32_t)(((kc >> 1) & 1) ^ 1), p.err, 1413);
-                if (!ok) break;
+                mbar_wait_on(bar(PR_KFULL + ks), (uint32_t)((kc / L::KST) & 1), p.err, 1412, patience);
+                mbar_wait_on(bar(PR_SEMPTY + sb), (uint32_t)(((kc >> 1) & 1) ^ 1), p.err, 1413, patience);
                 tc_fence_after();
                 const uint64_t dK = dK0 + (uint64_t)((ks * CFG::K_BYTES) >> 4);
                 if (elect_one()) {
@@ -843,12 +859,14 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 }
                 __syncwarp();
             }
-            if (ok && elect_one()) umma_commit(bar(PR_QEMPTY));       // the query tile may be replaced once these MMAs are done
+            if (elect_one()) umma_commit(bar(PR_QEMPTY));       // the query tile may be replaced once these MMAs are done
             __syncwarp();
             T += tiles;
         }
+        settle(patience != WAIT_LIMIT);
     } else if (warp == 3) {
         // ------------------------------------------------------------ MMA issuer of the values
+        uint32_t patience = WAIT_LIMIT;
         constexpr uint32_t ID_PV = idesc_bf16(128, PA_DV, 0, 1);
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         const uint64_t dP0 = smem_desc(base + L::OFF_P, 16, 1024), dC0 = smem_desc(base + L::OFF_C, PA_KT * 128, 1024);
@@ -861,19 +879,14 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             if (!ok || w < 0) break;
             const int tiles = __shfl_sync(0xffffffffu, it.nt - it.lo, 0);
             if (k > 0) {                         // the accumulator of the previous item has been read out
-                ok = mbar_wait(bar(PR_OFREE), (uint32_t)((k - 1) & 1), p.err, 1416);
+                ok = mbar_wait_warp(bar(PR_OFREE), (uint32_t)((k - 1) & 1), p.err, 1416);
                 if (!ok) break;
             }
-            for (int i = 0; i < tiles && ok; i++, T++) {
+#pragma unroll 1
+            for (int i = 0; i < tiles; i++, T++) {
                 const int pb = T & 3;
-                const bool own = (T & 1) == rank;
-                if (!own) {                          // (the peer's copy may be here before it is announced)
-                    if (elect_one()) mbar_expect_tx(bar(PR_PFULL + pb), PA_P_BYTES);
-                    __syncwarp();
-                }
-                ok = mbar_wait(bar(PR_CFULL + cs), (uint32_t)(cu & 1), p.err, 1414);
-                if (ok) ok = mbar_wait(bar(PR_PFULL + pb), (uint32_t)((T >> 2) & 1), p.err, 1415);
-                if (!ok) break;
+                mbar_wait_on(bar(PR_CFULL + cs), (uint32_t)(cu & 1), p.err, 1414, patience);
+                mbar_wait_on(bar(PR_PFULL + pb), (uint32_t)((T >> 2) & 1), p.err, 1415, patience);
                 tc_fence_after();
                 const uint64_t dP = dP0 + (uint64_t)((pb * PA_P_BYTES) >> 4), dC = dC0 + (uint64_t)((cs * PA_C_BYTES) >> 4);
                 if (elect_one()) {
@@ -887,29 +900,33 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 __syncwarp();
                 if (++cs == L::CST) { cs = 0; cu++; }
             }
-            if (ok && elect_one()) umma_commit(bar(PR_ODONE));
+            if (elect_one()) umma_commit(bar(PR_ODONE));
             __syncwarp();
         }
+        settle(patience != WAIT_LIMIT);
     } else if (warp == 20) {
         // ------------------------------------------------------------ sender of this CTA's P: as soon as it is there, whatever the values
         // wait for (in the values' issuer a tile's copy waited for the peer's copy of the tile before: 2.7 k cycles a tile)
         const uint32_t peer_p = cluster_addr(base + L::OFF_P, (uint32_t)(rank ^ 1)), peer_bar0 = cluster_addr(bar(PR_PFULL), (uint32_t)(rank ^ 1));
-        bool ok = true;
-        int T = 0;
-        for (int k = 0; ok; k++) {
-            int w;
-            AttnItem it;
-            ok = next_item(k, w, it);
-            if (!ok || w < 0) break;
-            const int end = __shfl_sync(0xffffffffu, T + it.nt - it.lo, 0);
-            for (T += (T ^ rank) & 1; T < end && ok; T += 2) {
-                const int pb = T & 3;
-                ok = mbar_wait(bar(PR_PFULL + pb), (uint32_t)((T >> 2) & 1), p.err, 1417);
+        if (lane == 0) {
+            bool ok = true;
+            int T = 0;
+            for (int k = 0; ok; k++) {
+                int w;
+                AttnItem it;
+                ok = mbar_wait(bar(PR_ITEM + (k & 7)), (uint32_t)((k >> 3) & 1), p.err, 1433);
                 if (!ok) break;
-                if (elect_one()) copy_to_peer(base + L::OFF_P + pb * PA_P_BYTES, PA_P_BYTES, peer_p + pb * PA_P_BYTES, peer_bar0 + 8u * (uint32_t)pb);
-                __syncwarp();
+                read_item(k, w, it);
+                if (w < 0) break;
+                const int end = T + it.nt - it.lo;
+                for (T += (T ^ rank) & 1; T < end && ok; T += 2) {
+                    const int pb = T & 3;
+                    ok = mbar_wait(bar(PR_PFULL + pb), (uint32_t)((T >> 2) & 1), p.err, 1417);
+                    if (ok) copy_to_peer(base + L::OFF_P + pb * PA_P_BYTES, PA_P_BYTES, peer_p + pb * PA_P_BYTES, peer_bar0 + 8u * (uint32_t)pb);
+                }
+                T = end;
             }
-            T = end;
+            settle(!ok);
         }
     } else {
         // ------------------------------------------------------------ softmax, epilogue
@@ -924,7 +941,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             if (lane == 0) mbar_arrive(bar(b));
         };
         auto buffer_free = [&](int T) {              // P buffer T % 4 is free for tile T: both CTAs are done with tile T - 4
-            return T < 4 || mbar_wait(bar(PR_PEMPTY + ((T - 4) & 7)), (uint32_t)(((T - 4) >> 3) & 1), p.err, 1423);
+            return T < 4 || mbar_wait_warp(bar(PR_PEMPTY + ((T - 4) & 7)), (uint32_t)(((T - 4) >> 3) & 1), p.err, 1423);
         };
         bool ok = true;
         int kc = 0, T = 0;                           // scored tiles so far (score buffer and its phase); number of the item's first tile
@@ -941,14 +958,14 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             // before the epilogue of the item before has left the P buffers.)
             auto reference = [&]() -> bool {
                 arrive(PR_XM);
-                if (!mbar_wait(bar(PR_XM), (uint32_t)(k & 1), p.err, 1426)) return false;
+                if (!mbar_wait_warp(bar(PR_XM), (uint32_t)(k & 1), p.err, 1426)) return false;
                 m = fmaxf(s_m[row], s_m[128 + row]);                 // the tile shows every row a key: finite
                 return true;
             };
-            if ((kc & 1) != set) ok = reference();
-            for (int e = (kc ^ set) & 1; e < mine && ok; e += 2) {
+            if ((kc & 1) != set && !reference()) break;
+            for (int e = (kc ^ set) & 1; e < mine; e += 2) {
                 const int d = nth(T, e), i = it.lo + d, sb = (kc + e) & 1, su = (kc + e) >> 1;
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(PR_SFULL + sb), (uint32_t)(su & 1), p.err, 1421));   // warp-uniform: the TMEM loads below are warp-wide
+                ok = mbar_wait_warp(bar(PR_SFULL + sb), (uint32_t)(su & 1), p.err, 1421);   // the TMEM loads below are warp-wide
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t v[NC];
@@ -998,7 +1015,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 float l0, l1;
                 unpack_f32x2(lsum, l0, l1);
                 l += l0 + l1;
-                ok = __all_sync(0xffffffffu, buffer_free(T + d));
+                ok = buffer_free(T + d);
                 if (!ok) break;
                 uint8_t *prow = sm + L::OFF_P + ((T + d) & 3) * PA_P_BYTES + row * 128;
 #pragma unroll
@@ -1017,7 +1034,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 ok = next_item(k + 1, wn, nx);
                 if (!ok) break;
                 if (wn >= 0) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(PR_QEMPTY), (uint32_t)(k & 1), p.err, 1425));
+                    ok = mbar_wait_warp(bar(PR_QEMPTY), (uint32_t)(k & 1), p.err, 1425);
                     if (!ok) break;
                     tc_fence_after();
                     load_query_tile<CFG, 4, false>(p, nx.q0, nx.h, row, wg, tlane, [&]() { arrive(PR_QFULL); });
@@ -1026,7 +1043,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             // ---- the row's sum: this CTA's four groups', then the peer's
             s_l[wg * 128 + row] = l;
             arrive(PR_XL);
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(PR_XL), (uint32_t)(k & 1), p.err, 1427));
+            ok = mbar_wait_warp(bar(PR_XL), (uint32_t)(k & 1), p.err, 1427);
             if (!ok) break;
             if (wg == 0) {
                 s_sum[(k & 1) * 128 + row] = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
@@ -1040,12 +1057,11 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             l = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
             // ---- epilogue of the item: O / l -> bf16 -> out[t][h][rank * 256 ..], through staging tiles in the buffers of this CTA's
             // own P (the peer may be filling the others): free when both CTAs are done with the last two own tiles
-            ok = mbar_wait(bar(PR_PEER + (k & 1)), (uint32_t)((k >> 1) & 1), p.err, 1428);
-            if (ok) ok = mbar_wait(bar(PR_ODONE), (uint32_t)(k & 1), p.err, 1424);
+            ok = mbar_wait_warp(bar(PR_PEER + (k & 1)), (uint32_t)((k >> 1) & 1), p.err, 1428);
+            if (ok) ok = mbar_wait_warp(bar(PR_ODONE), (uint32_t)(k & 1), p.err, 1424);
             const int next_own = T + ((T & 1) == rank ? 0 : 1);      // the own tile after this item, and the one behind it: in these buffers
             if (ok) ok = buffer_free(next_own);
             if (ok) ok = buffer_free(next_own + 2);
-            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
             l += s_peer[(k & 1) * 128 + row];
@@ -1342,7 +1358,7 @@ kexp_tc_kernel(const __grid_constant__ CUtensorMap tm_lat, const __grid_constant
                     *reinterpret_cast<uint4 *>(p.kx + ((int64_t)h * p.T + t0w + rr) * PaMla::DQK + KX_NOPE + jj * 8) = w;
                 }
             }
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(KB_DFULL + db), (uint32_t)((ti >> 1) & 1), p.err, 1107));
+            ok = mbar_wait_warp(bar(KB_DFULL + db), (uint32_t)((ti >> 1) & 1), p.err, 1107);
             if (!ok) break;
             tc_fence_after();
             {

@@ -9,6 +9,7 @@
 namespace {
 
 constexpr uint32_t WAIT_LIMIT = 1u << 22;   // try_wait iterations before a wait gives up
+constexpr uint32_t WAIT_SHORT = 1u << 10;   // ... where a warp's earlier wait has (mbar_wait_on)
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
@@ -46,6 +47,27 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *er
         if (mbar_try(bar, parity)) return true;
     atomicCAS(err, 0, code);
     return false;
+}
+// Bounded wait of a warp that issues MMAs tile by tile. Giving up records `code` and carries on with what is there: the loop runs to its end
+// whatever happens, with little patience from then on (WAIT_LIMIT at first), and the lanes have nothing to agree on on the way (a vote in these
+// loops, wherever it stood, was 2 to 5 % of a whole prompt; a word of the block in shared memory, which all would see, 2 % of a GQA prompt).
+// Only for loops whose MMAs and commits are all that they do: announcing bytes at a barrier, or sending them, again and again would run its
+// count over. settle() goes behind such a loop.
+__device__ __forceinline__ void mbar_wait_on(uint32_t bar, uint32_t parity, int *err, int code, uint32_t &patience) {
+    for (uint32_t i = 0; i < patience; i++)
+        if (mbar_try(bar, parity)) return;
+    atomicCAS(err, 0, code);
+    patience = WAIT_SHORT;
+}
+// The end of a role that issues MMAs or copies: where it gave up, the last of them may be under way with nobody waiting for them.
+__device__ __forceinline__ void settle(bool gave_up) {
+    if (gave_up)
+        for (const long long until = clock64() + 200000; clock64() < until;) { }      // (a tile's MMAs or copies take some thousand cycles)
+}
+// A whole warp's wait: all lanes give up if one does. A lane that left a loop alone would be waited for without limit at the warp's
+// next election, shuffle or tensor-memory access.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int *err, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code));
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *tm, int c0, int c1, int c2, uint32_t bar) {
     asm volatile(

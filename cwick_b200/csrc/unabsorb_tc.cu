@@ -131,8 +131,7 @@ unabsorb_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         for (int i = 0; i < nt && ok; i++) {
             const int db = i & 1;
             const int t0w = ((int)blockIdx.x + i * (int)gridDim.x) * UT_TOK + q4 * 32;       // first token row of this warp
-            ok = mbar_wait(bar(UB_DFULL + db), (uint32_t)((i >> 1) & 1), p.err, 917);
-            ok = __all_sync(0xffffffffu, ok);            // the TMEM loads below are warp-wide
+            ok = mbar_wait_warp(bar(UB_DFULL + db), (uint32_t)((i >> 1) & 1), p.err, 917);            // the TMEM loads below are warp-wide
             if (!ok) break;
             tc_fence_after();
             // A thread holds one token row of the accumulator, and rows of `out` lie nh * 256 bytes apart: the 64

@@ -43,22 +43,23 @@ class Bar:
 
 
 class Cta:
-    def __init__(self, rank, kst, pbars, arrivals):
+    def __init__(self, rank, kst, cst, pbars, arrivals):
         b = Bar
         self.rank = rank
         self.kfull, self.kempty = [b(1) for _ in range(kst)], [b(1) for _ in range(kst)]
+        self.cfull, self.cempty = [b(1) for _ in range(cst)], [b(1) for _ in range(cst)]
         self.sfull, self.sempty = [b(1), b(1)], [b(1), b(1)]
         self.pfull, self.pempty = [b(1) for _ in range(4)], [b(arrivals) for _ in range(pbars)]
         self.odone, self.qempty, self.qfull, self.ofree, self.xm, self.xl = b(1), b(1), b(2), b(2), b(2), b(2)
         self.peer = [b(1), b(1)]
-        self.k, self.s, self.p, self.readers = [None] * kst, [None, None], [None] * 4, [0] * 4
+        self.k, self.c, self.s, self.p, self.readers = [None] * kst, [None] * cst, [None, None], [None] * 4, [0] * 4
         self.sum, self.item_m, self.q = [None, None], None, None
 
 
-def model(items, seed, kst, pbars, told, arrivals=2):
+def model(items, seed, kst, cst, pbars, told, arrivals=2):
     """told(T, rank): the CTAs, as bits, that CTA `rank` tells of the end of its value products with tile T."""
     rnd = random.Random(seed)
-    ctas = [Cta(0, kst, pbars, arrivals), Cta(1, kst, pbars, arrivals)]
+    ctas = [Cta(0, kst, cst, pbars, arrivals), Cta(1, kst, cst, pbars, arrivals)]
     late = []                                                # completions under way in a CTA: a list per source, in order within it
     sent = []                                                # under way from one CTA to the other, in no order
 
@@ -90,6 +91,21 @@ def model(items, seed, kst, pbars, told, arrivals=2):
                 kc += 1
             T += tiles
 
+    def latents(c):                                          # announces the peer's P with the tile's latents
+        tma = [chain() for _ in range(cst)]
+        for T in range(sum(items)):
+            cs = T % cst
+            yield from wait(c.cempty[cs], (T // cst & 1) ^ 1)
+            if T & 1 != c.rank:
+                c.pfull[T & 3].arrive(1)
+            c.cfull[cs].arrive(1)
+
+            def land(cs=cs, T=T):
+                c.c[cs] = T
+                c.cfull[cs].bytes(1)
+            tma[cs].append(land)
+            yield
+
     def scores(c):
         kc, T, mma = 0, 0, chain()
         for k, tiles in enumerate(items):
@@ -119,16 +135,16 @@ def model(items, seed, kst, pbars, told, arrivals=2):
             if k:
                 yield from wait(c.ofree, k - 1 & 1)
             for _ in range(tiles):
-                pb, own = T & 3, T & 1 == c.rank
-                if not own:
-                    c.pfull[pb].arrive(1)
+                pb, cs = T & 3, T % cst
+                yield from wait(c.cfull[cs], T // cst & 1)
                 yield from wait(c.pfull[pb], T >> 2 & 1)
-                if c.p[pb] != T:
-                    raise Fault("values of tile %d with the P of %s" % (T, c.p[pb]))
+                if c.p[pb] != T or c.c[cs] != T:
+                    raise Fault("values of tile %d with the P of %s and the latents of %s" % (T, c.p[pb], c.c[cs]))
                 c.readers[pb] += 1
 
-                def end(pb=pb, T=T):
+                def end(pb=pb, cs=cs, T=T):
                     c.readers[pb] -= 1
+                    c.cempty[cs].arrive()
                     for x in ctas:
                         if told(T, c.rank) >> x.rank & 1:
                             if x is c:
@@ -221,7 +237,7 @@ def model(items, seed, kst, pbars, told, arrivals=2):
             c.ofree.arrive()
             yield
 
-    roles = [r for c in ctas for r in (keys(c), scores(c), values(c), sender(c), softmax(c, 0), softmax(c, 1))]
+    roles = [r for c in ctas for r in (keys(c), latents(c), scores(c), values(c), sender(c), softmax(c, 0), softmax(c, 1))]
     weight = [rnd.choice((1, 1, 4, 20)) for _ in roles]      # some roles are slow
     slow = rnd.random() < 0.5                                # the way between the CTAs: nothing arrives until all wait for it
     idle = 0
@@ -256,28 +272,28 @@ ITEMS = [[1], [2], [3], [1, 1, 1, 1, 1, 1, 1, 1, 1], [2, 1, 2, 1, 3, 1], [5, 4, 
 
 
 def source():
-    """Key slots, barriers of the P buffers and who is told of the end of a tile's value products, as the kernel has them."""
+    """Key and latent slots, barriers of the P buffers and who is told of the end of a tile's value products, as the kernel has them."""
     text = open(SRC).read()
-    kst = int(re.search(r"struct PrCfg \{\s*static constexpr int KST = (\d+)", text)[1])
+    kst, cst = map(int, re.search(r"struct PrCfg \{\s*static constexpr int KST = (\d+), CST = (\d+)", text).groups())
     pbars = int(re.search(r"PR_ODONE = PR_PEMPTY \+ (\d+)", text)[1])
     told = eval("lambda T, rank: " + re.search(r"umma_commit_to\(bar\(PR_PEMPTY \+ \(T & 7\)\), ([^;]+)\);", text)[1])
-    return kst, pbars, told
+    return kst, cst, pbars, told
 
 
 @pytest.mark.parametrize("items", ITEMS, ids=str)
 def test_the_pairs_protocol(items):
-    kst, pbars, told = source()
+    kst, cst, pbars, told = source()
     for seed in range(12):
-        model(items, seed, kst, pbars, told)
+        model(items, seed, kst, cst, pbars, told)
 
 
 def test_the_model_finds_buffers_freed_too_early():
     with pytest.raises(Fault):
         for seed in range(100):
-            model([7, 1, 6, 2, 9], seed, 2, 8, lambda T, rank: 1 << rank, arrivals=1)
+            model([7, 1, 6, 2, 9], seed, 2, 3, 8, lambda T, rank: 1 << rank, arrivals=1)
 
 
 def test_the_model_finds_arrivals_that_nobody_waits_for():
     with pytest.raises(Fault, match="has left"):
         for seed in range(100):
-            model([7, 1, 6, 2, 9], seed, 2, 8, lambda T, rank: 3)
+            model([7, 1, 6, 2, 9], seed, 2, 3, 8, lambda T, rank: 3)
