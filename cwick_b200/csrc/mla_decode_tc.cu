@@ -172,6 +172,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t bar0 = base + OFF_BAR;
     auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sm + OFF_MISC);
+    int *s_gave_up = reinterpret_cast<int *>(sm + OFF_MISC + 64);     // [3] a softmax thread's wait has: for a tile's scores (even, odd), for the output
     float *s_mref = reinterpret_cast<float *>(sm + OFF_MISC + 128);   // [64]
     float *s_alpha = s_mref + 64;                                     // [64]
     float *s_w = s_alpha + 64;                                        // [16 warps][16] per-warp max / sum
@@ -180,6 +181,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const int split = blockIdx.x;
     cwk_pdl_launch();
     if (tid == 0) {
+        s_gave_up[0] = s_gave_up[1] = s_gave_up[2] = 0;
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_q) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_kv) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_kr) : "memory");
@@ -485,8 +487,9 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
         for (int h = 0; h < HG; h++) lpart[h] = 0.f;
         for (int it = begin; it < end; it++) {
-            ok = mbar_wait_warp(bar(B_SFULL), (uint32_t)(it & 1), p.err, 301);
-            if (!ok) break;
+            // Giving up is told to all softmax threads, which leave together at the end of the tile: one that left alone would be waited for
+            // at their barriers. (Two words in turn: a thread reads a tile's while another may be a tile ahead.)
+            if (!mbar_wait(bar(B_SFULL), (uint32_t)(it & 1), p.err, 301)) s_gave_up[it & 1] = 1;
             if (st == 0) TRACE(2, it, 0);
             tc_fence_after();
             uint32_t sr[HG];
@@ -522,6 +525,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             uint32_t need;
             asm volatile("{\n.reg .pred pi, po;\nsetp.ne.b32 pi, %1, 0;\nbar.red.or.pred po, 1, 512, pi;\nselp.u32 %0, 1, 0, po;\n}\n"
                          : "=r"(need) : "r"((uint32_t)ex) : "memory");
+            const int gave_up = s_gave_up[it & 1];
             if (st == 0) TRACE(2, it, 6);
             if (need) {
                 // exact column maxima over the 128 tokens, new reference, rescale what exists
@@ -586,11 +590,16 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             tc_fence_before();
             mbar_arrive(bar(B_PFULL));
             if (st == 0) TRACE(2, it, 1);
+            if (gave_up) {
+                ok = false;
+                break;
+            }
         }
+        const bool scored = ok;
         // ---- epilogue: the row sums need only the last softmax; each 128-row block of O^T is written as soon
         // as its own MMAs have completed (their commit is the barrier that frees the block's latent slot), so
         // the write-out of block 0 runs under the MMAs of blocks 1-3
-        if (ok) {
+        if (scored) {
             const float mine = warp_transpose_reduce16<false>(lpart, lane);  // lane L: sum of head hb+(L&15) over this warp's rows
             if (lane < HG) s_w[(warp - 4) * HG + lane] = mine;
             if (st == 0) TRACE(2, 15, 3);
@@ -610,7 +619,10 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             if (st == 0) TRACE(2, 15, 4);
             for (int mb = mb0; mb < mb1 && ok; mb++) {
                 ok = mbar_wait_warp(bar(mb == 3 ? B_EMPTY_RP : B_EMPTY_L + mb), (uint32_t)((end - 1) & 1), p.err, 302);      // the TMEM load below is warp-wide
-                if (!ok) break;
+                if (!ok) {
+                    s_gave_up[2] = 1;
+                    break;
+                }
                 if (st == 0 && mb == 0) TRACE(2, 15, 2);
                 tc_fence_after();
                 uint32_t o[16];
@@ -629,9 +641,10 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 }
             }
         }
-        if (!RANGE || end >= n || !ok) break;
+        if (!RANGE || end >= n || !scored) break;
         tc_fence_before();                                // the accumulator has been read: these threads' next P lets its MMAs go ahead
         softmax_bar();                                    // the reference exponents and row sums have been read
+        if (s_gave_up[2]) break;
         next_segment(sg, n - end);
         begin = end;
         }

@@ -719,6 +719,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             if (i == PR_QFULL || i == PR_OFREE || i == PR_XM || i == PR_XL) count = 16;                  // every softmax warp
             if (i == PR_SEMPTY || i == PR_SEMPTY + 1) count = 8;                                         // the warps of a set
             if (i >= PR_PFULL && i < PR_PEMPTY) count = ((i - PR_PFULL) & 1) == rank ? 8 : 1;            // ... or the announcement of the peer's copy
+            if (i == PR_PEER || i == PR_PEER + 1) count = 4;                                             // the announcements of the warps that exchange row sums
             if (i >= PR_PEMPTY && i < PR_ODONE) count = 2;                                               // the value MMAs of both CTAs (own tiles' barriers)
             mbar_init(bar(i), count);
         }
@@ -1046,12 +1047,13 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             ok = mbar_wait_warp(bar(PR_XL), (uint32_t)(k & 1), p.err, 1427);
             if (!ok) break;
             if (wg == 0) {
+                // (each warp its own rows': a barrier of the four would be waited for without limit where one of them has given up)
                 s_sum[(k & 1) * 128 + row] = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (tid == 128) {
-                    mbar_expect_tx(bar(PR_PEER + (k & 1)), 512);
-                    copy_to_peer(smem_u32(s_sum + (k & 1) * 128), 512, peer_sum + (k & 1) * 512, peer_bar0 + 8u * (uint32_t)(k & 1));
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_expect_tx(bar(PR_PEER + (k & 1)), 128);
+                    copy_to_peer(smem_u32(s_sum + (k & 1) * 128 + row), 128, peer_sum + (k & 1) * 512 + row * 4, peer_bar0 + 8u * (uint32_t)(k & 1));
                 }
             }
             l = (s_l[row] + s_l[128 + row]) + (s_l[256 + row] + s_l[384 + row]);

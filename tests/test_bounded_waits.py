@@ -61,7 +61,7 @@ def test_a_warp_gives_up_as_a_whole(name):
         # voted on further down, with no way out in between; or told to the whole role, which looks at it together
         vote = text.find("__all_sync(0xffffffffu, here)", at)
         agreed = ("bool here =" in statement and 0 < vote < role[2] and not re.search(r"\b(break|continue|return)\b", text[at:vote])
-                  or re.match(r"[^;]*\)\) s_\w+\[\d\] = 1;", text[at:]))
+                  or re.match(r"[^;]*\)\) s_\w+\[[^\]]+\] = 1;", text[at:]))
         if not agreed and (lambda_ or WARP_WIDE.search(text[role[1]:role[2]])):
             bad.append("line %d: %s" % (text.count("\n", 0, at) + 1, text[at:text.index(";", at)]))
     assert not bad, "\n".join(bad)
@@ -79,3 +79,19 @@ def test_a_loop_that_carries_on_only_issues_and_commits(name):
         body, after = text[loop[1]:loop[2]], text[loop[2]:role[2]]
         assert not re.search(r"\b(break|continue|return|mbar_expect_tx|copy_to_peer|tma_load\w*)\b", body), body
         assert "&& ok" not in loop[0] and "settle(patience != WAIT_LIMIT);" in after, loop[0]
+
+
+@pytest.mark.parametrize("name", [n for n in SOURCES if re.search(r"softmax_bar\(|\bbar\.sync", open(os.path.join(CSRC, n)).read())])
+def test_a_role_gives_up_as_a_whole_where_its_warps_meet(name):
+    """Where a role has named barriers, a wait that gives up is told to all of it (a word in shared memory) before the next barrier in the text."""
+    text = strip(open(os.path.join(CSRC, name)).read())
+    meet = re.compile(r"softmax_bar\(\);|\"bar\.(?:sync|red)[^\"]* 1, \d+")
+    for m in re.finditer(r"\bmbar_wait(?:_warp)?\(", text):
+        inside = sorted((b for b in blocks(text) if b[1] < m.start() < b[2]), key=lambda b: b[1] - b[2], reverse=True)
+        if any(ONE_LANE.search(b[0]) for b in inside):
+            continue
+        role = next((b for b in inside if re.search(r"\bif \(.*\bwarp\b", b[0]) or b[0].endswith("else")), inside[-1])
+        if not meet.search(text[role[1]:role[2]]):
+            continue
+        nxt = meet.search(text, m.end())
+        assert re.search(r"\bs_\w+\[[^\]]+\] = 1;", text[m.end():nxt.start() if nxt and nxt.start() < role[2] else role[2]]), text[m.start():text.index(";", m.start())]
