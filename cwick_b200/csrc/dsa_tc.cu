@@ -342,6 +342,7 @@ __device__ __forceinline__ float e4m3_to_f32_i(uint32_t b) {
 constexpr int BC_KEYS = 64;                                   // band keys re-scored per pass and block
 constexpr int BC_QLD = IT_HD + 4;                             // padded q rows in shared memory
 constexpr int BC_BINS = 2 * TK_THREADS;                       // histogram bins (two per thread), in the place of the re-scored keys
+constexpr int BC_END = 128;                                   // scores in a bin at the band's end that are worth a second histogram
 constexpr int BC_LIST = 1024;                                 // a band of at most so many keys is ranked in shared memory
 constexpr int BC_SMEM = (IT_IH * BC_QLD + IT_IH + BC_KEYS * IT_HD + BC_KEYS * (IT_IH + 1) + BC_LIST + BC_LIST / TK_CL) * 4;
 static_assert(BC_BINS <= BC_KEYS * IT_HD, "the histogram lies in the place of the keys");
@@ -432,16 +433,26 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
     // Bins of equal width. No width (all scores alike), or scores that are not finite: one bin, and the whole row is re-scored.
     const float width = (mx - mn) * (1.0f / (BC_BINS - 1)), per_unit = 1.0f / width;
     const bool wide = width > 0.f && width < INFINITY && per_unit < INFINITY;
-    auto bin_of = [&](float a) { return !wide ? 0 : a == a ? max(0, min(BC_BINS - 1, (int)((a - mn) * per_unit))) : BC_BINS - 1; };      // rises with a
-    for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {
-        if (!sl.cached) tk_load(s, c0, sl.end, kc);
-        const int i0 = c0 + tid * TK_PT;
+    const float m = fmaxf(fabsf(mx), fabsf(mn));
+    const float eps = 2.0f * 0.001953125f * m;              // 2 * delta, delta = 2^-9 of the row's largest score
+    auto place = [&](float a) { return (a - mn) * per_unit; };      // in bins; rises with a
+    auto bin_of = [&](float a) { return !wide ? 0 : a == a ? max(0, min(BC_BINS - 1, (int)place(a))) : BC_BINS - 1; };
+    float from = 0.f, step = 1.f;             // the threshold lies in [from, from + step) bins
+    uint32_t left = (uint32_t)want;           // its rank among the scores of the histogram
+    bool fine = false;
+    while (true) {
+        for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {
+            if (!sl.cached) tk_load(s, c0, sl.end, kc);
+            const int i0 = c0 + tid * TK_PT;
 #pragma unroll
-        for (int j = 0; j < TK_PT; j++)
-            if (i0 + j < sl.end) atomicAdd(hist + bin_of(order_key_inverse(kc[j])), 1u);
-    }
-    cl.sync();
-    {
+            for (int j = 0; j < TK_PT; j++) {
+                const float a = order_key_inverse(kc[j]);
+                int k = bin_of(a);
+                if (fine) k = k != (int)from ? -1 : a == a ? max(0, min(BC_BINS - 1, (int)((place(a) - from) * BC_BINS))) : BC_BINS - 1;
+                if (i0 + j < sl.end && k >= 0) atomicAdd(hist + k, 1u);
+            }
+        }
+        cl.sync();
         uint2 c = make_uint2(0u, 0u);                       // bins 2 tid and 2 tid + 1 of the whole row
 #pragma unroll
         for (unsigned r = 0; r < TK_CL; r++) {
@@ -456,15 +467,34 @@ band_classify_kernel(const float *approx, int64_t stride, const int32_t *n, int 
         }
         if (lane == 0) sh.tot[warp] = incl;
         __syncthreads();
-        const uint32_t above = __reduce_add_sync(0xffffffffu, lane > warp ? sh.tot[lane] : 0u) + incl - (c.x + c.y), w = (uint32_t)want;
-        if (above < w && w <= above + c.x + c.y) sh.sel[0] = (uint32_t)(2 * tid) + (w <= above + c.y ? 1u : 0u);
+        const uint32_t above = __reduce_add_sync(0xffffffffu, lane > warp ? sh.tot[lane] : 0u) + incl - (c.x + c.y);
+        if (above < left && left <= above + c.x + c.y) {
+            const bool upper = left <= above + c.y;
+            sh.sel[0] = (uint32_t)(2 * tid) + (upper ? 1u : 0u);
+            sh.sel[1] = left - above - (upper ? 0u : c.y);
+        }
+        __syncthreads();
+        const float bin = (float)sh.sel[0];
+        if (fine) {
+            from += bin * (1.0f / BC_BINS);
+            step = 1.0f / BC_BINS;
+            break;
+        }
+        from = bin;
+        // The band's ends are a bin wide too. Where one of them has many scores in it -- a heavy tail, the threshold some eps above the bulk
+        // of the row -- a second histogram, of the threshold's bin, tells which of them the band needs.
+        const float e = eps * per_unit, d0 = floorf(bin - e), d1 = floorf(bin + e), k0 = (float)(2 * tid);
+        auto end = [&](float k) { return (k >= d0 && k <= d0 + 1.f) || (k >= d1 && k <= d1 + 1.f); };
+        fine = __syncthreads_or(wide && ((c.x > BC_END && end(k0)) || (c.y > BC_END && end(k0 + 1.f))));
+        if (!fine) break;
+        left = sh.sel[1];
+        cl.sync();                                          // the histograms have been read everywhere
+        *reinterpret_cast<uint2 *>(hist + 2 * tid) = make_uint2(0u, 0u);
         __syncthreads();
     }
     BTRACE(2);
-    const float m = fmaxf(fabsf(mx), fabsf(mn));
-    const float eps = 2.0f * 0.001953125f * m;              // 2 * delta, delta = 2^-9 of the row's largest score
-    // (a hundredth of a bin covers the roundings of bin_of and of these)
-    const float hi = wide ? mn + ((float)sh.sel[0] + 1.01f) * width + eps : INFINITY, lo = wide ? mn + ((float)sh.sel[0] - 0.01f) * width - eps : -INFINITY;
+    // (a hundredth of a bin covers the roundings of place and of these)
+    const float hi = wide ? mn + (from + step + 0.01f) * width + eps : INFINITY, lo = wide ? mn + (from - 0.01f) * width - eps : -INFINITY;
     int32_t *list = band_list + (int64_t)b * stride;
     uint32_t inb = 0;                                       // this thread's scores of the chunk that are in the band
     for (int c0 = sl.begin; c0 < sl.end; c0 += TK_CHUNK) {

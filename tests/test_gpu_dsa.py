@@ -210,6 +210,31 @@ def test_fused_selection_histogram_edges(attn, T, want, keep_self, keys):
     assert nsel[0] == ref.size and np.array_equal(sel[0, :nsel[0]].astype(np.int64), ref)
 
 
+@pytest.mark.parametrize("T,at", [(20000, 8.6), (20000, 40.4), (70000, 8.6)])
+def test_fused_selection_band_ends_inside_a_bin(attn, T, at):
+    """Scores with a heavy tail: the threshold lies `at` bins above the smallest score and the bulk of the row a little below the band, whose
+    half width is 8 of the 2047 bins. Only scores that the error bound cannot tell from the threshold may be re-scored: a band
+    that ended at the threshold's bin would take the bulk with it."""
+    want, step = 2048, 1.0 / 2047
+    codes, ks, q, wt = make_index_inputs(77, 1, T)
+    codes[0, :] = codes[0, 0]                                # scores in proportion to the keys' scales
+    rng = np.random.default_rng(T)
+    ks[0] = rng.uniform(0.02, 0.3, T) * step + max(0.0, at - 8.6) * step
+    where = rng.permutation(T)
+    ks[0, where[0]] = 1.0
+    ks[0, where[1:2001]] = rng.uniform(60, 200, 2000) * step
+    ks[0, where[2001:2201]] = (at + rng.uniform(-0.2, 0.2, 200)) * step
+    ks[0, where[2201]] = 0.0
+    lens = np.array([T], np.int32)
+    sel, nsel, refined = _select_both_ways(attn, codes, ks, q, wt, lens, want, False)
+    sc = oracle_scores(codes, ks, q, wt)[0]
+    assert sc.max() > 0
+    ref = oracle_select(sc, T, want, False)
+    assert nsel[0] == ref.size and np.array_equal(sel[0, :nsel[0]].astype(np.int64), ref)
+    reach = sc.max() * (2.0 ** -8 + 0.1 * step + 2.0 ** -16)          # the band, a tenth of a bin and the tensor-core scores' own error
+    assert np.isfinite(refined[0, :T]).sum() <= (np.abs(sc[:T] - np.sort(sc[:T])[-want]) <= reach).sum()
+
+
 def test_fused_selection_config4_size(attn):
     """BASELINE config 4 dimensions on two sequences: 65536 keys, top 2048."""
     B, T, want = 2, 65536, 2048
