@@ -431,80 +431,160 @@ static __global__ void __launch_bounds__(128) lse_merge_kernel(const float *part
 // The merge of many sequences with few records each, a warp per (sequence, head, 128 C columns) and no block barrier: a lane asks for
 // C pieces of sixteen bytes of the first AHEAD records at once. The kernel above is 128 threads, two barriers and some three
 // microseconds per 128 columns of a head, so that 64 sequences of 3 records (28 MB) took 25 us.
-template <int C, int AHEAD>
-static __global__ void __launch_bounds__(256) lse_merge_warp_kernel(const float *partial, int nsplit, int nh, int D, int items, uint16_t *out, const int2 *meta) {
+// With ranges (meta), a sequence of more than CWK_MERGE_LONG records is left to all blocks together (merge_long_rows below): a batch of one long
+// sequence among short ones has few records on average, and a warp that walks through most of them takes a trip to L2 for every four.
+constexpr int CWK_MERGE_LONG = 16;
+static __device__ __forceinline__ void merge_long_rows(const float *partial, int nh, int D, uint16_t *out, const int2 *meta, int B);
+
+template <int C, int AHEAD, bool RANGES>
+static __global__ void __launch_bounds__(256) lse_merge_warp_kernel(const float *partial, int nsplit, int nh, int D, int items, uint16_t *out, const int2 *meta, int B) {
     const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int chunks = D / (128 * C), chunk = item % chunks, bh = item / chunks, h = bh % nh, b = bh / nh;
     const int64_t rec_sz = (int64_t)nh * (D + 2);
     cwk_pdl_launch();
     cwk_pdl_wait();
-    if (item >= items) return;
     int64_t rec0 = (int64_t)b * nsplit;
-    if (meta) {
-        const int2 m = meta[b];
+    int looked = 0, looked2 = 0;                           // a thread looks at every 256th sequence, for the block; the first two are asked for with its own
+    if (RANGES) {
+        if ((int)threadIdx.x < B) looked = meta[threadIdx.x].y;
+        if ((int)threadIdx.x + 256 < B) looked2 = meta[threadIdx.x + 256].y;
+        const int2 m = meta[min(b, B - 1)];
         rec0 = m.x;
         nsplit = m.y;
     }
-    const float *base = partial + rec0 * rec_sz, *ml = base + h;
-    const float *col = base + 2 * nh + (int64_t)h * D + chunk * 128 * C + lane * 4;
-    float4 v[AHEAD][C];
+    if (item < items && !(RANGES && nsplit > CWK_MERGE_LONG)) {
+        const float *base = partial + rec0 * rec_sz, *ml = base + h;
+        const float *col = base + 2 * nh + (int64_t)h * D + chunk * 128 * C + lane * 4;
+        float4 v[AHEAD][C];
 #pragma unroll
-    for (int s = 0; s < AHEAD; s++)
+        for (int s = 0; s < AHEAD; s++)
 #pragma unroll
-        for (int c = 0; c < C; c++) v[s][c] = s < nsplit ? *reinterpret_cast<const float4 *>(col + s * rec_sz + c * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
-    // lane s: the record's reference exponent (-inf: nothing in it) and sum
-    auto mine = [&](int s, float &m, float &l) {
-        l = s < nsplit ? ml[s * rec_sz + nh] : 0.f;
-        m = l > 0.f ? ml[s * rec_sz] : -INFINITY;
-    };
-    float m0, l0, M;
-    mine(lane, m0, l0);
-    M = m0;
-    for (int s = lane + 32; s < nsplit; s += 32) {
-        float m, l;
-        mine(s, m, l);
-        M = fmaxf(M, m);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    auto weight = [&](float m) { return m == -INFINITY ? 0.f : __expf(m - M); };
-    float w = weight(m0), den = w * l0;                    // weights of records 0 .. 31
-    for (int s = lane + 32; s < nsplit; s += 32) {
-        float m, l;
-        mine(s, m, l);
-        den += weight(m) * l;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-    float4 a[C];
-#pragma unroll
-    for (int c = 0; c < C; c++) a[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s0 = 0; s0 < nsplit; s0 += AHEAD) {           // (AHEAD divides 32)
-        if (s0 > 0) {
-#pragma unroll
-            for (int s = 0; s < AHEAD; s++)
-#pragma unroll
-                for (int c = 0; c < C; c++) v[s][c] = s0 + s < nsplit ? *reinterpret_cast<const float4 *>(col + (s0 + s) * rec_sz + c * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if ((s0 & 31) == 0) {
-                float m, l;
-                mine(s0 + lane, m, l);
-                w = weight(m);
-            }
+            for (int c = 0; c < C; c++) v[s][c] = s < nsplit ? *reinterpret_cast<const float4 *>(col + s * rec_sz + c * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+        // lane s: the record's reference exponent (-inf: nothing in it) and sum
+        auto mine = [&](int s, float &m, float &l) {
+            l = s < nsplit ? ml[s * rec_sz + nh] : 0.f;
+            m = l > 0.f ? ml[s * rec_sz] : -INFINITY;
+        };
+        float m0, l0, M;
+        mine(lane, m0, l0);
+        M = m0;
+        for (int s = lane + 32; s < nsplit; s += 32) {
+            float m, l;
+            mine(s, m, l);
+            M = fmaxf(M, m);
         }
 #pragma unroll
-        for (int s = 0; s < AHEAD; s++) {
-            const float ws = __shfl_sync(0xffffffffu, w, (s0 + s) & 31);
-            if (s0 + s < nsplit) {                         // (a record without rows has weight 0 and defined values)
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        auto weight = [&](float m) { return m == -INFINITY ? 0.f : __expf(m - M); };
+        float w = weight(m0), den = w * l0;                    // weights of records 0 .. 31
+        for (int s = lane + 32; s < nsplit; s += 32) {
+            float m, l;
+            mine(s, m, l);
+            den += weight(m) * l;
+        }
 #pragma unroll
-                for (int c = 0; c < C; c++) { a[c].x += ws * v[s][c].x; a[c].y += ws * v[s][c].y; a[c].z += ws * v[s][c].z; a[c].w += ws * v[s][c].w; }
+        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+        float4 a[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) a[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s0 = 0; s0 < nsplit; s0 += AHEAD) {           // (AHEAD divides 32)
+            if (s0 > 0) {
+#pragma unroll
+                for (int s = 0; s < AHEAD; s++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) v[s][c] = s0 + s < nsplit ? *reinterpret_cast<const float4 *>(col + (s0 + s) * rec_sz + c * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if ((s0 & 31) == 0) {
+                    float m, l;
+                    mine(s0 + lane, m, l);
+                    w = weight(m);
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < AHEAD; s++) {
+                const float ws = __shfl_sync(0xffffffffu, w, (s0 + s) & 31);
+                if (s0 + s < nsplit) {                         // (a record without rows has weight 0 and defined values)
+#pragma unroll
+                    for (int c = 0; c < C; c++) { a[c].x += ws * v[s][c].x; a[c].y += ws * v[s][c].y; a[c].z += ws * v[s][c].z; a[c].w += ws * v[s][c].w; }
+                }
+            }
+        }
+        const float inv = den > 0.f ? 1.f / den : 0.f;
+        uint16_t *dst = out + ((int64_t)b * nh + h) * D + chunk * 128 * C + lane * 4;
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            *reinterpret_cast<uint2 *>(dst + c * 128) = make_uint2(pack_bf16x2(a[c].x * inv, a[c].y * inv), pack_bf16x2(a[c].z * inv, a[c].w * inv));
+    }
+    if (RANGES) {
+        bool any = max(looked, looked2) > CWK_MERGE_LONG;
+        for (int i = threadIdx.x + 512; i < B; i += 256) any |= meta[i].y > CWK_MERGE_LONG;
+        if (__syncthreads_or(any)) merge_long_rows(partial, nh, D, out, meta, B);
+    }
+}
+// The sequences among B that have more than CWK_MERGE_LONG records, by all blocks: a warp per head and 32 columns, every fourth record
+// for each eight of its lanes, sixteen records at a time. Whole calls, us: one block per 128 columns of every sequence (the kernel above) / a
+// warp for all of a sequence's records / this: 120000 rows + 63 x 1 119 / 143 / 103, 131072 + 63 x 2000 101 / 108 / 89, 32768 + 31 x
+// 1000 49 / 52 / 43, 120000 + 7 x 200 65 / 79 / 68. A batch without such a sequence pays for the
+// larger kernel from cold caches: 64 of 16384..32768 rows 374 -> 377, one after another no difference; with eight records a lane ahead, or sums
+// through shared memory, 379. A kernel of its own behind this one: 380, and 2 more for short batches.
+static __device__ __forceinline__ void merge_long_rows(const float *partial, int nh, int D, uint16_t *out, const int2 *meta, int B) {
+    constexpr int AHEAD = 4;
+    const int lane = threadIdx.x & 31, grp = lane >> 3, pieces = D / 32;
+    const int64_t rec_sz = (int64_t)nh * (D + 2);
+    for (int b0 = 0; b0 < B; b0 += 32) {
+        const int2 mt = b0 + lane < B ? meta[b0 + lane] : make_int2(0, 0);
+        for (uint32_t left = __ballot_sync(0xffffffffu, mt.y > CWK_MERGE_LONG); left; left &= left - 1) {
+            const int at = __ffs(left) - 1, n = __shfl_sync(0xffffffffu, mt.y, at);
+            const float *base = partial + __shfl_sync(0xffffffffu, mt.x, at) * rec_sz;
+#pragma unroll 1
+            for (int unit = (int)blockIdx.x * 8 + (threadIdx.x >> 5); unit < nh * pieces; unit += (int)gridDim.x * 8) {
+                const int h = unit / pieces, c0 = unit % pieces * 32 + (lane & 7) * 4;
+                const float *ml = base + h, *col = base + 2 * nh + (int64_t)h * D + c0;
+                auto mine = [&](int s, float &m, float &l) {
+                    l = s < n ? ml[s * rec_sz + nh] : 0.f;
+                    m = l > 0.f ? ml[s * rec_sz] : -INFINITY;
+                };
+                float4 v[AHEAD], a = make_float4(0.f, 0.f, 0.f, 0.f);
+                auto ask = [&](int s0) {
+#pragma unroll
+                    for (int k = 0; k < AHEAD; k++) {
+                        const int s = s0 + 4 * k + grp;
+                        v[k] = s < n ? *reinterpret_cast<const float4 *>(col + s * rec_sz) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                };
+                ask(0);
+                float M = -INFINITY, den = 0.f, m, l;
+#pragma unroll 2
+                for (int s = lane; s < n; s += 32) {
+                    mine(s, m, l);
+                    M = fmaxf(M, m);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+#pragma unroll 1
+                for (int s0 = 0; s0 < n; s0 += 4 * AHEAD) {
+                    if (s0 > 0) ask(s0);
+                    mine(s0 + (lane & 15), m, l);          // (both halves of the warp: the sum is halved at the end)
+                    const float w = m == -INFINITY ? 0.f : __expf(m - M);
+                    den += w * l;
+#pragma unroll
+                    for (int k = 0; k < AHEAD; k++) {      // (no record: weight and values are 0)
+                        const float ws = __shfl_sync(0xffffffffu, w, 4 * k + grp);
+                        a.x += ws * v[k].x; a.y += ws * v[k].y; a.z += ws * v[k].z; a.w += ws * v[k].w;
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+#pragma unroll
+                for (int o = 8; o < 32; o <<= 1) {
+                    a.x += __shfl_xor_sync(0xffffffffu, a.x, o); a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+                    a.z += __shfl_xor_sync(0xffffffffu, a.z, o); a.w += __shfl_xor_sync(0xffffffffu, a.w, o);
+                }
+                const float inv = den > 0.f ? 2.f / den : 0.f;
+                if (grp == 0)
+                    *reinterpret_cast<uint2 *>(out + ((int64_t)(b0 + at) * nh + h) * D + c0) = make_uint2(pack_bf16x2(a.x * inv, a.y * inv), pack_bf16x2(a.z * inv, a.w * inv));
             }
         }
     }
-    const float inv = den > 0.f ? 1.f / den : 0.f;
-    uint16_t *dst = out + ((int64_t)b * nh + h) * D + chunk * 128 * C + lane * 4;
-#pragma unroll
-    for (int c = 0; c < C; c++)
-        *reinterpret_cast<uint2 *>(dst + c * 128) = make_uint2(pack_bf16x2(a[c].x * inv, a[c].y * inv), pack_bf16x2(a[c].z * inv, a[c].w * inv));
 }
 // Whether it takes the merge: whole pieces of 128 columns, sixteen bytes aligned; at most 32 records a sequence (on average); and
 // work enough for its warps, where the kernel above would be 1024 blocks or more, 2048 where a warp goes round twice. Records of 64
@@ -516,8 +596,9 @@ static inline bool lse_merge_by_warps(const float *partial, int few, int nh, int
 }
 static inline void lse_merge_warps_launch(cudaStream_t st, const float *partial, int nsplit, int few, int nh, int D, int B, uint16_t *out, const int2 *meta) {
     const int most = few <= 4 ? 4 : few <= 8 ? 2 : 1, c = D % (128 * most) == 0 ? most : 1, items = B * nh * (D / (128 * c));
-    auto kern = c == 4 ? lse_merge_warp_kernel<4, 4> : c == 2 ? lse_merge_warp_kernel<2, 8> : lse_merge_warp_kernel<1, 16>;
-    (void)cwk_launch_early(kern, dim3((items + 7) / 8), dim3(256), 0, st, partial, nsplit, nh, D, items, out, meta);
+    auto kern = meta ? (c == 4 ? lse_merge_warp_kernel<4, 4, true> : c == 2 ? lse_merge_warp_kernel<2, 8, true> : lse_merge_warp_kernel<1, 16, true>)
+                     : (c == 4 ? lse_merge_warp_kernel<4, 4, false> : c == 2 ? lse_merge_warp_kernel<2, 8, false> : lse_merge_warp_kernel<1, 16, false>);
+    (void)cwk_launch_early(kern, dim3((items + 7) / 8), dim3(256), 0, st, partial, nsplit, nh, D, items, out, meta, B);
 }
 
 static inline void lse_combine_launch(cudaStream_t st, const float *partial, int nsplit, int nh, int D, int B,
