@@ -262,18 +262,21 @@ int cwk_mla_prefill_attn_tc(cwk_ctx *ctx, const void *Q, const float *rot, const
 
 // Which attention route is the faster one for a chunk of n queries behind pos0 rows. The expansion covers every cached
 // row once, whatever n, and its attention works in tiles of 128 queries; the absorbed route costs a pass of the decode
-// kernel per query. In microseconds, fitted to whole calls with 64 heads: expansion 0.012 per row; attention 0.64 per 64-key tile
-// and 5 per item (128 queries x head x half), the items dealt over the SMs; absorbed 0.033 per query and 128-key tile, 0.08 per
-// query around it (0.4 where the queries are more than the SMs: there the other route is far ahead anyway) and 18 for launches
-// that do not come up early. Calls measured near the line, absorbed / expanded:
-//   4 queries after 300 rows 81 / 73, after 1000 81 / 89;          16 after 300 84 / 73, after 1000 86 / 87, after 3000 95 / 127
-//   32 after 1000 97 / 90, after 3000 110 / 127;                   64 after 3000 136 / 129, after 8000 215 / 232
-//   96 after 8000 270 / 234, after 32000 759 / 736;                129 after 8000 341 / 319, after 16000 595 / 538, after 32000 1025 / 1023
+// kernel per query. In microseconds, fitted to whole calls with 64 heads (145 pairs of 1 to 512 queries and 0 to 32767 rows
+// before them): expansion 0.0109 per row; attention 0.51 per 64-key tile and 5 per item (128 queries x head), the items dealt to the
+// pairs of SMs in rounds; absorbed 0.0273 per query and 128-key tile, 0.02 per query around it and 21 for launches that do not come up
+// early. The route is the better one or within 2 % of it at all but one of them (80 after 12000, below). Near the line, absorbed / expanded, cold caches:
+//   4 queries after 300 rows 132 / 120, after 1000 132 / 132, after 2000 134 / 151;  16 after 1000 132 / 130, after 2000 136 / 149
+//   32 after 1000 146 / 132, after 2000 148 / 149, after 4000 165 / 194;             64 after 4000 196 / 196, after 8000 259 / 278
+//   80 after 12000 371 / 357;  85 after 28000 658 / 677;                             96 after 16000 474 / 439, after 32672 816 / 773
+//   129 after 8000 378 / 349, after 24000 853 / 806, after 32639 1080 / 1056;        130 after 28000 994 / 928
+// Other numbers of heads take a slower decode kernel: the estimate favours the absorbed route there (16 heads, 192 after 28000: 2741 / 314).
 static bool expanded_keys_pay(const cwk_ctx *ctx, int n, int64_t pos0, int nh) {
     const double T = (double)(pos0 + n), mean = (double)pos0 + 0.5 * n;
-    const double items = (double)((n + 127) / 128) * nh * 2, rounds = items <= ctx->sm_count ? 1.0 : items / ctx->sm_count + 0.5;
-    const double expanded = 0.012 * T * nh / 64 + rounds * (0.64 * (mean / 64 + 1) + 5.0);
-    const double absorbed = 18.0 + n * (0.033 * (mean / 128 + 1) + 0.08) * nh / 64;
+    const int pairs = std::max(1, ctx->sm_count / 2);
+    const double rounds = (double)(((int64_t)((n + 127) / 128) * nh + pairs - 1) / pairs);
+    const double expanded = 0.0109 * T * nh / 64 + rounds * (0.51 * (mean / 64 + 1) + 5.0);
+    const double absorbed = 21.0 + n * (0.0273 * (mean / 128 + 1) + 0.02) * nh / 64;
     return expanded < absorbed;
 }
 

@@ -239,6 +239,22 @@ def test_short_chunks_on_both_routes(attn, n, pos0, nh):
     close(bf16_to_np(gcache), bf16_to_np(ocache))
 
 
+@pytest.mark.parametrize("n,pos0,expanded", [(1, 300, True), (1, 4000, False), (32, 8000, False), (64, 12000, False), (96, 16000, True),
+                                             (129, 24000, True), (130, 28000, True)])
+def test_route_of_a_chunk(attn, n, pos0, expanded):
+    """The route that the estimate gives a chunk, at points where the routes' measured times are 6 % or more apart: the absorbed route is
+    the forced one bit for bit, the expanded one agrees with it within the rounding of its own operands."""
+    nh, H, q_lora = 64, 512, 256
+    m = make_model(83, H, q_lora, nh)
+    X = synth.normal_bf16(83, 9, (n, H))
+    cache0 = np.zeros((pos0 + n, LAT + ROPE), np.uint16)
+    cache0[:pos0] = synth.normal_bf16(83, 10, (pos0, LAT + ROPE))
+    got, _ = run_gpu(attn, m, X, cache0, pos0, nh)
+    absorbed, _ = _forced(attn, 2, lambda: run_gpu(attn, m, X, cache0, pos0, nh))
+    assert torch.equal(got, absorbed) == (not expanded)
+    close(bf16_to_np(got), bf16_to_np(absorbed))
+
+
 @pytest.mark.parametrize("n,pos0", [(200, 6000), (256, 8000)])
 def test_few_heads_in_shares(attn, n, pos0):
     """16 heads leave most of the pairs of blocks without an item: the key tiles are dealt out in shares and the parts joined.
