@@ -68,17 +68,18 @@ def test_ragged_batch_with_empty_sequence(attn, nsplit):
 
 
 @pytest.fixture(scope="module")
-def five_long():
-    q, cache = make_case(78, 5, 64, 4300)
-    lens = np.array([4300, 0, 1, 2100, 4225], np.int32)
+def eight_long():
+    q, cache = make_case(78, 8, 64, 4300)
+    lens = np.array([4300, 0, 1, 2100, 4225, 129, 3968, 640], np.int32)
     return to_bf16_cuda(q), to_bf16_cuda(cache), torch.from_numpy(lens).cuda(), oracle_out(q, cache, lens)
 
 
 @pytest.mark.parametrize("nsplit", [2, 4, 5, 8, 9, 16, 17, 32, 33])
-def test_merge_of_split_records(attn, five_long, nsplit):
+def test_merge_of_split_records(attn, eight_long, nsplit):
     """Both merges (a warp per row and chunk up to 32 records, blocks above) at the ends of their numbers of records ahead,
-    with empty and one-row sequences among the records."""
-    q, cache, lens, want = five_long
+    with empty and one-row sequences among the records. Eight sequences are 2048 pieces of 128 columns, enough for the warps
+    to go round twice (17 and 32 records, sixteen at a time)."""
+    q, cache, lens, want = eight_long
     g = bf16_to_np(attn.mla_decode(q, cache, lens, scale=SCALE, n_splits=nsplit))
     assert np.all(g[1] == 0)
     close(g, want)

@@ -65,8 +65,8 @@ def run_oracle(m, X, cache_init, pos0, nh, rows):
     return out, cache
 
 
-def run_oracle_rows(m, X, cache, nh, rows):
-    """Outputs of some query rows over a cache the oracle has already filled (n = 0: no row is rewritten)."""
+def run_oracle_rows(m, X, cache, nh, rows, pos0=0):
+    """Outputs of some query rows over a cache that is already filled (n = 0: no row is rewritten)."""
     o = orc.oracle()
     H = X.shape[1]
     q_lora = m["Wqa"].shape[0]
@@ -75,7 +75,7 @@ def run_oracle_rows(m, X, cache, nh, rows):
     out = np.empty((rows.size, nh, LAT), np.float32)
     o.orc_mla_prefill(P(Xf, f32p), P(m["Wqa"], u8p), P(m["Sqa"], f32p), P(m["Wqb"], u8p), P(m["Sqb"], f32p),
                       P(m["Wkva"], u8p), P(m["Skva"], f32p), P(m["qa_n"], u16p), P(m["kva_n"], u16p),
-                      P(m["Wuk"], u16p), P(cache, u16p), 0, 0, H, q_lora, nh, NOPE, ROPE, LAT, 1e-6, 10000.0,
+                      P(m["Wuk"], u16p), P(cache, u16p), pos0, 0, H, q_lora, nh, NOPE, ROPE, LAT, 1e-6, 10000.0,
                       1.0 / math.sqrt(NOPE + ROPE), P(rows, i32p), rows.size, P(out, f32p))
     return out
 
@@ -275,18 +275,26 @@ def test_few_heads_in_shares(attn, n, pos0):
     close(bf16_to_np(got), bf16_to_np(exact))
 
 
-@pytest.mark.parametrize("n,pos0", [(1, 3), (255, 0), (257, 64), (1030, 5), (2305, 0)])
+@pytest.mark.parametrize("n,pos0", [(1, 3), (255, 0), (257, 64), (509, 0), (1000, 5), (2305, 0)])
 def test_norm_adds_up_the_parts_of_cut_tiles(attn, n, pos0):
-    """The norms behind q_a and kv_a add up the tiles that their GEMM cut along K: all of them (up to two row tiles and five), or some (2305
-    tokens are 90 tiles: a wave of 74 whole, then the columns of kv_a from a row tile in their middle on). Cache rows against float64:
-    the reference's narrowing takes less than a bf16 step (2^-7 relative) off; the f32 sums of 2048 products are within 2^-24 * 16 blocks of
-    their magnitude (2^-20 * 4), and an angle of up to 2305 in f32 is off by 2^-24 * 2305 * 2, times values below 4: 1e-3 covers both."""
+    """The norms behind q_a and kv_a add up the tiles that their GEMM cut along K: all of them (up to four row tiles), or some (2305 tokens are
+    90 tiles: a wave of 74 whole, then the columns of kv_a from a row tile in their middle on; columns of q_a are cut together or not at
+    all on 148 SMs). Cache rows against float64: the reference's narrowing takes less than a bf16 step (2^-7 relative) off; the f32 sums of 2048
+    products are within 2^-24 * 16 blocks of their magnitude (2^-20 * 4), and an angle of up to 2305 in f32 is off by 2^-24 * 2305 * 2, times
+    values below 4: 1e-3 covers both. The rows of q_a only show in the attention's output: rows of every row tile against the oracle over
+    the same cache, with q_b weights x4, so that a part left out or taken twice in one of q_a's six column tiles moves the scores by more than
+    the tolerance."""
     H, nh = 2048, 2
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    tiles = (1536 // 256 + 3) * -(-n // 256)
+    assert min(pairs // (tiles % pairs), H // 128 // 4) > 1          # (the parts that the GEMM's launch cuts the last wave into)
     m = make_model(77, H, 1536, nh)
+    m["Sqb"] = (m["Sqb"] * np.float32(4.0)).astype(np.float32)
     X = synth.normal_bf16(n, 9, (n, H))
     cache0 = np.zeros((pos0 + n, LAT + ROPE), np.uint16)
     out, cache = run_gpu(attn, m, X, cache0, pos0, nh)
-    assert torch.isfinite(out.float()).all()
+    rows = np.unique(np.minimum(n - 1, np.arange(0, n + 255, 255)))
+    close(bf16_to_np(out)[rows], run_oracle_rows(m, X, cache.view(torch.int16).cpu().numpy().view(np.uint16), nh, rows, pos0))
     W = torch.from_numpy(m["Wkva"]).cuda().view(torch.float8_e4m3fn).double()
     W *= torch.from_numpy(m["Skva"]).cuda().double().repeat_interleave(128, 0)[:LAT + ROPE].repeat_interleave(128, 1)
     kv = to_bf16_cuda(X).double() @ W.T
