@@ -349,9 +349,9 @@ __global__ void __launch_bounds__(256) rms_scale_pair_kernel(float *xa, int na, 
 // q_a | kv_a projection (part [splits][n][na + nb]), then the q_a row leaves as three bf16 planes (the next projection's
 // operand), the kv_a row as the narrowed cache row and, where the caller's cache is f32, as f32. The sum of squares is a
 // sum of doubles, as in rms_scale_row, four columns at a time here.
-// A row is a few KB: what it takes is trips to L2, so a thread asks for two pieces of every partial sum and for its weights at
-// once and everything is read and written in pieces of four columns (one value at a time, 2-byte stores: 11 us for 128 tokens of
-// 1536 + 512 in sixteen parts, now 8).
+// A row is a few KB: what it takes is trips to L2, so a thread asks for two pieces of every partial sum at once and everything is
+// read and written in pieces of four columns (one value at a time, 2-byte stores: 11 us for 128 tokens of 1536 + 512 in sixteen
+// parts, now 8). The weights are read behind the sum.
 __global__ void __launch_bounds__(256) norm_chunk_kernel(const float *part, int splits, int n, int na, int nb, const uint16_t *wa, const uint16_t *wb,
                                                          float eps, uint16_t *planes, uint16_t *cache_rows, float *kv_out) {
     extern __shared__ __align__(16) float s_row[];
