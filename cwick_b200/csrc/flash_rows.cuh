@@ -433,7 +433,7 @@ static __global__ void __launch_bounds__(128) lse_merge_kernel(const float *part
 // microseconds per 128 columns of a head, so that 64 sequences of 3 records (28 MB) took 25 us.
 // With ranges (meta), a sequence of more than CWK_MERGE_LONG records is left to all blocks together (merge_long_rows below): a batch of one long
 // sequence among short ones has few records on average, and a warp that walks through most of them takes a trip to L2 for every four.
-constexpr int CWK_MERGE_LONG = 16;
+constexpr int CWK_MERGE_LONG = 32;
 static __device__ __forceinline__ void merge_long_rows(const float *partial, int nh, int D, uint16_t *out, const int2 *meta, int B);
 
 template <int C, int AHEAD, bool RANGES>
@@ -522,13 +522,17 @@ static __global__ void __launch_bounds__(256) lse_merge_warp_kernel(const float 
 }
 // The sequences among B that have more than CWK_MERGE_LONG records, by all blocks: a warp per head and 32 columns, every fourth record
 // for each eight of its lanes, sixteen records at a time. Whole calls, us: one block per 128 columns of every sequence (the kernel above) / a
-// warp for all of a sequence's records / this: 120000 rows + 63 x 1 119 / 143 / 103, 131072 + 63 x 2000 101 / 108 / 89, 32768 + 31 x
-// 1000 49 / 52 / 43, 120000 + 7 x 200 65 / 79 / 68. A batch without such a sequence pays for the
-// larger kernel from cold caches: 64 of 16384..32768 rows 374 -> 377, one after another no difference; with eight records a lane ahead, or sums
-// through shared memory, 379. A kernel of its own behind this one: 380, and 2 more for short batches.
+// warp for all of a sequence's records / this: 120000 rows + 63 x 1 119 / 143 / 103, 131072 + 63 x 2000 101 / 108 / 87, 32768 + 31 x
+// 1000 49 / 52 / 42, 120000 + 7 x 200 65 / 79 / 68, 2 x 100000 + 30 x 500 88 / 91 / 84. The line: sequences of up to 32 records are often many,
+// and warps of their own do them side by side (8 of 16384..32768 rows, 19 records each: 71, 86 with the line at 16); four of 36 beside 26 x 500
+// are 74 here and 70 on their own, one of 35 (32768 + 31 x 1000) the other way. A batch without such a sequence pays for the larger kernel
+// from cold caches: 64 of 16384..32768 rows 374 -> 377, one after another no difference; with eight records a lane ahead, or sums through shared
+// memory, 379. A kernel of its own behind this one: 380, and 2 more for short batches.
 static __device__ __forceinline__ void merge_long_rows(const float *partial, int nh, int D, uint16_t *out, const int2 *meta, int B) {
     constexpr int AHEAD = 4;
     const int lane = threadIdx.x & 31, grp = lane >> 3, pieces = D / 32;
+    const int units = nh * pieces, warps = (int)gridDim.x * 8;
+    int first = (int)blockIdx.x * 8 + (threadIdx.x >> 5);  // this warp's first unit; the next sequence begins with the warps after those that had one
     const int64_t rec_sz = (int64_t)nh * (D + 2);
     for (int b0 = 0; b0 < B; b0 += 32) {
         const int2 mt = b0 + lane < B ? meta[b0 + lane] : make_int2(0, 0);
@@ -536,7 +540,7 @@ static __device__ __forceinline__ void merge_long_rows(const float *partial, int
             const int at = __ffs(left) - 1, n = __shfl_sync(0xffffffffu, mt.y, at);
             const float *base = partial + __shfl_sync(0xffffffffu, mt.x, at) * rec_sz;
 #pragma unroll 1
-            for (int unit = (int)blockIdx.x * 8 + (threadIdx.x >> 5); unit < nh * pieces; unit += (int)gridDim.x * 8) {
+            for (int unit = first; unit < units; unit += warps) {
                 const int h = unit / pieces, c0 = unit % pieces * 32 + (lane & 7) * 4;
                 const float *ml = base + h, *col = base + 2 * nh + (int64_t)h * D + c0;
                 auto mine = [&](int s, float &m, float &l) {
@@ -583,6 +587,7 @@ static __device__ __forceinline__ void merge_long_rows(const float *partial, int
                 if (grp == 0)
                     *reinterpret_cast<uint2 *>(out + ((int64_t)(b0 + at) * nh + h) * D + c0) = make_uint2(pack_bf16x2(a.x * inv, a.y * inv), pack_bf16x2(a.z * inv, a.w * inv));
             }
+            first = (first + warps - units % warps) % warps;
         }
     }
 }

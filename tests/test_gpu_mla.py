@@ -395,12 +395,11 @@ def test_bad_arguments_are_reported_not_run(attn):
     [0, 40000, 0, 1, 129, 0, 70000, 128],            # empty sequences in front, between and inside; one block, many blocks
     [9000] * 13,                                     # alike, not a multiple of the blocks' share
     [1] * 300 + [120000],                            # blocks that pass through dozens of sequences
-    # records left to all blocks of the merge (more than sixteen of a sequence), behind each of its forms: 3, 5 and 19 records on average
+    # records left to all blocks of the merge (more than 32 of a sequence), behind each of its forms: 3, 5 and 19 records on average
     [120000] + [1] * 63,
     [90000] + [1] * 20 + [300] * 8 + [60000],
     [200] * 7 + [150000],
-    [13000] * 9,                                     # seventeen or eighteen records of every sequence
-    [12500] * 10,                                    # fifteen or sixteen: none of a sequence's records are
+    [29000, 30500, 29000] + [9500] * 5 + [1, 1],     # 34 records between sequences of 32 (on 148 SMs), which warps of their own merge
     [0, 0, 0],                                       # nothing at all
 ])
 def test_batch_in_equal_shares_of_tiles(attn, lens):
